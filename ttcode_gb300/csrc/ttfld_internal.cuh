@@ -176,9 +176,10 @@ __device__ __forceinline__ void atomic_max_nonneg(unsigned long long* a, double 
 // blocks are resident), on a monotonic 64-bit arrival counter that the host
 // zeroes before each launch: the k-th barrier of a launch is complete once
 // the counter has reached k * nblocks.  Thread 0 of each block releases the
-// block's writes (a block barrier, a fence, a release reduction) and polls
-// the counter with acquire loads, 32 ns apart, then a fence and a block
-// barrier order every thread's later loads after the other blocks' writes.
+// block's writes (a block barrier, then a release reduction, cumulative over
+// what the barrier ordered before it) and polls the counter with acquire
+// loads; a block barrier then orders every thread's later loads after the
+// other blocks' writes.
 // With no reset and no generation word, the last block to arrive adds one
 // round trip to L2 to the barrier.  `passed` counts this block's barriers
 // (the same value in every thread).  The wait is bounded: after
@@ -207,19 +208,16 @@ __device__ __forceinline__ bool grid_sync(SolverDev* sol, unsigned int nblocks, 
   ++passed;
   if (threadIdx.x == 0) {
     int ok = 1;
-    __threadfence();
     asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(&sol->arrivals) : "memory");
     const unsigned long long target = passed * nblocks;
     long long polls = 0;
     while (ld_acquire64(&sol->arrivals) < target) {
-      __nanosleep(32);
       if (give_up(++polls, sol)) {
         atomicExch(&sol->bar_timeout, 1);
         ok = 0;
         break;
       }
     }
-    __threadfence();
     ok_sh = ok;
   }
   __syncthreads();
