@@ -44,8 +44,8 @@ int pole_shift(ttfld_ctx* c, double* a) {
 // copied from UPPERBND-1.  kappa_P = kappa_A = kappa_R, zero T-derivatives
 // (the IKAPTYP=3 convention, pprphy.f:84-87).
 __device__ __forceinline__ double kap_formula(const Dev& d, double t, double rh, double kmul) {
-  double th = t / 1000.0;
-  return ((d.kap0 * sqrt(rh)) * (th * sqrt(th))) * kmul;
+  const double th = div_rn(t, 1000.0);
+  return ((d.kap0 * sqrt_rn(rh)) * (th * sqrt_rn(th))) * kmul;
 }
 
 // The opacity table of kappa_model 2 in device memory: an error word, then
@@ -315,9 +315,9 @@ static int qdens(ttfld_ctx* c) {
   Dev d = c->d;
   launch_box(c->stream, box(-1, d.nx + 2, -1, d.ny + 2, -1, d.nz + 2), [=] __device__(int i, int j, int k) {
     size_t q = hidx(d, i, j, k);
-    if (i >= 0) d.RHQX[q] = G(ddx1, i) * d.RH[q] + G(ddx0, i) * HA(RH, i - 1, j, k);
-    if (j >= 0) d.RHQY[q] = G(ddy1, j) * d.RH[q] + G(ddy0, j) * HA(RH, i, j - 1, k);
-    if (k >= 0) d.RHQZ[q] = G(ddz1, k) * d.RH[q] + G(ddz0, k) * HA(RH, i, j, k - 1);
+    if (i >= 0) d.RHQX[q] = mul_rn(G(ddx1, i), d.RH[q]) + G(ddx0, i) * HA(RH, i - 1, j, k);
+    if (j >= 0) d.RHQY[q] = mul_rn(G(ddy1, j), d.RH[q]) + G(ddy0, j) * HA(RH, i, j - 1, k);
+    if (k >= 0) d.RHQZ[q] = mul_rn(G(ddz1, k), d.RH[q]) + G(ddz0, k) * HA(RH, i, j, k - 1);
   });
   TT_CHECK_LAUNCH();
   return 0;
@@ -329,58 +329,58 @@ static int qdens(ttfld_ctx* c) {
 // and the fluxes of a face together (bit for bit the values of the separate
 // loops).
 
+// FLIM's flux limiter of a face (IFLIMTYP 2): the energy gradient's size over
+// den = rho kappa (E + E'), R, then (2 + R) / (6 + 3 R + R^2).  About 20
+// products, 20 sums, six quotients and a root per face in all: the quotients,
+// the root and half of the products run on the integer pipes
+// (ttfld_fp64.cuh), which then take about as long as the FP64 pipe's share.
+__device__ __forceinline__ double limiter(double gradx, double grady, double gradz, double den) {
+  const double grad = sqrt_rn(gradx * gradx + grady * grady + gradz * gradz) + 1.0e-50;
+  const double rr = div_rn(2.0 * grad, den);
+  return div_rn(2.0 + rr, 6.0 + 3.0 * rr + mul_rn(rr, rr));
+}
+
 // FLIM's x loop body, pprphy.f:414-448 (IFLIMTYP 2).
 __device__ __forceinline__ double flimx_calc(const Dev& d, int i, int j, int k) {
   const double sg = d.sigval;
-  double gradx = (HA(ER, i, j, k) - HA(ER, i - 1, j, k)) / G(dxb, i);
-  double grady = (G(ddx1, i) * (HA(ER, i, j + 1, k) - HA(ER, i, j - 1, k)) +
-                  G(ddx0, i) * (HA(ER, i - 1, j + 1, k) - HA(ER, i - 1, j - 1, k))) /
-                 (G(geoxga, i) * G(geozg, k) * (G(xyb, j + 1) - G(xyb, j - 1)));
-  double gradz = (G(ddx1, i) * (HA(ER, i, j, k + 1) - HA(ER, i, j, k - 1)) +
-                  G(ddx0, i) * (HA(ER, i - 1, j, k + 1) - HA(ER, i - 1, j, k - 1))) /
-                 (G(geoxha, i) * (G(xzb, k + 1) - G(xzb, k - 1)));
-  double grad = sqrt(gradx * gradx + grady * grady + gradz * gradz) + 1.0e-50;
-  double rrx = 2.0 * grad /
-               (HA(RHQX, i, j, k) *
-                (G(ddx1, i) * (HA(XKAPR, i, j, k) + sg) + G(ddx0, i) * (HA(XKAPR, i - 1, j, k) + sg)) *
-                (HA(ER, i, j, k) + HA(ER, i - 1, j, k)));
-  return (2.0 + rrx) / (6.0 + 3.0 * rrx + rrx * rrx);
+  double gradx = div_rn(HA(ER, i, j, k) - HA(ER, i - 1, j, k), G(dxb, i));
+  double grady = div_rn(G(ddx1, i) * (HA(ER, i, j + 1, k) - HA(ER, i, j - 1, k)) +
+                            G(ddx0, i) * (HA(ER, i - 1, j + 1, k) - HA(ER, i - 1, j - 1, k)),
+                        mul_rn(mul_rn(G(geoxga, i), G(geozg, k)), G(xyb, j + 1) - G(xyb, j - 1)));
+  double gradz = div_rn(G(ddx1, i) * (HA(ER, i, j, k + 1) - HA(ER, i, j, k - 1)) +
+                            G(ddx0, i) * (HA(ER, i - 1, j, k + 1) - HA(ER, i - 1, j, k - 1)),
+                        mul_rn(G(geoxha, i), G(xzb, k + 1) - G(xzb, k - 1)));
+  const double kap = mul_rn(G(ddx1, i), HA(XKAPR, i, j, k) + sg) + mul_rn(G(ddx0, i), HA(XKAPR, i - 1, j, k) + sg);
+  return limiter(gradx, grady, gradz, mul_rn(mul_rn(HA(RHQX, i, j, k), kap), HA(ER, i, j, k) + HA(ER, i - 1, j, k)));
 }
 
 // FLIM's y loop body, pprphy.f:462-484.
 __device__ __forceinline__ double flimy_calc(const Dev& d, int i, int j, int k) {
   const double sg = d.sigval;
-  double gradx = (G(ddy1, j) * (HA(ER, i + 1, j, k) - HA(ER, i - 1, j, k)) +
-                  G(ddy0, j) * (HA(ER, i + 1, j - 1, k) - HA(ER, i - 1, j - 1, k))) /
-                 (G(xxb, i + 1) - G(xxb, i - 1));
-  double grady = (HA(ER, i, j, k) - HA(ER, i, j - 1, k)) / (G(geoxg, i) * G(geozg, k) * G(dyb, j));
-  double gradz = (G(ddy1, j) * (HA(ER, i, j, k + 1) - HA(ER, i, j, k - 1)) +
-                  G(ddy0, j) * (HA(ER, i, j - 1, k + 1) - HA(ER, i, j - 1, k - 1))) /
-                 ((G(xzb, k + 1) - G(xzb, k - 1)) * G(geoxh, i));
-  double grad = sqrt(gradx * gradx + grady * grady + gradz * gradz) + 1.0e-50;
-  double rry = 2.0 * grad /
-               (HA(RHQY, i, j, k) *
-                (G(ddy1, j) * (HA(XKAPR, i, j, k) + sg) + G(ddy0, j) * (HA(XKAPR, i, j - 1, k) + sg)) *
-                (HA(ER, i, j, k) + HA(ER, i, j - 1, k)));
-  return (2.0 + rry) / (6.0 + 3.0 * rry + rry * rry);
+  double gradx = div_rn(G(ddy1, j) * (HA(ER, i + 1, j, k) - HA(ER, i - 1, j, k)) +
+                            G(ddy0, j) * (HA(ER, i + 1, j - 1, k) - HA(ER, i - 1, j - 1, k)),
+                        G(xxb, i + 1) - G(xxb, i - 1));
+  double grady =
+      div_rn(HA(ER, i, j, k) - HA(ER, i, j - 1, k), mul_rn(mul_rn(G(geoxg, i), G(geozg, k)), G(dyb, j)));
+  double gradz = div_rn(G(ddy1, j) * (HA(ER, i, j, k + 1) - HA(ER, i, j, k - 1)) +
+                            G(ddy0, j) * (HA(ER, i, j - 1, k + 1) - HA(ER, i, j - 1, k - 1)),
+                        mul_rn(G(xzb, k + 1) - G(xzb, k - 1), G(geoxh, i)));
+  const double kap = mul_rn(G(ddy1, j), HA(XKAPR, i, j, k) + sg) + mul_rn(G(ddy0, j), HA(XKAPR, i, j - 1, k) + sg);
+  return limiter(gradx, grady, gradz, mul_rn(mul_rn(HA(RHQY, i, j, k), kap), HA(ER, i, j, k) + HA(ER, i, j - 1, k)));
 }
 
 // FLIM's z loop body, pprphy.f:493-515.
 __device__ __forceinline__ double flimz_calc(const Dev& d, int i, int j, int k) {
   const double sg = d.sigval;
-  double gradx = (G(ddz1, k) * (HA(ER, i + 1, j, k) - HA(ER, i - 1, j, k)) +
-                  G(ddz0, k) * (HA(ER, i + 1, j, k - 1) - HA(ER, i - 1, j, k - 1))) /
-                 (G(xxb, i + 1) - G(xxb, i - 1));
-  double grady = (G(ddz1, k) * (HA(ER, i, j + 1, k) - HA(ER, i, j - 1, k)) +
-                  G(ddz0, k) * (HA(ER, i, j + 1, k - 1) - HA(ER, i, j - 1, k - 1))) /
-                 ((G(xyb, j + 1) - G(xyb, j - 1)) * G(geoxg, i) * G(geozga, k));
-  double gradz = (HA(ER, i, j, k) - HA(ER, i, j, k - 1)) / (G(geoxh, i) * G(dzb, k));
-  double grad = sqrt(gradx * gradx + grady * grady + gradz * gradz) + 1.0e-50;
-  double rrz = 2.0 * grad /
-               (HA(RHQZ, i, j, k) *
-                (G(ddz1, k) * (HA(XKAPR, i, j, k) + sg) + G(ddz0, k) * (HA(XKAPR, i, j, k - 1) + sg)) *
-                (HA(ER, i, j, k) + HA(ER, i, j, k - 1)));
-  return (2.0 + rrz) / (6.0 + 3.0 * rrz + rrz * rrz);
+  double gradx = div_rn(G(ddz1, k) * (HA(ER, i + 1, j, k) - HA(ER, i - 1, j, k)) +
+                            G(ddz0, k) * (HA(ER, i + 1, j, k - 1) - HA(ER, i - 1, j, k - 1)),
+                        G(xxb, i + 1) - G(xxb, i - 1));
+  double grady = div_rn(G(ddz1, k) * (HA(ER, i, j + 1, k) - HA(ER, i, j - 1, k)) +
+                            G(ddz0, k) * (HA(ER, i, j + 1, k - 1) - HA(ER, i, j - 1, k - 1)),
+                        mul_rn(mul_rn(G(xyb, j + 1) - G(xyb, j - 1), G(geoxg, i)), G(geozga, k)));
+  double gradz = div_rn(HA(ER, i, j, k) - HA(ER, i, j, k - 1), mul_rn(G(geoxh, i), G(dzb, k)));
+  const double kap = mul_rn(G(ddz1, k), HA(XKAPR, i, j, k) + sg) + mul_rn(G(ddz0, k), HA(XKAPR, i, j, k - 1) + sg);
+  return limiter(gradx, grady, gradz, mul_rn(mul_rn(HA(RHQZ, i, j, k), kap), HA(ER, i, j, k) + HA(ER, i, j, k - 1)));
 }
 
 // FLIMX(i,j,k) as FLIM leaves it: formed for i <= UPPERBND-1 (:414-448),
@@ -417,9 +417,8 @@ __device__ __forceinline__ double flimz_at(const Dev& d, int i, int j, int k) {
 // DIFF pprad.f:74-156, one face of each direction (with the ieta = 5 floor).
 __device__ __forceinline__ double difrx_of(const Dev& d, int i, int j, int k, double fl) {
   const double sg = d.sigval;
-  double v = TT_FD * fl /
-             (G(dxb, i) * HA(RHQX, i, j, k) *
-              (G(ddx1, i) * (HA(XKAPR, i, j, k) + sg) + G(ddx0, i) * (HA(XKAPR, i - 1, j, k) + sg)));
+  const double kap = mul_rn(G(ddx1, i), HA(XKAPR, i, j, k) + sg) + mul_rn(G(ddx0, i), HA(XKAPR, i - 1, j, k) + sg);
+  double v = div_rn(mul_rn(TT_FD, fl), mul_rn(mul_rn(G(dxb, i), HA(RHQX, i, j, k)), kap));
   if (d.ieta == 5) {
     double mn = HA(RHQX, i, j, k) * HA(CV, i, j, k) * d.xnue /
                 (G(dxb, i) * 4.0 * TT_ARAD * p3(G(ddx1, i) * HA(T, i, j, k) + G(ddx0, i) * HA(T, i - 1, j, k)) *
@@ -430,9 +429,9 @@ __device__ __forceinline__ double difrx_of(const Dev& d, int i, int j, int k, do
 }
 __device__ __forceinline__ double difry_of(const Dev& d, int i, int j, int k, double fl) {
   const double sg = d.sigval;
-  double v = TT_FD * fl /
-             (G(dyb, j) * G(geoxg, i) * G(geozg, k) * HA(RHQY, i, j, k) *
-              (G(ddy1, j) * (HA(XKAPR, i, j, k) + sg) + G(ddy0, j) * (HA(XKAPR, i, j - 1, k) + sg)));
+  const double kap = mul_rn(G(ddy1, j), HA(XKAPR, i, j, k) + sg) + mul_rn(G(ddy0, j), HA(XKAPR, i, j - 1, k) + sg);
+  const double h = mul_rn(mul_rn(G(dyb, j), G(geoxg, i)), G(geozg, k));
+  double v = div_rn(TT_FD * fl, mul_rn(h * HA(RHQY, i, j, k), kap));
   if (d.ieta == 5) {
     double mn = HA(RHQY, i, j, k) * HA(CV, i, j, k) * d.xnue /
                 (G(dyb, j) * G(geoxg, i) * G(geozg, k) * 4.0 * TT_ARAD *
@@ -443,9 +442,9 @@ __device__ __forceinline__ double difry_of(const Dev& d, int i, int j, int k, do
 }
 __device__ __forceinline__ double difrz_of(const Dev& d, int i, int j, int k, double fl) {
   const double sg = d.sigval;
-  double v = TT_FD * fl /
-             (G(dzb, k) * G(geoxh, i) * HA(RHQZ, i, j, k) *
-              (G(ddz1, k) * (HA(XKAPR, i, j, k) + sg) + G(ddz0, k) * (HA(XKAPR, i, j, k - 1) + sg)));
+  const double kap = mul_rn(G(ddz1, k), HA(XKAPR, i, j, k) + sg) + mul_rn(G(ddz0, k), HA(XKAPR, i, j, k - 1) + sg);
+  const double h = mul_rn(G(dzb, k), G(geoxh, i));
+  double v = div_rn(mul_rn(TT_FD, fl), mul_rn(h * HA(RHQZ, i, j, k), kap));
   if (d.ieta == 5) {
     double mn = HA(RHQZ, i, j, k) * HA(CV, i, j, k) * d.xnue /
                 (G(dzb, k) * G(geoxh, i) * 4.0 * TT_ARAD *
@@ -713,11 +712,17 @@ static int stellarinput_heating(ttfld_ctx* c) {
   // STELLAR_DTAU and STELLARINPUT of the same cell in one pass
   launch_box(c->stream, box(1, d.nx + 1, -1, d.ny + 2, -1, d.nz + 2), [=] __device__(int i, int j, int k) {
     int is = i < 2 ? 2 : (i > d.nx ? d.nx : i);  // dtaus(1)=dtaus(2), dtaus(NX+1)=dtaus(NX)
-    const double dtaus = (HA(STAU, is - 1, j, k) - HA(STAU, is + 1, j, k)) / 2.0;
+    const double dtaus = (HA(STAU, is - 1, j, k) - HA(STAU, is + 1, j, k)) * 0.5;
     HA(DTAUS, i, j, k) = dtaus;
     if (i > d.nx) return;
-    double tinc = PA(TINC, j, k), mu = PA(MU, j, k);
-    HA(SI, i, j, k) = TT_SBCONST * (p4(tinc) / mu) * (exp(-HA(STAU, i, j, k) / mu)) * dtaus / G(dxb, i);
+    const double tinc = PA(TINC, j, k), mu = PA(MU, j, k);
+    const double day = mul_rn(TT_SBCONST, div_rn(p4(tinc), mu));
+    // the night side (no incident flux) needs no exponential: any factor in
+    // (0, 1] gives the same signed zero, and an infinite tau has made dtaus
+    // non-finite too
+    const double tau = HA(STAU, i, j, k);
+    const double ex = day == 0.0 && tau >= 0.0 ? 1.0 : exp(div_rn(-tau, mu));
+    HA(SI, i, j, k) = div_rn(mul_rn(mul_rn(day, ex), dtaus), G(dxb, i));
   });
   TT_CHECK_LAUNCH();
   return 0;

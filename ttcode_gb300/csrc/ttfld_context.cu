@@ -192,6 +192,9 @@ int ttfld_create(ttfld_ctx** out, const ttfld_dims* dims, const ttfld_metrics* m
   Dev& d = c->d;
   d.nx = dims->nx; d.ny = dims->ny; d.nz = dims->nz;
   d.poles = dims->poles;
+  d.by_nx = fast_div(d.nx);
+  d.by_ny = fast_div(d.ny);
+  d.by_nxh = fast_div((d.nx + 1) / 2);
   apply_params(c);
 
   const size_t H = nhalo(d), Cn = ncell(d), Fn = nface(d), Pn = nplane(d);

@@ -9,6 +9,7 @@
 #include <stdio.h>
 
 #include "../../include/ttfld.h"
+#include "ttfld_fp64.cuh"
 
 // global_constants, ppmod.f:1074-1092: REAL*4 literals held in double.
 #define TT_FD ((double)2.99792458e10f)
@@ -77,6 +78,7 @@ struct Dev {
   int itmax, bcxmin, ibdrad, iflimtyp, f_incident, ieta, isigtyp, iii, kappa_model;
   SolverDev* sol;
   StepDev* stp;
+  FastDiv by_nx, by_ny, by_nxh;  // NX, NY and the (NX + 1) / 2 cells of a colour in a radial row
 };
 
 __host__ __device__ __forceinline__ size_t hidx(const Dev& d, int i, int j, int k) {
@@ -106,31 +108,39 @@ __host__ __device__ __forceinline__ size_t nplane(const Dev& d) { return (size_t
 #define FA(a, i, j, k) (d.a[fidx(d, i, j, k)])
 #define PA(a, j, k) (d.a[pidx(d, j, k)])
 
-__device__ __forceinline__ double p4(double x) { double x2 = x * x; return x2 * x2; }
-__device__ __forceinline__ double p3(double x) { return (x * x) * x; }
+__device__ __forceinline__ double p4(double x) { double x2 = mul_rn(x, x); return mul_rn(x2, x2); }
+__device__ __forceinline__ double p3(double x) { return mul_rn(mul_rn(x, x), x); }
+
+// (i, j, k) of cell t of the (1:NX,1:NY,1:NZ) order.
+__device__ __forceinline__ void cell_ijk(const Dev& d, unsigned int t, int& i, int& j, int& k) {
+  unsigned int r, q = div_rem(d.by_nx, t, r);
+  i = (int)r + 1;
+  k = (int)div_rem(d.by_ny, q, r) + 1;
+  j = (int)r + 1;
+}
 
 // An inclusive index box [i0,i1]x[j0,j1]x[k0,k1] walked i fastest.
 struct Box {
   int i0, j0, k0, ni, nj, nk;
+  FastDiv by_ni, by_nj;
 };
 inline Box box(int i0, int i1, int j0, int j1, int k0, int k1) {
-  Box b{i0, j0, k0, i1 - i0 + 1, j1 - j0 + 1, k1 - k0 + 1};
+  Box b{i0, j0, k0, i1 - i0 + 1, j1 - j0 + 1, k1 - k0 + 1, {}, {}};
   if (b.ni < 0) b.ni = 0;
   if (b.nj < 0) b.nj = 0;
   if (b.nk < 0) b.nk = 0;
+  if (b.ni > 0) b.by_ni = fast_div(b.ni);
+  if (b.nj > 0) b.by_nj = fast_div(b.nj);
   return b;
 }
 
 template <class Fn>
 __global__ void __launch_bounds__(kThreads) box_kernel(Box b, Fn fn) {
-  const long long n = (long long)b.ni * b.nj * b.nk;
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n;
-       t += (long long)gridDim.x * blockDim.x) {
-    int i = b.i0 + (int)(t % b.ni);
-    long long r = t / b.ni;
-    int j = b.j0 + (int)(r % b.nj);
-    int k = b.k0 + (int)(r / b.nj);
-    fn(i, j, k);
+  const unsigned int n = (unsigned int)b.ni * b.nj * b.nk;
+  for (unsigned int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+    unsigned int i, j;
+    const unsigned int k = div_rem(b.by_nj, div_rem(b.by_ni, t, i), j);
+    fn(b.i0 + (int)i, b.j0 + (int)j, b.k0 + (int)k);
   }
 }
 
@@ -345,13 +355,15 @@ struct EvalRow {
 };
 __device__ __forceinline__ EvalRow evalues_cell(const Dev& d, int i, int j, int k, double theta, double eta) {
   EvalRow r;
-  r.e1 = -G(surxa, i + 1) * FA(DIFRX, i + 1, j, k) / (G(surxb, i) * G(dxa, i));
-  r.e2 = -G(surxa, i) * FA(DIFRX, i, j, k) / (G(surxb, i) * G(dxa, i));
-  r.e3 = -FA(DIFRY, i, j + 1, k) / (G(xxb, i) * G(surzb, k) * G(dya, j));
-  r.e4 = -FA(DIFRY, i, j, k) / (G(xxb, i) * G(surzb, k) * G(dya, j));
-  r.e5 = -FA(DIFRZ, i, j, k + 1) * G(surza, k + 1) / (G(xxb, i) * G(surzb, k) * G(dza, k));
-  r.e6 = -FA(DIFRZ, i, j, k) * G(surza, k) / (G(xxb, i) * G(surzb, k) * G(dza, k));
-  r.e7 = 1.0 + (1.0 - eta) * d.delt * HA(RH, i, j, k) * HA(XKAPP, i, j, k) * TT_FD;
+  const double hx = G(surxb, i) * G(dxa, i), rz = mul_rn(G(xxb, i), G(surzb, k));
+  const double hy = rz * G(dya, j), hz = rz * G(dza, k);
+  r.e1 = div_rn(-G(surxa, i + 1) * FA(DIFRX, i + 1, j, k), hx);
+  r.e2 = div_rn(-G(surxa, i) * FA(DIFRX, i, j, k), hx);
+  r.e3 = div_rn(-FA(DIFRY, i, j + 1, k), hy);
+  r.e4 = div_rn(-FA(DIFRY, i, j, k), hy);
+  r.e5 = div_rn(-FA(DIFRZ, i, j, k + 1) * G(surza, k + 1), hz);
+  r.e6 = div_rn(-FA(DIFRZ, i, j, k) * G(surza, k), hz);
+  r.e7 = 1.0 + mul_rn((1.0 - eta) * d.delt * HA(RH, i, j, k) * HA(XKAPP, i, j, k), TT_FD);
   r.e8 = (eta * (1.0 - theta) - 1.0) * d.delt;
   r.e16 = r.e1 + r.e2 + r.e3 + r.e4 + r.e5 + r.e6;
   return r;
@@ -367,8 +379,8 @@ __device__ __forceinline__ void store_evalues(const Dev& d, size_t q, const Eval
 __device__ __forceinline__ bool sor_row(const Dev& d, int i, int j, int k, size_t q, const EvalRow& r) {
   double e8 = r.e8;
   double a = r.e7 + e8 * r.e16;
-  double b = -e8 * r.e2, cc = -e8 * r.e1, dd = -e8 * r.e4;
-  double e = -e8 * r.e3, f = -e8 * r.e6, g = -e8 * r.e5;
+  double b = mul_rn(-e8, r.e2), cc = mul_rn(-e8, r.e1), dd = mul_rn(-e8, r.e4);
+  double e = mul_rn(-e8, r.e3), f = mul_rn(-e8, r.e6), g = mul_rn(-e8, r.e5);
   int ub = PA(UB, j, k);
   // the theta edges are boundary rows only without poles (ppsor.f:228-272)
   bool ident = (i >= ub) || (i == d.nx) || (!d.poles && (k == 1 || k == d.nz));

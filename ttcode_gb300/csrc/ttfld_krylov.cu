@@ -111,19 +111,12 @@ __device__ __forceinline__ double b_of(const Dev& d, const double* b, size_t t, 
   return b[t];
 }
 
-__device__ __forceinline__ void cell_of(const Dev& d, long long t, int& i, int& j, int& k) {
-  i = (int)(t % d.nx) + 1;
-  const long long r = t / d.nx;
-  j = (int)(r % d.ny) + 1;
-  k = (int)(r / d.ny) + 1;
-}
-
 // W_n and Sigma_n (cell order).  A coupled row needs EVAL8 < 0.
 __global__ void __launch_bounds__(kThreads) kry_weights_kernel(Dev d, Kry kr, int hypre) {
-  const long long n = (long long)ncell(d);
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
+  const unsigned int n = (unsigned int)ncell(d);
+  for (unsigned int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
     int i, j, k;
-    cell_of(d, t, i, j, k);
+    cell_ijk(d, t, i, j, k);
     const Row r = row_of(d, t, i, j, k, hypre != 0);
     const bool decoupled = r.b == 0.0 && r.c == 0.0 && r.d == 0.0 && r.e == 0.0 && r.f == 0.0 && r.g == 0.0;
     const double v = G(surxb, i) * G(dxa, i) * G(dya, j) * G(surzb, k) * G(dza, k);
@@ -140,11 +133,11 @@ __global__ void __launch_bounds__(kThreads) kry_weights_kernel(Dev d, Kry kr, in
 // Couplings of S (the symmetric part of Sigma W A Sigma) to the +i, +j, +k
 // neighbours, written line-major.
 __global__ void __launch_bounds__(kThreads) kry_couplings_kernel(Dev d, Kry kr, int hypre) {
-  const long long n = (long long)ncell(d);
+  const unsigned int n = (unsigned int)ncell(d);
   const int nx = d.nx, ny = d.ny, nz = d.nz;
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
+  for (unsigned int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
     int i, j, k;
-    cell_of(d, t, i, j, k);
+    cell_ijk(d, t, i, j, k);
     const bool h = hypre != 0;
     const Row r = row_of(d, t, i, j, k, h);
     const double wn = kr.wgt[t], sn = kr.sig[t];
@@ -204,12 +197,12 @@ __global__ void __launch_bounds__(kThreads) kry_anchor_kernel(Dev d, Kry kr, con
   __shared__ double sh[32];
   __shared__ bool last;
   const int nx = d.nx, ny = d.ny;
-  const long long n = (long long)ncell(d);
+  const unsigned int n = (unsigned int)ncell(d);
   const size_t sj = (size_t)(nx + 4), sk = (size_t)(nx + 4) * (ny + 4);
   double s[4] = {0.0, 0.0, 0.0, 0.0};
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
+  for (unsigned int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
     int i, j, k;
-    cell_of(d, t, i, j, k);
+    cell_ijk(d, t, i, j, k);
     const Row r = row_of(d, t, i, j, k, hypre != 0);
     const size_t q = hidx(d, i, j, k);
     const size_t qjm = (j == 1) ? hidx(d, i, ny, k) : q - sj;
@@ -264,10 +257,10 @@ __global__ void __launch_bounds__(kThreads) kry_anchor_kernel(Dev d, Kry kr, con
 
 // x += Sigma e (x a halo array, e line-major).
 __global__ void __launch_bounds__(kThreads) kry_update_kernel(Dev d, Kry kr, double* x) {
-  const long long n = (long long)ncell(d);
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
+  const unsigned int n = (unsigned int)ncell(d);
+  for (unsigned int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
     int i, j, k;
-    cell_of(d, t, i, j, k);
+    cell_ijk(d, t, i, j, k);
     x[hidx(d, i, j, k)] += kr.sig[t] * (double)kr.e[lq(kr, i, j, k)];
   }
 }

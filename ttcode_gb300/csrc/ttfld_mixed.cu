@@ -32,6 +32,7 @@ struct Cmp {
   long long rows;       // ny * nz
   size_t csz;           // slots per colour array (no ghost planes)
   size_t gsz;           // slots per colour array with theta ghost planes
+  FastDiv by_pairs;     // nxp / 2
 };
 
 static Cmp make_cmp(const Dev& d) {
@@ -40,6 +41,7 @@ static Cmp make_cmp(const Dev& d) {
   g.poles = d.poles;
   int nxh = (d.nx + 1) / 2;
   g.nxp = (nxh + 3) / 4 * 4;
+  g.by_pairs = fast_div(g.nxp / 2);
   g.rows = (long long)d.ny * d.nz;
   g.csz = (size_t)g.rows * g.nxp;
   g.gsz = (size_t)(d.nz + 2) * d.ny * g.nxp;
@@ -155,15 +157,15 @@ static int prep32(ttfld_ctx* c) {
     size_t q = cidx(d, i, j, k);
     int col = (i + j + k) & 1;
     size_t s = cslot(g, j - 1, k - 1, (i - 1) >> 1);
-    double inv = 1.0 / d.SA[q];
-    m.a[0][col][s] = (float)(d.SB[q] * inv);
-    m.a[1][col][s] = (float)(d.SC[q] * inv);
-    m.a[2][col][s] = (float)(d.SD[q] * inv);
-    m.a[3][col][s] = (float)(d.SE[q] * inv);
-    m.a[4][col][s] = (float)(d.SF[q] * inv);
-    m.a[5][col][s] = (float)(d.SG[q] * inv);
-    m.ainv[col][s] = (float)inv;
-    m.diag[col][s] = (float)d.SA[q];
+    const double inv = div_rn(1.0, d.SA[q]);
+    m.a[0][col][s] = f32_rn(d.SB[q] * inv);
+    m.a[1][col][s] = f32_rn(d.SC[q] * inv);
+    m.a[2][col][s] = f32_rn(mul_rn(d.SD[q], inv));
+    m.a[3][col][s] = f32_rn(mul_rn(d.SE[q], inv));
+    m.a[4][col][s] = f32_rn(mul_rn(d.SF[q], inv));
+    m.a[5][col][s] = f32_rn(mul_rn(d.SG[q], inv));
+    m.ainv[col][s] = f32_rn(inv);
+    m.diag[col][s] = f32_rn(d.SA[q]);
   });
   TT_CHECK_LAUNCH();
   return 0;
@@ -173,8 +175,8 @@ __device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast
 __device__ __forceinline__ void st4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
 // Loads of the correction e are plain coherent loads, never the read-only
 // path: the persistent kernels write e in one half-sweep and read it, from
-// other SMs, in the next.  The wait between them (acquire loads and a fence
-// by the polling threads, then a block barrier) orders those loads after
+// other SMs, in the next.  The wait between them (acquire loads by the
+// polling threads, then a block barrier) orders those loads after
 // the other blocks' writes, as the PTX memory model defines it.
 __device__ __forceinline__ float4 lde4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ float lde(const float* p) { return *p; }
@@ -792,7 +794,7 @@ static int add_correction(ttfld_ctx* c, double* x) {
     int col = (i + j + k) & 1;
     const float* e = col ? e1 : e0;
     size_t q = hidx(d, i, j, k);
-    x[q] = x[q] + (double)e[gslot(g, j - 1, k - 1, (i - 1) >> 1)];
+    x[q] = x[q] + f64_of_f32(e[gslot(g, j - 1, k - 1, (i - 1) >> 1)]);
   });
   TT_CHECK_LAUNCH();
   return 0;
@@ -813,7 +815,7 @@ static int add_correction_unless(ttfld_ctx* c, double* x, int it0) {
     int col = (i + j + k) & 1;
     const float* e = col ? e1 : e0;
     size_t q = hidx(d, i, j, k);
-    x[q] = x[q] + (double)e[gslot(g, j - 1, k - 1, (i - 1) >> 1)];
+    x[q] = x[q] + f64_of_f32(e[gslot(g, j - 1, k - 1, (i - 1) >> 1)]);
   });
   TT_CHECK_LAUNCH();
   return 0;
@@ -825,13 +827,12 @@ __global__ void __launch_bounds__(kThreads) resid32_kernel(Dev d, Cmp g, Mix32 m
   __shared__ double sh[32];
   __shared__ bool last;
   const int nx = d.nx, ny = d.ny;
-  const long long n = (long long)nx * ny * sor_zmax(d);  // the rows the SOR solves
+  const unsigned int n = (unsigned int)nx * ny * sor_zmax(d);  // the rows the SOR solves
   const size_t sj = (size_t)(nx + 4), sk = (size_t)(nx + 4) * (ny + 4);
   double acc = 0.0;
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-    int i = (int)(t % nx) + 1;
-    long long r = t / nx;
-    int j = (int)(r % ny) + 1, k = (int)(r / ny) + 1;
+  for (unsigned int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+    int i, j, k;
+    cell_ijk(d, t, i, j, k);
     size_t q = hidx(d, i, j, k);
     size_t qjm = (j == 1) ? hidx(d, i, ny, k) : q - sj;
     size_t qjp = (j == ny) ? hidx(d, i, 1, k) : q + sj;
@@ -846,7 +847,7 @@ __global__ void __launch_bounds__(kThreads) resid32_kernel(Dev d, Cmp g, Mix32 m
     acc += fabs(rr);
     int col = (i + j + k) & 1;
     size_t s = cslot(g, j - 1, k - 1, (i - 1) >> 1);
-    m.rhat[col][s] = __double2float_rn(rr) * m.ainv[col][s];
+    m.rhat[col][s] = f32_rn(rr) * m.ainv[col][s];
   }
   double sblk = block_sum(acc, sh);
   if (threadIdx.x == 0) {
@@ -895,7 +896,7 @@ static int rhat_of_b(ttfld_ctx* c, const double* b) {
   launch_box(c->stream, box(1, d.nx, 1, d.ny, 1, d.nz), [=] __device__(int i, int j, int k) {
     const int col = (i + j + k) & 1;
     const size_t s = cslot(g, j - 1, k - 1, (i - 1) >> 1);
-    m.rhat[col][s] = __double2float_rn(b[cidx(d, i, j, k)]) * m.ainv[col][s];
+    m.rhat[col][s] = f32_rn(b[cidx(d, i, j, k)]) * m.ainv[col][s];
   });
   TT_CHECK_LAUNCH();
   return 0;
@@ -1284,19 +1285,18 @@ __global__ void __launch_bounds__(kThreads) sweep64_kernel(Dev d, Cmp g, Fast64 
   __shared__ double sh[32];
   __shared__ bool last;
   if (solver_done(d)) return;
-  const int nv = g.nxp >> 1;
-  const long long n = g.rows * nv;
+  const unsigned int n = (unsigned int)g.rows * g.by_pairs.d;
   const double* __restrict__ xo = m.x[1 - COL];
   double* __restrict__ xs = m.x[COL];
   const size_t plane = (size_t)g.ny * g.nxp;
   double acc = 0.0;
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-    const int hv = (int)(t % nv);
-    const long long rr = t / nv;
-    const int j0 = (int)(rr % g.ny), k0 = (int)(rr / g.ny);
+  for (unsigned int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+    unsigned int hv, ju;
+    const unsigned int rr = div_rem(g.by_pairs, t, hv);
+    const int k0 = (int)div_rem(d.by_ny, rr, ju), j0 = (int)ju;
     if (POLES && k0 == g.nz - 1) continue;  // zmax_sor_index = NZ-1 (ppsor.f:39-43)
     const int off = (1 + ((j0 + k0) & 1) + COL) & 1;
-    const int h0 = hv * 2;
+    const int h0 = (int)hv * 2;
     const int ncol = (g.nx - off + 1) >> 1;
     const size_t cb = (size_t)rr * g.nxp + h0;
     const size_t eb = gslot(g, j0, k0, h0);

@@ -99,24 +99,29 @@ static int rows(ttfld_ctx* c, double theta, bool divf_is_old) {
     const double divf = divf_is_old ? d.DIVF_OLD[q] : divf_cell(d, t, i, j, k);
     d.DIVF[q] = divf;
     double qq = d.Q[h], rh = d.RH[h], cv = d.CV[h], er = d.ER[h], kp = d.XKAPP[h];
-    double qr = qq / (rh * cv);
-    double bb = TT_ARAD * p4(qr);
+    // quotients and about half of the products on the integer pipes
+    // (ttfld_fp64.cuh); the common subexpressions of the reference's
+    // formulas are formed once, in its operand order
+    const double qr = div_rn(qq, rh * cv);
+    const double bb = TT_ARAD * p4(qr), gap = bb - er, dtc = div_rn(d.delt, cv);
+    const double emit = mul_rn(mul_rn(mul_rn(kp * 4.0, TT_ARAD), TT_FD), p3(qr));
+    const double turn = TT_FD * gap * d.DXKAPP[h];
+    const double couple = mul_rn(mul_rn(rh, kp), TT_FD) * gap;
     double fq, dfq;
-    double dfr = -((d.delt / cv) * (kp * 4.0 * TT_ARAD * TT_FD * p3(qr) + TT_FD * (bb - er) * d.DXKAPP[h]));
+    const double dfr = -(dtc * (emit + turn));
     if (d.f_incident > 1) {
       double si = d.SI[h];
-      double heat = si / (rh * d.XKAPA[h]);
-      fq = qq - d.Q_OLD[h] + d.delt * ((1 - theta) * (d.DIVF_OLD[q] - divf) + (rh * kp * TT_FD * (bb - er)) - si);
-      dfq = 1.0 + (d.delt / cv) * (kp * 4.0 * TT_ARAD * TT_FD * p3(qr) + (TT_FD * (bb - er) * d.DXKAPP[h]) -
-                                   heat * d.DXKAPA[h]);
+      double heat = div_rn(si, mul_rn(rh, d.XKAPA[h]));
+      fq = qq - d.Q_OLD[h] + d.delt * ((1 - theta) * (d.DIVF_OLD[q] - divf) + couple - si);
+      dfq = 1.0 + dtc * (emit + turn - heat * d.DXKAPA[h]);
     } else {
-      fq = qq - d.Q_OLD[h] + d.delt * ((1 - theta) * (d.DIVF_OLD[q] - divf) + rh * kp * TT_FD * (bb - er));
-      dfq = 1.0 + (d.delt / cv) * (kp * 4.0 * TT_ARAD * TT_FD * p3(qr) + TT_FD * (bb - er) * d.DXKAPP[h]);
+      fq = qq - d.Q_OLD[h] + d.delt * ((1 - theta) * (d.DIVF_OLD[q] - divf) + couple);
+      dfq = 1.0 + dtc * (emit + turn);
     }
-    double fr = er - d.ER_OLD[h] + d.delt * (divf - rh * kp * TT_FD * (bb - er));
+    double fr = er - d.ER_OLD[h] + mul_rn(d.delt, divf - couple);
     d.FQ[q] = fq; d.FR[q] = fr; d.DFQ[q] = dfq; d.DFR[q] = dfr;
     double eta;
-    if (dfq != 0.0) eta = -dfr / dfq;
+    if (dfq != 0.0) eta = div_rn(-dfr, dfq);
     else { eta = 0.0; d.stp->dfq_zero = 1; }
     d.ETA[q] = eta;
     const EvalRow e = evalues_cell(d, i, j, k, theta, eta);
@@ -132,32 +137,32 @@ static int rows(ttfld_ctx* c, double theta, bool divf_is_old) {
 // (ppenergy.f:379-541), fused with the damped update of :551-573 (each cell
 // reads only its own Q and E_R, which only it updates).
 __global__ void __launch_bounds__(kThreads) delta_q_kernel(Dev d, double theta, double conv) {
-  const int nx = d.nx, ny = d.ny, nz = d.nz;
-  const long long n = (long long)(nx - 1) * ny * nz;  // i = 2..NX
+  const int nx = d.nx, ny = d.ny;
+  const unsigned int n = (unsigned int)ncell(d);
   const size_t sj = (size_t)(nx + 4), sk = (size_t)(nx + 4) * (ny + 4);
   const double* x = d.DELTA_ER;
   double mq = 0.0, me = 0.0;
   int bad = 0;
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-    int i = 2 + (int)(t % (nx - 1));
-    long long r = t / (nx - 1);
-    int j = (int)(r % ny) + 1, k = (int)(r / ny) + 1;
+  for (unsigned int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+    int i, j, k;
+    cell_ijk(d, t, i, j, k);
     int xmax_index = PA(UB, j, k) - 1;
-    if (i > xmax_index || xmax_index > nx) continue;
+    if (i < 2 || i > xmax_index || xmax_index > nx) continue;  // i = 2..UPPERBND-1
     size_t h = hidx(d, i, j, k), q = cidx(d, i, j, k);
-    double q1 = -d.delt * (1.0 - theta);
-    double q2 = d.delt * d.RH[h] * d.XKAPP[h] * TT_FD;
-    double dq = (1.0 / d.DFQ[q]) *
-                (q1 * d.E16[q] * x[h] - q1 * d.E1[q] * x[h + 1] - q1 * d.E2[q] * x[h - 1] -
-                 q1 * d.E3[q] * x[h + sj] - q1 * d.E4[q] * x[h - sj] - q1 * d.E5[q] * x[h + sk] -
-                 q1 * d.E6[q] * x[h - sk] + q2 * x[h] - d.FQ[q]);
+    const double q1 = -d.delt * (1.0 - theta);
+    const double q2 = mul_rn(mul_rn(d.delt, d.RH[h]) * d.XKAPP[h], TT_FD);
+    double flow = 0.0;  // theta = 1 (ppenergy.f:60): the seven products are zeros
+    if (q1 != 0.0)
+      flow = q1 * d.E16[q] * x[h] - q1 * d.E1[q] * x[h + 1] - q1 * d.E2[q] * x[h - 1] - q1 * d.E3[q] * x[h + sj] -
+             q1 * d.E4[q] * x[h - sj] - q1 * d.E5[q] * x[h + sk] - q1 * d.E6[q] * x[h - sk];
+    const double dq = mul_rn(div_rn(1.0, d.DFQ[q]), flow + mul_rn(q2, x[h]) - d.FQ[q]);
     d.DQ[q] = dq;
     double qv = d.Q[h], erv = d.ER[h];
     if ((qv + conv * dq) <= 0.0) bad = 1;
-    mq = fmax(mq, fabs(dq / qv));
-    me = fmax(me, fabs(x[h] / erv));
+    mq = fmax(mq, fabs(div_rn(dq, qv)));
+    me = fmax(me, fabs(div_rn(x[h], erv)));
     d.ER[h] = erv + conv * x[h];
-    d.Q[h] = qv + conv * dq;
+    d.Q[h] = qv + mul_rn(conv, dq);
   }
   // max is exact in any order: reduce in the warp, one atomic per warp
   for (int o = 16; o > 0; o >>= 1) {
@@ -174,7 +179,7 @@ __global__ void __launch_bounds__(kThreads) delta_q_kernel(Dev d, double theta, 
 
 static int delta_q_update(ttfld_ctx* c, double theta, double conv) {
   const Dev& d = c->d;
-  delta_q_kernel<<<grid_for((long long)(d.nx - 1) * d.ny * d.nz), kThreads, 0, c->stream>>>(d, theta, conv);
+  delta_q_kernel<<<grid_for((long long)ncell(d)), kThreads, 0, c->stream>>>(d, theta, conv);
   count_launches(1);
   TT_CHECK_LAUNCH();
   return 0;
@@ -185,7 +190,7 @@ static int finish_step(ttfld_ctx* c) {  // ppenergy.f:787-789
   launch_box(c->stream, box(-1, d.nx + 2, -1, d.ny + 2, -1, d.nz + 2), [=] __device__(int i, int j, int k) {
     size_t h = hidx(d, i, j, k);
     d.DELTA_ER[h] = d.ER[h] - d.ER_OLD[h];
-    d.T[h] = d.Q[h] / (d.RH[h] * d.CV[h]);
+    d.T[h] = div_rn(d.Q[h], mul_rn(d.RH[h], d.CV[h]));
   });
   TT_CHECK_LAUNCH();
   return 0;
@@ -207,7 +212,7 @@ int coupled_energy_eqs(ttfld_ctx* c, int do_bounds, ttfld_step_stats* out) {
   if (do_bounds && (rc = asm_bounds(c))) return rc;                     // :63
   launch_box(c->stream, box(-1, d.nx + 2, -1, d.ny + 2, -1, d.nz + 2), [=] __device__(int i, int j, int k) {
     size_t h = hidx(d, i, j, k);
-    d.Q[h] = d.RH[h] * d.CV[h] * d.T[h];                                 // :65
+    d.Q[h] = mul_rn(d.RH[h], d.CV[h]) * d.T[h];                          // :65
   });
   TT_CHECK_LAUNCH();
   // Recomputations that reproduce their inputs bit for bit are left out:
