@@ -218,7 +218,7 @@ int ttfld_create(ttfld_ctx** out, const ttfld_dims* dims, const ttfld_metrics* m
   bytes += nh * align_up(H * 8, A) + nc * align_up(Cn * 8, A) + nf * align_up(Fn * 8, A);
   bytes += 3 * align_up(Pn * 8, A) + ng * align_up((size_t)n1 * 8, A);
   bytes += align_up(sizeof(SolverDev), A) + align_up(sizeof(StepDev), A);
-  bytes += align_up(2 * kMaxPartials * 8, A);
+  bytes += align_up(2 * kMaxPartials * 8, A) + align_up(kFlagBytes, A);
   size_t staging = H > Fn ? H : Fn;
   bytes += align_up(staging * 8, A);
   char* base = nullptr;
@@ -238,6 +238,7 @@ int ttfld_create(ttfld_ctx** out, const ttfld_dims* dims, const ttfld_metrics* m
   c->sol = (SolverDev*)take(sizeof(SolverDev));
   c->stp = (StepDev*)take(sizeof(StepDev));
   c->partials = (double*)take(2 * kMaxPartials * 8);
+  c->flags64 = (unsigned int*)take(kFlagBytes);
   c->staging = (double*)take(staging * 8);
   d.sol = c->sol;
   d.stp = c->stp;

@@ -128,35 +128,53 @@ TT_FP_HD double hw_div(double a, double b) { return a / b; }
 TT_FP_HD double hw_sqrt(double a) { return sqrt(a); }
 #endif
 
-// a b.  The mantissas (2^52..2^53) are taken times 2^11 and 2, so that the
-// high 64 bits of their product lie in [2^52, 2^54) and the low 64 bits are
-// the part that is rounded away.
+// a b.  The 106-bit product P of the mantissas is P2 (from bit 64 up), P1, P0;
+// c is 1 if it is 2^105 or more, and its leading 53 bits m and the part that
+// is rounded away, top-aligned in rh:rl, come by shifts of 20 + c and 12 - c.
+// m is rounded up if rh:rl is above half, or half with m odd: then
+// rh + 2^31 - 1 + odd carries (the bits of rl joined to rh's last one).  The
+// fast path is for operands and results in [2^-511, 2^512): the first two
+// exponent bits differ.
 TT_FP_HD double mul_rn(double a, double b) {
   const uint64_t ua = f64_bits(a), ub = f64_bits(b);
   const uint32_t ah = hi32(ua), al = lo32(ua), bh = hi32(ub), bl = lo32(ub);
-  const uint32_t ea = (ah >> 20) & 0x7ffu, eb = (bh >> 20) & 0x7ffu;
   const uint32_t mh = (ah & 0xfffffu) | 0x100000u, nh = (bh & 0xfffffu) | 0x100000u;
-  const uint32_t xh = (mh << 11) | (al >> 21), xl = al << 11;
-  const uint32_t yh = (nh << 1) | (bl >> 31), yl = bl << 1;
-  const uint64_t t0 = wide(xl, yl);
-  const uint64_t t1 = wide(xh, yl) + hi32(t0);
-  const uint64_t t2 = wide(xl, yh) + lo32(t1);
-  const uint64_t t3 = wide(xh, yh) + hi32(t1) + hi32(t2);
-  const uint32_t c = hi32(t3) >> 21;  // 1 if the product is 2^53 or more in units of the high part
-  const uint32_t m0 = shr64_lo(lo32(t3), hi32(t3), (int)c);
-  const uint32_t rh = shr64_lo(lo32(t2), lo32(t3), (int)c);  // first 32 bits rounded away
-  const uint32_t rl = lo32(t0) | (lo32(t2) & c);             // the rest (or its absence)
-  const uint32_t s = (rl != 0u ? 1u : 0u) | (m0 & 1u);
-  const uint64_t m = (t3 >> c) + (rh > 0x80000000u - s ? 1u : 0u);
-  const int32_t e = (int32_t)(ea + eb + c) - 1024;  // the leading mantissa bit adds the missing 1
-  // both operands normal, the result clear of either end of the range
-  if (ea - 1u < 2046u && eb - 1u < 2046u && (uint32_t)(e - 1) < 2043u) {
-    const uint32_t sign = (ah ^ bh) & 0x80000000u;
-    return f64_of((((uint64_t)((uint32_t)e << 20 | sign)) << 32) + m);
-  }
+  const uint64_t t0 = wide(al, bl), t1 = wide(mh, bl) + wide(al, nh), t2 = wide(mh, nh);  // t1 < 2^54
+  uint32_t p1, p2l, p2h;
+#if defined(__CUDA_ARCH__)
+  asm("add.cc.u32 %0, %3, %4;\n\taddc.cc.u32 %1, %5, %6;\n\taddc.u32 %2, %7, 0;"
+      : "=&r"(p1), "=&r"(p2l), "=r"(p2h)
+      : "r"(hi32(t0)), "r"(lo32(t1)), "r"(lo32(t2)), "r"(hi32(t1)), "r"(hi32(t2)));
+#else
+  const uint64_t w = (uint64_t)hi32(t0) + lo32(t1), v = t2 + hi32(t1) + (w >> 32);
+  p1 = lo32(w);
+  p2l = lo32(v);
+  p2h = hi32(v);
+#endif
+  const uint32_t c = p2h >> 9;
+  const uint32_t ml = shr64_lo(p1, p2l, (int)(20u + c));
+  const uint32_t mu = shr64_lo(p2l, p2h, (int)(20u + c));
+  const uint32_t rl = lo32(t0) << (12u - c);
+  const uint32_t rest = shr64_lo(lo32(t0), p1, (int)(20u + c)) | (rl < 1u ? rl : 1u);
+  const uint32_t half = 0x7fffffffu + (ml & 1u);
+  const uint32_t e = (ah & 0x7ff00000u) + (bh & 0x7ff00000u) + (c << 20) - (1024u << 20) + ((ah ^ bh) & 0x80000000u);
+  uint32_t ol, oh;
+#if defined(__CUDA_ARCH__)
+  uint32_t drop;
+  asm("add.cc.u32 %0, %3, %4;\n\taddc.cc.u32 %1, %5, 0;\n\taddc.u32 %2, %6, %7;"
+      : "=&r"(drop), "=&r"(ol), "=r"(oh)
+      : "r"(rest), "r"(half), "r"(ml), "r"(mu), "r"(e));
+#else
+  const uint64_t o = (((uint64_t)(mu + e) << 32) | ml) + (((uint64_t)rest + half) >> 32);
+  ol = lo32(o);
+  oh = hi32(o);
+#endif
+  if (((ah ^ (ah << 1)) & (bh ^ (bh << 1)) & (oh ^ (oh << 1)) & 0x40000000u) != 0u)
+    return f64_of(((uint64_t)oh << 32) | ol);
   // a zero operand (no flow across a face, a boundary row) needs no product
-  const uint32_t ma = (al | (ah << 1)) == 0u, mb = (bl | (bh << 1)) == 0u;
-  if ((ma && eb < 2047u) || (mb && ea < 2047u)) return f64_of((uint64_t)((ah ^ bh) & 0x80000000u) << 32);
+  const uint32_t ea = (ah >> 20) & 0x7ffu, eb = (bh >> 20) & 0x7ffu;
+  const bool za = (al | (ah << 1)) == 0u, zb = (bl | (bh << 1)) == 0u;
+  if ((za && eb < 2047u) || (zb && ea < 2047u)) return f64_of((uint64_t)((ah ^ bh) & 0x80000000u) << 32);
   return hw_mul(a, b);
 }
 

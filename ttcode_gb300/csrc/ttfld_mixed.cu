@@ -22,7 +22,7 @@
 // theta neighbours at the same h.
 #include <math.h>
 
-#include "ttfld_internal.cuh"
+#include "ttfld_sweep64.cuh"
 
 namespace ttfld {
 
@@ -62,11 +62,6 @@ struct Fast64 {
   double* diag[2];  // A
   double* x[2];     // iterate, with theta ghost planes
 };
-
-// Per-block flags of the neighbour-flag sweep form (below).
-constexpr int kFlagStride = 32;        // unsigned ints per flag: one 128-byte line per block
-constexpr int kMaxLocalBlocks = 1024;  // flags in the workspace
-constexpr size_t kFlagBytes = (size_t)kMaxLocalBlocks * kFlagStride * sizeof(unsigned int);
 
 struct MixWork {
   Cmp g;
@@ -406,55 +401,6 @@ __global__ void __launch_bounds__(kPersistThreads) sweeps32_persistent(Cmp g, Mi
 // faster per sweep at 100x128x128, 100x256x128, 100x256x160 and
 // 160x512x256, the same at 160x256x128 and 60x512x256 (a slow block holds
 // up only its neighbours, not the grid).
-
-__device__ __forceinline__ void st_release(unsigned int* p, unsigned int v) {
-  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
-// The block whose items [n b / nb, n (b + 1) / nb) hold item t (0 <= t < n).
-__device__ __forceinline__ int owner_block(long long t, long long n, int nb) {
-  int b = (int)(t * nb / n);
-  while (b + 1 < nb && n * (b + 1) / nb <= t) ++b;
-  while (b > 0 && n * b / nb > t) --b;
-  return b;
-}
-
-// This block has finished v half-sweeps: after every thread's stores.  The
-// block barrier orders them before thread 0's release, which is cumulative
-// (PTX memory model), so no fence of its own is needed; a fence there, one
-// after the acquire in wait_flags and a 32 ns sleep between polls cost 2-9 %
-// of a whole implicit step (1.158 against 1.080 ms at 40x64x32, 19.6 against
-// 19.1 ms at 100x256x128).
-__device__ __forceinline__ void publish_flag(unsigned int* flag, unsigned int v) {
-  __syncthreads();
-  if (threadIdx.x == 0) st_release(flag, v);
-}
-
-// Wait until blocks lo..hi other than this one have finished at least
-// `target` half-sweeps; warp 0 polls, one flag per lane.  Bounded like the
-// grid barriers: false after kBarrierSpins polls or once another block has
-// given up.
-__device__ __forceinline__ bool wait_flags(const unsigned int* flags, int lo, int hi, unsigned int target,
-                                           SolverDev* sol) {
-  __shared__ int ok_sh;
-  if (threadIdx.x < 32) {
-    int ok = 1;
-    long long polls = 0;
-    for (;;) {
-      bool ready = true;
-      for (int q = lo + (int)threadIdx.x; q <= hi; q += 32)
-        if (q != (int)blockIdx.x && (int)(ld_acquire(flags + (size_t)q * kFlagStride) - target) < 0) ready = false;
-      if (__all_sync(0xffffffffu, ready)) break;
-      if (__any_sync(0xffffffffu, give_up(++polls, sol))) { ok = 0; break; }
-    }
-    if (threadIdx.x == 0) {
-      if (!ok) atomicExch(&sol->bar_timeout, 1);
-      ok_sh = ok;
-    }
-  }
-  __syncthreads();
-  return ok_sh != 0;
-}
 
 template <bool POLES>
 __global__ void __launch_bounds__(kPersistThreads) sweeps32_local(Cmp g, Mix32 m, float omega, SolverDev* sol,
@@ -1236,7 +1182,7 @@ static int prep64(ttfld_ctx* c, const double* x, const double* b) {
     int col = (i + j + k) & 1;
     size_t s = cslot(g, j - 1, k - 1, (i - 1) >> 1);
     double a = d.SA[q];
-    double inv = 1.0 / a;
+    const double inv = div_rn(1.0, a);
     double bb = b[q];
     if (i == 1) bb = bb - d.SB[q] * x[hidx(d, 0, j, k)];
     if (i == d.nx) bb = bb - d.SC[q] * x[hidx(d, d.nx + 1, j, k)];
@@ -1244,12 +1190,12 @@ static int prep64(ttfld_ctx* c, const double* x, const double* b) {
     // cell's own value, and row NZ is not swept: nothing to fold
     if (!d.poles && k == 1) bb = bb - d.SF[q] * x[hidx(d, i, j, 0)];
     if (!d.poles && k == d.nz) bb = bb - d.SG[q] * x[hidx(d, i, j, d.nz + 1)];
-    m.a[0][col][s] = d.SB[q] * inv;
-    m.a[1][col][s] = d.SC[q] * inv;
-    m.a[2][col][s] = d.SD[q] * inv;
-    m.a[3][col][s] = d.SE[q] * inv;
-    m.a[4][col][s] = d.SF[q] * inv;
-    m.a[5][col][s] = d.SG[q] * inv;
+    m.a[0][col][s] = mul_rn(d.SB[q], inv);
+    m.a[1][col][s] = mul_rn(d.SC[q], inv);
+    m.a[2][col][s] = mul_rn(d.SD[q], inv);
+    m.a[3][col][s] = mul_rn(d.SE[q], inv);
+    m.a[4][col][s] = mul_rn(d.SF[q], inv);
+    m.a[5][col][s] = mul_rn(d.SG[q], inv);
     m.bhat[col][s] = bb * inv;
     m.diag[col][s] = a;
     m.x[col][gslot(g, j - 1, k - 1, (i - 1) >> 1)] = x[hidx(d, i, j, k)];
@@ -1350,7 +1296,85 @@ __global__ void __launch_bounds__(kThreads) sweep64_kernel(Dev d, Cmp g, Fast64 
   }
 }
 
+// The same two cells at a time for the persistent sweeps (ttfld_sweep64.cuh).
+// The seven fused multiply-adds and two sums of a cell stay on the FP64
+// pipe, the product of its norm goes to the integer pipes.
+struct FastRows {
+  typedef double2 Word;
+  static constexpr int kWords = 8, kThreads = 768;  // 196 KB for two stages
+  Fast64 m;
+  double omega;
+  long long rows;
+  int nx, ny, nz, nxp, poles;
+  FastDiv by_items, by_ny;
+  __device__ double norm(double sum) const { return sum; }
+  template <int COL>
+  __device__ void before(unsigned int, unsigned int) const {}
+  template <int COL>
+  __device__ void after(unsigned int, unsigned int, bool) const {}
+  template <int COL>
+  __device__ __forceinline__ void fetch(unsigned int row, unsigned int h, double2* to, unsigned int T) const {
+    const size_t c = (size_t)row * nxp + 2 * h;
+#pragma unroll
+    for (int q = 0; q < 6; ++q) copy_async(to + q * T, reinterpret_cast<const double2*>(m.a[q][COL] + c));
+    copy_async(to + 6 * T, reinterpret_cast<const double2*>(m.bhat[COL] + c));
+    copy_async(to + 7 * T, reinterpret_cast<const double2*>(m.diag[COL] + c));
+  }
+  template <int COL>
+  __device__ __forceinline__ double update(unsigned int row, unsigned int h, const double2* w, unsigned int T,
+                                           bool) const {
+    unsigned int j0;
+    const unsigned int k0 = div_rem(by_ny, row, j0);
+    const double* xo = m.x[1 - COL];
+    double* xs = m.x[COL];
+    const int off = (1 + ((j0 + k0) & 1) + COL) & 1, h0 = 2 * (int)h, ncol = (nx - off + 1) >> 1;
+    const size_t plane = (size_t)ny * nxp, eb = plane + (size_t)row * nxp + h0;  // a theta ghost plane first
+    const size_t ejm = j0 == 0 ? eb + (size_t)(ny - 1) * nxp : eb - nxp;
+    const size_t ejp = (int)j0 == ny - 1 ? eb - (size_t)(ny - 1) * nxp : eb + nxp;
+    const double2 o = ld2(xo + eb), s = ld2(xo + ejm), nn = ld2(xo + ejp), xv = ld2(xs + eb);
+    double xm0, xm1, xp0, xp1;
+    if (off == 0) {
+      xm0 = h0 > 0 ? xo[eb - 1] : 0.0; xm1 = o.x; xp0 = o.x; xp1 = o.y;
+    } else {
+      xm0 = o.x; xm1 = o.y; xp0 = o.y; xp1 = (h0 + 2 < nxp) ? xo[eb + 2] : 0.0;
+    }
+    const double2 bz = (poles && k0 == 0) ? xv : ld2(xo + eb - plane);
+    const double2 tz = (poles && (int)k0 == nz - 2) ? xv : ld2(xo + eb + plane);
+    double share = 0.0;
+    double2 out = make_double2(0.0, 0.0);
+#define TT_CELL(L, IDX, XM, XP)                                                                                     \
+    if (h0 + IDX < ncol) {                                                                                          \
+      const double rh = fma(w[0].L, XM, fma(w[T].L, XP, fma(w[2 * T].L, s.L, fma(w[3 * T].L, nn.L,                   \
+                        fma(w[4 * T].L, bz.L, fma(w[5 * T].L, tz.L, xv.L - w[6 * T].L))))));                          \
+      share += fabs(mul_rn(w[7 * T].L, rh));                                                                        \
+      out.L = fma(-omega, rh, xv.L);                                                                                \
+    }
+    TT_CELL(x, 0, xm0, xp0)
+    TT_CELL(y, 1, xm1, xp1)
+#undef TT_CELL
+    st2(xs + eb, out);
+    return share;
+  }
+};
+
+// nsweeps sweeps (fewer if the rule fires) in one launch; 1 where that is
+// not possible.
+static int launch_fast_persistent(ttfld_ctx* c, int nsweeps, int itmin, int itmax, double eps) {
+  MixWork* w = work(c);
+  const Cmp& g = w->g;
+  FastRows s;
+  s.m = w->m64;
+  s.omega = c->d.sorparam;
+  s.rows = (long long)g.ny * (g.poles ? g.nz - 1 : g.nz);  // zmax_sor_index (ppsor.f:39-43)
+  s.nx = g.nx; s.ny = g.ny; s.nz = g.nz; s.nxp = g.nxp; s.poles = g.poles;
+  s.by_items = g.by_pairs;
+  s.by_ny = c->d.by_ny;
+  return launch_sweeps64_persistent(s, c->stream, c->sol, c->partials, c->flags64, nsweeps, itmin, itmax, eps);
+}
+
 int launch_sweeps64(ttfld_ctx* c, int nsweeps, int itmin, int itmax, double eps) {
+  const int rc = launch_fast_persistent(c, nsweeps, itmin, itmax, eps);
+  if (rc <= 0) return rc;
   MixWork* w = work(c);
   const Cmp& g = w->g;
   long long nvec = g.rows * (g.nxp >> 1);
@@ -1383,10 +1407,11 @@ int solve_fast64(ttfld_ctx* c, double* x, const double* b, int itmin, int itmax,
   if ((rc = rhs_norm(c, b, nullptr))) return rc;
   int chunk = 4, launched = 0;
   for (;;) {
-    if ((rc = launch_sweeps64(c, chunk, itmin, itmax, c->d.epsmat))) return rc;
+    // the persistent kernel stops itself, at ITMAX at the latest
+    if ((rc = launch_fast_persistent(c, itmax, itmin, itmax, c->d.epsmat)) <= 0) chunk = itmax;
+    else rc = launch_sweeps64(c, chunk, itmin, itmax, c->d.epsmat);
+    if (rc || (rc = poll(c))) return rc;
     launched += chunk;
-    TT_CHECK(cudaMemcpyAsync(c->host_sol, c->sol, sizeof(SolverDev), cudaMemcpyDeviceToHost, c->stream));
-    TT_CHECK(cudaStreamSynchronize(c->stream));
     if (c->host_sol->done) break;
     if (launched >= itmax + 2) return TTFLD_E_CUDA;
     chunk = chunk < 128 ? chunk * 2 : 256;

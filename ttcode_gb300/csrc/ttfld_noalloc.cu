@@ -32,7 +32,7 @@
 //    synchronises its stream to read the stopping flag).
 #include <mutex>
 
-#include "ttfld_internal.cuh"
+#include "ttfld_sweep64.cuh"
 
 namespace ttfld {
 namespace {
@@ -40,22 +40,15 @@ namespace {
 constexpr int kNoAllocMaxRows = 131072;
 constexpr int kNoAllocMaxContexts = 64;
 
-struct NoAllocState {
-  double rhsnorm;
-  double rnorm;
-  int iter;
-  int done;
-  int maxit;
-  int nonfinite;
-  unsigned int ticket;
-  int pad[7];
-};
-
 struct NoAllocScratch {
-  NoAllocState st;                       // 64 B, cleared by every call
-  double pad[24];                        // keeps partials 256-B aligned
-  double partials[2][kNoAllocMaxRows];   // |resid| summed per (j,k) row and colour
+  SolverDev st;                          // cleared by every call
+  // |resid| summed per (j,k) row and colour (one launch per colour), or the
+  // blocks' partials and half-sweep flags of the persistent sweeps
+  double partials[2][kNoAllocMaxRows];
 };
+static_assert(sizeof(SolverDev) == 256, "the scratch is 2 MiB + 256 B, its partials 256-B aligned");
+static_assert(2 * kMaxPartials <= kNoAllocMaxRows && kFlagBytes <= kNoAllocMaxRows * sizeof(double),
+              "the persistent sweeps' partials and flags fit in the scratch");
 
 static __device__ __align__(256) NoAllocScratch g_noalloc_scratch;
 
@@ -182,10 +175,11 @@ __global__ void __launch_bounds__(kThreads) noalloc_sweep_kernel(
       const size_t qjm = (j == 1) ? q + sj * (size_t)(ny - 1) : q - sj;
       const size_t qjp = (j == ny) ? q - sj * (size_t)(ny - 1) : q + sj;
       const double xc = x[q];
-      const double resid = A[c] * xc + B[c] * x[q - 1] + C[c] * x[q + 1] + D[c] * x[qjm] + E[c] * x[qjp] +
-                           F[c] * x[q - sk] + G[c] * x[q + sk] - rhs[c];
+      const double a = A[c];
+      const double resid = mul_rn(a, xc) + mul_rn(B[c], x[q - 1]) + mul_rn(C[c], x[q + 1]) + mul_rn(D[c], x[qjm]) +
+                           mul_rn(E[c], x[qjp]) + mul_rn(F[c], x[q - sk]) + mul_rn(G[c], x[q + sk]) - rhs[c];
       acc = acc + fabs(resid);
-      x[q] = xc - omega * resid / A[c];
+      x[q] = xc - div_rn(omega * resid, a);
     }
     acc = warp_sum(acc);
     if (lane == 0) s->partials[COLOUR][warp] = acc;
@@ -194,7 +188,7 @@ __global__ void __launch_bounds__(kThreads) noalloc_sweep_kernel(
     double r0 = block_sum_array(s->partials[0], rows, sh);
     double r1 = block_sum_array(s->partials[1], rows, sh);
     if (threadIdx.x == 0) {
-      NoAllocState& st = s->st;
+      SolverDev& st = s->st;
       const double rnorm = r0 + r1;
       const int it = st.iter + 1;
       st.iter = it;
@@ -247,15 +241,32 @@ extern "C" int ttfld_sor_solve_noalloc(const double* sor_a, const double* sor_b,
   cudaStream_t st = (cudaStream_t)stream;
   const int rows = ny * nz;
   const int blocks = (int)(((long long)rows * 32 + kThreads - 1) / kThreads);
-  TT_CHECK(cudaMemsetAsync(&s->st, 0, sizeof(NoAllocState), st));
+  TT_CHECK(cudaMemsetAsync(&s->st, 0, sizeof(SolverDev), st));
   noalloc_rhs_kernel<<<blocks, kThreads, 0, st>>>(s, rhs, nx, rows);
   count_launches(1);
   TT_CHECK_LAUNCH();
-  NoAllocState h;
+  SolverDev h;
   int chunk = 4, launched = 0;
   double ratio_prev = 0.0;
   int iter_prev = 0;
-  for (;;) {
+  // the whole solve in one launch; the chunks below where that is not possible
+  const double* const coef[7] = {sor_a, sor_b, sor_c, sor_d, sor_e, sor_f, sor_g};
+  rc = launch_sweeps64_persistent(sor_rows(coef, rhs, x, nx, ny, nz, nz, 0, omega), st, &s->st, s->partials[0],
+                                  (unsigned int*)s->partials[1], itmax, itmin, itmax, epsmat);
+  if (rc < 0) return rc;
+  if (rc == 0) {
+    TT_CHECK(cudaMemcpyAsync(&h, &s->st, sizeof(h), cudaMemcpyDeviceToHost, st));
+    TT_CHECK(cudaStreamSynchronize(st));
+    if (h.bar_timeout) {
+      fprintf(stderr, "ttfld_sor_solve_noalloc: a wait of the persistent sweeps timed out\n");
+      return TTFLD_E_CUDA;
+    }
+    if (!h.done) {
+      fprintf(stderr, "ttfld_sor_solve_noalloc: the sweeps ended without the stopping flag\n");
+      return TTFLD_E_INTERNAL;
+    }
+  }
+  while (rc == 1) {
     for (int q = 0; q < chunk; ++q) {
       noalloc_sweep_kernel<0><<<blocks, kThreads, 0, st>>>(s, sor_a, sor_b, sor_c, sor_d, sor_e, sor_f, sor_g, rhs, x,
                                                            nx, ny, nz, omega, itmin, itmax, epsmat);

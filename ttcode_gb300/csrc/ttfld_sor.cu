@@ -1,7 +1,7 @@
 // ttfld_sor.cu -- FILL_SOR_MATRIX / B_VECTOR_BOUNDARIES and the FP64
 // red-black SOR of SOLVE_WITH_SOR (ppsor.f:2-329) on the device.
 //
-// The exact kernel evaluates each cell update with the reference's operand
+// The exact kernels evaluate each cell update with the reference's operand
 // order and no fused multiply-add, so every sweep leaves DELTA_ER bitwise
 // equal to the serial Fortran loop: within one colour no cell reads another
 // cell of the same colour, so the order of the updates inside a colour does
@@ -11,7 +11,7 @@
 // other colour).  The L1 norm of the in-sweep residuals is reduced in a
 // fixed order (block partials, then one block), so the sweep count is
 // reproducible run to run.
-#include "ttfld_internal.cuh"
+#include "ttfld_sweep64.cuh"
 
 namespace ttfld {
 
@@ -35,9 +35,9 @@ int fill_sor_matrix(ttfld_ctx* c, bool zero_rhs) {
 __global__ void __launch_bounds__(kThreads) rhsnorm_kernel(Dev d, const double* b, double* partials) {
   __shared__ double sh[32];
   __shared__ bool last;
-  const long long n = (long long)ncell(d);
+  const unsigned int n = (unsigned int)ncell(d);
   double acc = 0.0;
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x)
+  for (unsigned int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x)
     acc += fabs(b[t]);
   double s = block_sum(acc, sh);
   if (threadIdx.x == 0) {
@@ -66,25 +66,24 @@ __global__ void __launch_bounds__(kThreads) sor_exact_kernel(Dev d, double* __re
   __shared__ bool last;
   if (solver_done(d)) return;
   const int nx = d.nx, ny = d.ny;
-  const int nxh = (nx + 1) >> 1;
-  const long long n = (long long)nxh * ny * sor_zmax(d);  // rows k = 1..zmax_sor_index
+  const unsigned int n = d.by_nxh.d * (unsigned int)ny * sor_zmax(d);  // rows k = 1..zmax_sor_index
   const size_t sj = (size_t)(nx + 4), sk = (size_t)(nx + 4) * (ny + 4);
   double acc = 0.0;
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-    int h = (int)(t % nxh);
-    long long r = t / nxh;
-    int j = (int)(r % ny) + 1, k = (int)(r / ny) + 1;
-    int i = 2 - ((j + k + COLOUR) & 1) + 2 * h;
+  for (unsigned int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+    unsigned int h, j0;
+    const int k = (int)div_rem(d.by_ny, div_rem(d.by_nxh, t, h), j0) + 1, j = (int)j0 + 1;
+    const int i = 2 - ((j + k + COLOUR) & 1) + 2 * (int)h;
     if (i > nx) continue;
     size_t c = cidx(d, i, j, k);
     size_t q = hidx(d, i, j, k);
     size_t qjm = (j == 1) ? hidx(d, i, ny, k) : q - sj;
     size_t qjp = (j == ny) ? hidx(d, i, 1, k) : q + sj;
-    double xc = x[q];
-    double resid = d.SA[c] * xc + d.SB[c] * x[q - 1] + d.SC[c] * x[q + 1] + d.SD[c] * x[qjm] +
-                   d.SE[c] * x[qjp] + d.SF[c] * x_km(d, x, q, k, sk) + d.SG[c] * x_kp(d, x, q, k, sk) - b[c];
+    const double xc = x[q], a = d.SA[c];
+    const double resid = mul_rn(a, xc) + mul_rn(d.SB[c], x[q - 1]) + mul_rn(d.SC[c], x[q + 1]) +
+                         mul_rn(d.SD[c], x[qjm]) + mul_rn(d.SE[c], x[qjp]) +
+                         mul_rn(d.SF[c], x_km(d, x, q, k, sk)) + mul_rn(d.SG[c], x_kp(d, x, q, k, sk)) - b[c];
     acc = acc + fabs(resid);
-    x[q] = xc - omega * resid / d.SA[c];
+    x[q] = xc - div_rn(omega * resid, a);
   }
   double s = block_sum(acc, sh);
   if (threadIdx.x == 0) {
@@ -109,13 +108,12 @@ __global__ void __launch_bounds__(kThreads) resid_l1_kernel(Dev d, const double*
   __shared__ double sh[32];
   __shared__ bool last;
   const int nx = d.nx, ny = d.ny;
-  const long long n = (long long)nx * ny * sor_zmax(d);  // the rows the SOR solves
+  const unsigned int n = (unsigned int)nx * ny * sor_zmax(d);  // the rows the SOR solves
   const size_t sj = (size_t)(nx + 4), sk = (size_t)(nx + 4) * (ny + 4);
   double acc = 0.0;
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-    int i = (int)(t % nx) + 1;
-    long long r = t / nx;
-    int j = (int)(r % ny) + 1, k = (int)(r / ny) + 1;
+  for (unsigned int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+    int i, j, k;
+    cell_ijk(d, t, i, j, k);
     size_t q = hidx(d, i, j, k);
     size_t qjm = (j == 1) ? hidx(d, i, ny, k) : q - sj;
     size_t qjp = (j == ny) ? hidx(d, i, 1, k) : q + sj;
@@ -145,13 +143,12 @@ __global__ void __launch_bounds__(kThreads) resid_l1_kernel(Dev d, const double*
 __global__ void __launch_bounds__(kThreads) energy_sums_kernel(Dev d, double* part, int nbmax) {
   __shared__ double sh[32];
   __shared__ bool last;
-  const int nx = d.nx, ny = d.ny, nz = d.nz;
-  const long long n = (long long)nx * ny * nz;
+  const int nx = d.nx, nz = d.nz;
+  const unsigned int n = (unsigned int)ncell(d);
   double s[7] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(t % nx) + 1;
-    const long long r = t / nx;
-    const int j = (int)(r % ny) + 1, k = (int)(r / ny) + 1;
+  for (unsigned int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+    int i, j, k;
+    cell_ijk(d, t, i, j, k);
     const int ub = PA(UB, j, k);
     const int itop = (ub < nx ? ub : nx) - 1;  // last active cell of the column
     if (i > itop || k < 2 || k > nz - 1) continue;
@@ -221,8 +218,20 @@ static int sweep_blocks(const Dev& d) {
   return nb > kMaxPartials ? kMaxPartials : nb;
 }
 
-int launch_exact_sweeps(ttfld_ctx* c, double* x, const double* b, int nsweeps, int itmin, int itmax,
-                               double eps) {
+// nsweeps sweeps of the reference loop (fewer if its rule fires) in one
+// launch; 1 where that is not possible.
+static int launch_exact_persistent(ttfld_ctx* c, double* x, const double* b, int nsweeps, int itmin, int itmax,
+                                   double eps) {
+  const Dev& d = c->d;
+  const double* const coef[7] = {d.SA, d.SB, d.SC, d.SD, d.SE, d.SF, d.SG};
+  const SorRows sys = sor_rows(coef, b, x, d.nx, d.ny, d.nz, sor_zmax(d), d.poles, d.sorparam);
+  return launch_sweeps64_persistent(sys, c->stream, c->sol, c->partials, c->flags64, nsweeps, itmin, itmax, eps);
+}
+
+// The same, by two launches per sweep where one launch is not possible.
+int launch_exact_sweeps(ttfld_ctx* c, double* x, const double* b, int nsweeps, int itmin, int itmax, double eps) {
+  const int rc = launch_exact_persistent(c, x, b, nsweeps, itmin, itmax, eps);
+  if (rc <= 0) return rc;
   const int nb = sweep_blocks(c->d);
   const double omega = c->d.sorparam;
   for (int s = 0; s < nsweeps; ++s) {
@@ -231,6 +240,17 @@ int launch_exact_sweeps(ttfld_ctx* c, double* x, const double* b, int nsweeps, i
   }
   count_launches(2 * nsweeps);
   TT_CHECK_LAUNCH();
+  return 0;
+}
+
+// Read the solver's state back; an error if a wait of the sweeps ran out.
+static int read_sol(ttfld_ctx* c) {
+  TT_CHECK(cudaMemcpyAsync(c->host_sol, c->sol, sizeof(SolverDev), cudaMemcpyDeviceToHost, c->stream));
+  TT_CHECK(cudaStreamSynchronize(c->stream));
+  if (c->host_sol->bar_timeout) {
+    fprintf(stderr, "ttfld: a wait of the persistent FP64 sweeps timed out\n");
+    return TTFLD_E_CUDA;
+  }
   return 0;
 }
 
@@ -243,9 +263,6 @@ static void fill_stats(ttfld_ctx* c, ttfld_solve_stats* st, int status) {
   st->status = status;
 }
 
-// Red-black SOR to the ppsor.f:161-177 rule.  The host checks the device
-// flag after chunks of sweeps; sweeps queued after the rule fired return at
-// once, so the iteration count is exactly the reference's.
 // DIFFUSION's sweeps on a context with poles: every theta row k = 1..NZ
 // (ppdif.f:45-46, 93-94; no zmax_sor_index), the theta ghosts read as they
 // are, and the pole shifts of the scalar after each colour (ppdif.f:80-89,
@@ -269,8 +286,12 @@ static int launch_exact_sweeps_all_rows(ttfld_ctx* c, double* x, const double* b
   return 0;
 }
 
-// all_rows: DIFFUSION's row range and pole shifts (above) instead of
-// SOLVE_WITH_SOR's.
+// Red-black SOR to the ppsor.f:161-177 rule: one persistent launch, which
+// applies the rule after every sweep; or, with one launch per colour, the
+// host checks the device flag after chunks of sweeps, and sweeps queued
+// after the rule fired return at once.  The iteration count is exactly the
+// reference's.  all_rows: DIFFUSION's row range and pole shifts (above)
+// instead of SOLVE_WITH_SOR's.
 static int solve_exact_rows(ttfld_ctx* c, double* x, const double* b, int itmin, int itmax, ttfld_solve_stats* st,
                             bool all_rows) {
   all_rows = all_rows && c->d.poles;
@@ -279,12 +300,13 @@ static int solve_exact_rows(ttfld_ctx* c, double* x, const double* b, int itmin,
   if (rc) return rc;
   int chunk = 4, launched = 0;
   for (;;) {
-    rc = all_rows ? launch_exact_sweeps_all_rows(c, x, b, chunk, itmin, itmax, c->d.epsmat)
-                  : launch_exact_sweeps(c, x, b, chunk, itmin, itmax, c->d.epsmat);
-    if (rc) return rc;
+    // the persistent kernel stops itself, at ITMAX at the latest
+    if (!all_rows && (rc = launch_exact_persistent(c, x, b, itmax, itmin, itmax, c->d.epsmat)) <= 0) chunk = itmax;
+    else
+      rc = all_rows ? launch_exact_sweeps_all_rows(c, x, b, chunk, itmin, itmax, c->d.epsmat)
+                    : launch_exact_sweeps(c, x, b, chunk, itmin, itmax, c->d.epsmat);
+    if (rc || (rc = read_sol(c))) return rc;
     launched += chunk;
-    TT_CHECK(cudaMemcpyAsync(c->host_sol, c->sol, sizeof(SolverDev), cudaMemcpyDeviceToHost, c->stream));
-    TT_CHECK(cudaStreamSynchronize(c->stream));
     if (c->host_sol->done) break;
     if (launched >= itmax + 2) return TTFLD_E_CUDA;  // the rule must have fired by ITMAX
     chunk = chunk < 128 ? chunk * 2 : 256;
@@ -379,10 +401,9 @@ int solve_delta_er(ttfld_ctx* c, ttfld_solve_stats* st) {
         else TT_CHECK(cudaMemsetAsync(c->guess_tmp, 0, nhalo(d) * 8, c->stream));
         TT_CHECK(cudaMemsetAsync(c->sol, 0, sizeof(SolverDev), c->stream));
         if ((rc = rhs_norm(c, d.RHS, nullptr))) return rc;
-        if ((rc = launch_exact_sweeps(c, c->guess_tmp, d.RHS, race_sweeps, race_sweeps + 1, race_sweeps + 1, -1.0)))
+        if ((rc = launch_exact_sweeps(c, c->guess_tmp, d.RHS, race_sweeps, race_sweeps + 1, race_sweeps + 1, -1.0)) ||
+            (rc = read_sol(c)))
           return rc;
-        TT_CHECK(cudaMemcpyAsync(c->host_sol, c->sol, sizeof(SolverDev), cudaMemcpyDeviceToHost, c->stream));
-        TT_CHECK(cudaStreamSynchronize(c->stream));
         r2[q] = c->host_sol->rnorm;
       }
       reject = !(r2[0] < r2[1]);
@@ -442,9 +463,7 @@ int ttfld_sor_sweeps(ttfld_ctx* c, int n, double* rnorm, double* rhsnorm) {
   if (rc) return rc;
   // itmax beyond n so the rule never stops the requested sweeps
   if ((rc = launch_exact_sweeps(c, c->d.DELTA_ER, c->d.RHS, n, n + 1, n + 2, -1.0))) return rc;
-  if ((rc = halo_shift(c, c->d.DELTA_ER)) || (rc = pole_shift(c, c->d.DELTA_ER))) return rc;
-  TT_CHECK(cudaMemcpyAsync(c->host_sol, c->sol, sizeof(SolverDev), cudaMemcpyDeviceToHost, c->stream));
-  TT_CHECK(cudaStreamSynchronize(c->stream));
+  if ((rc = halo_shift(c, c->d.DELTA_ER)) || (rc = pole_shift(c, c->d.DELTA_ER)) || (rc = read_sol(c))) return rc;
   if (rnorm) *rnorm = c->host_sol->rnorm;
   if (rhsnorm) *rhsnorm = c->host_sol->rhsnorm;
   return c->host_sol->iter == n ? 0 : TTFLD_E_CUDA;
@@ -542,17 +561,21 @@ static int diffusion(ttfld_ctx* c, ttfld_solve_stats* st) {
   launch_box(c->stream, box(1, d.nx, 1, d.ny, 1, d.nz), [=] __device__(int i, int j, int k) {
     size_t q = cidx(d, i, j, k);
     d.RHS_DIF[q] = HA(SCALAR, i, j, k);
-    double dx1 = dconst / G(dxb, i + 1), dx2 = dconst / G(dxb, i);
-    double dy1 = dconst / (G(dyb, j + 1) * G(geoxg, i) * G(geozg, k));
-    double dy2 = dconst / (G(dyb, j) * G(geoxg, i) * G(geozg, k));
-    double dz1 = dconst / (G(dzb, k + 1) * G(geoxh, i));
-    double dz2 = dconst / (G(dzb, k) * G(geoxh, i));
-    double d1 = d.delt * G(surxa, i + 1) * dx1 / (G(surxb, i) * G(dxa, i));
-    double d2 = d.delt * G(surxa, i) * dx2 / (G(surxb, i) * G(dxa, i));
-    double d3 = d.delt * dy1 / (G(geoxg, i) * G(surzb, k) * G(dya, j));
-    double d4 = d.delt * dy2 / (G(geoxg, i) * G(surzb, k) * G(dya, j));
-    double d5 = d.delt * dz1 * G(surza, k + 1) / (G(geoxg, i) * G(surzb, k) * G(dza, k));
-    double d6 = d.delt * dz2 * G(surza, k) / (G(geoxg, i) * G(surzb, k) * G(dza, k));
+    // quotients and most products on the integer pipes (ttfld_fp64.cuh), in
+    // the reference's operand order
+    const double dx1 = div_rn(dconst, G(dxb, i + 1)), dx2 = div_rn(dconst, G(dxb, i));
+    const double dy1 = div_rn(dconst, mul_rn(mul_rn(G(dyb, j + 1), G(geoxg, i)), G(geozg, k)));
+    const double dy2 = div_rn(dconst, mul_rn(mul_rn(G(dyb, j), G(geoxg, i)), G(geozg, k)));
+    const double dz1 = div_rn(dconst, G(dzb, k + 1) * G(geoxh, i));
+    const double dz2 = div_rn(dconst, G(dzb, k) * G(geoxh, i));
+    const double hx = G(surxb, i) * G(dxa, i), rz = G(geoxg, i) * G(surzb, k);
+    const double hy = rz * G(dya, j), hz = rz * G(dza, k);
+    const double d1 = div_rn(mul_rn(d.delt * G(surxa, i + 1), dx1), hx);
+    const double d2 = div_rn(mul_rn(d.delt * G(surxa, i), dx2), hx);
+    const double d3 = div_rn(d.delt * dy1, hy);
+    const double d4 = div_rn(d.delt * dy2, hy);
+    const double d5 = div_rn(mul_rn(d.delt * dz1, G(surza, k + 1)), hz);
+    const double d6 = div_rn(mul_rn(d.delt * dz2, G(surza, k)), hz);
     double d16 = d1 + d2 + d3 + d4 + d5 + d6;
     if (i == d.nx) {  // XMAX zero-gradient row, ppdif.f:212-220
       d.SA[q] = 1.0 + d2; d.SB[q] = -d2; d.SC[q] = 0.0; d.SD[q] = 0.0;

@@ -1,0 +1,304 @@
+// ttfld_sweep64.cuh -- FP64 red-black sweeps with the reference's stopping
+// rule after every sweep, any number of them in one cooperative launch.
+//
+// One launch per colour leaves the chip idle between the launches, and a
+// grid of a few hundred thousand cells is a few microseconds of work per
+// colour: the waves of blocks, their partial sums and the launch gaps cost
+// several times that.  Here one block per SM owns a contiguous run of (j,k)
+// rows for all sweeps.  Between the colours it waits only for the blocks that
+// own rows within one theta plane of its own (wait_flags); after the second
+// colour a grid barrier carries the blocks' partial norms, so that every
+// block adds them in the same fixed order and takes the same stop decision.
+// The cells' updates and their operands are those of one launch per colour,
+// so the iterate is the same bit for bit; only the order in which the norm
+// is summed differs.
+//
+// What does not change during a solve (the coefficients and b) each thread
+// copies for its next item into its own slots of shared memory (cp.async)
+// before it updates the present one, across the colours too, so that these
+// reads, eight of the 16 values of a cell, wait for nothing.  Where a block's
+// share of them fits in shared memory (RESIDENT: 227 KB a block, 540,000
+// cells in all) it is copied once for all sweeps.
+//
+// A system is a struct with
+//   rows, by_items          (j,k) rows, and the items of a colour in a row
+//   kWords, Word            its coefficients of an item, as kWords of Word
+//   fetch<COL>(row, h, to)  queues their copies to to[0], to[T], to[2 T], ...
+//                           (T threads)
+//   update<COL>(row, h, w, T, first)  updates item h of a row with them, returns its
+//                           share of the norm; first: no colour has run yet
+//   before<COL>(r0, r1), after<COL>(r0, r1, first)  a block's own work around
+//                           a colour (all its threads; boundary values of its rows)
+//   norm(sum)               the norm from the sum of the shares
+#pragma once
+#include "ttfld_internal.cuh"
+
+namespace ttfld {
+
+// Sum over the warp in a fixed order, the same in every lane.
+__device__ __forceinline__ double warp_sum_all(double v) {
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// An asynchronous copy of one 8- or 16-byte word to shared memory.
+template <class W>
+__device__ __forceinline__ void copy_async(W* to, const W* from) {
+  const unsigned int dst = (unsigned int)__cvta_generic_to_shared(to);
+  if (sizeof(W) == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(from) : "memory");
+  else asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(from) : "memory");
+}
+
+// The items of one colour of a block's rows.  Not RESIDENT: the thread's
+// next item (of this colour, or its first of the other) is fetched before
+// the present one is updated.
+template <int COL, bool RESIDENT, class Sys>
+__device__ __forceinline__ double sweep_colour(const Sys& s, unsigned int r0, unsigned int n, bool first,
+                                               typename Sys::Word* slots, int& stage) {
+  double acc = 0.0;
+  const unsigned int T = blockDim.x;
+  for (unsigned int u = threadIdx.x; u < n; u += T) {
+    unsigned int h;
+    const unsigned int r = r0 + div_rem(s.by_items, u, h);
+    if (RESIDENT) {
+      acc += s.template update<COL>(r, h, slots + (size_t)COL * Sys::kWords * n + u, n, first);
+      continue;
+    }
+    typename Sys::Word* mine = slots + (size_t)stage * Sys::kWords * T + threadIdx.x;
+    stage ^= 1;
+    typename Sys::Word* next = slots + (size_t)stage * Sys::kWords * T + threadIdx.x;
+    unsigned int hn;
+    if (u + T < n) {
+      const unsigned int rn = r0 + div_rem(s.by_items, u + T, hn);
+      s.template fetch<COL>(rn, hn, next, T);
+    } else {
+      const unsigned int rn = r0 + div_rem(s.by_items, threadIdx.x, hn);
+      s.template fetch<1 - COL>(rn, hn, next, T);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    acc += s.template update<COL>(r, h, mine, T, first);
+  }
+  return acc;
+}
+
+template <class Sys, bool RESIDENT>
+__global__ void __launch_bounds__(Sys::kThreads, 1)
+    sweeps64_persistent(Sys s, SolverDev* sol, double* partials, unsigned int* flags, int nsweeps, int itmin,
+                        int itmax, double eps) {
+  __shared__ double sh[32];
+  __shared__ int stop_sh;
+  const int nb = (int)gridDim.x, b = (int)blockIdx.x;
+  if (*(volatile int*)&sol->done) return;  // set before the launch, so the same for every block
+  const long long rows = s.rows;
+  const unsigned int r0 = (unsigned int)(rows * b / nb), r1 = (unsigned int)(rows * (b + 1) / nb);
+  const long long ny = s.ny;
+  const int lo = owner_block(r0 > ny ? r0 - ny : 0, rows, nb);
+  const int hi = owner_block(r1 - 1 + ny < rows ? r1 - 1 + ny : rows - 1, rows, nb);
+  const unsigned int n = (r1 - r0) * s.by_items.d;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  const double rhsnorm = sol->rhsnorm;
+  int it = sol->iter;
+  unsigned long long passed = 0;
+  extern __shared__ __align__(16) unsigned char slots_raw[];
+  typename Sys::Word* slots = reinterpret_cast<typename Sys::Word*>(slots_raw);
+  int stage = 0;
+  if (RESIDENT) {  // each thread copies what it will read itself
+    for (unsigned int u = threadIdx.x; u < n; u += blockDim.x) {
+      unsigned int h;
+      const unsigned int r = r0 + div_rem(s.by_items, u, h);
+      s.template fetch<0>(r, h, slots + u, n);
+      s.template fetch<1>(r, h, slots + (size_t)Sys::kWords * n + u, n);
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+  } else if (threadIdx.x < n) {
+    unsigned int h;
+    const unsigned int r = r0 + div_rem(s.by_items, threadIdx.x, h);
+    s.template fetch<0>(r, h, slots + threadIdx.x, blockDim.x);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  for (int sw = 1; sw <= nsweeps; ++sw) {
+    s.template before<0>(r0, r1);
+    double acc = sweep_colour<0, RESIDENT>(s, r0, n, sw == 1, slots, stage);
+    s.template after<0>(r0, r1, sw == 1);
+    publish_flag(flags + (size_t)b * kFlagStride, (unsigned int)sw);
+    if (!wait_flags(flags, lo, hi, (unsigned int)sw, sol)) break;
+    s.template before<1>(r0, r1);
+    acc += sweep_colour<1, RESIDENT>(s, r0, n, false, slots, stage);
+    s.template after<1>(r0, r1, false);
+    // the norm and the grid barrier in one: warp 0 publishes the block's
+    // partial with its arrival and adds all partials once every block has
+    // arrived.  Partials alternate between two arrays, so that a block
+    // already in the next sweep does not overwrite one still being read.
+    acc = warp_sum_all(acc);
+    if (lane == 0) sh[warp] = acc;
+    __syncthreads();
+    ++passed;
+    ++it;
+    if (warp == 0) {
+      double* part = partials + (passed & 1) * kMaxPartials;
+      const double own = warp_sum_all(lane < nw ? sh[lane] : 0.0);
+      int ok = 1;
+      if (lane == 0) {
+        part[b] = own;
+        asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(&sol->arrivals) : "memory");
+        const unsigned long long target = passed * (unsigned long long)nb;
+        long long polls = 0;
+        while (ld_acquire64(&sol->arrivals) < target)
+          if (give_up(++polls, sol)) {
+            atomicExch(&sol->bar_timeout, 1);
+            ok = 0;
+            break;
+          }
+      }
+      __syncwarp();  // the other lanes' loads come after lane 0's acquire
+      ok = __shfl_sync(0xffffffffu, ok, 0);
+      double tot = 0.0;
+      if (ok)
+        for (int q = lane; q < nb; q += 32) tot += __ldcg(part + q);
+      tot = s.norm(warp_sum_all(tot));
+      const double ratio = tot / rhsnorm;
+      const bool fin = isfinite(tot);
+      const bool met = !(ratio > eps) && it >= itmin, out = it == itmax;
+      if (lane == 0) {
+        stop_sh = !ok ? 2 : (!fin || out || met || sw == nsweeps) ? 1 : 0;
+        if (stop_sh == 1 && b == 0) {
+          sol->iter = it;
+          sol->rnorm = tot;
+          sol->ratio = ratio;
+          if (!fin && sol->nonfinite == 0) sol->nonfinite = 1;
+          else if (out) sol->maxit = 1;
+          if (!fin || out || met) sol->done = 1;
+        }
+      }
+    }
+    __syncthreads();
+    if (stop_sh) break;
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+}
+
+// Queue nsweeps sweeps of a system (fewer if the rule fires).  1 where the
+// launch is not possible (no cooperative launch, or fewer SMs to be had than
+// blocks): the caller runs one launch per colour instead.
+template <class Sys>
+int launch_sweeps64_persistent(const Sys& s, cudaStream_t st, SolverDev* sol, double* partials, unsigned int* flags,
+                               int nsweeps, int itmin, int itmax, double eps) {
+  int dev = 0, sms = 0, coop = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (!coop || sms <= 0 || nsweeps <= 0) return 1;
+  if (sms > kMaxLocalBlocks) sms = kMaxLocalBlocks;
+  // one block per SM, but no block of less than two warps' items
+  const long long items = (long long)s.rows * s.by_items.d;
+  long long nb = (items + 63) / 64;
+  if (nb > sms) nb = sms;
+  if (nb > s.rows) nb = s.rows;
+  // threads for the fewest rounds over a block's items, evenly filled
+  const long long most = (s.rows + nb - 1) / nb * s.by_items.d;
+  const long long rounds = (most + Sys::kThreads - 1) / Sys::kThreads;
+  const int threads = (int)(((most + rounds - 1) / rounds + 31) / 32 * 32);
+  int room = 0;
+  cudaDeviceGetAttribute(&room, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  const size_t item = 2 * (size_t)Sys::kWords * sizeof(typename Sys::Word);  // both colours, or both stages
+  const bool resident = item * (size_t)most + 1024 <= (size_t)room;
+  const size_t smem = item * (size_t)(resident ? most : threads);
+  const void* kernel = resident ? (const void*)sweeps64_persistent<Sys, true> : (const void*)sweeps64_persistent<Sys, false>;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+    cudaGetLastError();
+    return 1;
+  }
+  TT_CHECK(cudaMemsetAsync(flags, 0, (size_t)nb * kFlagStride * sizeof(unsigned int), st));
+  TT_CHECK(cudaMemsetAsync(&sol->arrivals, 0, sizeof(unsigned long long), st));
+  Sys sys = s;
+  void* args[] = {&sys, &sol, &partials, &flags, &nsweeps, &itmin, &itmax, &eps};
+  const cudaError_t e =
+      cudaLaunchCooperativeKernel(kernel, dim3((unsigned int)nb), dim3(threads), args, smem, st);
+  if (e == cudaErrorCooperativeLaunchTooLarge) {
+    cudaGetLastError();
+    return 1;
+  }
+  TT_CHECK(e);
+  count_launches(1);
+  return 0;
+}
+
+// SOLVE_WITH_SOR's rows in the reference's layout and operand order
+// (ppsor.f:59-136): the coefficients and b in cell order, x a halo array
+// whose phi direction is read by wrapping j.  With poles the theta
+// neighbours across the edges are the cell itself (x_km, x_kp).  The
+// products and the quotient run on the integer pipes, the sums on the FP64
+// pipe (ttfld_fp64.cuh).
+struct SorRows {
+  typedef double Word;
+  static constexpr int kWords = 8, kThreads = 1024;
+  const double *a, *xm, *xp, *jm, *jp, *km, *kp, *b;
+  double* x;
+  double omega;
+  long long rows;  // ny times the theta rows that are swept
+  int nx, ny, nz, poles;
+  FastDiv by_items, by_ny;
+  template <int COL>
+  __device__ void before(unsigned int, unsigned int) const {}
+  template <int COL>
+  __device__ void after(unsigned int, unsigned int, bool) const {}
+  __device__ double norm(double sum) const { return sum; }
+  // radial index (from 0) of item h of a row: i + j + k, all from 1, has COL's parity
+  template <int COL>
+  __device__ __forceinline__ unsigned int cell(unsigned int row, unsigned int h, unsigned int& j0,
+                                               unsigned int& k0) const {
+    k0 = div_rem(by_ny, row, j0);
+    return 2 * h + ((j0 + k0 + COL + 1) & 1);
+  }
+  template <int COL>
+  __device__ __forceinline__ void fetch(unsigned int row, unsigned int h, double* to, unsigned int T) const {
+    unsigned int j0, k0;
+    const unsigned int i0 = cell<COL>(row, h, j0, k0);
+    if ((int)i0 >= nx) return;
+    const size_t c = i0 + (size_t)nx * row;
+    copy_async(to, a + c);
+    copy_async(to + T, xm + c);
+    copy_async(to + 2 * T, xp + c);
+    copy_async(to + 3 * T, jm + c);
+    copy_async(to + 4 * T, jp + c);
+    copy_async(to + 5 * T, km + c);
+    copy_async(to + 6 * T, kp + c);
+    copy_async(to + 7 * T, b + c);
+  }
+  template <int COL>
+  __device__ __forceinline__ double update(unsigned int row, unsigned int h, const double* w, unsigned int T,
+                                           bool) const {
+    unsigned int j0, k0;
+    const unsigned int i0 = cell<COL>(row, h, j0, k0);
+    if ((int)i0 >= nx) return 0.0;
+    const size_t sj = (size_t)(nx + 4), sk = sj * (size_t)(ny + 4);
+    const size_t q = (i0 + 2) + sj * (j0 + 2) + sk * (k0 + 2);
+    const size_t qjm = j0 == 0 ? q + sj * (size_t)(ny - 1) : q - sj;
+    const size_t qjp = (int)j0 == ny - 1 ? q - sj * (size_t)(ny - 1) : q + sj;
+    const double xc = x[q], ac = w[0];
+    const double xkm = poles && k0 == 0 ? xc : x[q - sk];
+    const double xkp = poles && (int)k0 == nz - 2 ? xc : x[q + sk];
+    const double resid = mul_rn(ac, xc) + mul_rn(w[T], x[q - 1]) + mul_rn(w[2 * T], x[q + 1]) +
+                         mul_rn(w[3 * T], x[qjm]) + mul_rn(w[4 * T], x[qjp]) + mul_rn(w[5 * T], xkm) +
+                         mul_rn(w[6 * T], xkp) - w[7 * T];
+    x[q] = xc - div_rn(omega * resid, ac);
+    return fabs(resid);
+  }
+};
+
+inline SorRows sor_rows(const double* const coef[7], const double* b, double* x, int nx, int ny, int nz, int zmax,
+                        int poles, double omega) {
+  SorRows s;
+  s.a = coef[0]; s.xm = coef[1]; s.xp = coef[2]; s.jm = coef[3]; s.jp = coef[4]; s.km = coef[5]; s.kp = coef[6];
+  s.b = b;
+  s.x = x;
+  s.omega = omega;
+  s.rows = (long long)ny * zmax;
+  s.nx = nx; s.ny = ny; s.nz = nz; s.poles = poles;
+  s.by_items = fast_div((nx + 1) / 2);
+  s.by_ny = fast_div(ny);
+  return s;
+}
+
+}  // namespace ttfld
