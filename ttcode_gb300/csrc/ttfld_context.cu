@@ -240,6 +240,7 @@ int ttfld_create(ttfld_ctx** out, const ttfld_dims* dims, const ttfld_metrics* m
   c->partials = (double*)take(2 * kMaxPartials * 8);
   c->flags64 = (unsigned int*)take(kFlagBytes);
   c->staging = (double*)take(staging * 8);
+  c->staging_bytes = staging * 8;
   d.sol = c->sol;
   d.stp = c->stp;
 

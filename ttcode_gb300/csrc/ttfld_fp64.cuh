@@ -160,9 +160,8 @@ TT_FP_HD double mul_rn(double a, double b) {
   const uint32_t e = (ah & 0x7ff00000u) + (bh & 0x7ff00000u) + (c << 20) - (1024u << 20) + ((ah ^ bh) & 0x80000000u);
   uint32_t ol, oh;
 #if defined(__CUDA_ARCH__)
-  uint32_t drop;
-  asm("add.cc.u32 %0, %3, %4;\n\taddc.cc.u32 %1, %5, 0;\n\taddc.u32 %2, %6, %7;"
-      : "=&r"(drop), "=&r"(ol), "=r"(oh)
+  asm("{\n\t.reg .u32 drop;\n\tadd.cc.u32 drop, %2, %3;\n\taddc.cc.u32 %0, %4, 0;\n\taddc.u32 %1, %5, %6;\n\t}"
+      : "=&r"(ol), "=r"(oh)
       : "r"(rest), "r"(half), "r"(ml), "r"(mu), "r"(e));
 #else
   const uint64_t o = (((uint64_t)(mu + e) << 32) | ml) + (((uint64_t)rest + half) >> 32);

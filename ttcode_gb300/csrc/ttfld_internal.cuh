@@ -263,26 +263,30 @@ __device__ __forceinline__ void publish_flag(unsigned int* flag, unsigned int v)
 }
 
 // Wait until blocks lo..hi other than this one have finished at least
-// `target` half-sweeps; warp 0 polls, one flag per lane.  Bounded like the
+// `target` half-sweeps: one warp polls, one flag per lane.  Bounded like the
 // grid barriers: false after kBarrierSpins polls or once another block has
 // given up.
+__device__ __forceinline__ bool poll_flags(const unsigned int* flags, int lo, int hi, unsigned int target,
+                                           SolverDev* sol) {
+  const int lane = threadIdx.x & 31;
+  long long polls = 0;
+  for (;;) {
+    bool ready = true;
+    for (int q = lo + lane; q <= hi; q += 32)
+      if (q != (int)blockIdx.x && (int)(ld_acquire(flags + (size_t)q * kFlagStride) - target) < 0) ready = false;
+    if (__all_sync(0xffffffffu, ready)) return true;
+    if (__any_sync(0xffffffffu, give_up(++polls, sol))) break;
+  }
+  if (lane == 0) atomicExch(&sol->bar_timeout, 1);
+  return false;
+}
+// The same for the block.
 __device__ __forceinline__ bool wait_flags(const unsigned int* flags, int lo, int hi, unsigned int target,
                                            SolverDev* sol) {
   __shared__ int ok_sh;
   if (threadIdx.x < 32) {
-    int ok = 1;
-    long long polls = 0;
-    for (;;) {
-      bool ready = true;
-      for (int q = lo + (int)threadIdx.x; q <= hi; q += 32)
-        if (q != (int)blockIdx.x && (int)(ld_acquire(flags + (size_t)q * kFlagStride) - target) < 0) ready = false;
-      if (__all_sync(0xffffffffu, ready)) break;
-      if (__any_sync(0xffffffffu, give_up(++polls, sol))) { ok = 0; break; }
-    }
-    if (threadIdx.x == 0) {
-      if (!ok) atomicExch(&sol->bar_timeout, 1);
-      ok_sh = ok;
-    }
+    const bool ok = poll_flags(flags, lo, hi, target, sol);
+    if (threadIdx.x == 0) ok_sh = ok;
   }
   __syncthreads();
   return ok_sh != 0;
@@ -326,7 +330,8 @@ struct ttfld_ctx {
   cudaEvent_t ev0, ev1, evg;
   void* slab;                // one allocation holding every array
   size_t slab_bytes;
-  double* staging;           // device staging for box-shaped transfers
+  double* staging;           // device staging for box-shaped transfers, values kept by the FP64 sweeps
+  size_t staging_bytes;
   double* partials;          // 2 * kMaxPartials sweep partials
   unsigned int* flags64;     // per-block half-sweep counters of the persistent FP64 sweeps
   ttfld::SolverDev* sol;

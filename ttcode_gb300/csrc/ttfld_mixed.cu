@@ -1301,6 +1301,7 @@ __global__ void __launch_bounds__(kThreads) sweep64_kernel(Dev d, Cmp g, Fast64 
 // pipe, the product of its norm goes to the integer pipes.
 struct FastRows {
   typedef double2 Word;
+  typedef double2 Kept;
   static constexpr int kWords = 8, kThreads = 768;  // 196 KB for two stages
   Fast64 m;
   double omega;
@@ -1321,8 +1322,8 @@ struct FastRows {
     copy_async(to + 7 * T, reinterpret_cast<const double2*>(m.diag[COL] + c));
   }
   template <int COL>
-  __device__ __forceinline__ double update(unsigned int row, unsigned int h, const double2* w, unsigned int T,
-                                           bool) const {
+  __device__ __forceinline__ double update(unsigned int row, unsigned int h, const double2* w, unsigned int T, bool,
+                                           double2* kept) const {
     unsigned int j0;
     const unsigned int k0 = div_rem(by_ny, row, j0);
     const double* xo = m.x[1 - COL];
@@ -1353,7 +1354,11 @@ struct FastRows {
     TT_CELL(y, 1, xm1, xp1)
 #undef TT_CELL
     st2(xs + eb, out);
+    if (kept) *kept = xv;
     return share;
+  }
+  __device__ __forceinline__ void restore(unsigned int row, unsigned int h, double2 kept) const {
+    st2(m.x[0] + (size_t)ny * nxp + (size_t)row * nxp + 2 * h, kept);
   }
 };
 
@@ -1369,7 +1374,8 @@ static int launch_fast_persistent(ttfld_ctx* c, int nsweeps, int itmin, int itma
   s.nx = g.nx; s.ny = g.ny; s.nz = g.nz; s.nxp = g.nxp; s.poles = g.poles;
   s.by_items = g.by_pairs;
   s.by_ny = c->d.by_ny;
-  return launch_sweeps64_persistent(s, c->stream, c->sol, c->partials, c->flags64, nsweeps, itmin, itmax, eps);
+  return launch_sweeps64_persistent(s, c->stream, c->sol, c->partials, c->flags64, c->staging, c->staging_bytes,
+                                    nsweeps, itmin, itmax, eps);
 }
 
 int launch_sweeps64(ttfld_ctx* c, int nsweeps, int itmin, int itmax, double eps) {

@@ -226,6 +226,7 @@ int radiativebound(ttfld_ctx* c, double d_t, double tinit_bottom) {
 // themselves are filled after the last sweep (radbound_ghost_bottom, radbound_ghost_theta).
 struct RadRows {
   typedef double Word;
+  typedef double Kept;
   static constexpr int kWords = 8, kThreads = 1024;
   Dev d;
   RadWork w;
@@ -290,7 +291,7 @@ struct RadRows {
   }
   template <int COL>
   __device__ __forceinline__ double update(unsigned int row, unsigned int h, const double* c, unsigned int T,
-                                           bool first) const {
+                                           bool first, double* kept) const {
     unsigned int j0, k0;
     const unsigned int i0 = cell<COL>(row, h, j0, k0);
     const int nx = d.nx, i = (int)i0 + 1;
@@ -310,7 +311,13 @@ struct RadRows {
     // i = 1 and i > upperbnd (at upperbnd only a moving top reads it) keep
     // their boundary values
     if (i != 1 && (i < ub || (moving_top && i == ub) || ub > nx)) er[q] = e - div_rn(om * x, b);
+    if (kept) *kept = e;
     return mul_rn(x, x);
+  }
+  __device__ __forceinline__ void restore(unsigned int row, unsigned int h, double kept) const {
+    unsigned int j0, k0;
+    const unsigned int i0 = cell<0>(row, h, j0, k0);
+    if ((int)i0 < d.nx) HA(ER, (int)i0 + 1, (int)j0 + 1, (int)k0 + 1) = kept;
   }
 };
 
@@ -348,8 +355,9 @@ int solvmat_persistent(ttfld_ctx* c, const RadWork& w, double d_t, double tinit_
   s.ny = d.ny;
   s.moving_top = d.ibdrad == 9 && d.iii > 1;
   s.by_items = d.by_nxh;
-  const int rc =
-      launch_sweeps64_persistent(s, c->stream, c->sol, c->partials, c->flags64, d.itmax, 5, d.itmax, d.epsmat);
+  // a moving top is not kept: its decisions are waited for
+  const int rc = launch_sweeps64_persistent(s, c->stream, c->sol, c->partials, c->flags64, c->staging,
+                                            s.moving_top ? 0 : c->staging_bytes, d.itmax, 5, d.itmax, d.epsmat);
   if (rc) return rc;
   radbound_ghost_bottom<<<grid_for((long long)(d.ny + 4) * (d.nz + 4)), kThreads, 0, c->stream>>>(d, d_t, tinit_bottom);
   radbound_ghost_theta<<<grid_for((long long)(d.nx + 4) * (d.ny + 4)), kThreads, 0, c->stream>>>(d);

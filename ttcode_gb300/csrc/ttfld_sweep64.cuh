@@ -5,13 +5,16 @@
 // grid of a few hundred thousand cells is a few microseconds of work per
 // colour: the waves of blocks, their partial sums and the launch gaps cost
 // several times that.  Here one block per SM owns a contiguous run of (j,k)
-// rows for all sweeps.  Between the colours it waits only for the blocks that
-// own rows within one theta plane of its own (wait_flags); after the second
-// colour a grid barrier carries the blocks' partial norms, so that every
-// block adds them in the same fixed order and takes the same stop decision.
-// The cells' updates and their operands are those of one launch per colour,
-// so the iterate is the same bit for bit; only the order in which the norm
-// is summed differs.
+// rows for all sweeps, and after each colour waits only for the blocks that
+// own rows within one theta plane of its own (wait_flags).  Every block adds
+// all blocks' shares of a sweep's norm in the same fixed order and takes the
+// same stop decision -- one colour later: it begins the next sweep, keeping
+// the values that its first colour replaces, and reads the shares, by then
+// there, before the second; if the rule says stop it puts those values back.
+// (Where the values cannot be kept, the decision is waited for.)  The cells'
+// updates and their operands are those of one launch per colour, so the
+// iterate is the same bit for bit; only the order in which the norm is
+// summed differs.
 //
 // What does not change during a solve (the coefficients and b) each thread
 // copies for its next item into its own slots of shared memory (cp.async)
@@ -25,8 +28,10 @@
 //   kWords, Word            its coefficients of an item, as kWords of Word
 //   fetch<COL>(row, h, to)  queues their copies to to[0], to[T], to[2 T], ...
 //                           (T threads)
-//   update<COL>(row, h, w, T, first)  updates item h of a row with them, returns its
-//                           share of the norm; first: no colour has run yet
+//   update<COL>(row, h, w, T, first, kept)  updates item h of a row with them,
+//                           returns its share of the norm; first: no colour
+//                           has run yet; kept: where the old value (Kept) goes
+//   restore(row, h, kept)   puts a value of the first colour back
 //   before<COL>(r0, r1), after<COL>(r0, r1, first)  a block's own work around
 //                           a colour (all its threads; boundary values of its rows)
 //   norm(sum)               the norm from the sum of the shares
@@ -41,6 +46,89 @@ __device__ __forceinline__ double warp_sum_all(double v) {
   return v;
 }
 
+// A block's share of a sweep's norm, with the sweep it belongs to: written
+// and read as one 128-bit word, so that no fence orders the two.  Sweeps
+// alternate between two of them a block: when a block writes that of sweep
+// k + 2 it has read every block's of sweep k + 1, which each wrote after
+// reading those of sweep k.
+struct __align__(16) Partial {
+  double part;
+  unsigned long long sweep;
+};
+__device__ __forceinline__ void put_partial(Partial* gather, int b, int sweep, double part) {
+  Partial* p = gather + 2 * (size_t)b + (sweep & 1);
+  asm volatile(
+      "{\n .reg .b128 v;\n mov.b128 v, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], v;\n}" ::"l"(p),
+      "l"(__double_as_longlong(part)), "l"((long long)sweep)
+      : "memory");
+}
+__device__ __forceinline__ bool get_partial(const Partial* gather, int b, int sweep, double& part) {
+  const Partial* p = gather + 2 * (size_t)b + (sweep & 1);
+  long long v, n;
+  asm volatile("{\n .reg .b128 v;\n ld.relaxed.gpu.global.b128 v, [%2];\n mov.b128 {%0, %1}, v;\n}"
+               : "=l"(v), "=l"(n)
+               : "l"(p)
+               : "memory");
+  part = __longlong_as_double(v);
+  return n == sweep;
+}
+
+// The norm of sweep sw from every block's share, added in the same order by
+// one warp of every block, and the reference's rule on it: 0 go on, 1 stop,
+// 2 a block has given up (every lane gets it).  Bounded like the other waits.
+// Block 0 records the sweep.
+constexpr int kGather = 5;  // partials a lane reads at once: 160 blocks
+template <class Sys>
+__device__ __forceinline__ int gather_norm(const Sys& s, const Partial* gather, int nb, int sw, int it0, int itmin,
+                                           int itmax, double eps, double rhsnorm, SolverDev* sol) {
+  const int lane = threadIdx.x & 31;
+  double tot = 0.0;
+  for (int q0 = lane; q0 - lane < nb; q0 += 32 * kGather) {
+    double v[kGather];
+    long long polls = 0;
+    for (;;) {
+      bool ready = true;
+#pragma unroll
+      for (int m = 0; m < kGather; ++m) {
+        v[m] = 0.0;
+        if (q0 + 32 * m < nb && !get_partial(gather, q0 + 32 * m, sw, v[m])) ready = false;
+      }
+      if (__all_sync(0xffffffffu, ready)) break;
+      if (__any_sync(0xffffffffu, give_up(++polls, sol))) {
+        if (lane == 0) atomicExch(&sol->bar_timeout, 1);
+        return 2;
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < kGather; ++m) tot += v[m];
+  }
+  tot = s.norm(warp_sum_all(tot));
+  const double ratio = tot / rhsnorm;
+  const int it = it0 + sw;
+  const bool fin = isfinite(tot), out = it == itmax, met = !(ratio > eps) && it >= itmin;
+  const int stop = !fin || out || met ? 1 : 0;
+  if (lane == 0 && blockIdx.x == 0) {
+    sol->iter = it;
+    sol->rnorm = tot;
+    sol->ratio = ratio;
+    if (!fin && sol->nonfinite == 0) sol->nonfinite = 1;
+    else if (out) sol->maxit = 1;
+    if (stop) sol->done = 1;
+  }
+  return stop;
+}
+
+// Put back the first colour's values from before the present sweep.
+template <class Sys>
+__device__ __forceinline__ void undo_colour(const Sys& s, unsigned int r0, unsigned int n,
+                                            const typename Sys::Kept* mine) {
+  for (unsigned int u = threadIdx.x; u < n; u += blockDim.x) {
+    unsigned int h;
+    const unsigned int r = r0 + div_rem(s.by_items, u, h);
+    s.restore(r, h, mine[u]);
+  }
+}
+
 // An asynchronous copy of one 8- or 16-byte word to shared memory.
 template <class W>
 __device__ __forceinline__ void copy_async(W* to, const W* from) {
@@ -51,20 +139,20 @@ __device__ __forceinline__ void copy_async(W* to, const W* from) {
 
 // The items of one colour of a block's rows.  Not RESIDENT: the thread's
 // next item (of this colour, or its first of the other) is fetched before
-// the present one is updated.
+// the present one is updated.  mine: where to keep the values replaced.
 template <int COL, bool RESIDENT, class Sys>
 __device__ __forceinline__ double sweep_colour(const Sys& s, unsigned int r0, unsigned int n, bool first,
-                                               typename Sys::Word* slots, int& stage) {
+                                               typename Sys::Word* slots, int& stage, typename Sys::Kept* mine) {
   double acc = 0.0;
   const unsigned int T = blockDim.x;
   for (unsigned int u = threadIdx.x; u < n; u += T) {
     unsigned int h;
     const unsigned int r = r0 + div_rem(s.by_items, u, h);
     if (RESIDENT) {
-      acc += s.template update<COL>(r, h, slots + (size_t)COL * Sys::kWords * n + u, n, first);
+      acc += s.template update<COL>(r, h, slots + (size_t)COL * Sys::kWords * n + u, n, first, mine ? mine + u : nullptr);
       continue;
     }
-    typename Sys::Word* mine = slots + (size_t)stage * Sys::kWords * T + threadIdx.x;
+    const typename Sys::Word* now = slots + (size_t)stage * Sys::kWords * T + threadIdx.x;
     stage ^= 1;
     typename Sys::Word* next = slots + (size_t)stage * Sys::kWords * T + threadIdx.x;
     unsigned int hn;
@@ -77,17 +165,21 @@ __device__ __forceinline__ double sweep_colour(const Sys& s, unsigned int r0, un
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
     asm volatile("cp.async.wait_group 1;" ::: "memory");
-    acc += s.template update<COL>(r, h, mine, T, first);
+    acc += s.template update<COL>(r, h, now, T, first, mine ? mine + u : nullptr);
   }
   return acc;
 }
 
 template <class Sys, bool RESIDENT>
 __global__ void __launch_bounds__(Sys::kThreads, 1)
-    sweeps64_persistent(Sys s, SolverDev* sol, double* partials, unsigned int* flags, int nsweeps, int itmin,
-                        int itmax, double eps) {
+    sweeps64_persistent(Sys s, SolverDev* sol, Partial* gather, unsigned int* flags, typename Sys::Kept* keep,
+                        int nsweeps, int itmin, int itmax, double eps) {
   __shared__ double sh[32];
-  __shared__ int stop_sh;
+  __shared__ int stop_sh, ok_sh;
+  if (threadIdx.x == 0) {  // read after block barriers only
+    stop_sh = 0;
+    ok_sh = 1;
+  }
   const int nb = (int)gridDim.x, b = (int)blockIdx.x;
   if (*(volatile int*)&sol->done) return;  // set before the launch, so the same for every block
   const long long rows = s.rows;
@@ -98,8 +190,7 @@ __global__ void __launch_bounds__(Sys::kThreads, 1)
   const unsigned int n = (r1 - r0) * s.by_items.d;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   const double rhsnorm = sol->rhsnorm;
-  int it = sol->iter;
-  unsigned long long passed = 0;
+  const int it0 = sol->iter;
   extern __shared__ __align__(16) unsigned char slots_raw[];
   typename Sys::Word* slots = reinterpret_cast<typename Sys::Word*>(slots_raw);
   int stage = 0;
@@ -117,63 +208,47 @@ __global__ void __launch_bounds__(Sys::kThreads, 1)
     s.template fetch<0>(r, h, slots + threadIdx.x, blockDim.x);
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
-  for (int sw = 1; sw <= nsweeps; ++sw) {
+  typename Sys::Kept* mine = keep ? keep + (size_t)r0 * s.by_items.d : nullptr;
+  unsigned int* own = flags + (size_t)b * kFlagStride;
+  unsigned int half = 0;  // half-sweeps this block has finished
+  int stop = 0;
+  for (int sw = 1; sw <= nsweeps && !stop; ++sw) {
+    if (sw > 1 && !wait_flags(flags, lo, hi, half, sol)) break;
     s.template before<0>(r0, r1);
-    double acc = sweep_colour<0, RESIDENT>(s, r0, n, sw == 1, slots, stage);
+    double acc = sweep_colour<0, RESIDENT>(s, r0, n, sw == 1, slots, stage, sw > 1 ? mine : nullptr);
     s.template after<0>(r0, r1, sw == 1);
-    publish_flag(flags + (size_t)b * kFlagStride, (unsigned int)sw);
-    if (!wait_flags(flags, lo, hi, (unsigned int)sw, sol)) break;
-    s.template before<1>(r0, r1);
-    acc += sweep_colour<1, RESIDENT>(s, r0, n, false, slots, stage);
-    s.template after<1>(r0, r1, false);
-    // the norm and the grid barrier in one: warp 0 publishes the block's
-    // partial with its arrival and adds all partials once every block has
-    // arrived.  Partials alternate between two arrays, so that a block
-    // already in the next sweep does not overwrite one still being read.
-    acc = warp_sum_all(acc);
-    if (lane == 0) sh[warp] = acc;
-    __syncthreads();
-    ++passed;
-    ++it;
-    if (warp == 0) {
-      double* part = partials + (passed & 1) * kMaxPartials;
-      const double own = warp_sum_all(lane < nw ? sh[lane] : 0.0);
-      int ok = 1;
-      if (lane == 0) {
-        part[b] = own;
-        asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(&sol->arrivals) : "memory");
-        const unsigned long long target = passed * (unsigned long long)nb;
-        long long polls = 0;
-        while (ld_acquire64(&sol->arrivals) < target)
-          if (give_up(++polls, sol)) {
-            atomicExch(&sol->bar_timeout, 1);
-            ok = 0;
-            break;
-          }
-      }
-      __syncwarp();  // the other lanes' loads come after lane 0's acquire
-      ok = __shfl_sync(0xffffffffu, ok, 0);
-      double tot = 0.0;
-      if (ok)
-        for (int q = lane; q < nb; q += 32) tot += __ldcg(part + q);
-      tot = s.norm(warp_sum_all(tot));
-      const double ratio = tot / rhsnorm;
-      const bool fin = isfinite(tot);
-      const bool met = !(ratio > eps) && it >= itmin, out = it == itmax;
-      if (lane == 0) {
-        stop_sh = !ok ? 2 : (!fin || out || met || sw == nsweeps) ? 1 : 0;
-        if (stop_sh == 1 && b == 0) {
-          sol->iter = it;
-          sol->rnorm = tot;
-          sol->ratio = ratio;
-          if (!fin && sol->nonfinite == 0) sol->nonfinite = 1;
-          else if (out) sol->maxit = 1;
-          if (!fin || out || met) sol->done = 1;
-        }
-      }
+    publish_flag(own, ++half);
+    // the first warp waits for the neighbours, the last takes the last
+    // sweep's rule, and with it whether this sweep begins at all
+    if (warp == 0 && !poll_flags(flags, lo, hi, half, sol) && lane == 0) ok_sh = 0;
+    if (warp == nw - 1 && mine && sw > 1) {
+      const int r = gather_norm(s, gather, nb, sw - 1, it0, itmin, itmax, eps, rhsnorm, sol);
+      if (lane == 0) stop_sh = r;
     }
     __syncthreads();
-    if (stop_sh) break;
+    stop = stop_sh;
+    if (stop || !ok_sh) {
+      if (stop == 1) undo_colour(s, r0, n, mine);
+      break;
+    }
+    s.template before<1>(r0, r1);
+    acc += sweep_colour<1, RESIDENT>(s, r0, n, false, slots, stage, nullptr);
+    s.template after<1>(r0, r1, false);
+    acc = warp_sum_all(acc);
+    if (lane == 0) sh[warp] = acc;
+    publish_flag(own, ++half);  // its block barrier also orders sh
+    if (warp == 0) {
+      const double part = warp_sum_all(lane < nw ? sh[lane] : 0.0);
+      if (lane == 0) put_partial(gather, b, sw, part);
+    }
+    if (!mine || sw == nsweeps) {
+      if (warp == nw - 1) {
+        const int r = gather_norm(s, gather, nb, sw, it0, itmin, itmax, eps, rhsnorm, sol);
+        if (lane == 0) stop_sh = r;
+      }
+      __syncthreads();
+      stop = stop_sh;
+    }
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
@@ -183,7 +258,7 @@ __global__ void __launch_bounds__(Sys::kThreads, 1)
 // blocks): the caller runs one launch per colour instead.
 template <class Sys>
 int launch_sweeps64_persistent(const Sys& s, cudaStream_t st, SolverDev* sol, double* partials, unsigned int* flags,
-                               int nsweeps, int itmin, int itmax, double eps) {
+                               void* kept, size_t kept_bytes, int nsweeps, int itmin, int itmax, double eps) {
   int dev = 0, sms = 0, coop = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
@@ -210,9 +285,12 @@ int launch_sweeps64_persistent(const Sys& s, cudaStream_t st, SolverDev* sol, do
     return 1;
   }
   TT_CHECK(cudaMemsetAsync(flags, 0, (size_t)nb * kFlagStride * sizeof(unsigned int), st));
-  TT_CHECK(cudaMemsetAsync(&sol->arrivals, 0, sizeof(unsigned long long), st));
+  Partial* gather = (Partial*)partials;  // two a block
+  TT_CHECK(cudaMemsetAsync(gather, 0, (size_t)nb * 2 * sizeof(Partial), st));
   Sys sys = s;
-  void* args[] = {&sys, &sol, &partials, &flags, &nsweeps, &itmin, &itmax, &eps};
+  typename Sys::Kept* keep =
+      (size_t)items * sizeof(typename Sys::Kept) <= kept_bytes ? (typename Sys::Kept*)kept : nullptr;
+  void* args[] = {&sys, &sol, &gather, &flags, &keep, &nsweeps, &itmin, &itmax, &eps};
   const cudaError_t e =
       cudaLaunchCooperativeKernel(kernel, dim3((unsigned int)nb), dim3(threads), args, smem, st);
   if (e == cudaErrorCooperativeLaunchTooLarge) {
@@ -232,6 +310,7 @@ int launch_sweeps64_persistent(const Sys& s, cudaStream_t st, SolverDev* sol, do
 // pipe (ttfld_fp64.cuh).
 struct SorRows {
   typedef double Word;
+  typedef double Kept;
   static constexpr int kWords = 8, kThreads = 1024;
   const double *a, *xm, *xp, *jm, *jp, *km, *kp, *b;
   double* x;
@@ -267,8 +346,8 @@ struct SorRows {
     copy_async(to + 7 * T, b + c);
   }
   template <int COL>
-  __device__ __forceinline__ double update(unsigned int row, unsigned int h, const double* w, unsigned int T,
-                                           bool) const {
+  __device__ __forceinline__ double update(unsigned int row, unsigned int h, const double* w, unsigned int T, bool,
+                                           double* kept) const {
     unsigned int j0, k0;
     const unsigned int i0 = cell<COL>(row, h, j0, k0);
     if ((int)i0 >= nx) return 0.0;
@@ -283,7 +362,13 @@ struct SorRows {
                          mul_rn(w[3 * T], x[qjm]) + mul_rn(w[4 * T], x[qjp]) + mul_rn(w[5 * T], xkm) +
                          mul_rn(w[6 * T], xkp) - w[7 * T];
     x[q] = xc - div_rn(omega * resid, ac);
+    if (kept) *kept = xc;
     return fabs(resid);
+  }
+  __device__ __forceinline__ void restore(unsigned int row, unsigned int h, double kept) const {
+    unsigned int j0, k0;
+    const unsigned int i0 = cell<0>(row, h, j0, k0);
+    if ((int)i0 < nx) x[(i0 + 2) + (size_t)(nx + 4) * ((j0 + 2) + (size_t)(ny + 4) * (k0 + 2))] = kept;
   }
 };
 
