@@ -10,9 +10,11 @@ namespace ttfld {
 // ---- PLANETSHIFT ppshift.f:1009-1214, one rank --------------------------
 // Only the "from lower" (:1096-1107) and "from upper" (:1164-1173) copies
 // act with one rank; z and corner partners are MPI_PROC_NULL.
-int halo_shift(ttfld_ctx* c, double* a) {
+// a2: a second array for the same launch, or none.
+static int halo_shift(ttfld_ctx* c, double* a1, double* a2) {
   Dev d = c->d;
-  launch_box(c->stream, box(-1, d.nx + 2, 0, 0, 1, d.nz), [=] __device__(int i, int, int k) {
+  launch_box(c->stream, box(-1, d.nx + 2, 1, a2 ? 2 : 1, 1, d.nz), [=] __device__(int i, int m, int k) {
+    double* a = m == 1 ? a1 : a2;
     a[hidx(d, i, 0, k)] = a[hidx(d, i, d.ny, k)];
     a[hidx(d, i, -1, k)] = a[hidx(d, i, d.ny - 1, k)];
     a[hidx(d, i, d.ny + 1, k)] = a[hidx(d, i, 1, k)];
@@ -21,16 +23,18 @@ int halo_shift(ttfld_ctx* c, double* a) {
   TT_CHECK_LAUNCH();
   return 0;
 }
+int halo_shift(ttfld_ctx* c, double* a) { return halo_shift(c, a, nullptr); }
 
 // NORTH_POLE_SHIFT / SOUTH_POLE_SHIFT ppshift.f:2217-2453 with one rank: the
 // partner across each pole (myid -/+ numprocs/2, ppshift.f:820-833) is the
 // rank itself, so planes NZ-1, NZ-2, NZ-3 are copied onto NZ, NZ+1, NZ+2 and
 // planes 1, 2 onto 0, -1, over the whole (i, j) extent with the ghosts.
 // Nothing without poles.
-int pole_shift(ttfld_ctx* c, double* a) {
+static int pole_shift(ttfld_ctx* c, double* a1, double* a2) {
   Dev d = c->d;
   if (!d.poles) return 0;
-  launch_box(c->stream, box(-1, d.nx + 2, -1, d.ny + 2, 0, 0), [=] __device__(int i, int j, int) {
+  launch_box(c->stream, box(-1, d.nx + 2, -1, d.ny + 2, 1, a2 ? 2 : 1), [=] __device__(int i, int j, int q) {
+    double* a = q == 1 ? a1 : a2;
     const int nz = d.nz;
     for (int m = 0; m < 3; ++m) a[hidx(d, i, j, nz + m)] = a[hidx(d, i, j, nz - 1 - m)];
     for (int m = 0; m < 2; ++m) a[hidx(d, i, j, -m)] = a[hidx(d, i, j, 1 + m)];
@@ -38,6 +42,7 @@ int pole_shift(ttfld_ctx* c, double* a) {
   TT_CHECK_LAUNCH();
   return 0;
 }
+int pole_shift(ttfld_ctx* c, double* a) { return pole_shift(c, a, nullptr); }
 
 // Synthetic analytic opacity in KAPPA's IKAPTYP 20:25 branch
 // (pprphy.f:321-351): evaluated for i = -1..UPPERBND, then i = UPPERBND..NX+2
@@ -55,6 +60,7 @@ struct OpacTab {
   int nt, nrh;
   int* err;
   const double *lt, *lrh, *ross, *plnk, *absk;
+  const double *t10, *plnk10, *absk10;  // pow(10, .) of the T nodes and of two of the means at the nodes
 };
 
 static OpacTab opac_tab(const ttfld_ctx* c) {
@@ -67,8 +73,23 @@ static OpacTab opac_tab(const ttfld_ctx* c) {
   t.lrh = p; p += t.nrh;
   t.ross = p; p += (size_t)t.nt * t.nrh;
   t.plnk = p; p += (size_t)t.nt * t.nrh;
-  t.absk = p;
+  t.absk = p; p += (size_t)t.nt * t.nrh;
+  t.t10 = p; p += t.nt;
+  t.plnk10 = p; p += (size_t)t.nt * t.nrh;
+  t.absk10 = p;
   return t;
+}
+
+// The first node above v (1-based; n + 1: none), as the reference's loop from
+// the first node up finds it; the nodes increase.
+__device__ __forceinline__ int first_above(const double* node, int n, double v) {
+  int lo = 0, hi = n;
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (node[mid] > v) hi = mid;
+    else lo = mid + 1;
+  }
+  return lo + 1;
 }
 
 // BurrowsOPC (pprphy.f:1005-1229) for the Rosseland, Planck and absorption
@@ -77,7 +98,9 @@ static OpacTab opac_tab(const ttfld_ctx* c) {
 // WS1/WS along T and WS2/WS3 along rho (:1081-1084, :1106-1109), 10^ of the
 // bilinear form (:1112-1135), the T-derivative stand-ins of :1180-1185.
 // Returns 0, or the reason the reference stops (1: T <= 0, 2: above the
-// table, 3: below it, 4: a non-positive opacity).
+// table, 3: below it, 4: a non-positive opacity).  The powers of ten of the
+// node values alone are formed once per table (ttfld_set_opacity_table): three
+// pow() per cell instead of nine.
 __device__ __forceinline__ int burrows_opc(const OpacTab& tb, double t, double rh, double& kp, double& kr,
                                            double& ka, double& dkp, double& dka) {
   if (!(t > 0.0)) return 1;
@@ -86,8 +109,7 @@ __device__ __forceinline__ int burrows_opc(const OpacTab& tb, double t, double r
   if (tm1 > (double)3.69889f) tm1 = (double)3.69888f;
   if (rh1 < (double)-11.9996f) rh1 = (double)-11.9995f;
   if (rh1 > (double)-1.99993f) rh1 = (double)-1.99994f;
-  int it = 1;
-  while (it <= tb.nt && !(tb.lt[it - 1] > tm1)) ++it;
+  const int it = first_above(tb.lt, tb.nt, tm1);
   if (it == tb.nt + 1) return 2;
   if (it == 1) return 3;
   const int it1 = it - 1;
@@ -95,8 +117,7 @@ __device__ __forceinline__ int burrows_opc(const OpacTab& tb, double t, double r
   double ws = tb.lt[it1 - 1] - tb.lt[it - 1];
   ws1 = ws1 / ws;
   ws = 1.0 - ws1;
-  int iw = 1;
-  while (iw <= tb.nrh && !(tb.lrh[iw - 1] > rh1)) ++iw;
+  const int iw = first_above(tb.lrh, tb.nrh, rh1);
   if (iw == tb.nrh + 1) return 2;
   if (iw == 1) return 3;
   const int iw1 = iw - 1;
@@ -114,9 +135,9 @@ __device__ __forceinline__ int burrows_opc(const OpacTab& tb, double t, double r
   kr = interp(tb.ross);
   kp = interp(tb.plnk);
   ka = interp(tb.absk);
-  const double dt = pow(10.0, tb.lt[it - 1]) - pow(10.0, tb.lt[it1 - 1]);
-  dkp = (pow(10.0, tb.plnk[n00]) - pow(10.0, tb.plnk[n01])) / dt;
-  dka = (pow(10.0, tb.absk[n00]) - pow(10.0, tb.absk[n01])) / dt;
+  const double dt = tb.t10[it - 1] - tb.t10[it1 - 1];
+  dkp = div_rn(tb.plnk10[n00] - tb.plnk10[n01], dt);
+  dka = div_rn(tb.absk10[n00] - tb.absk10[n01], dt);
   if (kr <= 0.0 || kp <= 0.0 || ka <= 0.0) return 4;
   return 0;
 }
@@ -131,8 +152,7 @@ __device__ __forceinline__ int burrows_wave(const OpacTab& tb, const double* wop
   if (tm1 > (double)3.69889f) tm1 = (double)3.69888f;
   if (rh1 < (double)-11.9996f) rh1 = (double)-11.9995f;
   if (rh1 > (double)-1.99993f) rh1 = (double)-1.99994f;
-  int it = 1;
-  while (it <= tb.nt && !(tb.lt[it - 1] > tm1)) ++it;
+  const int it = first_above(tb.lt, tb.nt, tm1);
   if (it == tb.nt + 1) return 2;
   if (it == 1) return 3;
   const int it1 = it - 1;
@@ -140,8 +160,7 @@ __device__ __forceinline__ int burrows_wave(const OpacTab& tb, const double* wop
   double ws = tb.lt[it1 - 1] - tb.lt[it - 1];
   ws1 = ws1 / ws;
   ws = 1.0 - ws1;
-  int iw = 1;
-  while (iw <= tb.nrh && !(tb.lrh[iw - 1] > rh1)) ++iw;
+  const int iw = first_above(tb.lrh, tb.nrh, rh1);
   if (iw == tb.nrh + 1) return 2;
   if (iw == 1) return 3;
   const int iw1 = iw - 1;
@@ -683,6 +702,56 @@ static int stellar_binned(ttfld_ctx* c) {
   return 0;
 }
 
+// CALCSTELLARTAU (pprad.f:191-221): per column the optical depth summed from
+// UPPERBND inward, one sum after another as the reference's loop has it, and
+// zero above it (where UPPERBND < NX).  A block takes 32 neighbouring columns:
+// all its threads form the products of kTauChunk radii, a warp per column
+// (coalesced), and 32 of them then run the columns' sums through shared
+// memory.  (One thread per column walking global memory, a stride of a whole
+// radial row between the threads of a warp: 50 us at 100x256x128, 20 us at
+// 40x64x32.)
+constexpr int kTauCols = 32, kTauChunk = 64;
+__global__ void __launch_bounds__(kThreads) stellar_tau_kernel(Dev d) {
+  __shared__ double s[kTauCols][kTauChunk + 1];
+  __shared__ int ubs[kTauCols];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const long long c0 = (long long)blockIdx.x * kTauCols, ncol = (long long)nplane(d);
+  if (threadIdx.x < kTauCols) {
+    const long long q = c0 + threadIdx.x;
+    int ub = q < ncol ? d.UB[q] : 0;
+    ubs[threadIdx.x] = ub > d.nx + 1 ? d.nx + 1 : ub;
+  }
+  const double dr = G(xxb, 2) - G(xxb, 1);
+  double tot = 0.0;  // of column c0 + lane, in warp 0
+  for (int top = d.nx + 1; top >= 1; top -= kTauChunk) {
+    const int low = top - kTauChunk + 1 > 1 ? top - kTauChunk + 1 : 1;
+    __syncthreads();
+    for (int m = warp; m < kTauCols; m += kThreads / 32) {
+      const long long q = c0 + m;
+      if (q >= ncol) break;
+      const size_t base = (size_t)(d.nx + 4) * (size_t)q + 1;  // halo index of i = 0
+      for (int i = low + lane; i <= top; i += 32)
+        s[m][i - low] = i <= ubs[m] ? mul_rn(mul_rn(d.XKAPA[base + i], d.RH[base + i]), dr) : 0.0;
+    }
+    __syncthreads();
+    if (warp == 0) {
+      const int first = ubs[lane] < top ? ubs[lane] : top;
+      for (int i = first; i >= low; --i) {
+        tot = tot + s[lane][i - low];
+        s[lane][i - low] = tot;
+      }
+    }
+    __syncthreads();
+    for (int m = warp; m < kTauCols; m += kThreads / 32) {
+      const long long q = c0 + m;
+      if (q >= ncol) break;
+      const size_t base = (size_t)(d.nx + 4) * (size_t)q + 1;
+      for (int i = low + lane; i <= top; i += 32)
+        if (i <= ubs[m] || ubs[m] < d.nx) d.STAU[base + i] = s[m][i - low];
+    }
+  }
+}
+
 static int stellarinput_heating(ttfld_ctx* c) {
   Dev d = c->d;
   if (d.f_incident == 0) {
@@ -696,18 +765,8 @@ static int stellarinput_heating(ttfld_ctx* c) {
     }
     return stellar_binned(c);
   }
-  launch_box(c->stream, box(0, 0, -1, d.ny + 2, -1, d.nz + 2), [=] __device__(int, int j, int k) {
-    double dr = G(xxb, 2) - G(xxb, 1);
-    int ub = PA(UB, j, k);
-    if (ub > d.nx + 1) ub = d.nx + 1;
-    if (ub < d.nx)
-      for (int i = ub + 1; i <= d.nx + 1; ++i) HA(STAU, i, j, k) = 0.0;
-    double tot = 0.0;
-    for (int i = ub; i >= 1; --i) {
-      tot = tot + (HA(XKAPA, i, j, k) * HA(RH, i, j, k) * dr);
-      HA(STAU, i, j, k) = tot;
-    }
-  });
+  stellar_tau_kernel<<<(unsigned int)((nplane(d) + kTauCols - 1) / kTauCols), kThreads, 0, c->stream>>>(d);
+  count_launches(1);
   TT_CHECK_LAUNCH();
   // STELLAR_DTAU and STELLARINPUT of the same cell in one pass
   launch_box(c->stream, box(1, d.nx + 1, -1, d.ny + 2, -1, d.nz + 2), [=] __device__(int i, int j, int k) {
@@ -728,6 +787,37 @@ static int stellarinput_heating(ttfld_ctx* c) {
   return 0;
 }
 
+// UPPERBND of every column (ppbou.f:124-138: the first i with RH below 1e-9,
+// else NX-1) and PASSUPPERBND's ghosts with one rank (ppbou.f:522-682: the j
+// ghosts by wrap for k = 1..NZ, then the k ghosts from k = 1 and NZ).  One
+// warp reads a column, 32 radii at once; its value goes to every place of the
+// plane that takes it.  (One thread per column, which reads its radii one
+// after another, and two more launches for the ghosts: 28 us at 100x256x128.)
+__global__ void __launch_bounds__(kThreads) upperbnd_kernel(Dev d) {
+  const unsigned int col = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31, ny = d.ny, nz = d.nz;
+  if (col >= (unsigned int)ny * nz) return;
+  unsigned int ju;
+  const int k = (int)div_rem(d.by_ny, col, ju) + 1, j = (int)ju + 1;
+  int ub = d.nx - 1;
+  for (int i0 = 1; i0 <= d.nx; i0 += 32) {
+    const int i = i0 + lane;
+    const unsigned int low =
+        __ballot_sync(0xffffffffu, i <= d.nx && HA(RH, i <= d.nx ? i : 1, j, k) < (double)1.0e-9f);
+    if (low) {
+      ub = i0 + __ffs(low) - 1;
+      break;
+    }
+  }
+  // the copies: j itself and its phi ghost, k itself and the two theta ghosts
+  const int jg = j <= 2 ? ny + j : (j >= ny - 1 ? j - ny : j);
+  if (lane >= 6) return;
+  const int jj = (lane & 1) ? jg : j, m = lane >> 1;
+  if (k == 1) PA(UB, jj, 1 - m) = ub;             // 1, 0, -1
+  else if (m == 0) PA(UB, jj, k) = ub;
+  if (k == nz && m > 0) PA(UB, jj, nz + m) = ub;  // NZ+1, NZ+2
+}
+
 // BOUNDS ppbou.f:1-92 for MODTYP=2 (MODVER 0,2-5), T/RH/UPPERBND only:
 // UPPERBND from density (ppbou.f:124-138), PASSUPPERBND one rank
 // (ppbou.f:522-682), BOUNDXMIN(9) (:1029-1049), BOUNDXMAX(2) (:1269-1384),
@@ -736,27 +826,13 @@ static int bounds(ttfld_ctx* c) {
   Dev d = c->d;
   int rc;
   if (d.bcxmin != 9) return TTFLD_E_UNSUPPORTED;
-  if ((rc = halo_shift(c, d.T)) || (rc = halo_shift(c, d.RH))) return rc;
-  if ((rc = pole_shift(c, d.T)) || (rc = pole_shift(c, d.RH))) return rc;
-  launch_box(c->stream, box(0, 0, 1, d.ny, 1, d.nz), [=] __device__(int, int j, int k) {
-    int ub = d.nx - 1;
-    for (int i = 1; i <= d.nx; ++i)
-      if (HA(RH, i, j, k) < (double)1.0e-9f) { ub = i; break; }
-    PA(UB, j, k) = ub;
-  });
-  TT_CHECK_LAUNCH();
-  // PASSUPPERBND one rank: j ghosts by wrap for k = 1..NZ, then edges.
-  launch_box(c->stream, box(0, 0, 0, 0, 1, d.nz), [=] __device__(int, int, int k) {
-    PA(UB, 0, k) = PA(UB, d.ny, k); PA(UB, -1, k) = PA(UB, d.ny - 1, k);
-    PA(UB, d.ny + 1, k) = PA(UB, 1, k); PA(UB, d.ny + 2, k) = PA(UB, 2, k);
-  });
-  TT_CHECK_LAUNCH();
-  launch_box(c->stream, box(0, 0, -1, d.ny + 2, 0, 0), [=] __device__(int, int j, int) {
-    const int nz = d.nz;
-    PA(UB, j, 0) = PA(UB, j, 1); PA(UB, j, -1) = PA(UB, j, 1);
-    PA(UB, j, nz + 1) = PA(UB, j, nz); PA(UB, j, nz + 2) = PA(UB, j, nz);
-  });
-  TT_CHECK_LAUNCH();
+  if ((rc = halo_shift(c, d.T, d.RH)) || (rc = pole_shift(c, d.T, d.RH))) return rc;
+  {
+    const long long lanes = (long long)d.ny * d.nz * 32;
+    upperbnd_kernel<<<(unsigned int)((lanes + kThreads - 1) / kThreads), kThreads, 0, c->stream>>>(d);
+    count_launches(1);
+    TT_CHECK_LAUNCH();
+  }
   // BOUNDXMIN(9); at III = 0 the opacity of cell (1,1,1) comes from the
   // opacity table (ppbou.f:1040-1044) where kappa_model 2 has one, else from
   // the analytic model
@@ -816,8 +892,7 @@ static int bounds(ttfld_ctx* c) {
     HA(T, i, j, nz + 2) = HA(T, i, j, nz);
   });
   TT_CHECK_LAUNCH();
-  if ((rc = halo_shift(c, d.T)) || (rc = halo_shift(c, d.RH))) return rc;
-  if ((rc = pole_shift(c, d.T)) || (rc = pole_shift(c, d.RH))) return rc;
+  if ((rc = halo_shift(c, d.T, d.RH)) || (rc = pole_shift(c, d.T, d.RH))) return rc;
   return 0;
 }
 
@@ -867,7 +942,8 @@ int ttfld_set_opacity_table(ttfld_ctx* c, const ttfld_opacity_table* t) {
       !t->log_abs)
     return TTFLD_E_ARGS;
   const size_t nn = (size_t)t->nt * t->nrh;
-  const size_t bytes = (1 + (size_t)t->nt + t->nrh + 3 * nn) * sizeof(double);
+  const size_t given = (size_t)t->nt + t->nrh + 3 * nn;
+  const size_t bytes = (1 + given + (size_t)t->nt + 2 * nn) * sizeof(double);
   TT_CHECK(cudaSetDevice(c->device));
   if (c->opac) {
     TT_CHECK(cudaStreamSynchronize(c->stream));
@@ -887,6 +963,16 @@ int ttfld_set_opacity_table(ttfld_ctx* c, const ttfld_opacity_table* t) {
   TT_CHECK(cudaMemcpy(p, t->log_plnk, nn * sizeof(double), cudaMemcpyHostToDevice));
   p += nn;
   TT_CHECK(cudaMemcpy(p, t->log_abs, nn * sizeof(double), cudaMemcpyHostToDevice));
+  // pow(10, .) of the T nodes and of the Planck and absorption means, on the
+  // device, whose pow() the interpolation uses
+  const OpacTab tb = opac_tab(c);
+  double* out = const_cast<double*>(tb.t10);
+  const int nt = t->nt, n2 = (int)(nt + 2 * nn);
+  launch_box(c->stream, box(0, n2 - 1, 0, 0, 0, 0), [=] __device__(int i, int, int) {
+    out[i] = pow(10.0, i < nt ? tb.lt[i] : tb.plnk[i - nt]);  // the two means lie one after the other
+  });
+  TT_CHECK_LAUNCH();
+  TT_CHECK(cudaStreamSynchronize(c->stream));
   return TTFLD_OK;
 }
 

@@ -23,39 +23,46 @@ int solve_delta_er(ttfld_ctx* c, ttfld_solve_stats* st);
 // j,k ghosts; those reads are clamped into the array here.  The cells they
 // feed (ghost corners and the i=NX+2 plane of E_R) are never read by the
 // step.
-static int upper_bc(ttfld_ctx* c) {
-  Dev d = c->d;
-  launch_box(c->stream, box(1, d.nx + 2, -1, d.ny + 2, -1, d.nz + 2), [=] __device__(int i, int j, int k) {
-    int ub = PA(UB, j, k);
-    if (i < ub || ub < 1) return;
-    double qupper = HA(RH, ub - 1, j, k) * HA(CV, ub - 1, j, k) * HA(T, ub, j, k);
-    int ic = i > d.nx + 1 ? d.nx + 1 : i;
-    int jc = j < 1 ? 1 : (j > d.ny ? d.ny : j);
-    int kc = k < 1 ? 1 : (k > d.nz ? d.nz : k);
-    HA(Q, i, j, k) = qupper;
-    HA(ER, i, j, k) = fabs(2.0 * FA(FLUXX, ic, jc, kc) / TT_FD);
-  });
-  TT_CHECK_LAUNCH();
-  return 0;
+__device__ __forceinline__ void upper_cell(const Dev& d, int i, int j, int k, int ub) {
+  const double qupper = mul_rn(mul_rn(HA(RH, ub - 1, j, k), HA(CV, ub - 1, j, k)), HA(T, ub, j, k));
+  const int ic = i > d.nx + 1 ? d.nx + 1 : i;
+  const int jc = j < 1 ? 1 : (j > d.ny ? d.ny : j);
+  const int kc = k < 1 ? 1 : (k > d.nz ? d.nz : k);
+  HA(Q, i, j, k) = qupper;
+  HA(ER, i, j, k) = fabs(div_rn(2.0 * FA(FLUXX, ic, jc, kc), TT_FD));
 }
 
 // Left (XMIN) boundary for BCXMIN=9, ppenergy.f:150-167 and :620-637.
-static int left_bc(ttfld_ctx* c) {
+__device__ __forceinline__ void left_column(const Dev& d, int j, int k) {
+  double dqdr;
+  if (d.ieta == 5)
+    dqdr = div_rn(-HA(RH, 1, j, k) * HA(CV, 1, j, k) * d.fbottom,
+                  HA(RH, 1, j, k) * HA(CV, 1, j, k) * (d.xnue / d.pr_num));
+  else
+    dqdr = -div_rn(HA(RH, 1, j, k) * HA(CV, 1, j, k) * 3.0 * d.fbottom * HA(XKAPR, 1, j, k) * HA(RH, 1, j, k),
+                   4.0 * TT_ARAD * TT_FD * p3(HA(T, 1, j, k)));
+  const double q1 = HA(Q, 1, j, k);
+  const double q0 = q1 - dqdr * (G(xxb, 1) - G(xxb, 0)), qm = q1 - dqdr * (G(xxb, 1) - G(xxb, -1));
+  HA(Q, 0, j, k) = q0;
+  HA(Q, -1, j, k) = qm;
+  HA(ER, 1, j, k) = TT_ARAD * p4(div_rn(q1, HA(RH, 1, j, k) * HA(CV, 1, j, k)));
+  HA(ER, 0, j, k) = TT_ARAD * p4(div_rn(q0, HA(RH, 0, j, k) * HA(CV, 0, j, k)));
+  HA(ER, -1, j, k) = TT_ARAD * p4(div_rn(qm, HA(RH, -1, j, k) * HA(CV, -1, j, k)));
+}
+
+// Both radial boundaries in one launch: the cells at i >= UPPERBND, and by the
+// thread of i = 1 the left one of its column.  They meet only in cell 1 of a
+// column with UPPERBND = 1, which that thread forms in the caller's order
+// (upper then left before the first outer iteration, ppenergy.f:80-167; left
+// then upper after each, :578-702).
+static int radial_bc(ttfld_ctx* c, bool upper_first) {
   Dev d = c->d;
   if (d.bcxmin != 9) return TTFLD_E_UNSUPPORTED;
-  launch_box(c->stream, box(0, 0, -1, d.ny + 2, -1, d.nz + 2), [=] __device__(int, int j, int k) {
-    double dqdr;
-    if (d.ieta == 5)
-      dqdr = -HA(RH, 1, j, k) * HA(CV, 1, j, k) * d.fbottom /
-             (HA(RH, 1, j, k) * HA(CV, 1, j, k) * (d.xnue / d.pr_num));
-    else
-      dqdr = -(HA(RH, 1, j, k) * HA(CV, 1, j, k) * 3.0 * d.fbottom * HA(XKAPR, 1, j, k) * HA(RH, 1, j, k) /
-               (4.0 * TT_ARAD * TT_FD * p3(HA(T, 1, j, k))));
-    HA(Q, 0, j, k) = HA(Q, 1, j, k) - dqdr * (G(xxb, 1) - G(xxb, 0));
-    HA(Q, -1, j, k) = HA(Q, 1, j, k) - dqdr * (G(xxb, 1) - G(xxb, -1));
-    HA(ER, 1, j, k) = TT_ARAD * p4(HA(Q, 1, j, k) / (HA(RH, 1, j, k) * HA(CV, 1, j, k)));
-    HA(ER, 0, j, k) = TT_ARAD * p4(HA(Q, 0, j, k) / (HA(RH, 0, j, k) * HA(CV, 0, j, k)));
-    HA(ER, -1, j, k) = TT_ARAD * p4(HA(Q, -1, j, k) / (HA(RH, -1, j, k) * HA(CV, -1, j, k)));
+  launch_box(c->stream, box(1, d.nx + 2, -1, d.ny + 2, -1, d.nz + 2), [=] __device__(int i, int j, int k) {
+    const int ub = PA(UB, j, k);
+    if (i == 1 && !upper_first) left_column(d, j, k);
+    if (i >= ub && ub >= 1) upper_cell(d, i, j, k, ub);
+    if (i == 1 && upper_first) left_column(d, j, k);
   });
   TT_CHECK_LAUNCH();
   return 0;
@@ -229,7 +236,7 @@ int coupled_energy_eqs(ttfld_ctx* c, int do_bounds, ttfld_step_stats* out) {
   // :74-75: only the top faces' fluxes are read (by :80-105) before :253-255
   // forms every face again
   if ((rc = asm_top_fluxes(c, kappa_done))) return rc;
-  if ((rc = upper_bc(c)) || (rc = left_bc(c)) || (rc = z_bc(c))) return rc;
+  if ((rc = radial_bc(c, true)) || (rc = z_bc(c))) return rc;
   if ((rc = halo_shift(c, d.ER)) || (rc = pole_shift(c, d.ER))) return rc;   // :230-245
   TT_CHECK(cudaMemcpyAsync(d.Q_OLD, d.Q, nhalo(d) * 8, cudaMemcpyDeviceToDevice, c->stream));
   TT_CHECK(cudaMemcpyAsync(d.ER_OLD, d.ER, nhalo(d) * 8, cudaMemcpyDeviceToDevice, c->stream));
@@ -264,7 +271,7 @@ int coupled_energy_eqs(ttfld_ctx* c, int do_bounds, ttfld_step_stats* out) {
       printf("MAX COUPLED SOR ITERATION %8d %8d %12.6e\n", c->params.iii, energy_iter, ss.rnorm / ss.rhsnorm);
     TT_CHECK(cudaMemsetAsync(c->stp, 0, sizeof(StepDev), c->stream));
     if ((rc = delta_q_update(c, theta, conv_parm))) return rc;          // :379-573
-    if ((rc = left_bc(c)) || (rc = upper_bc(c)) || (rc = z_bc(c))) return rc;  // :578-733
+    if ((rc = radial_bc(c, false)) || (rc = z_bc(c))) return rc;        // :578-733
     StepDev hs;
     TT_CHECK(cudaMemcpyAsync(&hs, c->stp, sizeof(StepDev), cudaMemcpyDeviceToHost, c->stream));
     TT_CHECK(cudaStreamSynchronize(c->stream));
