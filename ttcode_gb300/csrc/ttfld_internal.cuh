@@ -292,6 +292,77 @@ __device__ __forceinline__ bool wait_flags(const unsigned int* flags, int lo, in
   return ok_sh != 0;
 }
 
+// Sum over the warp in a fixed order, the same in every lane.
+__device__ __forceinline__ double warp_sum_all(double v) {
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// A block's share of a norm, with the norm's number (from 1 in each launch of
+// the persistent sweeps): written and read as one 128-bit word, so that no
+// fence orders the two.  Norms alternate between two words a block: when a
+// block writes that of norm k + 2 it has read every block's of norm k + 1,
+// which each wrote after reading those of norm k.
+struct __align__(16) Partial {
+  double part;
+  unsigned long long number;
+};
+__device__ __forceinline__ void put_partial(Partial* gather, int b, int number, double part) {
+  Partial* p = gather + 2 * (size_t)b + (number & 1);
+  asm volatile(
+      "{\n .reg .b128 v;\n mov.b128 v, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], v;\n}" ::"l"(p),
+      "l"(__double_as_longlong(part)), "l"((long long)number)
+      : "memory");
+}
+__device__ __forceinline__ bool get_partial(const Partial* gather, int b, int number, double& part) {
+  const Partial* p = gather + 2 * (size_t)b + (number & 1);
+  long long v, n;
+  asm volatile("{\n .reg .b128 v;\n ld.relaxed.gpu.global.b128 v, [%2];\n mov.b128 {%0, %1}, v;\n}"
+               : "=l"(v), "=l"(n)
+               : "l"(p)
+               : "memory");
+  part = __longlong_as_double(v);
+  return n == number;
+}
+
+// The sum of every block's share of a norm, added in the same order by every
+// block (one warp; every lane gets it).  Bounded like the other waits: false
+// once a block has given up.
+constexpr int kGather = 5;  // shares a lane reads at once: 160 blocks
+__device__ __forceinline__ bool gather_sum(const Partial* gather, int nb, int number, SolverDev* sol, double& tot) {
+  const int lane = threadIdx.x & 31;
+  tot = 0.0;
+  for (int q0 = lane; q0 - lane < nb; q0 += 32 * kGather) {
+    double v[kGather];
+    long long polls = 0;
+    for (;;) {
+      bool ready = true;
+#pragma unroll
+      for (int m = 0; m < kGather; ++m) {
+        v[m] = 0.0;
+        if (q0 + 32 * m < nb && !get_partial(gather, q0 + 32 * m, number, v[m])) ready = false;
+      }
+      if (__all_sync(0xffffffffu, ready)) break;
+      if (__any_sync(0xffffffffu, give_up(++polls, sol))) {
+        if (lane == 0) atomicExch(&sol->bar_timeout, 1);
+        return false;
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < kGather; ++m) tot += v[m];
+  }
+  tot = warp_sum_all(tot);
+  return true;
+}
+
+// An asynchronous copy of one 8- or 16-byte word to shared memory.
+template <class W>
+__device__ __forceinline__ void copy_async(W* to, const W* from) {
+  const unsigned int dst = (unsigned int)__cvta_generic_to_shared(to);
+  if (sizeof(W) == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(from) : "memory");
+  else asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(from) : "memory");
+}
+
 __device__ __forceinline__ bool solver_done(const Dev& d) {
   return *(volatile int*)&d.sol->done != 0;
 }
@@ -376,7 +447,7 @@ int check_cuda(cudaError_t e, const char* what);
 int solve_exact64(ttfld_ctx* c, double* x, const double* b, int itmin, int itmax, ttfld_solve_stats* st);
 int solve_fast64(ttfld_ctx* c, double* x, const double* b, int itmin, int itmax, ttfld_solve_stats* st);
 int solve_mixed(ttfld_ctx* c, double* x, const double* b, ttfld_solve_stats* st, int guess_test = 0,
-                int* fallback = nullptr);
+                int* fallback = nullptr, bool from_zero = false);
 int solve_pcg(ttfld_ctx* c, double* x, const double* b, ttfld_solve_stats* st, int guess_test = 0,
               int* fallback = nullptr);
 void krylov_free(ttfld_ctx* c);

@@ -32,7 +32,7 @@ struct Cmp {
   long long rows;       // ny * nz
   size_t csz;           // slots per colour array (no ghost planes)
   size_t gsz;           // slots per colour array with theta ghost planes
-  FastDiv by_pairs;     // nxp / 2
+  FastDiv by_pairs, by_quads, by_ny;  // nxp / 2, nxp / 4, ny
 };
 
 static Cmp make_cmp(const Dev& d) {
@@ -42,6 +42,8 @@ static Cmp make_cmp(const Dev& d) {
   int nxh = (d.nx + 1) / 2;
   g.nxp = (nxh + 3) / 4 * 4;
   g.by_pairs = fast_div(g.nxp / 2);
+  g.by_quads = fast_div(g.nxp / 4);
+  g.by_ny = fast_div(g.ny);
   g.rows = (long long)d.ny * d.nz;
   g.csz = (size_t)g.rows * g.nxp;
   g.gsz = (size_t)(d.nz + 2) * d.ny * g.nxp;
@@ -142,26 +144,58 @@ void mix_free(ttfld_ctx* c) {
 
 // ---- FP32 path ----------------------------------------------------------
 
-// Jacobi-scaled FP32 coefficients of the current SOR_A..G.
-static int prep32(ttfld_ctx* c) {
-  MixWork* w = work(c);
-  Dev d = c->d;
-  Cmp g = w->g;
-  Mix32 m = w->m32;
-  launch_box(c->stream, box(1, d.nx, 1, d.ny, 1, d.nz), [=] __device__(int i, int j, int k) {
-    size_t q = cidx(d, i, j, k);
-    int col = (i + j + k) & 1;
-    size_t s = cslot(g, j - 1, k - 1, (i - 1) >> 1);
-    const double inv = div_rn(1.0, d.SA[q]);
+// Jacobi-scaled FP32 coefficients of the current SOR_A..G, and of b: its norm
+// ||b||_1 (SolverDev::rhsnorm, fixed order) and rhat = b / A, the correction
+// equation of the zero iterate, whose residual b is.  A zero or non-finite
+// norm marks the solve done, so that sweeps queued behind do nothing.
+__global__ void __launch_bounds__(kThreads) prep32_kernel(Dev d, Cmp g, Mix32 m, const double* __restrict__ b,
+                                                          double* partials) {
+  __shared__ double sh[32];
+  __shared__ bool last;
+  const unsigned int n = (unsigned int)ncell(d);
+  double acc = 0.0;
+  for (unsigned int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
+    int i, j, k;
+    cell_ijk(d, q, i, j, k);
+    const int col = (i + j + k) & 1;
+    const size_t s = cslot(g, j - 1, k - 1, (i - 1) >> 1);
+    const double inv = div_rn(1.0, d.SA[q]), bb = b[q];
     m.a[0][col][s] = f32_rn(d.SB[q] * inv);
     m.a[1][col][s] = f32_rn(d.SC[q] * inv);
     m.a[2][col][s] = f32_rn(mul_rn(d.SD[q], inv));
     m.a[3][col][s] = f32_rn(mul_rn(d.SE[q], inv));
     m.a[4][col][s] = f32_rn(mul_rn(d.SF[q], inv));
     m.a[5][col][s] = f32_rn(mul_rn(d.SG[q], inv));
-    m.ainv[col][s] = f32_rn(inv);
+    const float ainv = f32_rn(inv);
+    m.ainv[col][s] = ainv;
     m.diag[col][s] = f32_rn(d.SA[q]);
-  });
+    m.rhat[col][s] = f32_rn(bb) * ainv;
+    acc += fabs(bb);
+  }
+  const double sb = block_sum(acc, sh);
+  if (threadIdx.x == 0) {
+    partials[blockIdx.x] = sb;
+    __threadfence();
+    last = (atomicAdd(&d.sol->ticket2, 1u) == gridDim.x - 1);
+  }
+  __syncthreads();
+  if (last) {
+    __threadfence();
+    const double tot = block_sum_array(partials, gridDim.x, sh);
+    if (threadIdx.x == 0) {
+      d.sol->rhsnorm = tot;
+      if (!(tot > 0.0) || !isfinite(tot)) d.sol->done = 1;
+      d.sol->ticket2 = 0;
+    }
+  }
+}
+
+static int prep32(ttfld_ctx* c, const double* b) {
+  MixWork* w = work(c);
+  int nb = grid_for((long long)ncell(c->d));
+  if (nb > kMaxPartials) nb = kMaxPartials;
+  prep32_kernel<<<nb, kThreads, 0, c->stream>>>(c->d, w->g, w->m32, b, c->partials);
+  count_launches(1);
   TT_CHECK_LAUNCH();
   return 0;
 }
@@ -200,15 +234,28 @@ __device__ __forceinline__ float4 ldc4(const float* p) {
 // compile-time copy of Cmp::poles, so that the kernels without poles carry
 // no test of it): theta rows 1 and NZ-1 take the cell itself as their
 // neighbour across the edge, and row NZ is not swept.
-template <int COL, bool NORM, bool POLES>
+// FAST_INDEX: the item's row by 32-bit invariant division, which is faster
+// where the coefficients are in shared memory and the index is on the path of
+// the only loads; beside loads of the coefficients the 64-bit one is (16.06
+// against 16.25 ms per step at 100x256x128).
+template <int COL, bool NORM, bool POLES, bool FAST_INDEX>
 __device__ __forceinline__ void update_vec(const Cmp& g, const Mix32& m, float omega, long long t, int nv,
                                            size_t plane, float4 aw, float4 ae, float4 as, float4 an, float4 ab,
                                            float4 at, float4 r, float4 dg, float& nacc) {
   const float* eo = m.e[1 - COL];
   float* es = m.e[COL];
-  const int hv = (int)(t % nv);
-  const long long rr = t / nv;
-  const int j0 = (int)(rr % g.ny), k0 = (int)(rr / g.ny);
+  int hv, j0, k0;
+  if (FAST_INDEX) {
+    unsigned int hu, ju;
+    k0 = (int)div_rem(g.by_ny, div_rem(g.by_quads, (unsigned int)t, hu), ju);
+    hv = (int)hu;
+    j0 = (int)ju;
+  } else {
+    hv = (int)(t % nv);
+    const long long rr = t / nv;
+    j0 = (int)(rr % g.ny);
+    k0 = (int)(rr / g.ny);
+  }
   if (POLES && k0 == g.nz - 1) return;  // the north pole's mirror row (zmax_sor_index, ppsor.f:39-43)
   const int off = (1 + ((j0 + k0) & 1) + COL) & 1;
   const int h0 = hv * 4;
@@ -258,7 +305,7 @@ __device__ __forceinline__ void sweep_vec(const Cmp& g, const Mix32& m, float om
   const float4 r = ldc4(m.rhat[COL] + cb);
   float4 dg = make_float4(0.f, 0.f, 0.f, 0.f);
   if (NORM) dg = ldc4(m.diag[COL] + cb);
-  update_vec<COL, NORM, POLES>(g, m, omega, t, nv, plane, aw, ae, as, an, ab, at, r, dg, nacc);
+  update_vec<COL, NORM, POLES, false>(g, m, omega, t, nv, plane, aw, ae, as, an, ab, at, r, dg, nacc);
 }
 
 // One colour per launch.  NORM launches of the second colour end with the
@@ -402,13 +449,50 @@ __global__ void __launch_bounds__(kPersistThreads) sweeps32_persistent(Cmp g, Mi
 // 160x512x256, the same at 160x256x128 and 60x512x256 (a slow block holds
 // up only its neighbours, not the grid).
 
-template <bool POLES>
+// RESIDENT: what does not change during a launch (the six couplings and r-hat
+// of an item, 112 of the 160 bytes of its update) is copied to shared memory
+// before the first sweep, where a block's share fits (1.2 million cells in
+// all); each thread copies what it reads itself.  Only e, which other blocks
+// write, is then read through L2 in a half-sweep.  Beyond that size the
+// coefficients come straight from global memory: copying each thread's next
+// item to shared memory ahead (cp.async, 172 KB a block) leaves too little L1
+// for the lines of e that items share, 18.0 against 16.1 ms per step at
+// 100x256x128 and 745 against 593 ms at 160x512x256.
+constexpr int kLocalWords = 7;  // float4 of an item: W E S N B T couplings, r-hat
+
+template <int COL>
+__device__ __forceinline__ void fetch_vec(const Mix32& m, long long t, float4* to, unsigned int stride) {
+  const size_t cb = (size_t)t * 4;
+#pragma unroll
+  for (int q = 0; q < 6; ++q) copy_async(to + q * stride, reinterpret_cast<const float4*>(m.a[q][COL] + cb));
+  copy_async(to + 6 * stride, reinterpret_cast<const float4*>(m.rhat[COL] + cb));
+}
+
+template <int COL, bool NORM, bool POLES, bool RESIDENT>
+__device__ __forceinline__ void sweep_local(const Cmp& g, const Mix32& m, float omega, long long t0, unsigned int n,
+                                            int nv, size_t plane, const float4* slots, float& nacc) {
+  for (unsigned int u = threadIdx.x; u < n; u += blockDim.x) {
+    const long long t = t0 + u;
+    if (RESIDENT) {
+      const float4* w = slots + (size_t)COL * kLocalWords * n + u;
+      const float4 dg = NORM ? ldc4(m.diag[COL] + (size_t)t * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+      update_vec<COL, NORM, POLES, true>(g, m, omega, t, nv, plane, w[0], w[n], w[2 * n], w[3 * n], w[4 * n], w[5 * n],
+                                   w[6 * n], dg, nacc);
+    } else {
+      sweep_vec<COL, NORM, POLES>(g, m, omega, t, nv, plane, nacc);
+    }
+  }
+}
+
+template <bool POLES, bool RESIDENT = false>
 __global__ void __launch_bounds__(kPersistThreads) sweeps32_local(Cmp g, Mix32 m, float omega, SolverDev* sol,
-                                                                 double* partials, double stop_ratio, int nsweeps,
+                                                                 Partial* gather, double stop_ratio, int nsweeps,
                                                                  int norm_every, int stall_check, unsigned int* flags,
                                                                  unsigned int base) {
   __shared__ double sh[32];
   __shared__ int stop_sh;
+  extern __shared__ __align__(16) unsigned char slots_raw[];
+  float4* slots = reinterpret_cast<float4*>(slots_raw);
   unsigned int* own = flags + (size_t)blockIdx.x * kFlagStride;
   const unsigned int fin = base + 2u * (unsigned int)nsweeps;
   if (*(volatile int*)&sol->done) {  // set before the launch, so the same for every block
@@ -420,43 +504,58 @@ __global__ void __launch_bounds__(kPersistThreads) sweeps32_local(Cmp g, Mix32 m
   const size_t plane = (size_t)g.ny * g.nxp;
   const int nb = (int)gridDim.x;
   const long long t0 = n * blockIdx.x / nb, t1 = n * (blockIdx.x + 1) / nb;
+  const unsigned int mine = (unsigned int)(t1 - t0);
   const long long reach = (long long)g.ny * nv;  // items within one theta plane
   const int lo = owner_block(t0 > reach ? t0 - reach : 0, n, nb);
   const int hi = owner_block(t1 - 1 + reach < n ? t1 - 1 + reach : n - 1, n, nb);
-  const long long ta = t0 + threadIdx.x;
-  const int bt = (int)blockDim.x;
-  double last_ratio = -1.0;
-  unsigned long long passed = 0;  // grid barriers this block has passed
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  if (RESIDENT) {
+    for (unsigned int u = threadIdx.x; u < mine; u += blockDim.x) {
+      fetch_vec<0>(m, t0 + u, slots + u, mine);
+      fetch_vec<1>(m, t0 + u, slots + (size_t)kLocalWords * mine + u, mine);
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+  }
+  double last_ratio = -1.0;  // in-sweep ratio of the previous norm sweep (lane 0 of the last warp)
+  const int it0 = sol->iter;
+  int norms = 0;
   unsigned int half = base;  // half-sweeps this block has finished
-  bool synced = true;        // every block has finished as many (launch start, grid barrier)
-  for (int sw = 1; sw <= nsweeps; ++sw) {
+  int sw = 1;
+  for (; sw <= nsweeps; ++sw) {
     const bool norm = norm_every > 0 && (sw % norm_every == 0 || sw == nsweeps);
     float nacc = 0.f;
-    if (!synced && !wait_flags(flags, lo, hi, half, sol)) break;
-    if (norm) { for (long long t = ta; t < t1; t += bt) sweep_vec<0, true, POLES>(g, m, omega, t, nv, plane, nacc); }
-    else { for (long long t = ta; t < t1; t += bt) sweep_vec<0, false, POLES>(g, m, omega, t, nv, plane, nacc); }
+    if (sw > 1 && !wait_flags(flags, lo, hi, half, sol)) break;
+    if (norm) sweep_local<0, true, POLES, RESIDENT>(g, m, omega, t0, mine, nv, plane, slots, nacc);
+    else sweep_local<0, false, POLES, RESIDENT>(g, m, omega, t0, mine, nv, plane, slots, nacc);
     publish_flag(own, ++half);
     if (!wait_flags(flags, lo, hi, half, sol)) break;
-    if (norm) { for (long long t = ta; t < t1; t += bt) sweep_vec<1, true, POLES>(g, m, omega, t, nv, plane, nacc); }
-    else { for (long long t = ta; t < t1; t += bt) sweep_vec<1, false, POLES>(g, m, omega, t, nv, plane, nacc); }
-    publish_flag(own, ++half);
-    synced = false;
+    if (norm) sweep_local<1, true, POLES, RESIDENT>(g, m, omega, t0, mine, nv, plane, slots, nacc);
+    else sweep_local<1, false, POLES, RESIDENT>(g, m, omega, t0, mine, nv, plane, slots, nacc);
     if (norm) {
-      const double sb = block_sum((double)nacc, sh);
-      if (threadIdx.x == 0) partials[blockIdx.x] = sb;
+      const double v = warp_sum_all((double)nacc);
+      if (lane == 0) sh[warp] = v;
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) sol->iter += 1;
+    publish_flag(own, ++half);  // its block barrier also orders sh
     if (norm) {
-      if (!grid_sync(sol, (unsigned int)nb, passed)) break;
-      synced = true;
-      const double tot = block_sum_array(partials, nb, sh);
-      if (threadIdx.x == 0) stop_sh = norm_stop(sol, tot, stop_ratio, stall_check, last_ratio);
+      ++norms;
+      if (warp == 0) {
+        const double part = warp_sum_all(lane < nw ? sh[lane] : 0.0);
+        if (lane == 0) put_partial(gather, (int)blockIdx.x, norms, part);
+      }
+      if (warp == nw - 1) {
+        double tot;
+        const bool ok = gather_sum(gather, nb, norms, sol, tot);
+        if (lane == 0) stop_sh = !ok ? 2 : norm_stop(sol, tot, stop_ratio, stall_check, last_ratio);
+      }
       __syncthreads();
       if (stop_sh) break;
     }
   }
   __syncthreads();
-  if (threadIdx.x == 0) *own = fin;
+  if (threadIdx.x == 0) {
+    *own = fin;
+    if (blockIdx.x == 0) sol->iter = it0 + (sw <= nsweeps ? sw : nsweeps);
+  }
 }
 
 // ---- temporal blocking through L2 (sweep_form 3) ---------------------------
@@ -694,8 +793,8 @@ __global__ void __launch_bounds__(kTmaThreads) sweeps32_tma(Cmp g, Mix32 m, floa
           const float4 dg = norm ? sb[7 * kTmaThreads] : make_float4(0.f, 0.f, 0.f, 0.f);
 #define UPD_ARGS g, m, omega, t, nv, plane, sb[0], sb[kTmaThreads], sb[2 * kTmaThreads], sb[3 * kTmaThreads], \
                  sb[4 * kTmaThreads], sb[5 * kTmaThreads], sb[6 * kTmaThreads], dg, nacc
-          if (col == 0) { if (norm) update_vec<0, true, POLES>(UPD_ARGS); else update_vec<0, false, POLES>(UPD_ARGS); }
-          else { if (norm) update_vec<1, true, POLES>(UPD_ARGS); else update_vec<1, false, POLES>(UPD_ARGS); }
+          if (col == 0) { if (norm) update_vec<0, true, POLES, false>(UPD_ARGS); else update_vec<0, false, POLES, false>(UPD_ARGS); }
+          else { if (norm) update_vec<1, true, POLES, false>(UPD_ARGS); else update_vec<1, false, POLES, false>(UPD_ARGS); }
 #undef UPD_ARGS
         }
         ++done_chunks;
@@ -833,21 +932,6 @@ static int resid32(ttfld_ctx* c, const double* x, const double* b, double* l1) {
   return 0;
 }
 
-// rhat = b / A: the correction equation of the zero initial guess.
-static int rhat_of_b(ttfld_ctx* c, const double* b) {
-  MixWork* w = work(c);
-  Dev d = c->d;
-  Cmp g = w->g;
-  Mix32 m = w->m32;
-  launch_box(c->stream, box(1, d.nx, 1, d.ny, 1, d.nz), [=] __device__(int i, int j, int k) {
-    const int col = (i + j + k) & 1;
-    const size_t s = cslot(g, j - 1, k - 1, (i - 1) >> 1);
-    m.rhat[col][s] = f32_rn(b[cidx(d, i, j, k)]) * m.ainv[col][s];
-  });
-  TT_CHECK_LAUNCH();
-  return 0;
-}
-
 // Grid of whole waves: the blocks that fit on the SMs at once (occupancy of
 // the kernel), walking the rest of the items by grid stride, so the last
 // wave of a short streaming kernel is never a partial one.
@@ -913,16 +997,39 @@ static int wave_planes(const Cmp& g) {
 // sized once per grid size and pole form.
 struct SweepGrids {
   int pers, tma, wave, local;
+  int local_threads, resident;
+  size_t local_smem;
 };
 template <bool POLES>
 static SweepGrids sweep_grids(long long nvec) {
-  static SweepGrids gr = {-1, -1, -1, -1};
+  static SweepGrids gr = {-1, -1, -1, -1, 0, 0, 0};
   static long long sized_for = -1;
   if (sized_for != nvec) {
     gr.tma = persistent_grid(sweeps32_tma<POLES>, kTmaThreads, kTmaSmem, nvec);
     gr.pers = persistent_grid(sweeps32_persistent<POLES>, kPersistThreads, 0, nvec);
     gr.wave = nvec < (1LL << 31) ? persistent_grid(sweeps32_wave<POLES>, kPersistThreads, 0, nvec) : 0;
-    gr.local = persistent_grid(sweeps32_local<POLES>, kPersistThreads, 0, nvec);
+    // one block per SM, none of less than two warps' items, with the items
+    // of both colours in shared memory where they fit
+    const size_t item = 2 * kLocalWords * sizeof(float4);  // both colours
+    int dev = 0, sms = 0, room = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaDeviceGetAttribute(&room, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    const long long want = (nvec + 63) / 64 < sms ? (nvec + 63) / 64 : sms;
+    const long long most = want > 0 ? (nvec + want - 1) / want : 0;
+    gr.resident = most > 0 && item * (size_t)most + 1024 <= (size_t)room;
+    if (gr.resident) {
+      const long long rounds = (most + kPersistThreads - 1) / kPersistThreads;
+      gr.local_threads = (int)(((most + rounds - 1) / rounds + 31) / 32 * 32);
+      gr.local_smem = item * (size_t)most;
+      gr.local = persistent_grid(sweeps32_local<POLES, true>, gr.local_threads, gr.local_smem, want * gr.local_threads);
+      if (gr.local != want) gr.resident = 0;
+    }
+    if (!gr.resident) {
+      gr.local_threads = kPersistThreads;
+      gr.local_smem = 0;
+      gr.local = persistent_grid(sweeps32_local<POLES>, kPersistThreads, 0, nvec);
+    }
     if (gr.local > kMaxLocalBlocks) gr.local = 0;
     sized_for = nvec;
   }
@@ -960,7 +1067,7 @@ static int launch_sweeps32_form(ttfld_ctx* c, int nsweeps, int norm_every, doubl
   int stall = stall_check ? 1 : 0;
   void* args[] = {&g, &m, &omega, &sol, &partials, &stop_ratio, &nsweeps, &norm_every, &stall};
   const SweepGrids gr = sweep_grids<POLES>(nvec);
-  if (form != kFormSplit)  // the grid barrier counts arrivals from zero
+  if (form != kFormSplit && form != kFormNeighbour)  // the grid barrier counts arrivals from zero
     TT_CHECK(cudaMemsetAsync(&sol->arrivals, 0, sizeof(unsigned long long), c->stream));
   if (form == kFormWave && gr.wave > 0) {
     int planes = wave_planes(g);
@@ -973,9 +1080,15 @@ static int launch_sweeps32_form(ttfld_ctx* c, int nsweeps, int norm_every, doubl
   if (form == kFormNeighbour && gr.local > 0) {
     unsigned int* flags = w->flags;
     unsigned int base = w->flag_base;
-    void* largs[] = {&g, &m, &omega, &sol, &partials, &stop_ratio, &nsweeps, &norm_every, &stall, &flags, &base};
-    TT_CHECK(cudaLaunchCooperativeKernel((const void*)sweeps32_local<POLES>, dim3(gr.local),
-                                         dim3(kPersistThreads), largs, 0, c->stream));
+    Partial* gather = (Partial*)partials;  // two a block
+    TT_CHECK(cudaMemsetAsync(gather, 0, (size_t)gr.local * 2 * sizeof(Partial), c->stream));
+    void* largs[] = {&g, &m, &omega, &sol, &gather, &stop_ratio, &nsweeps, &norm_every, &stall, &flags, &base};
+    if (gr.resident)
+      TT_CHECK(cudaLaunchCooperativeKernel((const void*)sweeps32_local<POLES, true>, dim3(gr.local),
+                                           dim3(gr.local_threads), largs, gr.local_smem, c->stream));
+    else
+      TT_CHECK(cudaLaunchCooperativeKernel((const void*)sweeps32_local<POLES>, dim3(gr.local), dim3(gr.local_threads),
+                                           largs, gr.local_smem, c->stream));
     w->flag_base = base + 2u * (unsigned int)nsweeps;  // every block leaves its flag there
     count_launches(1);
     return 0;
@@ -987,6 +1100,7 @@ static int launch_sweeps32_form(ttfld_ctx* c, int nsweeps, int norm_every, doubl
     return 0;
   }
   if (form != kFormSplit && gr.pers > 0) {
+    if (form == kFormNeighbour) TT_CHECK(cudaMemsetAsync(&sol->arrivals, 0, sizeof(unsigned long long), c->stream));
     TT_CHECK(cudaLaunchCooperativeKernel((const void*)sweeps32_persistent<POLES>, dim3(gr.pers),
                                          dim3(kPersistThreads), args, 0, c->stream));
     count_launches(1);
@@ -1036,16 +1150,21 @@ static int poll(ttfld_ctx* c) {
 // and the in-sweep norm of each n-th sweep (the residual the sweeps before
 // it left) decides.  The guess keeps its n sweeps and its residual as the
 // first anchor; a rejected guess is replaced by zero (*fallback = 1).
-int solve_mixed(ttfld_ctx* c, double* x, const double* b, ttfld_solve_stats* st, int guess_test, int* fallback) {
+//
+// from_zero: x is zero, so its residual is b (without poles, whose row NZ the
+// residual leaves out): the first anchor is what prep32 formed, and the first
+// sweeps are queued behind it without a residual pass or a readback.
+int solve_mixed(ttfld_ctx* c, double* x, const double* b, ttfld_solve_stats* st, int guess_test, int* fallback,
+                bool from_zero) {
   int rc;
-  if ((rc = ensure32(c)) || (rc = prep32(c))) return rc;
+  if ((rc = ensure32(c))) return rc;
   MixWork* w = work(c);
   const Cmp& g = w->g;
   TT_CHECK(cudaMemsetAsync(c->sol, 0, sizeof(SolverDev), c->stream));
   double bl1 = 0.0, l1 = 0.0;
   // ||b||_1 (SolverDev::rhsnorm, which nothing changes during the solve)
   // comes back with the first readback below
-  if ((rc = rhs_norm(c, b, nullptr))) return rc;
+  if ((rc = prep32(c, b))) return rc;
   const double tol = c->opts.tol;
   const long long budget = c->opts.max_sweeps > 0 ? c->opts.max_sweeps : (long long)c->d.itmax;
   const int period = 8;
@@ -1062,7 +1181,7 @@ int solve_mixed(ttfld_ctx* c, double* x, const double* b, ttfld_solve_stats* st,
   // one launch per anchor needs a persistent kernel (it stops itself)
   const bool one_launch = one_launch_form(sweep_grids_of(g), form);
   if (guess_test) {
-    if ((rc = rhat_of_b(c, b))) return rc;
+    TT_CHECK(cudaMemsetAsync(&c->sol->done, 0, sizeof(int), c->stream));
     TT_CHECK(cudaMemsetAsync(w->m32.e[0], 0, 2 * g.gsz * sizeof(float), c->stream));
     if ((rc = launch_sweeps32(c, guess_test, guess_test, -1.0, form))) return rc;
     // the guess's FP64 residual (and its r-hat) queued behind the sweeps from
@@ -1086,6 +1205,13 @@ int solve_mixed(ttfld_ctx* c, double* x, const double* b, ttfld_solve_stats* st,
     }
   }
   bool anchor_due = !resume;  // the residual of x is still to be formed
+  // the anchor of x = 0, its norm not read back yet: l1 / bl1 = 1 in its place
+  bool unread = !guess_test && from_zero && one_launch && !g.poles && tol < 1.0 && budget > 0;
+  if (unread) {
+    anchor_due = false;
+    c->host_sol->iter = 0;
+    l1 = bl1 = 1.0;
+  }
   for (;;) {
     if (anchor_due) {
       if ((rc = resid32(c, x, b, &l1))) return rc;
@@ -1101,7 +1227,7 @@ int solve_mixed(ttfld_ctx* c, double* x, const double* b, ttfld_solve_stats* st,
     const double stop = fmax(tol * tight, anchor * pow(10.0, -c->opts.inner_digits));
     hit_tol = stop <= tol;
     if (!resume) TT_CHECK(cudaMemsetAsync(w->m32.e[0], 0, 2 * g.gsz * sizeof(float), c->stream));  // e[0], e[1] adjacent
-    TT_CHECK(cudaMemsetAsync(&c->sol->done, 0, sizeof(int), c->stream));
+    if (!unread) TT_CHECK(cudaMemsetAsync(&c->sol->done, 0, sizeof(int), c->stream));
     resume = false;
     int it0 = c->host_sol->iter;
     double r_prev = anchor;
@@ -1124,6 +1250,12 @@ int solve_mixed(ttfld_ctx* c, double* x, const double* b, ttfld_solve_stats* st,
         TT_CHECK(cudaMemsetAsync(&c->sol->stalled, 0, sizeof(int), c->stream));
       }
       l1 = c->host_sol->true_l1;
+      if (unread) {
+        bl1 = c->host_sol->rhsnorm;
+        if (!isfinite(bl1)) { status = TTFLD_E_NONFINITE; break; }
+        if (!(bl1 > 0.0)) break;  // b = 0: x = 0 solves it
+        unread = false;
+      }
     }
     for (; !one_launch;) {
       if ((rc = launch_sweeps32(c, chunk, chunk <= period ? 1 : period, stop, kFormSplit))) return rc;
@@ -1462,7 +1594,8 @@ int time_sweeps(ttfld_ctx* c, int solver, int n, double* ms) {
     ~PlanesOverride() { g_wave_planes = 0; }
   } planes_override(solver >= 16 ? solver - 16 : 0);
   if (mixed) {
-    if ((rc = ensure32(c)) || (rc = prep32(c))) return rc;
+    if ((rc = ensure32(c)) || (rc = prep32(c, c->d.RHS))) return rc;
+    TT_CHECK(cudaMemsetAsync(&c->sol->done, 0, sizeof(int), c->stream));
     double l1;
     if ((rc = resid32(c, c->d.DELTA_ER, c->d.RHS, &l1))) return rc;
     if ((rc = launch_sweeps32(c, 8, 8, -1.0, form, false))) return rc;  // warm

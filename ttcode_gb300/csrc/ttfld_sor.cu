@@ -329,11 +329,13 @@ using namespace ttfld;
 
 namespace {
 
-int solve_current(ttfld_ctx* c, double* x, const double* b, int itmin, int itmax, ttfld_solve_stats* st) {
+// from_zero: x is zero
+int solve_current(ttfld_ctx* c, double* x, const double* b, int itmin, int itmax, ttfld_solve_stats* st,
+                  bool from_zero) {
   switch (c->opts.solver) {
     case TTFLD_SOLVER_SOR64_EXACT: return solve_exact64(c, x, b, itmin, itmax, st);
     case TTFLD_SOLVER_SOR64_FAST: return solve_fast64(c, x, b, itmin, itmax, st);
-    case TTFLD_SOLVER_MIXED: return solve_mixed(c, x, b, st);
+    case TTFLD_SOLVER_MIXED: return solve_mixed(c, x, b, st, 0, nullptr, from_zero);
     case TTFLD_SOLVER_PCG: return solve_pcg(c, x, b, st);
   }
   return TTFLD_E_ARGS;
@@ -348,7 +350,7 @@ int solve_delta_er(ttfld_ctx* c, ttfld_solve_stats* st) {
   ttfld_solve_stats local{};
   if (!st) st = &local;
   int fallback = 0;
-  bool race = false;
+  bool race = false, from_zero = false;
   // the network makes the guess where the run has no previous solution (its
   // first solve, or after ttfld_begin_step(ctx, 1)); once there is one, the
   // previous solution is the better guess (it beats the network's
@@ -359,6 +361,7 @@ int solve_delta_er(ttfld_ctx* c, ttfld_solve_stats* st) {
   TT_CHECK(cudaEventRecord(c->ev0, c->stream));
   if (guess == TTFLD_GUESS_ZERO || (guess == TTFLD_GUESS_PREVIOUS && !c->have_prev)) {
     TT_CHECK(cudaMemsetAsync(d.DELTA_ER, 0, nhalo(d) * 8, c->stream));  // ppsor.f:29
+    from_zero = true;
   } else {
     // initial iterate in the interior; ghosts zero as in ppsor.f:29
     double* x = d.DELTA_ER;
@@ -412,13 +415,14 @@ int solve_delta_er(ttfld_ctx* c, ttfld_solve_stats* st) {
     if (reject) {
       TT_CHECK(cudaMemsetAsync(x, 0, nhalo(d) * 8, c->stream));
       fallback = 1;
+      from_zero = true;
     }
   }
   TT_CHECK(cudaEventRecord(c->evg, c->stream));
   int rc;
   if (race && c->opts.solver == TTFLD_SOLVER_PCG) rc = solve_pcg(c, d.DELTA_ER, d.RHS, st, 1, &fallback);
   else if (race) rc = solve_mixed(c, d.DELTA_ER, d.RHS, st, c->opts.fallback_rule == 3 ? 5 : 2, &fallback);
-  else rc = solve_current(c, d.DELTA_ER, d.RHS, 1, d.itmax, st);
+  else rc = solve_current(c, d.DELTA_ER, d.RHS, 1, d.itmax, st, from_zero);
   TT_CHECK(cudaEventRecord(c->ev1, c->stream));
   TT_CHECK(cudaEventSynchronize(c->ev1));
   float ms = 0.f, gms = 0.f;

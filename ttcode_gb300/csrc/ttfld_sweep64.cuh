@@ -40,69 +40,16 @@
 
 namespace ttfld {
 
-// Sum over the warp in a fixed order, the same in every lane.
-__device__ __forceinline__ double warp_sum_all(double v) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
-// A block's share of a sweep's norm, with the sweep it belongs to: written
-// and read as one 128-bit word, so that no fence orders the two.  Sweeps
-// alternate between two of them a block: when a block writes that of sweep
-// k + 2 it has read every block's of sweep k + 1, which each wrote after
-// reading those of sweep k.
-struct __align__(16) Partial {
-  double part;
-  unsigned long long sweep;
-};
-__device__ __forceinline__ void put_partial(Partial* gather, int b, int sweep, double part) {
-  Partial* p = gather + 2 * (size_t)b + (sweep & 1);
-  asm volatile(
-      "{\n .reg .b128 v;\n mov.b128 v, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], v;\n}" ::"l"(p),
-      "l"(__double_as_longlong(part)), "l"((long long)sweep)
-      : "memory");
-}
-__device__ __forceinline__ bool get_partial(const Partial* gather, int b, int sweep, double& part) {
-  const Partial* p = gather + 2 * (size_t)b + (sweep & 1);
-  long long v, n;
-  asm volatile("{\n .reg .b128 v;\n ld.relaxed.gpu.global.b128 v, [%2];\n mov.b128 {%0, %1}, v;\n}"
-               : "=l"(v), "=l"(n)
-               : "l"(p)
-               : "memory");
-  part = __longlong_as_double(v);
-  return n == sweep;
-}
-
-// The norm of sweep sw from every block's share, added in the same order by
-// one warp of every block, and the reference's rule on it: 0 go on, 1 stop,
-// 2 a block has given up (every lane gets it).  Bounded like the other waits.
-// Block 0 records the sweep.
-constexpr int kGather = 5;  // partials a lane reads at once: 160 blocks
+// The norm of sweep sw from every block's share and the reference's rule on
+// it, by one warp of every block: 0 go on, 1 stop, 2 a block has given up
+// (every lane gets it).  Block 0 records the sweep.
 template <class Sys>
 __device__ __forceinline__ int gather_norm(const Sys& s, const Partial* gather, int nb, int sw, int it0, int itmin,
                                            int itmax, double eps, double rhsnorm, SolverDev* sol) {
   const int lane = threadIdx.x & 31;
-  double tot = 0.0;
-  for (int q0 = lane; q0 - lane < nb; q0 += 32 * kGather) {
-    double v[kGather];
-    long long polls = 0;
-    for (;;) {
-      bool ready = true;
-#pragma unroll
-      for (int m = 0; m < kGather; ++m) {
-        v[m] = 0.0;
-        if (q0 + 32 * m < nb && !get_partial(gather, q0 + 32 * m, sw, v[m])) ready = false;
-      }
-      if (__all_sync(0xffffffffu, ready)) break;
-      if (__any_sync(0xffffffffu, give_up(++polls, sol))) {
-        if (lane == 0) atomicExch(&sol->bar_timeout, 1);
-        return 2;
-      }
-    }
-#pragma unroll
-    for (int m = 0; m < kGather; ++m) tot += v[m];
-  }
-  tot = s.norm(warp_sum_all(tot));
+  double tot;
+  if (!gather_sum(gather, nb, sw, sol, tot)) return 2;
+  tot = s.norm(tot);
   const double ratio = tot / rhsnorm;
   const int it = it0 + sw;
   const bool fin = isfinite(tot), out = it == itmax, met = !(ratio > eps) && it >= itmin;
@@ -127,14 +74,6 @@ __device__ __forceinline__ void undo_colour(const Sys& s, unsigned int r0, unsig
     const unsigned int r = r0 + div_rem(s.by_items, u, h);
     s.restore(r, h, mine[u]);
   }
-}
-
-// An asynchronous copy of one 8- or 16-byte word to shared memory.
-template <class W>
-__device__ __forceinline__ void copy_async(W* to, const W* from) {
-  const unsigned int dst = (unsigned int)__cvta_generic_to_shared(to);
-  if (sizeof(W) == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(from) : "memory");
-  else asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(from) : "memory");
 }
 
 // The items of one colour of a block's rows.  Not RESIDENT: the thread's
