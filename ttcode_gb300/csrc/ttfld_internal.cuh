@@ -355,6 +355,47 @@ __device__ __forceinline__ bool gather_sum(const Partial* gather, int nb, int nu
   return true;
 }
 
+// A grid barrier that also adds up one value per thread: warp 0 publishes the
+// block's sum with the block's arrival and, once every block has arrived,
+// adds all of them in the same order, so that every block gets the same
+// total.  Sums alternate between the two halves of partials, so that a block
+// past the barrier does not overwrite one still being read.  sh: 33 doubles.
+__device__ __forceinline__ bool grid_sum(SolverDev* sol, unsigned int nblocks, unsigned long long& passed, double v,
+                                         double* partials, double* sh, double& total) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  __shared__ int ok_sh;
+  v = warp_sum_all(v);
+  if (lane == 0) sh[warp] = v;
+  __syncthreads();  // every thread's stores, before thread 0's release
+  ++passed;
+  if (warp == 0) {
+    double* part = partials + (passed & 1) * kMaxPartials;
+    const double own = warp_sum_all(lane < nw ? sh[lane] : 0.0);
+    int ok = 1;
+    if (lane == 0) {
+      part[blockIdx.x] = own;
+      asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(&sol->arrivals) : "memory");
+      const unsigned long long target = passed * nblocks;
+      long long polls = 0;
+      while (ld_acquire64(&sol->arrivals) < target)
+        if (give_up(++polls, sol)) {
+          atomicExch(&sol->bar_timeout, 1);
+          ok = 0;
+          break;
+        }
+      ok_sh = ok;
+    }
+    __syncwarp();  // the other lanes' loads come after lane 0's acquire
+    double t = 0.0;
+    for (unsigned int q = lane; q < nblocks; q += 32) t += __ldcg(part + q);
+    t = warp_sum_all(t);
+    if (lane == 0) sh[32] = t;
+  }
+  __syncthreads();
+  total = sh[32];
+  return ok_sh != 0;
+}
+
 // An asynchronous copy of one 8- or 16-byte word to shared memory.
 template <class W>
 __device__ __forceinline__ void copy_async(W* to, const W* from) {

@@ -51,7 +51,10 @@
 namespace ttfld {
 namespace {
 
-constexpr int kPcgThreads = 256;   // one block per SM; 248 registers for the batched passes
+// one block per SM: 256 threads with up to 255 registers for the batched line
+// passes, or 768 in groups for the line Gauss-Seidel tiles
+constexpr int kJacobiThreads = 256, kGsThreads = 768;
+extern __shared__ __align__(128) float tile_sh[];
 constexpr int kPcgStall = 25;      // iterations without a new minimum of r.z end an inner run
 constexpr double kInnerReduce = 1e-4;  // relative reduction of sqrt(r.z) asked of one inner run
 constexpr int kMaxGsSweeps = 32;       // symmetric line Gauss-Seidel sweeps per preconditioner application
@@ -69,6 +72,7 @@ struct Kry {
 struct KryWork {
   Kry k;
   void* mem;
+  float* tiles;  // line tiles in global memory (lines too long for shared memory)
 };
 
 __host__ __device__ __forceinline__ size_t lq(const Kry& k, int i, int j, int kk) {
@@ -119,66 +123,122 @@ __global__ void __launch_bounds__(kThreads) kry_weights_kernel(Dev d, Kry kr, in
     cell_ijk(d, t, i, j, k);
     const Row r = row_of(d, t, i, j, k, hypre != 0);
     const bool decoupled = r.b == 0.0 && r.c == 0.0 && r.d == 0.0 && r.e == 0.0 && r.f == 0.0 && r.g == 0.0;
-    const double v = G(surxb, i) * G(dxa, i) * G(dya, j) * G(surzb, k) * G(dza, k);
+    const double v = mul_rn(mul_rn(mul_rn(mul_rn(G(surxb, i), G(dxa, i)), G(dya, j)), G(surzb, k)), G(dza, k));
     const double e8 = d.E8[t];
-    const double w = decoupled ? v : v / (-e8);
-    const double dd = w * r.a;
+    const double w = decoupled ? v : div_rn(v, -e8);
+    const double dd = mul_rn(w, r.a);
     bool ok = (decoupled || e8 < 0.0) && dd > 0.0 && isfinite(dd);
     kr.wgt[t] = ok ? w : 0.0;
-    kr.sig[t] = ok ? rsqrt(dd) : 0.0;  // any positive scaling serves; it is used consistently
+    kr.sig[t] = ok ? div_rn(1.0, sqrt_rn(dd)) : 0.0;  // any positive scaling serves; it is used consistently
     if (!ok) atomicExch(&d.sol->bad_weights, 1);
   }
 }
 
+// The kernels between the cell order (radius fastest) and the line-major
+// order (phi fastest) work in strips of kStripCols neighbouring columns of
+// one theta row: NX * kStripCols consecutive cells, walked in cell order, with
+// the line-major side going through shared memory, so that both sides are
+// coalesced.  (A warp that writes its 32 radii straight to the line-major
+// arrays writes 32 sectors of 32 bytes for 4 bytes each: 140 us an anchor at
+// 100x256x128.)
+constexpr int kStripCols = 32;
+struct Strip {
+  int j0, k, cols;        // columns j0 .. j0 + cols - 1 (from 1) of theta row k
+  unsigned int t0;        // first cell
+};
+__device__ __forceinline__ Strip strip_of(const Dev& d, unsigned int m) {
+  const unsigned int per = ((unsigned int)d.ny + kStripCols - 1) / kStripCols;
+  Strip p;
+  p.k = (int)(m / per) + 1;
+  p.j0 = (int)(m % per) * kStripCols + 1;
+  p.cols = d.ny - p.j0 + 1 < kStripCols ? d.ny - p.j0 + 1 : kStripCols;
+  p.t0 = (unsigned int)cidx(d, 1, p.j0, p.k);
+  return p;
+}
+constexpr int kStripPitch = kStripCols + 1;
+// Write the staged values of a strip, stage[(i - 1) * kStripPitch + column], to
+// a line-major array.
+__device__ __forceinline__ void strip_out(const Kry& kr, const Strip& p, const float* stage, float* to) {
+  const int lane = threadIdx.x & 31;
+  if (lane < p.cols)
+    for (int i = threadIdx.x >> 5; i < kr.nx; i += blockDim.x >> 5)
+      to[(size_t)i * kr.ncol + (size_t)(p.k - 1) * kr.ny + (size_t)(p.j0 - 1 + lane)] = stage[i * kStripPitch + lane];
+}
+
 // Couplings of S (the symmetric part of Sigma W A Sigma) to the +i, +j, +k
-// neighbours, written line-major.
-__global__ void __launch_bounds__(kThreads) kry_couplings_kernel(Dev d, Kry kr, int hypre) {
-  const unsigned int n = (unsigned int)ncell(d);
+// neighbours, written line-major; stage holds three strips.
+__global__ void __launch_bounds__(kThreads) kry_couplings_kernel(Dev d, Kry kr, int hypre, unsigned int strips,
+                                                                 int staged) {
+  extern __shared__ float stage[];
   const int nx = d.nx, ny = d.ny, nz = d.nz;
-  for (unsigned int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-    int i, j, k;
-    cell_ijk(d, t, i, j, k);
-    const bool h = hypre != 0;
-    const Row r = row_of(d, t, i, j, k, h);
-    const double wn = kr.wgt[t], sn = kr.sig[t];
-    float cr = 0.f, cp = 0.f, ct = 0.f;
-    if (i < nx) {
-      const size_t m = t + 1;
-      const Row rm = row_of(d, m, i + 1, j, k, h);
-      cr = (float)(0.5 * (wn * r.c + kr.wgt[m] * rm.b) * sn * kr.sig[m]);
+  const bool h = hypre != 0;
+  const int one = nx * kStripPitch;
+  for (unsigned int m = blockIdx.x; m < strips; m += gridDim.x) {
+    const Strip p = strip_of(d, m);
+    for (unsigned int u = threadIdx.x; u < (unsigned int)(nx * p.cols); u += blockDim.x) {
+      unsigned int iu;
+      const int col = (int)div_rem(d.by_nx, u, iu), i = (int)iu + 1, j = p.j0 + col, k = p.k;
+      const size_t t = p.t0 + u;
+      const Row r = row_of(d, t, i, j, k, h);
+      const double wn = kr.wgt[t], sn = kr.sig[t];
+      float cr = 0.f, cp = 0.f, ct = 0.f;
+      if (i < nx) {
+        const size_t q = t + 1;
+        const Row rm = row_of(d, q, i + 1, j, k, h);
+        cr = f32_rn(mul_rn(mul_rn(0.5 * (mul_rn(wn, r.c) + mul_rn(kr.wgt[q], rm.b)), sn), kr.sig[q]));
+      }
+      {
+        const int jp = j == ny ? 1 : j + 1;
+        const size_t q = cidx(d, i, jp, k);
+        const Row rm = row_of(d, q, i, jp, k, h);
+        cp = f32_rn(mul_rn(mul_rn(0.5 * (mul_rn(wn, r.e) + mul_rn(kr.wgt[q], rm.d)), sn), kr.sig[q]));
+      }
+      if (k < nz) {
+        const size_t q = cidx(d, i, j, k + 1);
+        const Row rm = row_of(d, q, i, j, k + 1, h);
+        ct = f32_rn(mul_rn(mul_rn(0.5 * (mul_rn(wn, r.g) + mul_rn(kr.wgt[q], rm.f)), sn), kr.sig[q]));
+      }
+      if (staged) {
+        const int o = (int)iu * kStripPitch + col;
+        stage[o] = cr;
+        stage[one + o] = cp;
+        stage[2 * one + o] = ct;
+      } else {
+        const size_t q = lq(kr, i, j, k);
+        kr.cr[q] = cr;
+        kr.cp[q] = cp;
+        kr.ct[q] = ct;
+      }
     }
-    {
-      const int jp = j == ny ? 1 : j + 1;
-      const size_t m = cidx(d, i, jp, k);
-      const Row rm = row_of(d, m, i, jp, k, h);
-      cp = (float)(0.5 * (wn * r.e + kr.wgt[m] * rm.d) * sn * kr.sig[m]);
-    }
-    if (k < nz) {
-      const size_t m = cidx(d, i, j, k + 1);
-      const Row rm = row_of(d, m, i, j, k + 1, h);
-      ct = (float)(0.5 * (wn * r.g + kr.wgt[m] * rm.f) * sn * kr.sig[m]);
-    }
-    const size_t q = lq(kr, i, j, k);
-    kr.cr[q] = cr;
-    kr.cp[q] = cp;
-    kr.ct[q] = ct;
+    if (!staged) continue;
+    __syncthreads();
+    strip_out(kr, p, stage, kr.cr);
+    strip_out(kr, p, stage + one, kr.cp);
+    strip_out(kr, p, stage + 2 * one, kr.ct);
+    __syncthreads();
   }
 }
 
 // Reciprocal pivots of every radial line (diagonal 1, off-diagonal cr):
 // u_1 = 1, u_i = 1 - cr_{i-1}^2 / u_{i-1}; g = 1/u.  One thread per column;
 // FP32 (the factorisation only preconditions).
-__global__ void __launch_bounds__(kThreads) kry_factor_kernel(Kry kr, SolverDev* sol) {
-  for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < kr.ncol;
-       c += (long long)gridDim.x * blockDim.x) {
-    float g = 1.f, cprev = 0.f;
-    size_t q = (size_t)c;
-    for (int i = 0; i < kr.nx; ++i, q += kr.ncol) {
-      const float u = fmaf(-cprev * cprev, g, 1.f);
-      if (!(u > 0.f)) atomicExch(&sol->bad_weights, 1);
-      g = 1.f / u;
-      kr.g[q] = g;
-      cprev = kr.cr[q];
+__global__ void __launch_bounds__(32) kry_factor_kernel(Kry kr, SolverDev* sol) {
+  constexpr int U = 16;  // loads in flight: the recurrence waits one memory latency per 16 radii
+  const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= kr.ncol) return;
+  float g = 1.f, cprev = 0.f;
+  for (int i0 = 0; i0 < kr.nx; i0 += U) {
+    float cc[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) cc[u] = i0 + u < kr.nx ? kr.cr[(size_t)(i0 + u) * kr.ncol + c] : 0.f;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (i0 + u >= kr.nx) break;
+      const float piv = fmaf(-cprev * cprev, g, 1.f);
+      if (!(piv > 0.f)) atomicExch(&sol->bad_weights, 1);
+      g = 1.f / piv;
+      kr.g[(size_t)(i0 + u) * kr.ncol + c] = g;
+      cprev = cc[u];
     }
   }
 }
@@ -193,42 +253,58 @@ __global__ void __launch_bounds__(kThreads) kry_factor_kernel(Kry kr, SolverDev*
 template <bool L2, bool WITH_B>
 __global__ void __launch_bounds__(kThreads) kry_anchor_kernel(Dev d, Kry kr, const double* __restrict__ x,
                                                               const double* __restrict__ b, int hypre,
-                                                              double* partials, int nbmax) {
+                                                              double* partials, int nbmax, unsigned int strips,
+                                                              int staged) {
+  extern __shared__ float stage[];
   __shared__ double sh[32];
   __shared__ bool last;
   const int nx = d.nx, ny = d.ny;
-  const unsigned int n = (unsigned int)ncell(d);
   const size_t sj = (size_t)(nx + 4), sk = (size_t)(nx + 4) * (ny + 4);
   double s[4] = {0.0, 0.0, 0.0, 0.0};
-  for (unsigned int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-    int i, j, k;
-    cell_ijk(d, t, i, j, k);
-    const Row r = row_of(d, t, i, j, k, hypre != 0);
-    const size_t q = hidx(d, i, j, k);
-    const size_t qjm = (j == 1) ? hidx(d, i, ny, k) : q - sj;
-    const size_t qjp = (j == ny) ? hidx(d, i, 1, k) : q + sj;
-    const double bb = b_of(d, b, t, i, j, k, hypre != 0);
-    // a zero coupling contributes nothing, whatever the ghost it points at holds
-    double ax = r.a * x[q];
-    ax = fma(r.b, r.b != 0.0 ? x[q - 1] : 0.0, ax);
-    ax = fma(r.c, r.c != 0.0 ? x[q + 1] : 0.0, ax);
-    ax = fma(r.d, r.d != 0.0 ? x[qjm] : 0.0, ax);
-    ax = fma(r.e, r.e != 0.0 ? x[qjp] : 0.0, ax);
-    ax = fma(r.f, r.f != 0.0 ? x[q - sk] : 0.0, ax);
-    ax = fma(r.g, r.g != 0.0 ? x[q + sk] : 0.0, ax);
-    const double rr = bb - ax;
-    const double sw = kr.sig[t] * kr.wgt[t];
-    const double rs = sw * rr;
-    s[0] += fabs(rr);
-    if (L2) s[1] = fma(rs, rs, s[1]);
-    if (WITH_B) {
-      const double bs = sw * bb;
-      s[2] += fabs(hypre ? bb : b[t]);  // RHSNORM over every row (ppsor.f:33)
-      s[3] = fma(bs, bs, s[3]);
+  for (unsigned int m = blockIdx.x; m < strips; m += gridDim.x) {
+    const Strip p = strip_of(d, m);
+    for (unsigned int u = threadIdx.x; u < (unsigned int)(nx * p.cols); u += blockDim.x) {
+      unsigned int iu;
+      const int col = (int)div_rem(d.by_nx, u, iu), i = (int)iu + 1, j = p.j0 + col, k = p.k;
+      const size_t t = p.t0 + u;
+      const Row r = row_of(d, t, i, j, k, hypre != 0);
+      const size_t q = hidx(d, i, j, k);
+      const size_t qjm = (j == 1) ? hidx(d, i, ny, k) : q - sj;
+      const size_t qjp = (j == ny) ? hidx(d, i, 1, k) : q + sj;
+      const double bb = b_of(d, b, t, i, j, k, hypre != 0);
+      // a zero coupling contributes nothing, whatever the ghost it points at holds
+      double ax = r.a * x[q];
+      ax = fma(r.b, r.b != 0.0 ? x[q - 1] : 0.0, ax);
+      ax = fma(r.c, r.c != 0.0 ? x[q + 1] : 0.0, ax);
+      ax = fma(r.d, r.d != 0.0 ? x[qjm] : 0.0, ax);
+      ax = fma(r.e, r.e != 0.0 ? x[qjp] : 0.0, ax);
+      ax = fma(r.f, r.f != 0.0 ? x[q - sk] : 0.0, ax);
+      ax = fma(r.g, r.g != 0.0 ? x[q + sk] : 0.0, ax);
+      const double rr = bb - ax;
+      const double sw = mul_rn(kr.sig[t], kr.wgt[t]);
+      const double rs = mul_rn(sw, rr);
+      s[0] += fabs(rr);
+      if (L2) s[1] = fma(rs, rs, s[1]);
+      if (WITH_B) {
+        const double bs = mul_rn(sw, bb);
+        s[2] += fabs(hypre ? bb : b[t]);  // RHSNORM over every row (ppsor.f:33)
+        s[3] = fma(bs, bs, s[3]);
+      }
+      if (staged) {
+        stage[(int)iu * kStripPitch + col] = f32_rn(rs);
+      } else {
+        const size_t l = lq(kr, i, j, k);
+        kr.r[l] = f32_rn(rs);
+        kr.e[l] = 0.f;
+      }
     }
-    const size_t l = lq(kr, i, j, k);
-    kr.r[l] = (float)rs;
-    kr.e[l] = 0.f;
+    if (!staged) continue;
+    __syncthreads();
+    strip_out(kr, p, stage, kr.r);
+    if ((threadIdx.x & 31) < p.cols)
+      for (int i = threadIdx.x >> 5; i < nx; i += blockDim.x >> 5)
+        kr.e[(size_t)i * kr.ncol + (size_t)(p.k - 1) * ny + (size_t)(p.j0 - 1 + (threadIdx.x & 31))] = 0.f;
+    __syncthreads();
   }
   for (int m = 0; m < 4; ++m) {
     const double v = block_sum(s[m], sh);
@@ -256,32 +332,55 @@ __global__ void __launch_bounds__(kThreads) kry_anchor_kernel(Dev d, Kry kr, con
 }
 
 // x += Sigma e (x a halo array, e line-major).
-__global__ void __launch_bounds__(kThreads) kry_update_kernel(Dev d, Kry kr, double* x) {
-  const unsigned int n = (unsigned int)ncell(d);
-  for (unsigned int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-    int i, j, k;
-    cell_ijk(d, t, i, j, k);
-    x[hidx(d, i, j, k)] += kr.sig[t] * (double)kr.e[lq(kr, i, j, k)];
+__global__ void __launch_bounds__(kThreads) kry_update_kernel(Dev d, Kry kr, double* x, unsigned int strips, int staged) {
+  extern __shared__ float stage[];
+  const int nx = d.nx, lane = threadIdx.x & 31;
+  for (unsigned int m = blockIdx.x; m < strips; m += gridDim.x) {
+    const Strip p = strip_of(d, m);
+    if (staged) {
+      __syncthreads();
+      if (lane < p.cols)
+        for (int i = threadIdx.x >> 5; i < nx; i += blockDim.x >> 5)
+          stage[i * kStripPitch + lane] =
+              kr.e[(size_t)i * kr.ncol + (size_t)(p.k - 1) * kr.ny + (size_t)(p.j0 - 1 + lane)];
+      __syncthreads();
+    }
+    for (unsigned int u = threadIdx.x; u < (unsigned int)(nx * p.cols); u += blockDim.x) {
+      unsigned int iu;
+      const int col = (int)div_rem(d.by_nx, u, iu), i = (int)iu + 1, j = p.j0 + col;
+      const float e = staged ? stage[(int)iu * kStripPitch + col] : kr.e[lq(kr, i, j, p.k)];
+      x[hidx(d, i, j, p.k)] += mul_rn(kr.sig[p.t0 + u], f64_of_f32(e));
+    }
   }
 }
 
-// One radial line of the inner iteration for column c.  With UPDATE, first
-// r -= alpha s along the line.  Then z = T^-1 r by the factored tridiagonal
-// T (forward: y_i = r_i - cr_{i-1} g_{i-1} y_{i-1}, kept in z; backward:
-// z_i = (y_i - cr_i z_{i+1}) g_i).  Returns this line's share of r.z.  The
-// loads of kLineBatch radii are issued before any of their stores (the
-// compiler may not move a load above a store it cannot prove independent,
-// and a warp stalls at the first use of a pending load), so a pass waits
-// one memory latency per batch, not per radius.
+// Column m of colour C (0: (j+k) even, 1: odd) in the red-black order of
+// the columns; NY is even, so each theta row holds NY/2 of each colour.
+__device__ __forceinline__ long long col_of(long long m, int C, int ny) {
+  const long long half = ny >> 1;
+  const long long k0 = m / half;
+  const long long jj = m - k0 * half;
+  return k0 * ny + 2 * jj + ((k0 + C) & 1);
+}
+
+// One radial line of block Jacobi for column c, by one thread.  With UPDATE,
+// first r -= alpha s along the line.  Then z = T^-1 r by the factored
+// tridiagonal T (forward: y_i = r_i - cr_{i-1} g_{i-1} y_{i-1}; backward:
+// z_i = (y_i - cr_i z_{i+1}) g_i).  Returns this line's share of r.z, which is
+// sum y_i^2 g_i.  y waits in shared memory (SHARED: `y`, one value per radius
+// and thread), so that the backward pass reads two arrays and not four; where
+// NX is too long for that it waits in z.  The loads of kLineBatch radii are
+// issued before any of their stores (the compiler may not move a load above a
+// store it cannot prove independent, and a warp stalls at the first use of a
+// pending load), so a pass waits one memory latency per batch, not per radius.
 constexpr int kLineBatch = 16;
-template <bool UPDATE>
-__device__ __forceinline__ float line_pass(const Kry& k, long long c, float alpha) {
+template <bool UPDATE, bool SHARED>
+__device__ __forceinline__ float line_pass(const Kry& k, unsigned int c0, float alpha, float* y) {
   constexpr int U = kLineBatch;
   // 32-bit offsets (a context holds fewer than 2^31 cells per array)
   const unsigned int ncol = (unsigned int)k.ncol;
-  const unsigned int c0 = (unsigned int)c;
   const int nx = k.nx;
-  float yprev = 0.f, lprev = 0.f;
+  float yprev = 0.f, lprev = 0.f, dot = 0.f;
   for (int i0 = 0; i0 < nx; i0 += U) {
     const unsigned int qb = c0 + (unsigned int)i0 * ncol;
     float rr[U], cc[U], gg[U], ss[U];
@@ -304,26 +403,26 @@ __device__ __forceinline__ float line_pass(const Kry& k, long long c, float alph
           ri = fmaf(-alpha, ss[u], ri);
           k.r[q] = ri;
         }
-        const float y = fmaf(-lprev, yprev, ri);
-        k.z[q] = y;
+        const float v = fmaf(-lprev, yprev, ri);
+        if (SHARED) y[(i0 + u) * kJacobiThreads] = v;
+        else k.z[q] = v;
+        dot = fmaf(v * gg[u], v, dot);
         lprev = cc[u] * gg[u];
-        yprev = y;
+        yprev = v;
       }
     }
   }
-  float dot = 0.f;
   float znext = 0.f;
   for (int i1 = nx - 1; i1 >= 0; i1 -= U) {
     const unsigned int qb = c0 + (unsigned int)i1 * ncol;
-    float yy[U], cc[U], gg[U], rr[U];
+    float yy[U], cc[U], gg[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       if (i1 - u >= 0) {
         const unsigned int q = qb - (unsigned int)u * ncol;
-        yy[u] = k.z[q];
+        yy[u] = SHARED ? y[(i1 - u) * kJacobiThreads] : k.z[q];
         cc[u] = k.cr[q];
         gg[u] = k.g[q];
-        rr[u] = k.r[q];
       }
     }
 #pragma unroll
@@ -333,98 +432,174 @@ __device__ __forceinline__ float line_pass(const Kry& k, long long c, float alph
         const float zi = fmaf(-cc[u], znext, yy[u]) * gg[u];
         k.z[q] = zi;
         znext = zi;
-        dot = fmaf(rr[u], zi, dot);
       }
     }
   }
   return dot;
 }
 
-// One radial line of the red-black line Gauss-Seidel preconditioner for
-// column c (j0, k0): with UPDATE first r -= alpha s; then
-// z = T^-1 (r - the couplings to the four phi/theta neighbour columns, which
-// all have the other colour, times their z).  Returns r.z of the line.
-constexpr int kGsBatch = 4;
-template <bool UPDATE>
-__device__ __forceinline__ float line_gs(const Kry& k, long long c, float alpha) {
-  constexpr int U = kGsBatch;
-  const unsigned int ncol = (unsigned int)k.ncol;
-  const int nx = k.nx, ny = k.ny;
-  const int j0 = (int)(c % ny), k0 = (int)(c / ny);
-  const unsigned int c0 = (unsigned int)c;
-  // neighbour columns (theta neighbours outside the grid read column c with a zero coupling)
-  const unsigned int cjp = j0 == ny - 1 ? c0 - (ny - 1) : c0 + 1;
-  const unsigned int cjm = j0 == 0 ? c0 + (ny - 1) : c0 - 1;
-  const bool hkp = k0 + 1 < k.nz, hkm = k0 > 0;
-  const unsigned int ckp = hkp ? c0 + ny : c0, ckm = hkm ? c0 - ny : c0;
-  float yprev = 0.f, lprev = 0.f;
-  for (int i0 = 0; i0 < nx; i0 += U) {
-    const unsigned int qb = (unsigned int)i0 * ncol;
-    float rr[U], ss[U], cc[U], gg[U], nb[U];
+// Line Gauss-Seidel in tiles of kTileCols radial lines, a tile by a group of threads:
+// the group copies the lines to shared memory together (cp.async, everything
+// in flight at once), forms the right-hand sides there, and one lane per line
+// runs the recurrences on shared memory (forward y_i = b_i - cr_{i-1} g_{i-1}
+// y_{i-1}, backward z_i = (y_i - cr_i z_{i+1}) g_i).  What bounded a pass with
+// one thread per line on global memory was the memory latency per batch of
+// radii, with seven warps (32,768 columns) or one (the 4,096 of a colour of
+// 8,192) per SM.  A tile holds b (r), cr, g and s, each nx x kTileCols.
+// (Block Jacobi, whose tiles are many, is faster with one thread per line: two
+// tiles in flight per group take 205 KB of shared memory, and what L1 is left
+// then holds too few copies in flight, 27-44 us a pass at 100x256x128.)
+constexpr int kTileCols = 32;
+__device__ __forceinline__ void group_sync(int group, int threads) {
+  asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void copy_async4(float* to, const float* from) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned int)__cvta_generic_to_shared(to)), "l"(from)
+               : "memory");
+}
+// The threads of a group, and its tile (from value `at` on, in shared memory if
+// SHARED, else in `global`).
+struct Group {
+  int id, threads, tid;
+  unsigned int at;
+  float* global;
+};
+
+// The recurrences of one lane's line; NB: z takes its share of r.z with the
+// residual in the fourth array, else r.z = sum y_i^2 g_i.  Shared memory is
+// read in batches of R radii before the batch's first write (the compiler
+// cannot tell the arrays apart itself, and would wait for each read).
+// Not inlined: among the other passes' live registers the recurrences were
+// scheduled read by read, 60 clocks a radius instead of 12.
+template <bool NB, bool SHARED>
+__device__ __noinline__ float solve_line(int nx, unsigned int ncol, float* z, float* global, unsigned int at, int lane,
+                                         bool valid, unsigned int c0) {
+  constexpr int R = 8;
+  float* tile = SHARED ? tile_sh + at : global + at;
+  float *sb = tile + lane, *sc = sb + nx * kTileCols, *sg = sc + nx * kTileCols, *sr = sg + nx * kTileCols;
+  float dot = 0.f, yprev = 0.f, lprev = 0.f;
+  int i = 0;
+  for (; i + R <= nx; i += R) {
+    float bb[R], cc[R], gg[R];
+#pragma unroll
+    for (int u = 0; u < R; ++u) {
+      bb[u] = sb[(i + u) * kTileCols];
+      cc[u] = sc[(i + u) * kTileCols];
+      gg[u] = sg[(i + u) * kTileCols];
+    }
+#pragma unroll
+    for (int u = 0; u < R; ++u) {
+      bb[u] = fmaf(-lprev, yprev, bb[u]);
+      if (!NB) dot = fmaf(bb[u] * gg[u], bb[u], dot);
+      lprev = cc[u] * gg[u];
+      yprev = bb[u];
+    }
+#pragma unroll
+    for (int u = 0; u < R; ++u) sb[(i + u) * kTileCols] = bb[u];
+  }
+  for (; i < nx; ++i) {
+    const float g = sg[i * kTileCols], y = fmaf(-lprev, yprev, sb[i * kTileCols]);
+    sb[i * kTileCols] = y;
+    if (!NB) dot = fmaf(y * g, y, dot);
+    lprev = sc[i * kTileCols] * g;
+    yprev = y;
+  }
+  float znext = 0.f;
+  for (i = nx - 1; i >= R - 1; i -= R) {
+    float bb[R], cc[R], gg[R], rr[R];
+#pragma unroll
+    for (int u = 0; u < R; ++u) {
+      bb[u] = sb[(i - u) * kTileCols];
+      cc[u] = sc[(i - u) * kTileCols];
+      gg[u] = sg[(i - u) * kTileCols];
+      if (NB) rr[u] = sr[(i - u) * kTileCols];
+    }
+#pragma unroll
+    for (int u = 0; u < R; ++u) {
+      znext = fmaf(-cc[u], znext, bb[u]) * gg[u];
+      if (NB) dot = fmaf(rr[u], znext, dot);
+      if (valid) z[(unsigned int)(i - u) * ncol + c0] = znext;
+    }
+  }
+  for (; i >= 0; --i) {
+    znext = fmaf(-sc[i * kTileCols], znext, sb[i * kTileCols]) * sg[i * kTileCols];
+    if (NB) dot = fmaf(sr[i * kTileCols], znext, dot);
+    if (valid) z[(unsigned int)i * ncol + c0] = znext;
+  }
+  return valid ? dot : 0.f;
+}
+
+// One tile of lines of one colour (line `col` of this lane).  NB: the couplings
+// to the four phi/theta neighbour columns, which all have the other colour,
+// times their z are taken off the right-hand side (the red-black line
+// Gauss-Seidel step).  Returns this thread's share of r.z.
+template <bool UPDATE, bool NB, bool SHARED>
+__device__ __forceinline__ float colour_lines(const Kry& k, const Group& g, long long col, bool valid, float alpha) {
+  constexpr int U = 4;
+  const int W = g.threads >> 5, nx = k.nx, lane = threadIdx.x & 31, warp = g.tid >> 5;
+  // 32-bit offsets (a context holds fewer than 2^31 cells per array)
+  const unsigned int ncol = (unsigned int)k.ncol, c0 = (unsigned int)(valid ? col : 0);
+  float* tile = SHARED ? tile_sh + g.at : g.global + g.at;
+  float *sb = tile + lane, *sc = sb + nx * kTileCols, *sg = sc + nx * kTileCols, *sr = sg + nx * kTileCols;
+  unsigned int cjp = c0, cjm = c0, ckp = c0, ckm = c0;
+  bool hkm = false;
+  if (NB) {  // theta neighbours outside the grid read column c0 with a zero coupling
+    const unsigned int ny = (unsigned int)k.ny, k0 = c0 / ny, j0 = c0 - k0 * ny;
+    cjp = j0 == ny - 1 ? c0 - (ny - 1) : c0 + 1;
+    cjm = j0 == 0 ? c0 + (ny - 1) : c0 - 1;
+    hkm = k0 > 0;
+    if ((int)k0 + 1 < k.nz) ckp = c0 + ny;
+    if (hkm) ckm = c0 - ny;
+  }
+  group_sync(g.id, g.threads);  // the tile before this one is solved
+  // each thread copies the values that it alone reads back
+  for (int i = warp; i < nx; i += W) {
+    const unsigned int q = (unsigned int)i * ncol + c0;
+    const int o = i * kTileCols;
+    if (SHARED) {
+      copy_async4(sb + o, k.r + q);
+      if (UPDATE) copy_async4(sr + o, k.s + q);
+      copy_async4(sc + o, k.cr + q);
+      copy_async4(sg + o, k.g + q);
+    } else {
+      sb[o] = k.r[q];
+      if (UPDATE) sr[o] = k.s[q];
+      sc[o] = k.cr[q];
+      sg[o] = k.g[q];
+    }
+  }
+  bool waited = false;
+  for (int i0 = warp; i0 < nx; i0 += W * U) {
+    float nb[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      if (i0 + u < nx) {
-        const unsigned int o = qb + (unsigned int)u * ncol;
-        rr[u] = k.r[o + c0];
-        if (UPDATE) ss[u] = k.s[o + c0];
-        cc[u] = k.cr[o + c0];
-        gg[u] = k.g[o + c0];
+      const int i = i0 + W * u;
+      nb[u] = 0.f;
+      if (NB && i < nx) {
+        const unsigned int o = (unsigned int)i * ncol;
         const float ctm = hkm ? k.ct[o + ckm] : 0.f;
         nb[u] = fmaf(k.cp[o + c0], k.z[o + cjp],
                 fmaf(k.cp[o + cjm], k.z[o + cjm], fmaf(k.ct[o + c0], k.z[o + ckp], ctm * k.z[o + ckm])));
       }
     }
+    if (!waited) asm volatile("cp.async.wait_all;" ::: "memory");
+    waited = true;
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      if (i0 + u < nx) {
-        const unsigned int q = qb + (unsigned int)u * ncol + c0;
-        float ri = rr[u];
+      const int i = i0 + W * u, o = i * kTileCols;
+      if (i < nx) {
+        float ri = sb[o];
         if (UPDATE) {
-          ri = fmaf(-alpha, ss[u], ri);
-          k.r[q] = ri;
+          ri = fmaf(-alpha, sr[o], ri);
+          if (valid) k.r[(unsigned int)i * ncol + c0] = ri;
         }
-        const float y = fmaf(-lprev, yprev, ri - nb[u]);
-        k.z[q] = y;
-        lprev = cc[u] * gg[u];
-        yprev = y;
+        if (NB) sr[o] = ri;
+        sb[o] = NB ? ri - nb[u] : ri;
       }
     }
   }
-  float dot = 0.f, znext = 0.f;
-  for (int i1 = nx - 1; i1 >= 0; i1 -= U) {
-    const unsigned int qb = c0 + (unsigned int)i1 * ncol;
-    float yy[U], cc[U], gg[U], rr[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      if (i1 - u >= 0) {
-        const unsigned int q = qb - (unsigned int)u * ncol;
-        yy[u] = k.z[q];
-        cc[u] = k.cr[q];
-        gg[u] = k.g[q];
-        rr[u] = k.r[q];
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      if (i1 - u >= 0) {
-        const unsigned int q = qb - (unsigned int)u * ncol;
-        const float zi = fmaf(-cc[u], znext, yy[u]) * gg[u];
-        k.z[q] = zi;
-        znext = zi;
-        dot = fmaf(rr[u], zi, dot);
-      }
-    }
-  }
-  return dot;
-}
-
-// Column m of colour C (0: (j+k) even, 1: odd) in the red-black order of
-// the columns; NY is even, so each theta row holds NY/2 of each colour.
-__device__ __forceinline__ long long col_of(long long m, int C, int ny) {
-  const long long half = ny >> 1;
-  const long long k0 = m / half;
-  const long long jj = m - k0 * half;
-  return k0 * ny + 2 * jj + ((k0 + C) & 1);
+  group_sync(g.id, g.threads);
+  return g.tid < 32 ? solve_line<NB, SHARED>(nx, ncol, k.z, g.global, g.at, lane, valid, c0) : 0.f;
 }
 
 __device__ __forceinline__ float4 ldf4(const float* p) { return *reinterpret_cast<const float4*>(p); }
@@ -520,33 +695,40 @@ __device__ __forceinline__ float op_one(const Kry& k, const float* po, float* pn
 // preconditioner; otherwise the radial line solve of every column (block
 // Jacobi).  acc gains this thread's share of r.z (from each colour's last
 // pass).  False if a barrier gave up.
-template <bool UPDATE, bool SGS>
-__device__ __forceinline__ bool precondition(const Kry& k, SolverDev* sol, unsigned int nb, long long col0,
-                                             long long colstride, float alpha, float& acc, int sweeps,
-                                             unsigned long long& passed) {
-  if (!SGS) {
-    for (long long c = col0; c < k.ncol; c += colstride) acc += line_pass<UPDATE>(k, c, alpha);
+template <bool UPDATE, bool SGS, bool SHARED>
+__device__ __forceinline__ bool precondition(const Kry& k, SolverDev* sol, unsigned int nb, float alpha, float& acc,
+                                             int sweeps, unsigned long long& passed, const Group& g) {
+  if (!SGS) {  // the warps of all blocks take groups of 32 neighbouring columns in turn
+    const long long stride = (long long)(blockDim.x >> 5) * nb * 32;
+    for (long long c = ((long long)(threadIdx.x >> 5) * nb + blockIdx.x) * 32 + (threadIdx.x & 31); c < k.ncol; c += stride)
+      acc += line_pass<UPDATE, SHARED>(k, (unsigned int)c, alpha, tile_sh + threadIdx.x);
     return true;
   }
+  // tiles are dealt to the blocks first, then to the groups of a block
+  const int groups = (int)blockDim.x / g.threads, lane = threadIdx.x & 31;
+  const long long first = (long long)g.id * nb + blockIdx.x, step = (long long)groups * nb;
   const long long half = k.ncol >> 1;
-  for (long long m = col0; m < half; m += colstride) (void)line_pass<UPDATE>(k, col_of(m, 0, k.ny), alpha);
+  for (long long m0 = first * kTileCols; m0 < half; m0 += step * kTileCols)
+    (void)colour_lines<UPDATE, false, SHARED>(k, g, col_of(m0 + lane, 0, k.ny), m0 + lane < half, alpha);
   if (!grid_sync(sol, nb, passed)) return false;
   float ab = 0.f;  // r.z of the black lines' first pass (their last with one sweep)
-  for (long long m = col0; m < half; m += colstride) ab += line_gs<UPDATE>(k, col_of(m, 1, k.ny), alpha);
+  for (long long m0 = first * kTileCols; m0 < half; m0 += step * kTileCols)
+    ab += colour_lines<UPDATE, true, SHARED>(k, g, col_of(m0 + lane, 1, k.ny), m0 + lane < half, alpha);
   if (sweeps == 1) acc += ab;
 #pragma unroll 1
   for (int p = 2; p <= 2 * sweeps; ++p) {
     if (!grid_sync(sol, nb, passed)) return false;
     float ap = 0.f;
-    for (long long m = col0; m < half; m += colstride) ap += line_gs<false>(k, col_of(m, p & 1, k.ny), 0.f);
+    for (long long m0 = first * kTileCols; m0 < half; m0 += step * kTileCols)
+      ap += colour_lines<false, true, SHARED>(k, g, col_of(m0 + lane, p & 1, k.ny), m0 + lane < half, 0.f);
     if (p >= 2 * sweeps - 1) acc += ap;  // the last pass of its colour
   }
   return true;
 }
 
 // The FP32 PCG iteration on S e = r from e = 0 (r, e set by the anchor).
-// Line phases: the warps of all blocks are dealt round-robin over groups of
-// 32 consecutive columns.  Operator phase: p_new = z + beta p (p read from
+// Line phases: tiles of 32 columns, dealt to the groups of threads of all
+// blocks.  Operator phase: p_new = z + beta p (p read from
 // p[cur], written to p[1-cur], so that neighbours read the old values),
 // s = S p_new, and the previous iteration's e += alpha p.  Every block forms
 // alpha and beta from all block partials in the same fixed order, so all
@@ -555,39 +737,33 @@ __device__ __forceinline__ bool precondition(const Kry& k, SolverDev* sol, unsig
 // FP32 floor), on a non-positive p.s, or after maxit iterations; the last
 // iteration's e update is then applied.  maxit = 0 only computes r0.z0
 // (sol->scratch[2]).
-template <bool SGS>
-__global__ void __launch_bounds__(kPcgThreads, 1) pcg32_persistent(Kry k, SolverDev* sol, double* partials,
-                                                                   int maxit, double stop_ratio, int sweeps) {
-  __shared__ double sh[32];
-  __shared__ double bc[3];
+template <bool SGS, bool SHARED>
+__global__ void __launch_bounds__(SGS ? kGsThreads : kJacobiThreads, 1) pcg32_persistent(Kry k, SolverDev* sol, double* partials,
+                                                                   int maxit, double stop_ratio, int sweeps,
+                                                                   float* tiles, int groups) {
+  __shared__ double sh[33];
   const unsigned int nb = gridDim.x;
+  const int it0 = sol->iter;
   unsigned long long passed = 0;  // grid barriers this block has passed
   const long long n = k.n;
   const int ny = k.ny;
   const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long nth = (long long)gridDim.x * blockDim.x;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long long col0 = ((long long)warp * nb + blockIdx.x) * 32 + lane;
-  const long long colstride = (long long)(blockDim.x >> 5) * nb * 32;
-  double* pa = partials;                 // operator-phase partials
-  double* pb = partials + kMaxPartials;  // line-phase partials
+  Group g;
+  g.threads = (int)blockDim.x / groups;
+  g.id = (int)threadIdx.x / g.threads;
+  g.tid = (int)threadIdx.x - g.id * g.threads;
+  const unsigned int len = 4u * (unsigned int)k.nx * kTileCols;
+  g.at = (unsigned int)g.id * len;
+  g.global = SHARED ? nullptr : tiles + (size_t)blockIdx.x * groups * len;
 
   // z0 = T^-1 r0, gamma0 = r0.z0.  Per-thread partial sums (a few hundred
   // terms) are FP32 -- GB300's FP64 pipe is narrow -- and widened to FP64
   // for the block and grid sums.
   float acc = 0.f;
-  if (!precondition<false, SGS>(k, sol, nb, col0, colstride, 0.f, acc, sweeps, passed)) return;
-  {
-    const double v = block_sum((double)acc, sh);
-    if (threadIdx.x == 0) pb[blockIdx.x] = v;
-  }
-  if (!grid_sync(sol, nb, passed)) return;
-  {
-    const double tot = block_sum_array(pb, nb, sh);
-    if (threadIdx.x == 0) bc[0] = tot;
-    __syncthreads();
-  }
-  double gamma = bc[0];
+  if (!precondition<false, SGS, SHARED>(k, sol, nb, 0.f, acc, sweeps, passed, g)) return;
+  double gamma;
+  if (!grid_sum(sol, nb, passed, (double)acc, partials, sh, gamma)) return;
   const double gamma0 = gamma;
   if (blockIdx.x == 0 && threadIdx.x == 0) sol->scratch[2] = gamma0;
   if (maxit <= 0 || !(gamma0 > 0.0) || !isfinite(gamma0)) {
@@ -612,17 +788,8 @@ __global__ void __launch_bounds__(kPcgThreads, 1) pcg32_persistent(Kry k, Solver
       for (long long q = tid; q < n; q += nth) acc += op_one(k, po, pn, beta, ap, q);
     }
     pending = false;
-    {
-      const double v = block_sum((double)acc, sh);
-      if (threadIdx.x == 0) pa[blockIdx.x] = v;
-    }
-    if (!grid_sync(sol, nb, passed)) return;
-    {
-      const double tot = block_sum_array(pa, nb, sh);
-      if (threadIdx.x == 0) bc[1] = tot;
-      __syncthreads();
-    }
-    const double ps = bc[1];
+    double ps;
+    if (!grid_sum(sol, nb, passed, (double)acc, partials, sh, ps)) return;
     if (!(ps > 0.0) || !isfinite(ps)) {  // breakdown: S p_new not positive (rounding)
       if (blockIdx.x == 0 && threadIdx.x == 0) {
         sol->stalled = 1;
@@ -633,22 +800,13 @@ __global__ void __launch_bounds__(kPcgThreads, 1) pcg32_persistent(Kry k, Solver
     const float alpha = (float)(gamma / ps);
     // line phase: r -= alpha s, z = M^-1 r, r.z
     acc = 0.f;
-    if (!precondition<true, SGS>(k, sol, nb, col0, colstride, alpha, acc, sweeps, passed)) return;
-    {
-      const double v = block_sum((double)acc, sh);
-      if (threadIdx.x == 0) pb[blockIdx.x] = v;
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) sol->iter += 1;
+    if (!precondition<true, SGS, SHARED>(k, sol, nb, alpha, acc, sweeps, passed, g)) return;
     alpha_prev = alpha;
     pending = true;
     cur = 1 - cur;  // p[cur] is now this iteration's p
-    if (!grid_sync(sol, nb, passed)) return;
-    {
-      const double tot = block_sum_array(pb, nb, sh);
-      if (threadIdx.x == 0) bc[2] = tot;
-      __syncthreads();
-    }
-    const double gnew = bc[2];
+    double gnew;
+    if (!grid_sum(sol, nb, passed, (double)acc, partials, sh, gnew)) return;
+    if (blockIdx.x == 0 && threadIdx.x == 0) sol->iter = it0 + it;
     if (!isfinite(gnew)) {
       if (blockIdx.x == 0 && threadIdx.x == 0) sol->nonfinite = 1;
       break;
@@ -713,29 +871,66 @@ int poll_sol(ttfld_ctx* c) {
   return 0;
 }
 
-int pcg_blocks(long long ncells) {
-  static int blocks = -1;
-  if (blocks < 0) {
-    int dev = 0, sms = 0, per_sm = 0, coop = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    int per_sm_gs = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pcg32_persistent<false>, kPcgThreads, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_gs, pcg32_persistent<true>, kPcgThreads, 0);
-    if (per_sm_gs < per_sm) per_sm = per_sm_gs;
-    long long b = coop ? (long long)sms * per_sm : 0;
-    blocks = (int)(b > kMaxPartials ? kMaxPartials : b);
+// Launch shape of the PCG kernel, one block per SM.  Line Gauss-Seidel: a
+// colour has few tiles, and what they wait for is the reads of their
+// neighbours, so a block has as many groups as it has tiles, up to three and
+// to what fits in shared memory; a line too long for that (NX > 440) keeps its
+// tile in global memory.  Block Jacobi: the forward results of a line wait in
+// shared memory up to kJacobiShared, beyond which L1 would get too small for
+// the loads in flight.
+constexpr size_t kJacobiShared = 168 * 1024;
+struct PcgShape {
+  int blocks, threads, groups;
+  size_t smem;
+  bool shared;
+};
+const void* pcg_kernel(bool gs, bool shared) {
+  if (shared) return gs ? (const void*)pcg32_persistent<true, true> : (const void*)pcg32_persistent<false, true>;
+  return gs ? (const void*)pcg32_persistent<true, false> : (const void*)pcg32_persistent<false, false>;
+}
+PcgShape pcg_shape(const Kry& k, bool gs) {
+  int dev = 0, sms = 0, coop = 0, room = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  cudaDeviceGetAttribute(&room, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  PcgShape p{0, gs ? kGsThreads : kJacobiThreads, 1, 0, false};
+  if (!coop || sms <= 0) return p;
+  if (gs) {
+    const size_t tile = (size_t)4 * k.nx * kTileCols * sizeof(float);
+    const int fit = (int)(((size_t)room - 1024) / tile);
+    p.shared = fit > 0;
+    if (p.shared) {
+      const long long tiles = (k.ncol / 2 + kTileCols - 1) / kTileCols, per = (tiles + sms - 1) / sms;
+      p.groups = per < 3 ? (int)per : 3;
+      if (p.groups > fit) p.groups = fit;
+      p.smem = (size_t)p.groups * tile;
+    }
+  } else {
+    const size_t y = (size_t)k.nx * kJacobiThreads * sizeof(float);
+    p.shared = y <= kJacobiShared;
+    p.smem = p.shared ? y : 0;
   }
-  const long long need = (ncells + kPcgThreads - 1) / kPcgThreads;
-  return (int)(need < blocks ? need : blocks);
+  const void* kern = pcg_kernel(gs, p.shared);
+  int per_sm = 0;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, p.threads, p.smem) != cudaSuccess || per_sm < 1) {
+    cudaGetLastError();
+    return p;
+  }
+  const long long need = (k.n + 255) / 256;
+  p.blocks = (int)(need < sms ? need : sms);
+  if (p.blocks > kMaxPartials) p.blocks = kMaxPartials;
+  return p;
 }
 
 // One inner run; returns its iterations in *its.
 // gs: 0 block-Jacobi radial lines, m >= 1 m symmetric line Gauss-Seidel sweeps.
 int launch_inner(ttfld_ctx* c, KryWork* w, int maxit, double stop_ratio, int gs, int* its) {
-  const int nb = pcg_blocks(w->k.n);
-  if (nb <= 0) {
+  const PcgShape shape = pcg_shape(w->k, gs > 0);
+  if (shape.blocks > 0 && gs > 0 && !shape.shared && !w->tiles)
+    TT_CHECK(cudaMalloc((void**)&w->tiles, (size_t)shape.blocks * 4 * w->k.nx * kTileCols * sizeof(float)));
+  if (shape.blocks <= 0) {
     fprintf(stderr, "ttfld: the PCG solver needs cooperative launch\n");
     return TTFLD_E_UNSUPPORTED;
   }
@@ -747,10 +942,12 @@ int launch_inner(ttfld_ctx* c, KryWork* w, int maxit, double stop_ratio, int gs,
   SolverDev* sol = c->sol;
   double* partials = c->partials;
   int sweeps = gs > 0 ? gs : 1;
-  void* args[] = {&k, &sol, &partials, &maxit, &stop_ratio, &sweeps};
-  const void* kern = gs > 0 ? (const void*)pcg32_persistent<true> : (const void*)pcg32_persistent<false>;
+  float* tiles = w->tiles;
+  int groups = shape.groups;
+  void* args[] = {&k, &sol, &partials, &maxit, &stop_ratio, &sweeps, &tiles, &groups};
+  const void* kern = pcg_kernel(gs > 0, shape.shared);
   TT_CHECK(cudaMemsetAsync(&sol->arrivals, 0, sizeof(unsigned long long), c->stream));  // grid barrier
-  TT_CHECK(cudaLaunchCooperativeKernel(kern, dim3(nb), dim3(kPcgThreads), args, 0, c->stream));
+  TT_CHECK(cudaLaunchCooperativeKernel(kern, dim3(shape.blocks), dim3(shape.threads), args, shape.smem, c->stream));
   count_launches(1);
   int rc = poll_sol(c);
   if (rc) return rc;
@@ -759,16 +956,43 @@ int launch_inner(ttfld_ctx* c, KryWork* w, int maxit, double stop_ratio, int gs,
   return 0;
 }
 
-int anchor(ttfld_ctx* c, KryWork* w, const double* x, const double* b, bool hypre, bool l2, bool with_b) {
-  const int nb = grid_cells(w->k.n);
-  const int h = hypre ? 1 : 0;
-  if (l2 && with_b) kry_anchor_kernel<true, true><<<nb, kThreads, 0, c->stream>>>(c->d, w->k, x, b, h, c->partials, 1024);
-  else if (l2) kry_anchor_kernel<true, false><<<nb, kThreads, 0, c->stream>>>(c->d, w->k, x, b, h, c->partials, 1024);
-  else if (with_b) kry_anchor_kernel<false, true><<<nb, kThreads, 0, c->stream>>>(c->d, w->k, x, b, h, c->partials, 1024);
-  else kry_anchor_kernel<false, false><<<nb, kThreads, 0, c->stream>>>(c->d, w->k, x, b, h, c->partials, 1024);
+// The strips of a grid, the blocks that walk them, and the shared memory of
+// `arrays` staged strips (0 and not staged where NX is too long for 200 KB).
+struct StripShape {
+  unsigned int strips;
+  int blocks, staged;
+  size_t smem;
+};
+StripShape strip_shape(const Kry& k, const void* kernel, int arrays) {
+  StripShape s;
+  s.strips = (unsigned int)k.nz * (((unsigned int)k.ny + kStripCols - 1) / kStripCols);
+  s.blocks = s.strips < 1024 ? (int)s.strips : 1024;
+  s.smem = (size_t)arrays * k.nx * kStripPitch * sizeof(float);
+  s.staged = s.smem <= 200 * 1024;
+  if (s.staged && s.smem > 48 * 1024 &&
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.smem) != cudaSuccess) {
+    cudaGetLastError();
+    s.staged = 0;
+  }
+  if (!s.staged) s.smem = 0;
+  return s;
+}
+
+template <bool L2, bool WITH_B>
+int launch_anchor(ttfld_ctx* c, KryWork* w, const double* x, const double* b, int h) {
+  const StripShape s = strip_shape(w->k, (const void*)kry_anchor_kernel<L2, WITH_B>, 1);
+  kry_anchor_kernel<L2, WITH_B><<<s.blocks, kThreads, s.smem, c->stream>>>(c->d, w->k, x, b, h, c->partials, 1024,
+                                                                           s.strips, s.staged);
   count_launches(1);
   TT_CHECK_LAUNCH();
-  return poll_sol(c);
+  return 0;
+}
+
+int anchor(ttfld_ctx* c, KryWork* w, const double* x, const double* b, bool hypre, bool l2, bool with_b) {
+  const int h = hypre ? 1 : 0;
+  const int rc = l2 ? (with_b ? launch_anchor<true, true>(c, w, x, b, h) : launch_anchor<true, false>(c, w, x, b, h))
+                    : (with_b ? launch_anchor<false, true>(c, w, x, b, h) : launch_anchor<false, false>(c, w, x, b, h));
+  return rc ? rc : poll_sol(c);
 }
 
 // Factor the system (weights, couplings, line pivots).
@@ -776,8 +1000,9 @@ int prepare(ttfld_ctx* c, KryWork* w, bool hypre) {
   const int nb = grid_cells(w->k.n);
   TT_CHECK(cudaMemsetAsync(&c->sol->bad_weights, 0, sizeof(int), c->stream));
   kry_weights_kernel<<<nb, kThreads, 0, c->stream>>>(c->d, w->k, hypre ? 1 : 0);
-  kry_couplings_kernel<<<nb, kThreads, 0, c->stream>>>(c->d, w->k, hypre ? 1 : 0);
-  kry_factor_kernel<<<grid_cells(w->k.ncol), kThreads, 0, c->stream>>>(w->k, c->sol);
+  const StripShape s = strip_shape(w->k, (const void*)kry_couplings_kernel, 3);
+  kry_couplings_kernel<<<s.blocks, kThreads, s.smem, c->stream>>>(c->d, w->k, hypre ? 1 : 0, s.strips, s.staged);
+  kry_factor_kernel<<<(unsigned int)((w->k.ncol + 31) / 32), 32, 0, c->stream>>>(w->k, c->sol);
   count_launches(3);
   TT_CHECK_LAUNCH();
   return 0;
@@ -849,7 +1074,8 @@ int pcg_core(ttfld_ctx* c, double* x, const double* b, bool hypre, double tol, l
     total += its;
     ++anchors;
     if (c->host_sol->stalled) ++stalls;
-    kry_update_kernel<<<grid_cells(w->k.n), kThreads, 0, c->stream>>>(c->d, w->k, x);
+    const StripShape up = strip_shape(w->k, (const void*)kry_update_kernel, 1);
+    kry_update_kernel<<<up.blocks, kThreads, up.smem, c->stream>>>(c->d, w->k, x, up.strips, up.staged);
     count_launches(1);
     TT_CHECK_LAUNCH();
     if ((rc = anchor(c, w, x, b, hypre, l2, false))) return rc;
@@ -882,6 +1108,7 @@ void krylov_free(ttfld_ctx* c) {
   KryWork* w = (KryWork*)c->krylov;
   if (!w) return;
   if (w->mem) cudaFree(w->mem);
+  if (w->tiles) cudaFree(w->tiles);
   free(w);
   c->krylov = nullptr;
 }
