@@ -21,8 +21,8 @@
 // B = weights of one tap).  Activations are channels-last BF16 (voxel-major,
 // channels contiguous), so an A fragment row is one voxel's channels.
 // Backward-data is the same kernel on flipped, transposed weights; the weight
-// gradient is a GEMM over voxels (A = gradient^T, B = shifted input) reduced
-// with FP32 atomics (so training is not bitwise reproducible; inference is).
+// gradient is a GEMM over voxels (A = gradient^T, B = shifted input) whose
+// chunks are added in a fixed order (so training is bitwise reproducible).
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <math.h>
@@ -76,8 +76,10 @@ struct Net {
   float *pred_half, *gpred_half;   // network output on level 0
   float *pred, *gpred, *target;    // on the grid, one channel
   unsigned char* mask;             // active cells of the grid
-  double* loss_acc;
+  double* loss_acc;            // the loss, then the count of active cells
   void* act_mem;
+  void* grad_mem;              // gradient workspace (first training call)
+  float* feat_stage;           // features on the grid (first call with host features)
   // dataset (captured pairs)
   int cap, count, capture_next;
   bf16* ds_feat;       // [cap][level-0 vox][kFeatPad] pooled features
@@ -762,20 +764,37 @@ struct WgradArgs {
   long long chunk;      // voxels per warp (multiple of 16)
 };
 
-__device__ __forceinline__ long long shifted(long long v, int X, int Y, int Z, int dx, int dy, int dz) {
-  const int x = (int)(v % X);
-  const int y = (int)((v / X) % Y);
-  const int z = (int)(v / ((long long)X * Y));
-  const int xx = x + dx, zz = z + dz;
-  if (xx < 0 || xx >= X || zz < 0 || zz >= Z) return -1;
-  int yy = y + dy;
-  yy = yy < 0 ? yy + Y : (yy >= Y ? yy - Y : yy);
-  return ((long long)zz * Y + yy) * X + xx;
+// The voxel shifted by the tap, or -1 outside (zero padding in r and theta,
+// periodic phi).
+__device__ __forceinline__ int shifted(unsigned int v, unsigned int X, unsigned int Y, unsigned int Z, int dx, int dy,
+                                       int dz) {
+  const unsigned int row = v / X, z = row / Y;
+  const int xx = (int)(v - row * X) + dx, zz = (int)z + dz;
+  if (xx < 0 || xx >= (int)X || zz < 0 || zz >= (int)Z) return -1;
+  int yy = (int)(row - z * Y) + dy;
+  yy = yy < 0 ? yy + (int)Y : (yy >= (int)Y ? yy - (int)Y : yy);
+  return (zz * (int)Y + yy) * (int)X + xx;
 }
 
+// Both operands of a 16-voxel step are read 16 bytes (8 channels) a lane, one
+// step ahead, and go through shared memory: voxel-major rows there, which
+// ldmatrix.trans turns into the fragments (A row = output channel, B column =
+// input channel, voxels along k).  Reading the fragments' elements straight
+// from global memory took 8 + 4 NB two-byte loads a lane and step: 88-122 us a
+// level-0 layer at 64x128x64, 23-31 us with the rows.
+__device__ __forceinline__ void ldmatrix4_trans(uint32_t* r, const bf16* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"((uint32_t)__cvta_generic_to_shared(p))
+               : "memory");
+}
 template <int NB>
 __global__ void __launch_bounds__(256) conv3_wgrad_kernel(WgradArgs a) {
-  const int lane = threadIdx.x & 31;
+  constexpr int ZP = 16 + 8, XP = NB * 8 + 8;  // row pitches (16-byte rows fall on other banks)
+  constexpr int XU = (16 * NB + 31) / 32;      // 16-byte units of x a lane reads per step
+  __shared__ __align__(16) bf16 zs[8][16 * ZP];
+  __shared__ __align__(16) bf16 xs[8][16 * XP];
+  const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
   const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long V = (long long)a.X * a.Y * a.Z;
   const long long nchunks = (V + a.chunk - 1) / a.chunk;
@@ -787,34 +806,52 @@ __global__ void __launch_bounds__(256) conv3_wgrad_kernel(WgradArgs a) {
   const long long ck = warp / (27LL * cot);
   const int dz = tap / 9 - 1, dy = (tap / 3) % 3 - 1, dx = tap % 3 - 1;
   const int r = lane >> 2, cq = (lane & 3) * 2;
-  const int co = ct * 16 + r;
   float acc[NB][4];
 #pragma unroll
   for (int nb = 0; nb < NB; ++nb) acc[nb][0] = acc[nb][1] = acc[nb][2] = acc[nb][3] = 0.f;
-  const bf16 zero = __float2bfloat16_rn(0.f);
-  const long long v_end = min(V, (ck + 1) * a.chunk);
-  for (long long v0 = ck * a.chunk; v0 < v_end; v0 += 16) {
-    long long vv[4] = {v0 + cq, v0 + cq + 1, v0 + cq + 8, v0 + cq + 9};
-    bf16 za[4], zb[4];
-    long long sv[4];
+  const unsigned int v_end = (unsigned int)min(V, (ck + 1) * a.chunk);
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  uint4 zr, xr[XU];
+  auto fetch = [&](unsigned int v0) {
+    // lane q < 16: the shifted voxel of step row q; every lane reads units of rows
+    const unsigned int vq = v0 + (lane & 15);
+    const int sq = vq < v_end ? shifted(vq, a.X, a.Y, a.Z, dx, dy, dz) : -1;
+    const unsigned int vz = v0 + (lane >> 1);
+    zr = vz < v_end ? *reinterpret_cast<const uint4*>(a.dz + (size_t)vz * a.dz_cs + a.dz_co + ct * 16 + (lane & 1) * 8)
+                    : zero;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const bool in = vv[q] < v_end;
-      za[q] = in ? a.dz[(size_t)vv[q] * a.dz_cs + a.dz_co + co] : zero;
-      zb[q] = in ? a.dz[(size_t)vv[q] * a.dz_cs + a.dz_co + co + 8] : zero;
-      sv[q] = in ? shifted(vv[q], a.X, a.Y, a.Z, dx, dy, dz) : -1;
+    for (int m = 0; m < XU; ++m) {
+      const int u = lane + 32 * m, row = u / NB, part = u - row * NB;
+      const int sv = __shfl_sync(0xffffffffu, sq, row & 15);
+      xr[m] = u < 16 * NB && sv >= 0
+                  ? *reinterpret_cast<const uint4*>(a.x + (size_t)sv * a.x_cs + a.x_co + part * 8)
+                  : zero;
     }
-    // A fragment (row = co, col = voxel): a0 (r, cq..cq+1), a1 (r+8, cq..), a2 (r, cq+8..), a3 (r+8, cq+8..)
-    const uint32_t a0 = pack2(za[0], za[1]), a1 = pack2(zb[0], zb[1]);
-    const uint32_t a2 = pack2(za[2], za[3]), a3 = pack2(zb[2], zb[3]);
+  };
+  const unsigned int v_begin = (unsigned int)(ck * a.chunk);
+  fetch(v_begin);
+  bf16 *zt = zs[wi], *xt = xs[wi];
+  const int mat = lane >> 3, mr = lane & 7;
+  const bf16* za = zt + (mr + (mat >= 2 ? 8 : 0)) * ZP + (mat & 1) * 8;   // k = voxel rows, m = channel
+  const bf16* xb = xt + (mr + (mat & 1) * 8) * XP + (mat >> 1) * 8;       // k = voxel rows, two column blocks
+  for (unsigned int v0 = v_begin; v0 < v_end; v0 += 16) {
+    __syncwarp();  // the last step's fragments are read
+    *reinterpret_cast<uint4*>(zt + (lane >> 1) * ZP + (lane & 1) * 8) = zr;
 #pragma unroll
-    for (int nb = 0; nb < NB; ++nb) {
-      const int ci = nb * 8 + r;  // B column n = groupID
-      bf16 x0 = sv[0] >= 0 ? a.x[(size_t)sv[0] * a.x_cs + a.x_co + ci] : zero;
-      bf16 x1 = sv[1] >= 0 ? a.x[(size_t)sv[1] * a.x_cs + a.x_co + ci] : zero;
-      bf16 x2 = sv[2] >= 0 ? a.x[(size_t)sv[2] * a.x_cs + a.x_co + ci] : zero;
-      bf16 x3 = sv[3] >= 0 ? a.x[(size_t)sv[3] * a.x_cs + a.x_co + ci] : zero;
-      mma_bf16(acc[nb], a0, a1, a2, a3, pack2(x0, x1), pack2(x2, x3));
+    for (int m = 0; m < XU; ++m) {
+      const int u = lane + 32 * m, row = u / NB, part = u - row * NB;
+      if (u < 16 * NB) *reinterpret_cast<uint4*>(xt + row * XP + part * 8) = xr[m];
+    }
+    __syncwarp();
+    if (v0 + 16 < v_end) fetch(v0 + 16);
+    uint32_t fa[4];
+    ldmatrix4_trans(fa, za);
+#pragma unroll
+    for (int nb = 0; nb < NB; nb += 2) {
+      uint32_t fb[4];
+      ldmatrix4_trans(fb, xb + nb * 8);
+      mma_bf16(acc[nb], fa[0], fa[1], fa[2], fa[3], fb[0], fb[1]);
+      mma_bf16(acc[nb + 1], fa[0], fa[1], fa[2], fa[3], fb[2], fb[3]);
     }
   }
   // C: (row = co r / r+8, col = ci nb*8+cq, +1), into this chunk's slice
@@ -828,12 +865,23 @@ __global__ void __launch_bounds__(256) conv3_wgrad_kernel(WgradArgs a) {
 }
 
 // out[c] = sum over b = 0..nb-1 of part[b * C + c], added in b order
-// (accumulate: out[c] += that sum).
+// (accumulate: out[c] += that sum); 16 parts are read before the first of
+// them is added (a memory latency per part made this 160 us for the loss's
+// 2048 blocks and 38 us for a level-0 layer).
 template <class T>
 __global__ void sum_parts_kernel(const T* part, int nb, long long C, T* out, int accumulate) {
+  constexpr int U = 16;
   for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < C; c += (long long)gridDim.x * blockDim.x) {
     T s = 0;
-    for (int b = 0; b < nb; ++b) s += part[(size_t)b * C + c];
+    int b = 0;
+    for (; b + U <= nb; b += U) {
+      T v[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) v[u] = part[(size_t)(b + u) * C + c];
+#pragma unroll
+      for (int u = 0; u < U; ++u) s += v[u];
+    }
+    for (; b < nb; ++b) s += part[(size_t)b * C + c];
     out[c] = accumulate ? out[c] + s : s;
   }
 }
@@ -888,9 +936,19 @@ __global__ void bias_grad_kernel(const bf16* dz, int cs, int co, int C, long lon
   __shared__ float sh[64 * 8];
   const int c = threadIdx.x % C, lanes = blockDim.x / C, l = threadIdx.x / C;
   float acc = 0.f;
-  if (threadIdx.x < C * lanes)
-    for (long long v = blockIdx.x * (long long)lanes + l; v < V; v += (long long)gridDim.x * lanes)
-      acc += __bfloat162float(dz[(size_t)v * cs + co + c]);
+  if (threadIdx.x < C * lanes) {
+    constexpr int U = 16;  // voxels read before the first of them is added
+    const long long step = (long long)gridDim.x * lanes;
+    long long v = blockIdx.x * (long long)lanes + l;
+    for (; v + (U - 1) * step < V; v += U * step) {
+      bf16 t[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) t[u] = dz[(size_t)(v + u * step) * cs + co + c];
+#pragma unroll
+      for (int u = 0; u < U; ++u) acc += __bfloat162float(t[u]);
+    }
+    for (; v < V; v += step) acc += __bfloat162float(dz[(size_t)v * cs + co + c]);
+  }
   if (threadIdx.x < C * lanes) sh[threadIdx.x] = acc;
   __syncthreads();
   if (threadIdx.x < C) {
@@ -991,9 +1049,19 @@ __global__ void head_fwd_kernel(const bf16* a13, const float* w, float* pred, lo
   }
 }
 
-__global__ void loss_kernel(const float* pred, const float* target, const unsigned char* mask, long long V, double inv_n,
-                            float* gpred, double* part) {
+// Sum of the mask's bytes (the number of active cells); *count is zeroed before.
+__global__ void mask_count_kernel(const unsigned char* mask, long long V, unsigned long long* count) {
+  unsigned long long n = 0;
+  for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < V; v += (long long)gridDim.x * blockDim.x)
+    n += mask[v];
+  for (int o = 16; o > 0; o >>= 1) n += __shfl_down_sync(0xffffffffu, n, o);
+  if ((threadIdx.x & 31) == 0 && n) atomicAdd(count, n);
+}
+
+__global__ void loss_kernel(const float* pred, const float* target, const unsigned char* mask, long long V,
+                            const unsigned long long* count, float* gpred, double* part) {
   __shared__ double sh[32];
+  const double inv_n = 1.0 / (double)(*count > 0 ? *count : 1);
   double acc = 0.0;
   for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < V; v += (long long)gridDim.x * blockDim.x) {
     const float d = mask[v] ? pred[v] - target[v] : 0.f;
@@ -1408,17 +1476,12 @@ int backward(ttfld_ctx* c, GradWork* gw, double* loss_out) {
   int rc;
   TT_CHECK(cudaMemsetAsync(n->g, 0, n->nparams * 4, s));
   TT_CHECK(cudaMemsetAsync(n->loss_acc, 0, sizeof(double), s));
-  // number of active cells
-  long long nmask = 0;
-  {
-    std::vector<unsigned char> hm((size_t)VF);
-    TT_CHECK(cudaMemcpyAsync(hm.data(), n->mask, (size_t)VF, cudaMemcpyDeviceToHost, s));
-    TT_CHECK(cudaStreamSynchronize(s));
-    for (unsigned char m : hm) nmask += m;
-  }
-  const double inv_n = 1.0 / (double)(nmask > 0 ? nmask : 1);
   const int lblocks = GRID(VF), hblocks = GRID(V0);
-  loss_kernel<<<lblocks, 256, 0, s>>>(n->pred, n->target, n->mask, VF, inv_n, n->gpred, gw->lpart);
+  unsigned long long* count = reinterpret_cast<unsigned long long*>(n->loss_acc + 1);  // number of active cells
+  TT_CHECK(cudaMemsetAsync(count, 0, sizeof(*count), s));
+  mask_count_kernel<<<lblocks, 256, 0, s>>>(n->mask, VF, count);
+  count_launches(1);
+  loss_kernel<<<lblocks, 256, 0, s>>>(n->pred, n->target, n->mask, VF, count, n->gpred, gw->lpart);
   sum_parts_kernel<double><<<1, 32, 0, s>>>(gw->lpart, lblocks, 1, n->loss_acc, 0);
   pred_down_kernel<<<GRID(V0), 256, 0, s>>>(n->gpred, n->full, n->gpred_half, L(0));
   head_bwd_kernel<<<hblocks, 256, 0, s>>>(n->gpred_half, n->a13, n->p + n->hoff, n->g_a13, gw->hpart, V0);
@@ -1480,13 +1543,14 @@ size_t max_wpad(const Net* n) {
   return m;
 }
 
-// One allocation for the gradient workspace (freed with cudaFree(gw->gpad)).
-int alloc_gradwork(const Net* n, GradWork* gw) {
+// The gradient workspace: one allocation, made by the first training call and
+// kept with the network (an allocation and a free per call cost 0.4 ms).
+int grad_work(Net* n, GradWork* gw) {
   const size_t a = align256(max_wpad(n) * 4), b = align256(max_wpart() * 4);
   const size_t c = align256((size_t)kMaxGradBlocks * 64 * 4), d = align256((size_t)kMaxGradBlocks * 17 * 4);
   const size_t e = align256((size_t)kMaxGradBlocks * 8);
-  char* p = nullptr;
-  TT_CHECK(cudaMalloc((void**)&p, a + b + c + d + e));
+  if (!n->grad_mem) TT_CHECK(cudaMalloc(&n->grad_mem, a + b + c + d + e));
+  char* p = (char*)n->grad_mem;
   gw->gpad = (float*)p;
   gw->wpart = (float*)(p + a);
   gw->bpart = (float*)(p + a + b);
@@ -1530,23 +1594,28 @@ int make_features(ttfld_ctx* c, bf16* feat0, unsigned char* mask) {
 int upload_features(ttfld_ctx* c, const float* feat) {
   Net* n = net_of(c);
   const Level fi = n->full, l0 = n->lv[0];
-  std::vector<bf16> hf((size_t)l0.vox() * kFeatPad);
-  for (int z = 0; z < l0.Z; ++z)
-    for (int y = 0; y < l0.Y; ++y)
-      for (int x = 0; x < l0.X; ++x) {
-        float acc[kFeat] = {0.f, 0.f, 0.f, 0.f, 0.f};
-        int cnt = 0;
-        for (int q = 0; q < 8; ++q) {
-          const int xx = 2 * x + (q & 1), yy = 2 * y + ((q >> 1) & 1), zz = 2 * z + (q >> 2);
-          if (xx >= fi.X || yy >= fi.Y || zz >= fi.Z) continue;
-          const float* f = feat + (((size_t)zz * fi.Y + yy) * fi.X + xx) * kFeat;
-          for (int t = 0; t < kFeat; ++t) acc[t] += f[t];
-          ++cnt;
-        }
-        bf16* o = hf.data() + (((size_t)z * l0.Y + y) * l0.X + x) * kFeatPad;
-        for (int t = 0; t < kFeatPad; ++t) o[t] = __float2bfloat16_rn(t < kFeat ? acc[t] / (float)cnt : 0.f);
-      }
-  TT_CHECK(cudaMemcpyAsync(n->feat, hf.data(), hf.size() * 2, cudaMemcpyHostToDevice, c->stream));
+  const size_t bytes = (size_t)fi.vox() * kFeat * sizeof(float);
+  if (!n->feat_stage) TT_CHECK(cudaMalloc((void**)&n->feat_stage, bytes));
+  TT_CHECK(cudaMemcpyAsync(n->feat_stage, feat, bytes, cudaMemcpyHostToDevice, c->stream));
+  const float* in = n->feat_stage;
+  bf16* out = n->feat;
+  launch_box(c->stream, box(0, l0.X - 1, 0, l0.Y - 1, 0, l0.Z - 1), [=] __device__(int x, int y, int z) {
+    float acc[kFeat] = {0.f, 0.f, 0.f, 0.f, 0.f};
+    int cnt = 0;
+    for (int q = 0; q < 8; ++q) {
+      const int xx = 2 * x + (q & 1), yy = 2 * y + ((q >> 1) & 1), zz = 2 * z + (q >> 2);
+      if (xx >= fi.X || yy >= fi.Y || zz >= fi.Z) continue;
+      const float* f = in + (((size_t)zz * fi.Y + yy) * fi.X + xx) * kFeat;
+      for (int t = 0; t < kFeat; ++t) acc[t] += f[t];
+      ++cnt;
+    }
+    __align__(16) bf16 o[kFeatPad];
+    for (int t = 0; t < kFeatPad; ++t) o[t] = __float2bfloat16_rn(t < kFeat ? acc[t] / (float)cnt : 0.f);
+    uint4* dst = reinterpret_cast<uint4*>(out + (((size_t)z * l0.Y + y) * l0.X + x) * kFeatPad);
+    dst[0] = reinterpret_cast<const uint4*>(o)[0];
+    dst[1] = reinterpret_cast<const uint4*>(o)[1];
+  });
+  TT_CHECK_LAUNCH();
   return check_cuda(cudaStreamSynchronize(c->stream), "upload features");
 }
 
@@ -1560,6 +1629,8 @@ void unet_free(ttfld_ctx* c) {
   if (n->p) cudaFree(n->p);
   if (n->w16) cudaFree(n->w16);
   if (n->act_mem) cudaFree(n->act_mem);
+  if (n->grad_mem) cudaFree(n->grad_mem);
+  if (n->feat_stage) cudaFree(n->feat_stage);
   if (n->ds_feat) cudaFree(n->ds_feat);
   free(n);
   c->unet = nullptr;
@@ -1656,7 +1727,7 @@ int ttfld_guess_train(ttfld_ctx* c, int epochs, double lr, uint64_t seed, double
   if (n->count < 1) return TTFLD_E_ARGS;
   const long long V0 = L(0).vox(), VF = n->full.vox();
   GradWork gw;
-  int rc0 = alloc_gradwork(n, &gw);
+  int rc0 = grad_work(n, &gw);
   if (rc0) return rc0;
   std::vector<int> order(n->count);
   uint64_t st = seed * 0x9E3779B97F4A7C15ULL + 1;
@@ -1697,7 +1768,6 @@ int ttfld_guess_train(ttfld_ctx* c, int epochs, double lr, uint64_t seed, double
     }
   }
   cudaStreamSynchronize(c->stream);
-  cudaFree(gw.gpad);
   if (rc) return rc;
   if (mean_loss) *mean_loss = cnt ? tot / cnt : 0.0;
   c->have_model = 1;
@@ -1718,12 +1788,11 @@ int ttfld_guess_gradients(ttfld_ctx* c, const float* feat, const float* target, 
   TT_CHECK(cudaMemcpy(n->target, target, (size_t)VF * 4, cudaMemcpyHostToDevice));
   TT_CHECK(cudaMemcpy(n->mask, mask, (size_t)VF, cudaMemcpyHostToDevice));
   GradWork gw;
-  if ((rc = alloc_gradwork(n, &gw))) return rc;
+  if ((rc = grad_work(n, &gw))) return rc;
   rc = prep_weights(c);
   if (!rc) rc = forward(c);
   if (!rc) rc = backward(c, &gw, loss);
   cudaStreamSynchronize(c->stream);
-  cudaFree(gw.gpad);
   if (rc) return rc;
   if (grads) TT_CHECK(cudaMemcpy(grads, n->g, n->nparams * 4, cudaMemcpyDeviceToHost));
   return 0;
