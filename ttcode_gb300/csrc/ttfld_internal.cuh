@@ -396,6 +396,36 @@ __device__ __forceinline__ bool grid_sum(SolverDev* sol, unsigned int nblocks, u
   return ok_sh != 0;
 }
 
+// Which part of a sweep's arrays stays in L2 from sweep to sweep.  Where they
+// are larger than L2, each array's lines are gone again before the next
+// sweep wants them; so a fixed part of the lines, chosen by the hardware's
+// hash of the address, is marked to be evicted last and the rest first.  The
+// iterate goes first (it is read twice and written once per sweep), then the
+// coefficients.
+struct L2Keep {
+  float iter, coef;  // fractions of the lines
+};
+// Of what the L2 holds, 0.55 (70 of 126 MB): over unique footprints of 79 to
+// 671 MB of the FP32 sweeps 60 to 80 MB is best, 90 MB up to 12 % slower.
+inline L2Keep l2_keep(double iter_bytes, double coef_bytes) {
+  int dev = 0, l2 = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev);
+  const double room = 0.55 * l2;
+  L2Keep k;
+  k.iter = (float)(iter_bytes <= room ? 1.0 : room / iter_bytes);
+  k.coef = (float)(iter_bytes >= room ? 0.0 : coef_bytes <= room - iter_bytes ? 1.0 : (room - iter_bytes) / coef_bytes);
+  return k;
+}
+__device__ __forceinline__ uint64_t l2_policy(float keep) {
+  uint64_t p;
+  if (keep > 0.f)
+    asm("createpolicy.fractional.L2::evict_last.L2::evict_first.b64 %0, %1;" : "=l"(p) : "f"(keep));
+  else
+    asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+  return p;
+}
+
 // An asynchronous copy of one 8- or 16-byte word to shared memory.
 template <class W>
 __device__ __forceinline__ void copy_async(W* to, const W* from) {

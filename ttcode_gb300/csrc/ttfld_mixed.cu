@@ -223,6 +223,36 @@ __device__ __forceinline__ float4 ldc4(const float* p) {
   return v;
 }
 
+// The same accesses with a part of the lines kept in L2 (L2Keep).
+struct KeepPolicy {
+  uint64_t coef, iter;
+};
+__device__ __forceinline__ float4 ldc4(const float* p, const KeepPolicy& k) {
+  float4 v;
+  asm("ld.global.L1::no_allocate.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;"
+      : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+      : "l"(p), "l"(k.coef));
+  return v;
+}
+__device__ __forceinline__ float4 lde4(const float* p, const KeepPolicy& k) {
+  float4 v;
+  asm volatile("ld.global.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "l"(p), "l"(k.iter)
+               : "memory");
+  return v;
+}
+__device__ __forceinline__ void st4(float* p, float4 v, const KeepPolicy& k) {
+  asm volatile("st.global.L2::cache_hint.v4.f32 [%4], {%0, %1, %2, %3}, %5;" ::"f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w),
+               "l"(p), "l"(k.iter)
+               : "memory");
+}
+// No hint.
+struct KeepNone {};
+__device__ __forceinline__ float4 ldc4(const float* p, const KeepNone&) { return ldc4(p); }
+__device__ __forceinline__ float4 lde4(const float* p, const KeepNone&) { return lde4(p); }
+__device__ __forceinline__ void st4(float* p, float4 v, const KeepNone&) { st4(p, v); }
+
 // One colour of FP32 red-black SOR on A e = r (Jacobi-scaled), 4 cells per
 // thread: res = (e + sum a_nb e_nb) - rhat (the reference's in-sweep residual
 // divided by A, ppsor.f:64-71), e -= omega * res.  NORM sweeps also sum
@@ -238,10 +268,10 @@ __device__ __forceinline__ float4 ldc4(const float* p) {
 // where the coefficients are in shared memory and the index is on the path of
 // the only loads; beside loads of the coefficients the 64-bit one is (16.06
 // against 16.25 ms per step at 100x256x128).
-template <int COL, bool NORM, bool POLES, bool FAST_INDEX>
+template <int COL, bool NORM, bool POLES, bool FAST_INDEX, class Keep>
 __device__ __forceinline__ void update_vec(const Cmp& g, const Mix32& m, float omega, long long t, int nv,
                                            size_t plane, float4 aw, float4 ae, float4 as, float4 an, float4 ab,
-                                           float4 at, float4 r, float4 dg, float& nacc) {
+                                           float4 at, float4 r, float4 dg, float& nacc, const Keep& keep) {
   const float* eo = m.e[1 - COL];
   float* es = m.e[COL];
   int hv, j0, k0;
@@ -263,7 +293,7 @@ __device__ __forceinline__ void update_vec(const Cmp& g, const Mix32& m, float o
   const size_t eb = gslot(g, j0, k0, h0);
   const int jm = j0 == 0 ? g.ny - 1 : j0 - 1;
   const int jp = j0 == g.ny - 1 ? 0 : j0 + 1;
-  const float4 o = lde4(eo + eb);
+  const float4 o = lde4(eo + eb, keep);
   float xm0, xm1, xm2, xm3, xp0, xp1, xp2, xp3;
   if (off == 0) {
     xm0 = h0 > 0 ? lde(eo + eb - 1) : 0.f; xm1 = o.x; xm2 = o.y; xm3 = o.z;
@@ -272,12 +302,12 @@ __device__ __forceinline__ void update_vec(const Cmp& g, const Mix32& m, float o
     xm0 = o.x; xm1 = o.y; xm2 = o.z; xm3 = o.w;
     xp0 = o.y; xp1 = o.z; xp2 = o.w; xp3 = (h0 + 4 < g.nxp) ? lde(eo + eb + 4) : 0.f;
   }
-  const float4 s = lde4(eo + gslot(g, jm, k0, h0));
-  const float4 nn = lde4(eo + gslot(g, jp, k0, h0));
-  const float4 e = lde4(es + eb);
+  const float4 s = lde4(eo + gslot(g, jm, k0, h0), keep);
+  const float4 nn = lde4(eo + gslot(g, jp, k0, h0), keep);
+  const float4 e = lde4(es + eb, keep);
   // with poles the theta neighbour across either edge is the cell itself
-  const float4 b = (POLES && k0 == 0) ? e : lde4(eo + eb - plane);
-  const float4 tt = (POLES && k0 == g.nz - 2) ? e : lde4(eo + eb + plane);
+  const float4 b = (POLES && k0 == 0) ? e : lde4(eo + eb - plane, keep);
+  const float4 tt = (POLES && k0 == g.nz - 2) ? e : lde4(eo + eb + plane, keep);
   float4 out;
 #define UPD(L, IDX, XM, XP)                                                                \
   {                                                                                        \
@@ -290,22 +320,22 @@ __device__ __forceinline__ void update_vec(const Cmp& g, const Mix32& m, float o
   }
   UPD(x, 0, xm0, xp0) UPD(y, 1, xm1, xp1) UPD(z, 2, xm2, xp2) UPD(w, 3, xm3, xp3)
 #undef UPD
-  st4(es + eb, out);
+  st4(es + eb, out, keep);
 }
 
 // The same with the coefficients loaded from global memory (item t's four
 // slots are floats 4t .. 4t+3 of each coefficient array).
-template <int COL, bool NORM, bool POLES>
+template <int COL, bool NORM, bool POLES, class Keep = KeepNone>
 __device__ __forceinline__ void sweep_vec(const Cmp& g, const Mix32& m, float omega, long long t, int nv,
-                                          size_t plane, float& nacc) {
+                                          size_t plane, float& nacc, const Keep& keep = Keep()) {
   const size_t cb = (size_t)t * 4;
-  const float4 aw = ldc4(m.a[0][COL] + cb), ae = ldc4(m.a[1][COL] + cb);
-  const float4 as = ldc4(m.a[2][COL] + cb), an = ldc4(m.a[3][COL] + cb);
-  const float4 ab = ldc4(m.a[4][COL] + cb), at = ldc4(m.a[5][COL] + cb);
-  const float4 r = ldc4(m.rhat[COL] + cb);
+  const float4 aw = ldc4(m.a[0][COL] + cb, keep), ae = ldc4(m.a[1][COL] + cb, keep);
+  const float4 as = ldc4(m.a[2][COL] + cb, keep), an = ldc4(m.a[3][COL] + cb, keep);
+  const float4 ab = ldc4(m.a[4][COL] + cb, keep), at = ldc4(m.a[5][COL] + cb, keep);
+  const float4 r = ldc4(m.rhat[COL] + cb, keep);
   float4 dg = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (NORM) dg = ldc4(m.diag[COL] + cb);
-  update_vec<COL, NORM, POLES, false>(g, m, omega, t, nv, plane, aw, ae, as, an, ab, at, r, dg, nacc);
+  if (NORM) dg = ldc4(m.diag[COL] + cb, keep);
+  update_vec<COL, NORM, POLES, false>(g, m, omega, t, nv, plane, aw, ae, as, an, ab, at, r, dg, nacc, keep);
 }
 
 // One colour per launch.  NORM launches of the second colour end with the
@@ -468,18 +498,34 @@ __device__ __forceinline__ void fetch_vec(const Mix32& m, long long t, float4* t
   copy_async(to + 6 * stride, reinterpret_cast<const float4*>(m.rhat[COL] + cb));
 }
 
+// Not RESIDENT, the arrays exceed L2 (or nearly): a part of their lines is
+// marked to stay (keep), and every other sweep goes through the block's items
+// from the last to the first, so that it begins with what the sweep before
+// left in L2.  A norm sweep always goes forward: its sum has one order.
+// Per sweep at 96, 128 and 160 theta planes of 100x256 cells 15.4, 18.9 and
+// 22.4 us before, 12.4, 15.9 and 18.9 with both (the marks without the order
+// 12.6, 16.1 and 19.1); 26.8 -> 22.8 at 160x256x128, 38.2 -> 35.7 at
+// 160x256x192, 117 -> 111 at 160x512x256.  Loads without a mark but with
+// allocation in L2 as usual are 50.8 and 148 us at the last two sizes, the
+// same as the marks at the first.  Bulk prefetches of the next items to L2
+// made every size slower (16.0 -> 16.8, 111 -> 143).
 template <int COL, bool NORM, bool POLES, bool RESIDENT>
 __device__ __forceinline__ void sweep_local(const Cmp& g, const Mix32& m, float omega, long long t0, unsigned int n,
-                                            int nv, size_t plane, const float4* slots, float& nacc) {
-  for (unsigned int u = threadIdx.x; u < n; u += blockDim.x) {
-    const long long t = t0 + u;
-    if (RESIDENT) {
+                                            int nv, size_t plane, const float4* slots, float& nacc,
+                                            const KeepPolicy& keep, bool back) {
+  if constexpr (!RESIDENT) {
+    const unsigned int rounds = (n + blockDim.x - 1) / blockDim.x;
+    for (unsigned int q = 0; q < rounds; ++q) {
+      const unsigned int u = threadIdx.x + (!NORM && back ? rounds - 1 - q : q) * blockDim.x;
+      if (u < n) sweep_vec<COL, NORM, POLES>(g, m, omega, t0 + u, nv, plane, nacc, keep);
+    }
+  } else {
+    for (unsigned int u = threadIdx.x; u < n; u += blockDim.x) {
+      const long long t = t0 + u;
       const float4* w = slots + (size_t)COL * kLocalWords * n + u;
       const float4 dg = NORM ? ldc4(m.diag[COL] + (size_t)t * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
-      update_vec<COL, NORM, POLES, true>(g, m, omega, t, nv, plane, w[0], w[n], w[2 * n], w[3 * n], w[4 * n], w[5 * n],
-                                   w[6 * n], dg, nacc);
-    } else {
-      sweep_vec<COL, NORM, POLES>(g, m, omega, t, nv, plane, nacc);
+      update_vec<COL, NORM, POLES, true>(g, m, omega, t, nv, plane, w[0], w[n], w[2 * n], w[3 * n], w[4 * n],
+                                         w[5 * n], w[6 * n], dg, nacc, KeepNone());
     }
   }
 }
@@ -488,7 +534,7 @@ template <bool POLES, bool RESIDENT = false>
 __global__ void __launch_bounds__(kPersistThreads) sweeps32_local(Cmp g, Mix32 m, float omega, SolverDev* sol,
                                                                  Partial* gather, double stop_ratio, int nsweeps,
                                                                  int norm_every, int stall_check, unsigned int* flags,
-                                                                 unsigned int base) {
+                                                                 unsigned int base, L2Keep l2) {
   __shared__ double sh[32];
   __shared__ int stop_sh;
   extern __shared__ __align__(16) unsigned char slots_raw[];
@@ -517,6 +563,7 @@ __global__ void __launch_bounds__(kPersistThreads) sweeps32_local(Cmp g, Mix32 m
     asm volatile("cp.async.wait_all;" ::: "memory");
   }
   double last_ratio = -1.0;  // in-sweep ratio of the previous norm sweep (lane 0 of the last warp)
+  const KeepPolicy keep = {l2_policy(l2.coef), l2_policy(l2.iter)};
   const int it0 = sol->iter;
   int norms = 0;
   unsigned int half = base;  // half-sweeps this block has finished
@@ -525,12 +572,12 @@ __global__ void __launch_bounds__(kPersistThreads) sweeps32_local(Cmp g, Mix32 m
     const bool norm = norm_every > 0 && (sw % norm_every == 0 || sw == nsweeps);
     float nacc = 0.f;
     if (sw > 1 && !wait_flags(flags, lo, hi, half, sol)) break;
-    if (norm) sweep_local<0, true, POLES, RESIDENT>(g, m, omega, t0, mine, nv, plane, slots, nacc);
-    else sweep_local<0, false, POLES, RESIDENT>(g, m, omega, t0, mine, nv, plane, slots, nacc);
+    if (norm) sweep_local<0, true, POLES, RESIDENT>(g, m, omega, t0, mine, nv, plane, slots, nacc, keep, (sw & 1) != 0);
+    else sweep_local<0, false, POLES, RESIDENT>(g, m, omega, t0, mine, nv, plane, slots, nacc, keep, (sw & 1) != 0);
     publish_flag(own, ++half);
     if (!wait_flags(flags, lo, hi, half, sol)) break;
-    if (norm) sweep_local<1, true, POLES, RESIDENT>(g, m, omega, t0, mine, nv, plane, slots, nacc);
-    else sweep_local<1, false, POLES, RESIDENT>(g, m, omega, t0, mine, nv, plane, slots, nacc);
+    if (norm) sweep_local<1, true, POLES, RESIDENT>(g, m, omega, t0, mine, nv, plane, slots, nacc, keep, (sw & 1) != 0);
+    else sweep_local<1, false, POLES, RESIDENT>(g, m, omega, t0, mine, nv, plane, slots, nacc, keep, (sw & 1) != 0);
     if (norm) {
       const double v = warp_sum_all((double)nacc);
       if (lane == 0) sh[warp] = v;
@@ -792,7 +839,7 @@ __global__ void __launch_bounds__(kTmaThreads) sweeps32_tma(Cmp g, Mix32 m, floa
           const float4* sb = reinterpret_cast<const float4*>(stages + (size_t)st * kStageBytes) + threadIdx.x;
           const float4 dg = norm ? sb[7 * kTmaThreads] : make_float4(0.f, 0.f, 0.f, 0.f);
 #define UPD_ARGS g, m, omega, t, nv, plane, sb[0], sb[kTmaThreads], sb[2 * kTmaThreads], sb[3 * kTmaThreads], \
-                 sb[4 * kTmaThreads], sb[5 * kTmaThreads], sb[6 * kTmaThreads], dg, nacc
+                 sb[4 * kTmaThreads], sb[5 * kTmaThreads], sb[6 * kTmaThreads], dg, nacc, KeepNone()
           if (col == 0) { if (norm) update_vec<0, true, POLES, false>(UPD_ARGS); else update_vec<0, false, POLES, false>(UPD_ARGS); }
           else { if (norm) update_vec<1, true, POLES, false>(UPD_ARGS); else update_vec<1, false, POLES, false>(UPD_ARGS); }
 #undef UPD_ARGS
@@ -999,10 +1046,11 @@ struct SweepGrids {
   int pers, tma, wave, local;
   int local_threads, resident;
   size_t local_smem;
+  L2Keep l2;
 };
 template <bool POLES>
 static SweepGrids sweep_grids(long long nvec) {
-  static SweepGrids gr = {-1, -1, -1, -1, 0, 0, 0};
+  static SweepGrids gr = {-1, -1, -1, -1, 0, 0, 0, {1.f, 1.f}};
   static long long sized_for = -1;
   if (sized_for != nvec) {
     gr.tma = persistent_grid(sweeps32_tma<POLES>, kTmaThreads, kTmaSmem, nvec);
@@ -1031,6 +1079,7 @@ static SweepGrids sweep_grids(long long nvec) {
       gr.local = persistent_grid(sweeps32_local<POLES>, kPersistThreads, 0, nvec);
     }
     if (gr.local > kMaxLocalBlocks) gr.local = 0;
+    gr.l2 = l2_keep(32.0 * (double)nvec, 7 * 32.0 * (double)nvec);  // e; the couplings and r-hat, of both colours
     sized_for = nvec;
   }
   return gr;
@@ -1082,7 +1131,8 @@ static int launch_sweeps32_form(ttfld_ctx* c, int nsweeps, int norm_every, doubl
     unsigned int base = w->flag_base;
     Partial* gather = (Partial*)partials;  // two a block
     TT_CHECK(cudaMemsetAsync(gather, 0, (size_t)gr.local * 2 * sizeof(Partial), c->stream));
-    void* largs[] = {&g, &m, &omega, &sol, &gather, &stop_ratio, &nsweeps, &norm_every, &stall, &flags, &base};
+    L2Keep l2 = gr.l2;
+    void* largs[] = {&g, &m, &omega, &sol, &gather, &stop_ratio, &nsweeps, &norm_every, &stall, &flags, &base, &l2};
     if (gr.resident)
       TT_CHECK(cudaLaunchCooperativeKernel((const void*)sweeps32_local<POLES, true>, dim3(gr.local),
                                            dim3(gr.local_threads), largs, gr.local_smem, c->stream));
