@@ -433,6 +433,15 @@ __device__ __forceinline__ void copy_async(W* to, const W* from) {
   if (sizeof(W) == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(from) : "memory");
   else asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(from) : "memory");
 }
+// The same with an L2 policy (l2_policy).
+template <class W>
+__device__ __forceinline__ void copy_async(W* to, const W* from, uint64_t pol) {
+  const unsigned int dst = (unsigned int)__cvta_generic_to_shared(to);
+  if (sizeof(W) == 16)
+    asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;" ::"r"(dst), "l"(from), "l"(pol) : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global.L2::cache_hint [%0], [%1], 8, %2;" ::"r"(dst), "l"(from), "l"(pol) : "memory");
+}
 
 __device__ __forceinline__ bool solver_done(const Dev& d) {
   return *(volatile int*)&d.sol->done != 0;

@@ -1496,12 +1496,12 @@ struct FastRows {
   template <int COL>
   __device__ void after(unsigned int, unsigned int, bool) const {}
   template <int COL>
-  __device__ __forceinline__ void fetch(unsigned int row, unsigned int h, double2* to, unsigned int T) const {
+  __device__ __forceinline__ void fetch(unsigned int row, unsigned int h, double2* to, unsigned int T, uint64_t pol) const {
     const size_t c = (size_t)row * nxp + 2 * h;
 #pragma unroll
-    for (int q = 0; q < 6; ++q) copy_async(to + q * T, reinterpret_cast<const double2*>(m.a[q][COL] + c));
-    copy_async(to + 6 * T, reinterpret_cast<const double2*>(m.bhat[COL] + c));
-    copy_async(to + 7 * T, reinterpret_cast<const double2*>(m.diag[COL] + c));
+    for (int q = 0; q < 6; ++q) copy_async(to + q * T, reinterpret_cast<const double2*>(m.a[q][COL] + c), pol);
+    copy_async(to + 6 * T, reinterpret_cast<const double2*>(m.bhat[COL] + c), pol);
+    copy_async(to + 7 * T, reinterpret_cast<const double2*>(m.diag[COL] + c), pol);
   }
   template <int COL>
   __device__ __forceinline__ double update(unsigned int row, unsigned int h, const double2* w, unsigned int T, bool,

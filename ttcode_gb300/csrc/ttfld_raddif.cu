@@ -275,19 +275,19 @@ struct RadRows {
     }
   }
   template <int COL>
-  __device__ __forceinline__ void fetch(unsigned int row, unsigned int h, double* to, unsigned int T) const {
+  __device__ __forceinline__ void fetch(unsigned int row, unsigned int h, double* to, unsigned int T, uint64_t pol) const {
     unsigned int j0, k0;
     const unsigned int i0 = cell<COL>(row, h, j0, k0);
     if ((int)i0 >= d.nx) return;
     const size_t c = i0 + (size_t)d.nx * row;
-    copy_async(to, w.b + c);
-    copy_async(to + T, w.rhs + c);
-    copy_async(to + 2 * T, w.ax + c);
-    copy_async(to + 3 * T, w.cx + c);
-    copy_async(to + 4 * T, w.ay + c);
-    copy_async(to + 5 * T, w.cy + c);
-    copy_async(to + 6 * T, w.az + c);
-    copy_async(to + 7 * T, w.cz + c);
+    copy_async(to, w.b + c, pol);
+    copy_async(to + T, w.rhs + c, pol);
+    copy_async(to + 2 * T, w.ax + c, pol);
+    copy_async(to + 3 * T, w.cx + c, pol);
+    copy_async(to + 4 * T, w.ay + c, pol);
+    copy_async(to + 5 * T, w.cy + c, pol);
+    copy_async(to + 6 * T, w.az + c, pol);
+    copy_async(to + 7 * T, w.cz + c, pol);
   }
   template <int COL>
   __device__ __forceinline__ double update(unsigned int row, unsigned int h, const double* c, unsigned int T,

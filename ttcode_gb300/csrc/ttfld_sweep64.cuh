@@ -21,7 +21,10 @@
 // before it updates the present one, across the colours too, so that these
 // reads, eight of the 16 values of a cell, wait for nothing.  Where a block's
 // share of them fits in shared memory (RESIDENT: 227 KB a block, 540,000
-// cells in all) it is copied once for all sweeps.
+// cells in all) it is copied once for all sweeps.  Beyond L2 most of their
+// lines are marked to be evicted first (l2_keep), so that the iterate stays:
+// 52.2 -> 50.0 ms for the scaled SOR and 5.06 -> 4.75 ms for DIFFUSION at
+// 100x256x128, 11.9 -> 11.3 ms for DIFFUSION at 160x256x192.
 //
 // A system is a struct with
 //   rows, by_items          (j,k) rows, and the items of a colour in a row
@@ -81,7 +84,8 @@ __device__ __forceinline__ void undo_colour(const Sys& s, unsigned int r0, unsig
 // the present one is updated.  mine: where to keep the values replaced.
 template <int COL, bool RESIDENT, class Sys>
 __device__ __forceinline__ double sweep_colour(const Sys& s, unsigned int r0, unsigned int n, bool first,
-                                               typename Sys::Word* slots, int& stage, typename Sys::Kept* mine) {
+                                               typename Sys::Word* slots, int& stage, typename Sys::Kept* mine,
+                                               uint64_t pol) {
   double acc = 0.0;
   const unsigned int T = blockDim.x;
   for (unsigned int u = threadIdx.x; u < n; u += T) {
@@ -97,10 +101,10 @@ __device__ __forceinline__ double sweep_colour(const Sys& s, unsigned int r0, un
     unsigned int hn;
     if (u + T < n) {
       const unsigned int rn = r0 + div_rem(s.by_items, u + T, hn);
-      s.template fetch<COL>(rn, hn, next, T);
+      s.template fetch<COL>(rn, hn, next, T, pol);
     } else {
       const unsigned int rn = r0 + div_rem(s.by_items, threadIdx.x, hn);
-      s.template fetch<1 - COL>(rn, hn, next, T);
+      s.template fetch<1 - COL>(rn, hn, next, T, pol);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
     asm volatile("cp.async.wait_group 1;" ::: "memory");
@@ -112,7 +116,7 @@ __device__ __forceinline__ double sweep_colour(const Sys& s, unsigned int r0, un
 template <class Sys, bool RESIDENT>
 __global__ void __launch_bounds__(Sys::kThreads, 1)
     sweeps64_persistent(Sys s, SolverDev* sol, Partial* gather, unsigned int* flags, typename Sys::Kept* keep,
-                        int nsweeps, int itmin, int itmax, double eps) {
+                        int nsweeps, int itmin, int itmax, double eps, float coef_keep) {
   __shared__ double sh[32];
   __shared__ int stop_sh, ok_sh;
   if (threadIdx.x == 0) {  // read after block barriers only
@@ -132,19 +136,20 @@ __global__ void __launch_bounds__(Sys::kThreads, 1)
   const int it0 = sol->iter;
   extern __shared__ __align__(16) unsigned char slots_raw[];
   typename Sys::Word* slots = reinterpret_cast<typename Sys::Word*>(slots_raw);
+  const uint64_t pol = l2_policy(RESIDENT ? 0.f : coef_keep);  // resident: read once
   int stage = 0;
   if (RESIDENT) {  // each thread copies what it will read itself
     for (unsigned int u = threadIdx.x; u < n; u += blockDim.x) {
       unsigned int h;
       const unsigned int r = r0 + div_rem(s.by_items, u, h);
-      s.template fetch<0>(r, h, slots + u, n);
-      s.template fetch<1>(r, h, slots + (size_t)Sys::kWords * n + u, n);
+      s.template fetch<0>(r, h, slots + u, n, pol);
+      s.template fetch<1>(r, h, slots + (size_t)Sys::kWords * n + u, n, pol);
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
   } else if (threadIdx.x < n) {
     unsigned int h;
     const unsigned int r = r0 + div_rem(s.by_items, threadIdx.x, h);
-    s.template fetch<0>(r, h, slots + threadIdx.x, blockDim.x);
+    s.template fetch<0>(r, h, slots + threadIdx.x, blockDim.x, pol);
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
   typename Sys::Kept* mine = keep ? keep + (size_t)r0 * s.by_items.d : nullptr;
@@ -154,7 +159,7 @@ __global__ void __launch_bounds__(Sys::kThreads, 1)
   for (int sw = 1; sw <= nsweeps && !stop; ++sw) {
     if (sw > 1 && !wait_flags(flags, lo, hi, half, sol)) break;
     s.template before<0>(r0, r1);
-    double acc = sweep_colour<0, RESIDENT>(s, r0, n, sw == 1, slots, stage, sw > 1 ? mine : nullptr);
+    double acc = sweep_colour<0, RESIDENT>(s, r0, n, sw == 1, slots, stage, sw > 1 ? mine : nullptr, pol);
     s.template after<0>(r0, r1, sw == 1);
     publish_flag(own, ++half);
     // the first warp waits for the neighbours, the last takes the last
@@ -171,7 +176,7 @@ __global__ void __launch_bounds__(Sys::kThreads, 1)
       break;
     }
     s.template before<1>(r0, r1);
-    acc += sweep_colour<1, RESIDENT>(s, r0, n, false, slots, stage, nullptr);
+    acc += sweep_colour<1, RESIDENT>(s, r0, n, false, slots, stage, nullptr, pol);
     s.template after<1>(r0, r1, false);
     acc = warp_sum_all(acc);
     if (lane == 0) sh[warp] = acc;
@@ -229,7 +234,9 @@ int launch_sweeps64_persistent(const Sys& s, cudaStream_t st, SolverDev* sol, do
   Sys sys = s;
   typename Sys::Kept* keep =
       (size_t)items * sizeof(typename Sys::Kept) <= kept_bytes ? (typename Sys::Kept*)kept : nullptr;
-  void* args[] = {&sys, &sol, &gather, &flags, &keep, &nsweeps, &itmin, &itmax, &eps};
+  const double word = 2.0 * (double)items * sizeof(typename Sys::Word);  // an array of both colours
+  float coef_keep = l2_keep(word, Sys::kWords * word).coef;
+  void* args[] = {&sys, &sol, &gather, &flags, &keep, &nsweeps, &itmin, &itmax, &eps, &coef_keep};
   const cudaError_t e =
       cudaLaunchCooperativeKernel(kernel, dim3((unsigned int)nb), dim3(threads), args, smem, st);
   if (e == cudaErrorCooperativeLaunchTooLarge) {
@@ -270,19 +277,19 @@ struct SorRows {
     return 2 * h + ((j0 + k0 + COL + 1) & 1);
   }
   template <int COL>
-  __device__ __forceinline__ void fetch(unsigned int row, unsigned int h, double* to, unsigned int T) const {
+  __device__ __forceinline__ void fetch(unsigned int row, unsigned int h, double* to, unsigned int T, uint64_t pol) const {
     unsigned int j0, k0;
     const unsigned int i0 = cell<COL>(row, h, j0, k0);
     if ((int)i0 >= nx) return;
     const size_t c = i0 + (size_t)nx * row;
-    copy_async(to, a + c);
-    copy_async(to + T, xm + c);
-    copy_async(to + 2 * T, xp + c);
-    copy_async(to + 3 * T, jm + c);
-    copy_async(to + 4 * T, jp + c);
-    copy_async(to + 5 * T, km + c);
-    copy_async(to + 6 * T, kp + c);
-    copy_async(to + 7 * T, b + c);
+    copy_async(to, a + c, pol);
+    copy_async(to + T, xm + c, pol);
+    copy_async(to + 2 * T, xp + c, pol);
+    copy_async(to + 3 * T, jm + c, pol);
+    copy_async(to + 4 * T, jp + c, pol);
+    copy_async(to + 5 * T, km + c, pol);
+    copy_async(to + 6 * T, kp + c, pol);
+    copy_async(to + 7 * T, b + c, pol);
   }
   template <int COL>
   __device__ __forceinline__ double update(unsigned int row, unsigned int h, const double* w, unsigned int T, bool,
