@@ -80,6 +80,10 @@ struct Net {
   void* act_mem;
   void* grad_mem;              // gradient workspace (first training call)
   float* feat_stage;           // features on the grid (first call with host features)
+  // beside the backward pass's chain: the weight and the bias gradients
+  cudaStream_t side[2];
+  cudaEvent_t dz_ready, done[2];
+  int joined;                  // the streams and events exist
   // dataset (captured pairs)
   int cap, count, capture_next;
   bf16* ds_feat;       // [cap][level-0 vox][kFeatPad] pooled features
@@ -864,30 +868,49 @@ __global__ void __launch_bounds__(256) conv3_wgrad_kernel(WgradArgs a) {
   }
 }
 
-// out[c] = sum over b = 0..nb-1 of part[b * C + c], added in b order
-// (accumulate: out[c] += that sum); 16 parts are read before the first of
-// them is added (a memory latency per part made this 160 us for the loss's
-// 2048 blocks and 38 us for a level-0 layer).
-template <class T>
-__global__ void sum_parts_kernel(const T* part, int nb, long long C, T* out, int accumulate) {
-  constexpr int U = 16;
-  for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < C; c += (long long)gridDim.x * blockDim.x) {
-    T s = 0;
-    int b = 0;
-    for (; b + U <= nb; b += U) {
-      T v[U];
+// Sum over b = 0..nb-1 of part[b * C], added in b order; 32 parts are read
+// before the first of them is added (a memory latency per part made a level-0
+// layer's sums 38 us).
+__device__ __forceinline__ float sum_of_parts(const float* part, int nb, long long C) {
+  constexpr int U = 32;
+  float s = 0;
+  int b = 0;
+  for (; b + U <= nb; b += U) {
+    float v[U];
 #pragma unroll
-      for (int u = 0; u < U; ++u) v[u] = part[(size_t)(b + u) * C + c];
+    for (int u = 0; u < U; ++u) v[u] = part[(size_t)(b + u) * C];
 #pragma unroll
-      for (int u = 0; u < U; ++u) s += v[u];
-    }
-    for (; b < nb; ++b) s += part[(size_t)b * C + c];
-    out[c] = accumulate ? out[c] + s : s;
+    for (int u = 0; u < U; ++u) s += v[u];
+  }
+  for (; b < nb; ++b) s += part[(size_t)b * C];
+  return s;
+}
+// The weight gradient's: the chunks' sums [27][cout][cin_pad] added into the
+// gradient of the real [27][cout][cin] weights.
+__global__ void sum_wgrad_kernel(const float* part, int nb, int cin, int cin_pad, int cout, float* g) {
+  const int n = 27 * cout * cin;
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+    const int rest = t / cin, ci = t - rest * cin;
+    g[t] += sum_of_parts(part + (size_t)rest * cin_pad + ci, nb, 27LL * cout * cin_pad);
   }
 }
+__global__ void sum_parts_kernel(const float* part, int nb, long long C, float* out) {
+  for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < C; c += (long long)gridDim.x * blockDim.x)
+    out[c] += sum_of_parts(part + c, nb, C);
+}
 
-// Weight gradient of one layer into dw [27][cout][cin] (written).
-static int conv_wgrad(cudaStream_t s, WgradArgs a, float* dw) {
+// *out = the sum of the blocks' losses, by one block in a fixed order (one
+// thread's chain of FP64 additions was 120 us for 2048 blocks).
+__global__ void sum_loss_kernel(const double* part, int nb, double* out) {
+  __shared__ double sh[32];
+  double t = 0.0;
+  for (int b = threadIdx.x; b < nb; b += blockDim.x) t += part[b];
+  t = block_sum(t, sh);
+  if (threadIdx.x == 0) *out = t;
+}
+
+// Weight gradient of one layer, added into g [27][cout][cin] (cin real input channels).
+static int conv_wgrad(cudaStream_t s, WgradArgs a, int cin, float* g) {
   if (a.cout % 16 || a.cin % 8) return TTFLD_E_ARGS;
   const long long V = (long long)a.X * a.Y * a.Z;
   // at most one full wave of warps, each summing a long run of voxels
@@ -910,23 +933,31 @@ static int conv_wgrad(cudaStream_t s, WgradArgs a, float* dw) {
     case 16: conv3_wgrad_kernel<16><<<blocks, 256, 0, s>>>(a); break;
     default: return TTFLD_E_UNSUPPORTED;
   }
-  const long long C = 27LL * a.cout * a.cin;
-  sum_parts_kernel<float><<<grid_for(C), 256, 0, s>>>(a.part, (int)nch, C, dw, 0);
+  const int threads = 64;  // few weights and long sums: as many SMs as there are
+  sum_wgrad_kernel<<<(27 * a.cout * cin + threads - 1) / threads, threads, 0, s>>>(a.part, (int)nch, cin, a.cin, a.cout, g);
   count_launches(2);
   TT_CHECK_LAUNCH();
   return 0;
 }
 
 // ---- elementwise pieces -------------------------------------------------
-// dZ = dY * leaky'(Y) in place, on a channel slice
+// dZ = dY * leaky'(Y) in place, on a channel slice (8 channels a thread; the
+// channel strides, offsets and counts are multiples of 8)
 __global__ void act_bwd_kernel(bf16* dy, int dy_cs, int dy_co, const bf16* y, int y_cs, int y_co, int C, long long V) {
-  const long long n = V * C;
+  const int C8 = C >> 3;
+  const long long n = V * C8;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-    const long long v = t / C;
-    const int c = (int)(t % C);
-    bf16* p = dy + (size_t)v * dy_cs + dy_co + c;
-    const float yv = __bfloat162float(y[(size_t)v * y_cs + y_co + c]);
-    if (!(yv > 0.f)) *p = __float2bfloat16_rn(__bfloat162float(*p) * kLeak);
+    const long long v = t / C8;
+    const int c = (int)(t % C8) * 8;
+    uint4* p = reinterpret_cast<uint4*>(dy + (size_t)v * dy_cs + dy_co + c);
+    uint4 d = *p;
+    const uint4 yv = *reinterpret_cast<const uint4*>(y + (size_t)v * y_cs + y_co + c);
+    bf16* db = reinterpret_cast<bf16*>(&d);
+    const bf16* yb = reinterpret_cast<const bf16*>(&yv);
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
+      if (!(__bfloat162float(yb[e]) > 0.f)) db[e] = __float2bfloat16_rn(__bfloat162float(db[e]) * kLeak);
+    *p = d;
   }
 }
 
@@ -1216,17 +1247,6 @@ __global__ void adam_kernel(float* p, const float* g, float* m, float* v, size_t
   }
 }
 
-// wgrad accumulates [27][cout][cin_pad]; fold it into the FP32 gradient of
-// the real [27][cout][cin] weights
-__global__ void wgrad_fold_kernel(const float* gpad, int cin, int cin_pad, int cout, float* g) {
-  const long long n = 27LL * cout * cin;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-    const int ci = (int)(t % cin);
-    const long long rest = t / cin;
-    g[t] += gpad[rest * cin_pad + ci];
-  }
-}
-
 // ---- features from the step's state ------------------------------------
 // L0 voxel (x,y,z) = interior cell (i,j,k) = (x+1, y+1, z+1)
 // In FP32: the features are rounded to BF16 anyway, and FP64 logarithms
@@ -1426,18 +1446,23 @@ int forward(ttfld_ctx* c) {
 
 // Backward of one conv layer: dY (in place -> dZ), weight/bias gradients,
 // and (when gx != null) the input gradient, written or accumulated.
-// Gradient workspace of one training call: the padded weight gradient of a
-// layer, the per-chunk weight-gradient sums, and the per-block sums of the
-// bias, head and loss reductions (each added in a fixed order).
+// Gradient workspace of one training call: the per-chunk weight-gradient sums
+// of a layer, and the per-block sums of the bias, head and loss reductions
+// (each added in a fixed order).
 constexpr int kMaxGradBlocks = 4096;  // >= any grid_for() grid
 struct GradWork {
-  float* gpad;   // max_wpad()
   float* wpart;  // max_wpart()
   float* bpart;  // kMaxGradBlocks x 64
   float* hpart;  // kMaxGradBlocks x 17
   double* lpart; // kMaxGradBlocks
 };
 
+// The chain through the layers (leaky', backward-data) runs on the context's
+// stream; once dZ is there, the layer's weight and bias gradients, which the
+// chain does not wait for and which alone leave most SMs idle, run on two side
+// streams.  Nothing writes dZ again in this pass, the layers share the partial
+// sums' workspace in stream order, and backward() joins the streams: 2.1 -> 1.6
+// ms per loss and gradient at 64x128x64 (with the sums below batched).
 int conv_backward(ttfld_ctx* c, GradWork* gw, int l, bf16* gy, int gy_cs, int gy_co, const bf16* y, int y_cs, int y_co,
                   const bf16* x, int x_cs, int x_co, bf16* gx, int gx_cs, int gx_co, int accum, int lev) {
   Net* n = net_of(c);
@@ -1445,15 +1470,17 @@ int conv_backward(ttfld_ctx* c, GradWork* gw, int l, bf16* gy, int gy_cs, int gy
   cudaStream_t st = c->stream;
   const long long V = L(lev).vox();
   int rc;
-  act_bwd_kernel<<<GRID(V * s.cout), 256, 0, st>>>(gy, gy_cs, gy_co, y, y_cs, y_co, s.cout, V);
+  act_bwd_kernel<<<GRID(V * s.cout / 8), 256, 0, st>>>(gy, gy_cs, gy_co, y, y_cs, y_co, s.cout, V);
+  cudaStream_t sw = n->side[0], sb = n->side[1];
+  TT_CHECK(cudaEventRecord(n->dz_ready, st));
+  TT_CHECK(cudaStreamWaitEvent(sw, n->dz_ready, 0));
+  TT_CHECK(cudaStreamWaitEvent(sb, n->dz_ready, 0));
   const int bblocks = GRID(V / 8 + 1);
-  bias_grad_kernel<<<bblocks, 512, 0, st>>>(gy, gy_cs, gy_co, s.cout, V, gw->bpart);
-  sum_parts_kernel<float><<<1, 64, 0, st>>>(gw->bpart, bblocks, s.cout, n->g + n->boff[l], 1);
+  bias_grad_kernel<<<bblocks, 512, 0, sb>>>(gy, gy_cs, gy_co, s.cout, V, gw->bpart);
+  sum_parts_kernel<<<1, 64, 0, sb>>>(gw->bpart, bblocks, s.cout, n->g + n->boff[l]);
   count_launches(3);
   WgradArgs wa{gy, gy_cs, gy_co, s.cout, x, x_cs, x_co, s.cin_pad, gw->wpart, L(lev).X, L(lev).Y, L(lev).Z, 0};
-  if ((rc = conv_wgrad(st, wa, gw->gpad))) return rc;
-  wgrad_fold_kernel<<<GRID(27LL * s.cout * s.cin), 256, 0, st>>>(gw->gpad, s.cin, s.cin_pad, s.cout, n->g + n->woff[l]);
-  count_launches(1);
+  if ((rc = conv_wgrad(sw, wa, s.cin, n->g + n->woff[l]))) return rc;
   if (gx) {
     ConvArgs a;
     a.in = gy; a.in_cs = gy_cs; a.in_co = gy_co; a.cin = s.cout;
@@ -1468,8 +1495,7 @@ int conv_backward(ttfld_ctx* c, GradWork* gw, int l, bf16* gy, int gy_cs, int gy
   return 0;
 }
 
-// Loss against n->target/mask and the gradients of every parameter (n->g).
-int backward(ttfld_ctx* c, GradWork* gw, double* loss_out) {
+int backward_layers(ttfld_ctx* c, GradWork* gw) {
   Net* n = net_of(c);
   cudaStream_t s = c->stream;
   const long long V0 = L(0).vox(), VF = n->full.vox();
@@ -1482,10 +1508,10 @@ int backward(ttfld_ctx* c, GradWork* gw, double* loss_out) {
   mask_count_kernel<<<lblocks, 256, 0, s>>>(n->mask, VF, count);
   count_launches(1);
   loss_kernel<<<lblocks, 256, 0, s>>>(n->pred, n->target, n->mask, VF, count, n->gpred, gw->lpart);
-  sum_parts_kernel<double><<<1, 32, 0, s>>>(gw->lpart, lblocks, 1, n->loss_acc, 0);
+  sum_loss_kernel<<<1, 256, 0, s>>>(gw->lpart, lblocks, n->loss_acc);
   pred_down_kernel<<<GRID(V0), 256, 0, s>>>(n->gpred, n->full, n->gpred_half, L(0));
   head_bwd_kernel<<<hblocks, 256, 0, s>>>(n->gpred_half, n->a13, n->p + n->hoff, n->g_a13, gw->hpart, V0);
-  sum_parts_kernel<float><<<1, 32, 0, s>>>(gw->hpart, hblocks, 17, n->g + n->hoff, 1);
+  sum_parts_kernel<<<1, 32, 0, s>>>(gw->hpart, hblocks, 17, n->g + n->hoff);
   count_launches(5);
 #define BWD(l, gy, gcs, gco, y, ycs, yco, x, xcs, xco, gx, gxcs, gxco, acc, lev)                                  \
   if ((rc = conv_backward(c, gw, l, gy, gcs, gco, y, ycs, yco, x, xcs, xco, gx, gxcs, gxco, acc, lev))) return rc;
@@ -1512,7 +1538,19 @@ int backward(ttfld_ctx* c, GradWork* gw, double* loss_out) {
 #undef BWD
   count_launches(6);
   TT_CHECK_LAUNCH();
-  if ((rc = check_umma(s))) return rc;
+  return 0;
+}
+
+// Loss against n->target/mask and the gradients of every parameter (n->g).
+int backward(ttfld_ctx* c, GradWork* gw, double* loss_out) {
+  Net* n = net_of(c);
+  cudaStream_t s = c->stream;
+  int rc = backward_layers(c, gw);
+  for (int q = 0; q < 2; ++q) {  // also after an error
+    TT_CHECK(cudaEventRecord(n->done[q], n->side[q]));
+    TT_CHECK(cudaStreamWaitEvent(s, n->done[q], 0));
+  }
+  if (rc || (rc = check_umma(s))) return rc;
   if (loss_out) {
     double h = 0.0;
     TT_CHECK(cudaMemcpyAsync(&h, n->loss_acc, sizeof(double), cudaMemcpyDeviceToHost, s));
@@ -1533,29 +1571,27 @@ size_t max_wpart() {
   return m;
 }
 
-// Largest [27][cout][cin_pad] of the layers (the padded weight-gradient buffer).
-size_t max_wpad(const Net* n) {
-  size_t m = 0;
-  for (int l = 0; l < kNumConv; ++l) {
-    size_t v = (size_t)27 * kLayers[l].cout * kLayers[l].cin_pad;
-    if (v > m) m = v;
-  }
-  return m;
-}
-
-// The gradient workspace: one allocation, made by the first training call and
-// kept with the network (an allocation and a free per call cost 0.4 ms).
+// The gradient workspace (one allocation) and the side streams, made by the
+// first training call and kept with the network (an allocation and a free per
+// call cost 0.4 ms).
 int grad_work(Net* n, GradWork* gw) {
-  const size_t a = align256(max_wpad(n) * 4), b = align256(max_wpart() * 4);
+  const size_t b = align256(max_wpart() * 4);
   const size_t c = align256((size_t)kMaxGradBlocks * 64 * 4), d = align256((size_t)kMaxGradBlocks * 17 * 4);
   const size_t e = align256((size_t)kMaxGradBlocks * 8);
-  if (!n->grad_mem) TT_CHECK(cudaMalloc(&n->grad_mem, a + b + c + d + e));
+  if (!n->grad_mem) TT_CHECK(cudaMalloc(&n->grad_mem, b + c + d + e));
   char* p = (char*)n->grad_mem;
-  gw->gpad = (float*)p;
-  gw->wpart = (float*)(p + a);
-  gw->bpart = (float*)(p + a + b);
-  gw->hpart = (float*)(p + a + b + c);
-  gw->lpart = (double*)(p + a + b + c + d);
+  gw->wpart = (float*)p;
+  gw->bpart = (float*)(p + b);
+  gw->hpart = (float*)(p + b + c);
+  gw->lpart = (double*)(p + b + c + d);
+  if (!n->joined) {
+    for (int q = 0; q < 2; ++q) {
+      if (!n->side[q]) TT_CHECK(cudaStreamCreateWithFlags(&n->side[q], cudaStreamNonBlocking));
+      if (!n->done[q]) TT_CHECK(cudaEventCreateWithFlags(&n->done[q], cudaEventDisableTiming));
+    }
+    if (!n->dz_ready) TT_CHECK(cudaEventCreateWithFlags(&n->dz_ready, cudaEventDisableTiming));
+    n->joined = 1;
+  }
   return 0;
 }
 
@@ -1631,6 +1667,11 @@ void unet_free(ttfld_ctx* c) {
   if (n->act_mem) cudaFree(n->act_mem);
   if (n->grad_mem) cudaFree(n->grad_mem);
   if (n->feat_stage) cudaFree(n->feat_stage);
+  for (int q = 0; q < 2; ++q) {
+    if (n->side[q]) cudaStreamDestroy(n->side[q]);
+    if (n->done[q]) cudaEventDestroy(n->done[q]);
+  }
+  if (n->dz_ready) cudaEventDestroy(n->dz_ready);
   if (n->ds_feat) cudaFree(n->ds_feat);
   free(n);
   c->unet = nullptr;
