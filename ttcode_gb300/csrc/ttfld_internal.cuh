@@ -488,6 +488,8 @@ struct ttfld_ctx {
   ttfld::SolverDev* sol;
   ttfld::StepDev* stp;
   ttfld::SolverDev* host_sol;  // pinned mirror
+  void* sweep_copy;          // coefficients in the order of the FP64 sweeps (allocated on first use)
+  size_t sweep_copy_bytes;
   // mixed-precision workspace (allocated on first use)
   void* mix_slab;
   size_t mix_bytes;

@@ -1485,6 +1485,7 @@ struct FastRows {
   typedef double2 Word;
   typedef double2 Kept;
   static constexpr int kWords = 8, kThreads = 768;  // 196 KB for two stages
+  static constexpr bool kStrided = false;
   Fast64 m;
   double omega;
   long long rows;
@@ -1557,7 +1558,7 @@ static int launch_fast_persistent(ttfld_ctx* c, int nsweeps, int itmin, int itma
   s.by_items = g.by_pairs;
   s.by_ny = c->d.by_ny;
   return launch_sweeps64_persistent(s, c->stream, c->sol, c->partials, c->flags64, c->staging, c->staging_bytes,
-                                    nsweeps, itmin, itmax, eps);
+                                    nsweeps, itmin, itmax, eps, c);
 }
 
 int launch_sweeps64(ttfld_ctx* c, int nsweeps, int itmin, int itmax, double eps) {

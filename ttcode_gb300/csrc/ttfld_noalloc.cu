@@ -253,7 +253,8 @@ extern "C" int ttfld_sor_solve_noalloc(const double* sor_a, const double* sor_b,
   const double* const coef[7] = {sor_a, sor_b, sor_c, sor_d, sor_e, sor_f, sor_g};
   rc = launch_sweeps64_persistent(sor_rows(coef, rhs, x, nx, ny, nz, nz, 0, omega), st, &s->st, s->partials[0],
                                   (unsigned int*)s->partials[1], s->partials[0] + 2 * kMaxPartials,
-                                  (kNoAllocMaxRows - 2 * kMaxPartials) * sizeof(double), itmax, itmin, itmax, epsmat);
+                                  (kNoAllocMaxRows - 2 * kMaxPartials) * sizeof(double), itmax, itmin, itmax, epsmat,
+                                  nullptr);
   if (rc < 0) return rc;
   if (rc == 0) {
     TT_CHECK(cudaMemcpyAsync(&h, &s->st, sizeof(h), cudaMemcpyDeviceToHost, st));

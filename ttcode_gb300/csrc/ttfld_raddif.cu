@@ -228,6 +228,7 @@ struct RadRows {
   typedef double Word;
   typedef double Kept;
   static constexpr int kWords = 8, kThreads = 1024;
+  static constexpr bool kStrided = true;
   Dev d;
   RadWork w;
   double om, d_t, tinit_bottom;
@@ -357,7 +358,7 @@ int solvmat_persistent(ttfld_ctx* c, const RadWork& w, double d_t, double tinit_
   s.by_items = d.by_nxh;
   // a moving top is not kept: its decisions are waited for
   const int rc = launch_sweeps64_persistent(s, c->stream, c->sol, c->partials, c->flags64, c->staging,
-                                            s.moving_top ? 0 : c->staging_bytes, d.itmax, 5, d.itmax, d.epsmat);
+                                            s.moving_top ? 0 : c->staging_bytes, d.itmax, 5, d.itmax, d.epsmat, c);
   if (rc) return rc;
   radbound_ghost_bottom<<<grid_for((long long)(d.ny + 4) * (d.nz + 4)), kThreads, 0, c->stream>>>(d, d_t, tinit_bottom);
   radbound_ghost_theta<<<grid_for((long long)(d.nx + 4) * (d.ny + 4)), kThreads, 0, c->stream>>>(d);

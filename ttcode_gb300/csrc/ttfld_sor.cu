@@ -226,7 +226,7 @@ static int launch_exact_persistent(ttfld_ctx* c, double* x, const double* b, int
   const double* const coef[7] = {d.SA, d.SB, d.SC, d.SD, d.SE, d.SF, d.SG};
   const SorRows sys = sor_rows(coef, b, x, d.nx, d.ny, d.nz, sor_zmax(d), d.poles, d.sorparam);
   return launch_sweeps64_persistent(sys, c->stream, c->sol, c->partials, c->flags64, c->staging, c->staging_bytes,
-                                    nsweeps, itmin, itmax, eps);
+                                    nsweeps, itmin, itmax, eps, c);
 }
 
 // The same, by two launches per sweep where one launch is not possible.

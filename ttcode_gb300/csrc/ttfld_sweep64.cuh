@@ -26,6 +26,14 @@
 // 52.2 -> 50.0 ms for the scaled SOR and 5.06 -> 4.75 ms for DIFFUSION at
 // 100x256x128, 11.9 -> 11.3 ms for DIFFUSION at 160x256x192.
 //
+// Where a system's items are every other cell of its arrays (kStrided), each
+// colour's pass reads the lines of both colours.  Not RESIDENT, the first
+// sweep therefore stores what each thread has fetched for its items, in the
+// order in which it will want it, and later sweeps fetch from that copy, half
+// the bytes: DIFFUSION 4.72 -> 4.46 ms at 100x256x128 and 11.3 -> 10.4 at
+// 160x256x192, the exact SOR 58.9 -> 56.5 ms at 100x256x100, RADDIF 25.2 ->
+// 24.2 there.  (The FP64 pipe is then busy two thirds of the time.)
+//
 // A system is a struct with
 //   rows, by_items          (j,k) rows, and the items of a colour in a row
 //   kWords, Word            its coefficients of an item, as kWords of Word
@@ -35,6 +43,7 @@
 //                           returns its share of the norm; first: no colour
 //                           has run yet; kept: where the old value (Kept) goes
 //   restore(row, h, kept)   puts a value of the first colour back
+//   kStrided                the items of a colour are not contiguous in memory
 //   before<COL>(r0, r1), after<COL>(r0, r1, first)  a block's own work around
 //                           a colour (all its threads; boundary values of its rows)
 //   norm(sum)               the norm from the sum of the shares
@@ -79,13 +88,37 @@ __device__ __forceinline__ void undo_colour(const Sys& s, unsigned int r0, unsig
   }
 }
 
+// The copy that later sweeps fetch from: word q of item u of a block at
+// at[COL][q * n + u] (null: none, or not yet written).
+template <class Word>
+struct SweepCopy {
+  const Word* now;   // of this colour
+  const Word* next;  // of the colour that follows
+  Word* store;       // written in the first sweep
+};
+
+// Queue the copies of item u of a block's n.
+template <int COL, class Sys>
+__device__ __forceinline__ void fetch_item(const Sys& s, unsigned int r0, unsigned int n, unsigned int u,
+                                           const typename Sys::Word* copy, typename Sys::Word* to, unsigned int T,
+                                           uint64_t pol) {
+  if (Sys::kStrided && copy) {
+#pragma unroll
+    for (int q = 0; q < Sys::kWords; ++q) copy_async(to + q * T, copy + (size_t)q * n + u, pol);
+    return;
+  }
+  unsigned int h;
+  const unsigned int r = r0 + div_rem(s.by_items, u, h);
+  s.template fetch<COL>(r, h, to, T, pol);
+}
+
 // The items of one colour of a block's rows.  Not RESIDENT: the thread's
 // next item (of this colour, or its first of the other) is fetched before
 // the present one is updated.  mine: where to keep the values replaced.
 template <int COL, bool RESIDENT, class Sys>
 __device__ __forceinline__ double sweep_colour(const Sys& s, unsigned int r0, unsigned int n, bool first,
                                                typename Sys::Word* slots, int& stage, typename Sys::Kept* mine,
-                                               uint64_t pol) {
+                                               uint64_t pol, const SweepCopy<typename Sys::Word>& copy) {
   double acc = 0.0;
   const unsigned int T = blockDim.x;
   for (unsigned int u = threadIdx.x; u < n; u += T) {
@@ -98,16 +131,14 @@ __device__ __forceinline__ double sweep_colour(const Sys& s, unsigned int r0, un
     const typename Sys::Word* now = slots + (size_t)stage * Sys::kWords * T + threadIdx.x;
     stage ^= 1;
     typename Sys::Word* next = slots + (size_t)stage * Sys::kWords * T + threadIdx.x;
-    unsigned int hn;
-    if (u + T < n) {
-      const unsigned int rn = r0 + div_rem(s.by_items, u + T, hn);
-      s.template fetch<COL>(rn, hn, next, T, pol);
-    } else {
-      const unsigned int rn = r0 + div_rem(s.by_items, threadIdx.x, hn);
-      s.template fetch<1 - COL>(rn, hn, next, T, pol);
-    }
+    if (u + T < n) fetch_item<COL>(s, r0, n, u + T, copy.now, next, T, pol);
+    else fetch_item<1 - COL>(s, r0, n, threadIdx.x, copy.next, next, T, pol);
     asm volatile("cp.async.commit_group;" ::: "memory");
     asm volatile("cp.async.wait_group 1;" ::: "memory");
+    if (Sys::kStrided && copy.store) {
+#pragma unroll
+      for (int q = 0; q < Sys::kWords; ++q) copy.store[(size_t)q * n + u] = now[q * T];
+    }
     acc += s.template update<COL>(r, h, now, T, first, mine ? mine + u : nullptr);
   }
   return acc;
@@ -116,7 +147,8 @@ __device__ __forceinline__ double sweep_colour(const Sys& s, unsigned int r0, un
 template <class Sys, bool RESIDENT>
 __global__ void __launch_bounds__(Sys::kThreads, 1)
     sweeps64_persistent(Sys s, SolverDev* sol, Partial* gather, unsigned int* flags, typename Sys::Kept* keep,
-                        int nsweeps, int itmin, int itmax, double eps, float coef_keep) {
+                        int nsweeps, int itmin, int itmax, double eps, float coef_keep,
+                        typename Sys::Word* copy) {
   __shared__ double sh[32];
   __shared__ int stop_sh, ok_sh;
   if (threadIdx.x == 0) {  // read after block barriers only
@@ -152,6 +184,9 @@ __global__ void __launch_bounds__(Sys::kThreads, 1)
     s.template fetch<0>(r, h, slots + threadIdx.x, blockDim.x, pol);
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
+  typedef SweepCopy<typename Sys::Word> Copy;
+  typename Sys::Word* copy0 = copy ? copy + (size_t)r0 * s.by_items.d * 2 * Sys::kWords : nullptr;
+  typename Sys::Word* copy1 = copy ? copy0 + (size_t)Sys::kWords * n : nullptr;
   typename Sys::Kept* mine = keep ? keep + (size_t)r0 * s.by_items.d : nullptr;
   unsigned int* own = flags + (size_t)b * kFlagStride;
   unsigned int half = 0;  // half-sweeps this block has finished
@@ -159,7 +194,8 @@ __global__ void __launch_bounds__(Sys::kThreads, 1)
   for (int sw = 1; sw <= nsweeps && !stop; ++sw) {
     if (sw > 1 && !wait_flags(flags, lo, hi, half, sol)) break;
     s.template before<0>(r0, r1);
-    double acc = sweep_colour<0, RESIDENT>(s, r0, n, sw == 1, slots, stage, sw > 1 ? mine : nullptr, pol);
+    double acc = sweep_colour<0, RESIDENT>(s, r0, n, sw == 1, slots, stage, sw > 1 ? mine : nullptr, pol,
+                                            sw > 1 ? Copy{copy0, copy1, nullptr} : Copy{nullptr, nullptr, copy0});
     s.template after<0>(r0, r1, sw == 1);
     publish_flag(own, ++half);
     // the first warp waits for the neighbours, the last takes the last
@@ -176,7 +212,8 @@ __global__ void __launch_bounds__(Sys::kThreads, 1)
       break;
     }
     s.template before<1>(r0, r1);
-    acc += sweep_colour<1, RESIDENT>(s, r0, n, false, slots, stage, nullptr, pol);
+    acc += sweep_colour<1, RESIDENT>(s, r0, n, false, slots, stage, nullptr, pol,
+                                      sw > 1 ? Copy{copy1, copy0, nullptr} : Copy{nullptr, copy0, copy1});
     s.template after<1>(r0, r1, false);
     acc = warp_sum_all(acc);
     if (lane == 0) sh[warp] = acc;
@@ -197,12 +234,31 @@ __global__ void __launch_bounds__(Sys::kThreads, 1)
   asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
+// The context's copy of a system's coefficients, 64 bytes a cell, allocated by
+// the first solve that wants it; null where there is no room.
+inline void* sweep_copy(ttfld_ctx* c, size_t bytes) {
+  if (c->sweep_copy_bytes < bytes) {
+    if (c->sweep_copy) cudaFree(c->sweep_copy);
+    c->sweep_copy = nullptr;
+    c->sweep_copy_bytes = 0;
+    if (cudaMalloc(&c->sweep_copy, bytes) != cudaSuccess) {
+      cudaGetLastError();
+      c->sweep_copy = nullptr;
+      return nullptr;
+    }
+    c->sweep_copy_bytes = bytes;
+  }
+  return c->sweep_copy;
+}
+
 // Queue nsweeps sweeps of a system (fewer if the rule fires).  1 where the
 // launch is not possible (no cooperative launch, or fewer SMs to be had than
-// blocks): the caller runs one launch per colour instead.
+// blocks): the caller runs one launch per colour instead.  owner: the context
+// that holds the copy of the coefficients (null: none is made).
 template <class Sys>
 int launch_sweeps64_persistent(const Sys& s, cudaStream_t st, SolverDev* sol, double* partials, unsigned int* flags,
-                               void* kept, size_t kept_bytes, int nsweeps, int itmin, int itmax, double eps) {
+                               void* kept, size_t kept_bytes, int nsweeps, int itmin, int itmax, double eps,
+                               ttfld_ctx* owner) {
   int dev = 0, sms = 0, coop = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
@@ -236,7 +292,11 @@ int launch_sweeps64_persistent(const Sys& s, cudaStream_t st, SolverDev* sol, do
       (size_t)items * sizeof(typename Sys::Kept) <= kept_bytes ? (typename Sys::Kept*)kept : nullptr;
   const double word = 2.0 * (double)items * sizeof(typename Sys::Word);  // an array of both colours
   float coef_keep = l2_keep(word, Sys::kWords * word).coef;
-  void* args[] = {&sys, &sol, &gather, &flags, &keep, &nsweeps, &itmin, &itmax, &eps, &coef_keep};
+  // the first sweep's stores cost about what half a sweep's reads do
+  typename Sys::Word* copy = nullptr;
+  if (Sys::kStrided && !resident && owner && nsweeps >= 4)
+    copy = (typename Sys::Word*)sweep_copy(owner, (size_t)(Sys::kWords * word));
+  void* args[] = {&sys, &sol, &gather, &flags, &keep, &nsweeps, &itmin, &itmax, &eps, &coef_keep, &copy};
   const cudaError_t e =
       cudaLaunchCooperativeKernel(kernel, dim3((unsigned int)nb), dim3(threads), args, smem, st);
   if (e == cudaErrorCooperativeLaunchTooLarge) {
@@ -258,6 +318,7 @@ struct SorRows {
   typedef double Word;
   typedef double Kept;
   static constexpr int kWords = 8, kThreads = 1024;
+  static constexpr bool kStrided = true;
   const double *a, *xm, *xp, *jm, *jp, *km, *kp, *b;
   double* x;
   double omega;
