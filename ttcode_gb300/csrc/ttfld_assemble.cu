@@ -713,6 +713,7 @@ static int stellar_binned(ttfld_ctx* c) {
 // 40x64x32.)
 constexpr int kTauCols = 32, kTauChunk = 64;
 __global__ void __launch_bounds__(kThreads) stellar_tau_kernel(Dev d) {
+  start_after();
   __shared__ double s[kTauCols][kTauChunk + 1];
   __shared__ int ubs[kTauCols];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -766,7 +767,7 @@ static int stellarinput_heating(ttfld_ctx* c) {
     }
     return stellar_binned(c);
   }
-  stellar_tau_kernel<<<(unsigned int)((nplane(d) + kTauCols - 1) / kTauCols), kThreads, 0, c->stream>>>(d);
+  launch_after(stellar_tau_kernel, (unsigned int)((nplane(d) + kTauCols - 1) / kTauCols), kThreads, 0, c->stream, d);
   count_launches(1);
   TT_CHECK_LAUNCH();
   // STELLAR_DTAU and STELLARINPUT of the same cell in one pass
@@ -795,6 +796,7 @@ static int stellarinput_heating(ttfld_ctx* c) {
 // plane that takes it.  (One thread per column, which reads its radii one
 // after another, and two more launches for the ghosts: 28 us at 100x256x128.)
 __global__ void __launch_bounds__(kThreads) upperbnd_kernel(Dev d) {
+  start_after();
   const unsigned int col = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31, ny = d.ny, nz = d.nz;
   if (col >= (unsigned int)ny * nz) return;
@@ -830,7 +832,7 @@ static int bounds(ttfld_ctx* c) {
   if ((rc = halo_shift(c, d.T, d.RH)) || (rc = pole_shift(c, d.T, d.RH))) return rc;
   {
     const long long lanes = (long long)d.ny * d.nz * 32;
-    upperbnd_kernel<<<(unsigned int)((lanes + kThreads - 1) / kThreads), kThreads, 0, c->stream>>>(d);
+    launch_after(upperbnd_kernel, (unsigned int)((lanes + kThreads - 1) / kThreads), kThreads, 0, c->stream, d);
     count_launches(1);
     TT_CHECK_LAUNCH();
   }

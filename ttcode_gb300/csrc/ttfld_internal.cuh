@@ -134,8 +134,37 @@ inline Box box(int i0, int i1, int j0, int j1, int k0, int k1) {
   return b;
 }
 
+// The kernels of a step follow one another on one stream, and the small ones
+// last a few microseconds, of which starting the next one's blocks is a good
+// part.  launch_after starts them while the kernel before is still running
+// (programmatic stream serialisation), and every kernel launched so begins
+// with start_after, which waits for that kernel's end and its writes before
+// anything is read or written, and then lets the next kernel's blocks start.
+// Implicit step 810 -> 764 us at 40x64x32, 1.60 -> 1.53 ms at 53x90x47 with
+// poles, 13.62 -> 13.56 ms at 100x256x128.
+__device__ __forceinline__ void start_after() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <class... Par, class... Arg>
+inline void launch_after(void (*kernel)(Par...), unsigned int blocks, unsigned int threads, size_t smem, cudaStream_t s,
+                         Arg&&... arg) {
+  cudaLaunchAttribute after;
+  after.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  after.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &after;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, Par(arg)...);
+}
+
 template <class Fn>
 __global__ void __launch_bounds__(kThreads) box_kernel(Box b, Fn fn) {
+  start_after();
   const unsigned int n = (unsigned int)b.ni * b.nj * b.nk;
   for (unsigned int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
     unsigned int i, j;
@@ -151,7 +180,7 @@ template <class Fn>
 inline void launch_box(cudaStream_t s, Box b, Fn fn) {
   long long n = (long long)b.ni * b.nj * b.nk;
   if (n <= 0) return;
-  box_kernel<<<grid_for(n), kThreads, 0, s>>>(b, fn);
+  launch_after(box_kernel<Fn>, grid_for(n), kThreads, 0, s, b, fn);
   count_launches(1);
 }
 

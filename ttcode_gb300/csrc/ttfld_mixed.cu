@@ -150,6 +150,7 @@ void mix_free(ttfld_ctx* c) {
 // norm marks the solve done, so that sweeps queued behind do nothing.
 __global__ void __launch_bounds__(kThreads) prep32_kernel(Dev d, Cmp g, Mix32 m, const double* __restrict__ b,
                                                           double* partials) {
+  start_after();
   __shared__ double sh[32];
   __shared__ bool last;
   const unsigned int n = (unsigned int)ncell(d);
@@ -194,7 +195,7 @@ static int prep32(ttfld_ctx* c, const double* b) {
   MixWork* w = work(c);
   int nb = grid_for((long long)ncell(c->d));
   if (nb > kMaxPartials) nb = kMaxPartials;
-  prep32_kernel<<<nb, kThreads, 0, c->stream>>>(c->d, w->g, w->m32, b, c->partials);
+  launch_after(prep32_kernel, nb, kThreads, 0, c->stream, c->d, w->g, w->m32, b, c->partials);
   count_launches(1);
   TT_CHECK_LAUNCH();
   return 0;
@@ -916,6 +917,7 @@ static int add_correction_unless(ttfld_ctx* c, double* x, int it0) {
 // r = b - A x in FP64 (FMA), its L1 norm (fixed-order) and rhat = r/A in FP32.
 __global__ void __launch_bounds__(kThreads) resid32_kernel(Dev d, Cmp g, Mix32 m, const double* __restrict__ x,
                                                            const double* __restrict__ b, double* partials) {
+  start_after();
   __shared__ double sh[32];
   __shared__ bool last;
   const int nx = d.nx, ny = d.ny;
@@ -964,7 +966,7 @@ static int resid32_launch(ttfld_ctx* c, const double* x, const double* b) {
   MixWork* w = work(c);
   int nb = grid_for((long long)ncell(c->d));
   if (nb > kMaxPartials) nb = kMaxPartials;
-  resid32_kernel<<<nb, kThreads, 0, c->stream>>>(c->d, w->g, w->m32, x, b, c->partials + kMaxPartials);
+  launch_after(resid32_kernel, nb, kThreads, 0, c->stream, c->d, w->g, w->m32, x, b, c->partials + kMaxPartials);
   count_launches(1);
   TT_CHECK_LAUNCH();
   return 0;

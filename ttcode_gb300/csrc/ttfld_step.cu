@@ -144,6 +144,7 @@ static int rows(ttfld_ctx* c, double theta, bool divf_is_old) {
 // (ppenergy.f:379-541), fused with the damped update of :551-573 (each cell
 // reads only its own Q and E_R, which only it updates).
 __global__ void __launch_bounds__(kThreads) delta_q_kernel(Dev d, double theta, double conv) {
+  start_after();
   const int nx = d.nx, ny = d.ny;
   const unsigned int n = (unsigned int)ncell(d);
   const size_t sj = (size_t)(nx + 4), sk = (size_t)(nx + 4) * (ny + 4);
@@ -186,7 +187,7 @@ __global__ void __launch_bounds__(kThreads) delta_q_kernel(Dev d, double theta, 
 
 static int delta_q_update(ttfld_ctx* c, double theta, double conv) {
   const Dev& d = c->d;
-  delta_q_kernel<<<grid_for((long long)ncell(d)), kThreads, 0, c->stream>>>(d, theta, conv);
+  launch_after(delta_q_kernel, grid_for((long long)ncell(d)), kThreads, 0, c->stream, d, theta, conv);
   count_launches(1);
   TT_CHECK_LAUNCH();
   return 0;
