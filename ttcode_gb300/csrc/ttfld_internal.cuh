@@ -327,8 +327,8 @@ __device__ __forceinline__ double warp_sum_all(double v) {
   return v;
 }
 
-// A block's share of a norm, with the norm's number (from 1 in each launch of
-// the persistent sweeps): written and read as one 128-bit word, so that no
+// A block's share of a norm, with the norm's number (from 1, in the persistent
+// FP64 sweeps for each launch): written and read as one 128-bit word, so that no
 // fence orders the two.  Norms alternate between two words a block: when a
 // block writes that of norm k + 2 it has read every block's of norm k + 1,
 // which each wrote after reading those of norm k.
@@ -336,14 +336,14 @@ struct __align__(16) Partial {
   double part;
   unsigned long long number;
 };
-__device__ __forceinline__ void put_partial(Partial* gather, int b, int number, double part) {
+__device__ __forceinline__ void put_partial(Partial* gather, int b, long long number, double part) {
   Partial* p = gather + 2 * (size_t)b + (number & 1);
   asm volatile(
       "{\n .reg .b128 v;\n mov.b128 v, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], v;\n}" ::"l"(p),
-      "l"(__double_as_longlong(part)), "l"((long long)number)
+      "l"(__double_as_longlong(part)), "l"(number)
       : "memory");
 }
-__device__ __forceinline__ bool get_partial(const Partial* gather, int b, int number, double& part) {
+__device__ __forceinline__ bool get_partial(const Partial* gather, int b, long long number, double& part) {
   const Partial* p = gather + 2 * (size_t)b + (number & 1);
   long long v, n;
   asm volatile("{\n .reg .b128 v;\n ld.relaxed.gpu.global.b128 v, [%2];\n mov.b128 {%0, %1}, v;\n}"
@@ -358,7 +358,7 @@ __device__ __forceinline__ bool get_partial(const Partial* gather, int b, int nu
 // block (one warp; every lane gets it).  Bounded like the other waits: false
 // once a block has given up.
 constexpr int kGather = 5;  // shares a lane reads at once: 160 blocks
-__device__ __forceinline__ bool gather_sum(const Partial* gather, int nb, int number, SolverDev* sol, double& tot) {
+__device__ __forceinline__ bool gather_sum(const Partial* gather, int nb, long long number, SolverDev* sol, double& tot) {
   const int lane = threadIdx.x & 31;
   tot = 0.0;
   for (int q0 = lane; q0 - lane < nb; q0 += 32 * kGather) {

@@ -74,6 +74,8 @@ struct MixWork {
   Fast64 m64;
   unsigned int* flags;     // per-block half-sweep counters of the neighbour-flag sweep form
   unsigned int flag_base;  // their value when the next launch of that form starts
+  Partial* gather;         // its norm shares, two a block
+  long long norm_base;     // the norms numbered so far
 };
 
 __host__ __device__ __forceinline__ size_t cslot(const Cmp& g, int j0, int k0, int h) {
@@ -97,7 +99,8 @@ static int ensure32(ttfld_ctx* c) {
   if (w->have32) return 0;
   const Cmp& g = w->g;
   const size_t flag_floats = kFlagBytes / sizeof(float);  // the flags first: 128-byte lines
-  size_t n = flag_floats + 2 * (6 + 3) * g.csz + 2 * g.gsz;
+  const size_t gather_floats = (size_t)kMaxLocalBlocks * 2 * sizeof(Partial) / sizeof(float);
+  size_t n = flag_floats + gather_floats + 2 * (6 + 3) * g.csz + 2 * g.gsz;
   float* p = nullptr;
   TT_CHECK(cudaMalloc((void**)&p, n * sizeof(float)));
   TT_CHECK(cudaMemset(p, 0, n * sizeof(float)));
@@ -105,6 +108,9 @@ static int ensure32(ttfld_ctx* c) {
   w->flags = reinterpret_cast<unsigned int*>(p);
   w->flag_base = 0;
   p += flag_floats;
+  w->gather = reinterpret_cast<Partial*>(p);
+  w->norm_base = 0;
+  p += gather_floats;
   for (int q = 0; q < 6; ++q)
     for (int col = 0; col < 2; ++col) { w->m32.a[q][col] = p; p += g.csz; }
   for (int col = 0; col < 2; ++col) { w->m32.ainv[col] = p; p += g.csz; }
@@ -535,7 +541,7 @@ template <bool POLES, bool RESIDENT = false>
 __global__ void __launch_bounds__(kPersistThreads) sweeps32_local(Cmp g, Mix32 m, float omega, SolverDev* sol,
                                                                  Partial* gather, double stop_ratio, int nsweeps,
                                                                  int norm_every, int stall_check, unsigned int* flags,
-                                                                 unsigned int base, L2Keep l2) {
+                                                                 unsigned int base, long long norms, L2Keep l2) {
   __shared__ double sh[32];
   __shared__ int stop_sh;
   extern __shared__ __align__(16) unsigned char slots_raw[];
@@ -566,7 +572,6 @@ __global__ void __launch_bounds__(kPersistThreads) sweeps32_local(Cmp g, Mix32 m
   double last_ratio = -1.0;  // in-sweep ratio of the previous norm sweep (lane 0 of the last warp)
   const KeepPolicy keep = {l2_policy(l2.coef), l2_policy(l2.iter)};
   const int it0 = sol->iter;
-  int norms = 0;
   unsigned int half = base;  // half-sweeps this block has finished
   int sw = 1;
   for (; sw <= nsweeps; ++sw) {
@@ -895,20 +900,22 @@ static int add_correction(ttfld_ctx* c, double* x) {
 
 // The same, queued behind the sweeps before their state is read back: it
 // does nothing when they made no progress (SOR_ITER still it0) or met a
-// non-finite norm, the cases in which the solve loop leaves x as it is.
+// non-finite norm, the cases in which the solve loop leaves x as it is.  e is
+// zero afterwards, for the next sweeps.
 static int add_correction_unless(ttfld_ctx* c, double* x, int it0) {
   MixWork* w = work(c);
   Dev d = c->d;
   Cmp g = w->g;
-  const float* e0 = w->m32.e[0];
-  const float* e1 = w->m32.e[1];
+  float* e0 = w->m32.e[0];
+  float* e1 = w->m32.e[1];
   const SolverDev* sol = c->sol;
   launch_box(c->stream, box(1, d.nx, 1, d.ny, 1, d.nz), [=] __device__(int i, int j, int k) {
     if (sol->iter == it0 || sol->nonfinite) return;
     int col = (i + j + k) & 1;
-    const float* e = col ? e1 : e0;
+    float* e = (col ? e1 : e0) + gslot(g, j - 1, k - 1, (i - 1) >> 1);
     size_t q = hidx(d, i, j, k);
-    x[q] = x[q] + f64_of_f32(e[gslot(g, j - 1, k - 1, (i - 1) >> 1)]);
+    x[q] = x[q] + f64_of_f32(*e);
+    *e = 0.f;
   });
   TT_CHECK_LAUNCH();
   return 0;
@@ -956,12 +963,13 @@ __global__ void __launch_bounds__(kThreads) resid32_kernel(Dev d, Cmp g, Mix32 m
     if (threadIdx.x == 0) {
       d.sol->true_l1 = tot;
       d.sol->ticket2 = 0;
+      d.sol->done = 0;
     }
   }
 }
 
 // The FP64 anchor queued: SolverDev::true_l1 holds ||b - A x||_1 once it has
-// run (read back with the next poll).
+// run (read back with the next poll), and SolverDev::done is 0.
 static int resid32_launch(ttfld_ctx* c, const double* x, const double* b) {
   MixWork* w = work(c);
   int nb = grid_for((long long)ncell(c->d));
@@ -1131,10 +1139,10 @@ static int launch_sweeps32_form(ttfld_ctx* c, int nsweeps, int norm_every, doubl
   if (form == kFormNeighbour && gr.local > 0) {
     unsigned int* flags = w->flags;
     unsigned int base = w->flag_base;
-    Partial* gather = (Partial*)partials;  // two a block
-    TT_CHECK(cudaMemsetAsync(gather, 0, (size_t)gr.local * 2 * sizeof(Partial), c->stream));
+    Partial* gather = w->gather;
+    long long norms = w->norm_base;  // no number is used twice, so nothing is cleared between launches
     L2Keep l2 = gr.l2;
-    void* largs[] = {&g, &m, &omega, &sol, &gather, &stop_ratio, &nsweeps, &norm_every, &stall, &flags, &base, &l2};
+    void* largs[] = {&g, &m, &omega, &sol, &gather, &stop_ratio, &nsweeps, &norm_every, &stall, &flags, &base, &norms, &l2};
     if (gr.resident)
       TT_CHECK(cudaLaunchCooperativeKernel((const void*)sweeps32_local<POLES, true>, dim3(gr.local),
                                            dim3(gr.local_threads), largs, gr.local_smem, c->stream));
@@ -1142,6 +1150,7 @@ static int launch_sweeps32_form(ttfld_ctx* c, int nsweeps, int norm_every, doubl
       TT_CHECK(cudaLaunchCooperativeKernel((const void*)sweeps32_local<POLES>, dim3(gr.local), dim3(gr.local_threads),
                                            largs, gr.local_smem, c->stream));
     w->flag_base = base + 2u * (unsigned int)nsweeps;  // every block leaves its flag there
+    w->norm_base = norms + nsweeps;
     count_launches(1);
     return 0;
   }
@@ -1224,6 +1233,7 @@ int solve_mixed(ttfld_ctx* c, double* x, const double* b, ttfld_solve_stats* st,
   double tight = 1.0;  // halved each time the in-sweep norm met tol but the FP64 residual did not
   bool hit_tol = false;
   bool resume = false;  // the first anchor and its first sweeps are done already
+  bool e_zero = false;  // add_correction_unless has left e so
   if (fallback) *fallback = 0;
   const SweepForm form = c->opts.sweep_form == 1   ? kFormTma
                          : c->opts.sweep_form == 2 ? kFormSplit
@@ -1278,8 +1288,8 @@ int solve_mixed(ttfld_ctx* c, double* x, const double* b, ttfld_solve_stats* st,
     const double anchor = l1 / bl1;
     const double stop = fmax(tol * tight, anchor * pow(10.0, -c->opts.inner_digits));
     hit_tol = stop <= tol;
-    if (!resume) TT_CHECK(cudaMemsetAsync(w->m32.e[0], 0, 2 * g.gsz * sizeof(float), c->stream));  // e[0], e[1] adjacent
-    if (!unread) TT_CHECK(cudaMemsetAsync(&c->sol->done, 0, sizeof(int), c->stream));
+    if (!resume && !e_zero) TT_CHECK(cudaMemsetAsync(w->m32.e[0], 0, 2 * g.gsz * sizeof(float), c->stream));  // e[0], e[1] adjacent
+    if (resume) TT_CHECK(cudaMemsetAsync(&c->sol->done, 0, sizeof(int), c->stream));  // else the anchor's work, or unread
     resume = false;
     int it0 = c->host_sol->iter;
     double r_prev = anchor;
@@ -1296,6 +1306,7 @@ int solve_mixed(ttfld_ctx* c, double* x, const double* b, ttfld_solve_stats* st,
       if ((rc = launch_sweeps32(c, n, period, stop, form)) || (rc = add_correction_unless(c, x, it0)) ||
           (rc = resid32_launch(c, x, b)) || (rc = poll(c)))
         return rc;
+      e_zero = true;
       if (c->host_sol->nonfinite) status = TTFLD_E_NONFINITE;
       if (c->host_sol->stalled) {
         ++stalls;
