@@ -129,6 +129,7 @@ struct ConvArgs {
 // would otherwise leave most SMs idle while a few warps walk all 27 taps.
 template <int KS>
 __global__ void __launch_bounds__(256) conv3_fwd_kernel(ConvArgs a) {
+  start_after();
   constexpr int TPC = 8 / KS;  // tiles per CTA
   __shared__ float red[KS > 1 ? 8 : 1][8][32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -227,6 +228,7 @@ static size_t conv_smem_bytes(int cin, int cout, bool with_w) {
 
 template <int NB>
 __global__ void __launch_bounds__(256) conv3_smem_kernel(ConvArgs a, int w_in_smem) {
+  start_after();
   extern __shared__ __align__(16) unsigned char csm[];
   const int cst = a.cin + 8;  // padded row, in bf16
   bf16* tin = reinterpret_cast<bf16*>(csm);
@@ -320,7 +322,7 @@ static int launch_conv_smem(cudaStream_t s, const ConvArgs& a) {
     opted = 200 * 1024;
   }
   const long long blocks = (long long)((a.X + kTX - 1) / kTX) * ((a.Y + kTY - 1) / kTY) * ((a.Z + kTZ - 1) / kTZ);
-  conv3_smem_kernel<NB><<<(unsigned)blocks, 256, smem, s>>>(a, with_w ? 1 : 0);
+  launch_after(conv3_smem_kernel<NB>, (unsigned)blocks, 256, smem, s, a, with_w ? 1 : 0);
   count_launches(1);
   TT_CHECK_LAUNCH();
   return 0;
@@ -449,6 +451,7 @@ __device__ __forceinline__ void tc_issue(const CUtensorMap* tm, const CUtensorMa
 template <int N>
 __global__ void __launch_bounds__(128, 1) conv3_tc_kernel(ConvArgs a, const __grid_constant__ CUtensorMap tmain,
                                                           const __grid_constant__ CUtensorMap trow, long long ntiles) {
+  start_after();
   extern __shared__ __align__(128) unsigned char usm_raw[];
   unsigned char* usm = (unsigned char*)(((uintptr_t)usm_raw + 127) & ~(uintptr_t)127);
   __shared__ __align__(8) uint64_t full_bar[2];
@@ -692,7 +695,7 @@ static int launch_conv_tc(cudaStream_t s, const ConvArgs& a) {
   const long long ntiles = (long long)((a.X + kUX - 1) / kUX) * ((a.Y + kUY - 1) / kUY) * a.Z;
   const long long slots = (long long)sms * per_sm;
   const int blocks = (int)(ntiles < slots ? ntiles : slots);
-  conv3_tc_kernel<N><<<blocks, 128, smem, s>>>(a, tm, tr, ntiles);
+  launch_after(conv3_tc_kernel<N>, blocks, 128, smem, s, a, tm, tr, ntiles);
   count_launches(1);
   TT_CHECK_LAUNCH();
   return 0;
@@ -741,10 +744,10 @@ static int conv_fwd(cudaStream_t s, const ConvArgs& a) {
   const long long tpc = 8 / ks;
   const int blocks = (int)((tiles + tpc - 1) / tpc);
   switch (ks) {
-    case 1: conv3_fwd_kernel<1><<<blocks, 256, 0, s>>>(a); break;
-    case 2: conv3_fwd_kernel<2><<<blocks, 256, 0, s>>>(a); break;
-    case 4: conv3_fwd_kernel<4><<<blocks, 256, 0, s>>>(a); break;
-    default: conv3_fwd_kernel<8><<<blocks, 256, 0, s>>>(a); break;
+    case 1: launch_after(conv3_fwd_kernel<1>, blocks, 256, 0, s, a); break;
+    case 2: launch_after(conv3_fwd_kernel<2>, blocks, 256, 0, s, a); break;
+    case 4: launch_after(conv3_fwd_kernel<4>, blocks, 256, 0, s, a); break;
+    default: launch_after(conv3_fwd_kernel<8>, blocks, 256, 0, s, a); break;
   }
   count_launches(1);
   TT_CHECK_LAUNCH();
@@ -888,6 +891,7 @@ __device__ __forceinline__ float sum_of_parts(const float* part, int nb, long lo
 // The weight gradient's: the chunks' sums [27][cout][cin_pad] added into the
 // gradient of the real [27][cout][cin] weights.
 __global__ void sum_wgrad_kernel(const float* part, int nb, int cin, int cin_pad, int cout, float* g) {
+  start_after();
   const int n = 27 * cout * cin;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
     const int rest = t / cin, ci = t - rest * cin;
@@ -895,6 +899,7 @@ __global__ void sum_wgrad_kernel(const float* part, int nb, int cin, int cin_pad
   }
 }
 __global__ void sum_parts_kernel(const float* part, int nb, long long C, float* out) {
+  start_after();
   for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < C; c += (long long)gridDim.x * blockDim.x)
     out[c] += sum_of_parts(part + c, nb, C);
 }
@@ -902,6 +907,7 @@ __global__ void sum_parts_kernel(const float* part, int nb, long long C, float* 
 // *out = the sum of the blocks' losses, by one block in a fixed order (one
 // thread's chain of FP64 additions was 120 us for 2048 blocks).
 __global__ void sum_loss_kernel(const double* part, int nb, double* out) {
+  start_after();
   __shared__ double sh[32];
   double t = 0.0;
   for (int b = threadIdx.x; b < nb; b += blockDim.x) t += part[b];
@@ -934,7 +940,7 @@ static int conv_wgrad(cudaStream_t s, WgradArgs a, int cin, float* g) {
     default: return TTFLD_E_UNSUPPORTED;
   }
   const int threads = 64;  // few weights and long sums: as many SMs as there are
-  sum_wgrad_kernel<<<(27 * a.cout * cin + threads - 1) / threads, threads, 0, s>>>(a.part, (int)nch, cin, a.cin, a.cout, g);
+  launch_after(sum_wgrad_kernel, (27 * a.cout * cin + threads - 1) / threads, threads, 0, s, a.part, (int)nch, cin, a.cin, a.cout, g);
   count_launches(2);
   TT_CHECK_LAUNCH();
   return 0;
@@ -944,6 +950,7 @@ static int conv_wgrad(cudaStream_t s, WgradArgs a, int cin, float* g) {
 // dZ = dY * leaky'(Y) in place, on a channel slice (8 channels a thread; the
 // channel strides, offsets and counts are multiples of 8)
 __global__ void act_bwd_kernel(bf16* dy, int dy_cs, int dy_co, const bf16* y, int y_cs, int y_co, int C, long long V) {
+  start_after();
   const int C8 = C >> 3;
   const long long n = V * C8;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
@@ -995,6 +1002,7 @@ __global__ void bias_grad_kernel(const bf16* dz, int cs, int co, int C, long lon
 // multiples of 8.
 __global__ void pool8_fwd_kernel(const bf16* in, int in_cs, int in_co, Level fi, bf16* out, int out_cs, int out_co,
                                  Level co_, int C) {
+  start_after();
   const int C8 = C >> 3;
   const long long n = co_.vox() * C8;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
@@ -1022,6 +1030,7 @@ __global__ void pool8_fwd_kernel(const bf16* in, int in_cs, int in_co, Level fi,
 
 __global__ void up8_fwd_kernel(const bf16* in, int in_cs, Level co_, bf16* out, int out_cs, int out_co, Level fi,
                                int C) {
+  start_after();
   const int C8 = C >> 3;
   const long long n = fi.vox() * C8;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
@@ -1036,6 +1045,7 @@ __global__ void up8_fwd_kernel(const bf16* in, int in_cs, Level co_, bf16* out, 
 // d(fine) += d(coarse) / count (accumulate into a slice of the fine gradient)
 __global__ void pool_bwd_kernel(const bf16* gco, int g_cs, int g_co, Level co_, bf16* gfi, int f_cs, int f_co, Level fi,
                                 int C) {
+  start_after();
   const long long n = fi.vox() * C;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
     const int c = (int)(t % C);
@@ -1055,6 +1065,7 @@ __global__ void pool_bwd_kernel(const bf16* gco, int g_cs, int g_co, Level co_, 
 
 // d(coarse) = sum of d(fine children) (written, not accumulated)
 __global__ void up_bwd_kernel(const bf16* gfi, int f_cs, int f_co, Level fi, bf16* gco, int g_cs, Level co_, int C) {
+  start_after();
   const long long n = co_.vox() * C;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
     const int c = (int)(t % C);
@@ -1072,6 +1083,7 @@ __global__ void up_bwd_kernel(const bf16* gfi, int f_cs, int f_co, Level fi, bf1
 
 // head: pred = w . a13 + b (FP32); loss = sum mask (pred - target)^2 / nmask
 __global__ void head_fwd_kernel(const bf16* a13, const float* w, float* pred, long long V) {
+  start_after();
   for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < V; v += (long long)gridDim.x * blockDim.x) {
     float s = w[16];
 #pragma unroll
@@ -1082,6 +1094,7 @@ __global__ void head_fwd_kernel(const bf16* a13, const float* w, float* pred, lo
 
 // Sum of the mask's bytes (the number of active cells); *count is zeroed before.
 __global__ void mask_count_kernel(const unsigned char* mask, long long V, unsigned long long* count) {
+  start_after();
   unsigned long long n = 0;
   for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < V; v += (long long)gridDim.x * blockDim.x)
     n += mask[v];
@@ -1091,6 +1104,7 @@ __global__ void mask_count_kernel(const unsigned char* mask, long long V, unsign
 
 __global__ void loss_kernel(const float* pred, const float* target, const unsigned char* mask, long long V,
                             const unsigned long long* count, float* gpred, double* part) {
+  start_after();
   __shared__ double sh[32];
   const double inv_n = 1.0 / (double)(*count > 0 ? *count : 1);
   double acc = 0.0;
@@ -1106,6 +1120,7 @@ __global__ void loss_kernel(const float* pred, const float* target, const unsign
 // d(a13)[v][c] = gpred[v] * w[c]; per block: part[block][c] = sum gpred * a13,
 // part[block][16] = sum gpred (added in block order afterwards)
 __global__ void head_bwd_kernel(const float* gpred, const bf16* a13, const float* w, bf16* ga13, float* part, long long V) {
+  start_after();
   __shared__ float sh[17][32];
   float acc[17];
   for (int c = 0; c < 17; ++c) acc[c] = 0.f;
@@ -1179,6 +1194,7 @@ __device__ __forceinline__ int interp1_window(int c, int nf, bool periodic, int*
 }
 
 __global__ void pred_up_kernel(const float* half, Level co_, float* full, Level fi) {
+  start_after();
   const long long n = fi.vox();
   for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < n; v += (long long)gridDim.x * blockDim.x) {
     const int x = (int)(v % fi.X), y = (int)((v / fi.X) % fi.Y), z = (int)(v / ((long long)fi.X * fi.Y));
@@ -1196,6 +1212,7 @@ __global__ void pred_up_kernel(const float* half, Level co_, float* full, Level 
 
 // adjoint of pred_up_kernel, as a gather over each coarse cell's window
 __global__ void pred_down_kernel(const float* gfull, Level fi, float* ghalf, Level co_) {
+  start_after();
   const long long n = co_.vox();
   for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < n; v += (long long)gridDim.x * blockDim.x) {
     const int x = (int)(v % co_.X), y = (int)((v / co_.X) % co_.Y), z = (int)(v / ((long long)co_.X * co_.Y));
@@ -1222,6 +1239,7 @@ __global__ void pred_down_kernel(const float* gfull, Level fi, float* ghalf, Lev
 // FP32 master weights -> BF16 [tap][cout][cin_pad] and the flipped transpose
 // [26 - tap][cin_pad][cout] used by backward-data
 __global__ void wprep_kernel(const float* w, int cin, int cin_pad, int cout, bf16* w16, bf16* w16t) {
+  start_after();
   const long long n = 27LL * cout * cin_pad;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
     const int ci = (int)(t % cin_pad);
@@ -1385,7 +1403,7 @@ int prep_weights(ttfld_ctx* c) {
   if (!n->wdirty) return 0;
   for (int l = 0; l < kNumConv; ++l) {
     const LayerSpec& s = kLayers[l];
-    wprep_kernel<<<grid_for(27LL * s.cout * s.cin_pad), 256, 0, c->stream>>>(
+    launch_after(wprep_kernel, grid_for(27LL * s.cout * s.cin_pad), 256, 0, c->stream,
         n->p + n->woff[l], s.cin, s.cin_pad, s.cout, n->w16 + n->w16off[l], n->w16t + n->w16off[l]);
     count_launches(1);
   }
@@ -1418,27 +1436,27 @@ int forward(ttfld_ctx* c) {
   if ((rc = conv_fwd(s, conv_args(n, l, in, ics, ico, out, ocs, oco, lev)))) return rc;
   CONV(0, n->feat, 16, 0, n->a0, 16, 0, 0);
   CONV(1, n->a0, 16, 0, n->cat0, 48, 32, 0);                // s0 -> cat0[32:48]
-  pool8_fwd_kernel<<<GRID(L(1).vox() * 2), 256, 0, s>>>(n->cat0, 48, 32, L(0), n->p0, 16, 0, L(1), 16);
+  launch_after(pool8_fwd_kernel, GRID(L(1).vox() * 2), 256, 0, s, n->cat0, 48, 32, L(0), n->p0, 16, 0, L(1), 16);
   CONV(2, n->p0, 16, 0, n->a2, 32, 0, 1);
   CONV(3, n->a2, 32, 0, n->cat1, 96, 64, 1);                // s1 -> cat1[64:96]
-  pool8_fwd_kernel<<<GRID(L(2).vox() * 4), 256, 0, s>>>(n->cat1, 96, 64, L(1), n->p1, 32, 0, L(2), 32);
+  launch_after(pool8_fwd_kernel, GRID(L(2).vox() * 4), 256, 0, s, n->cat1, 96, 64, L(1), n->p1, 32, 0, L(2), 32);
   CONV(4, n->p1, 32, 0, n->a4, 64, 0, 2);
   CONV(5, n->a4, 64, 0, n->cat2, 128, 64, 2);               // s2 -> cat2[64:128]
-  pool8_fwd_kernel<<<GRID(L(3).vox() * 8), 256, 0, s>>>(n->cat2, 128, 64, L(2), n->p2, 64, 0, L(3), 64);
+  launch_after(pool8_fwd_kernel, GRID(L(3).vox() * 8), 256, 0, s, n->cat2, 128, 64, L(2), n->p2, 64, 0, L(3), 64);
   CONV(6, n->p2, 64, 0, n->a6, 64, 0, 3);
   CONV(7, n->a6, 64, 0, n->a7, 64, 0, 3);
-  up8_fwd_kernel<<<GRID(L(2).vox() * 8), 256, 0, s>>>(n->a7, 64, L(3), n->cat2, 128, 0, L(2), 64);
+  launch_after(up8_fwd_kernel, GRID(L(2).vox() * 8), 256, 0, s, n->a7, 64, L(3), n->cat2, 128, 0, L(2), 64);
   CONV(8, n->cat2, 128, 0, n->a8, 64, 0, 2);
   CONV(9, n->a8, 64, 0, n->a9, 64, 0, 2);
-  up8_fwd_kernel<<<GRID(L(1).vox() * 8), 256, 0, s>>>(n->a9, 64, L(2), n->cat1, 96, 0, L(1), 64);
+  launch_after(up8_fwd_kernel, GRID(L(1).vox() * 8), 256, 0, s, n->a9, 64, L(2), n->cat1, 96, 0, L(1), 64);
   CONV(10, n->cat1, 96, 0, n->a10, 32, 0, 1);
   CONV(11, n->a10, 32, 0, n->a11, 32, 0, 1);
-  up8_fwd_kernel<<<GRID(L(0).vox() * 4), 256, 0, s>>>(n->a11, 32, L(1), n->cat0, 48, 0, L(0), 32);
+  launch_after(up8_fwd_kernel, GRID(L(0).vox() * 4), 256, 0, s, n->a11, 32, L(1), n->cat0, 48, 0, L(0), 32);
   CONV(12, n->cat0, 48, 0, n->a12, 16, 0, 0);
   CONV(13, n->a12, 16, 0, n->a13, 16, 0, 0);
 #undef CONV
-  head_fwd_kernel<<<GRID(L(0).vox()), 256, 0, s>>>(n->a13, n->p + n->hoff, n->pred_half, L(0).vox());
-  pred_up_kernel<<<GRID(n->full.vox()), 256, 0, s>>>(n->pred_half, L(0), n->pred, n->full);
+  launch_after(head_fwd_kernel, GRID(L(0).vox()), 256, 0, s, n->a13, n->p + n->hoff, n->pred_half, L(0).vox());
+  launch_after(pred_up_kernel, GRID(n->full.vox()), 256, 0, s, n->pred_half, L(0), n->pred, n->full);
   count_launches(7);
   TT_CHECK_LAUNCH();
   return check_umma(s);
@@ -1470,14 +1488,14 @@ int conv_backward(ttfld_ctx* c, GradWork* gw, int l, bf16* gy, int gy_cs, int gy
   cudaStream_t st = c->stream;
   const long long V = L(lev).vox();
   int rc;
-  act_bwd_kernel<<<GRID(V * s.cout / 8), 256, 0, st>>>(gy, gy_cs, gy_co, y, y_cs, y_co, s.cout, V);
+  launch_after(act_bwd_kernel, GRID(V * s.cout / 8), 256, 0, st, gy, gy_cs, gy_co, y, y_cs, y_co, s.cout, V);
   cudaStream_t sw = n->side[0], sb = n->side[1];
   TT_CHECK(cudaEventRecord(n->dz_ready, st));
   TT_CHECK(cudaStreamWaitEvent(sw, n->dz_ready, 0));
   TT_CHECK(cudaStreamWaitEvent(sb, n->dz_ready, 0));
   const int bblocks = GRID(V / 8 + 1);
   bias_grad_kernel<<<bblocks, 512, 0, sb>>>(gy, gy_cs, gy_co, s.cout, V, gw->bpart);
-  sum_parts_kernel<<<1, 64, 0, sb>>>(gw->bpart, bblocks, s.cout, n->g + n->boff[l]);
+  launch_after(sum_parts_kernel, 1, 64, 0, sb, gw->bpart, bblocks, s.cout, n->g + n->boff[l]);
   count_launches(3);
   WgradArgs wa{gy, gy_cs, gy_co, s.cout, x, x_cs, x_co, s.cin_pad, gw->wpart, L(lev).X, L(lev).Y, L(lev).Z, 0};
   if ((rc = conv_wgrad(sw, wa, s.cin, n->g + n->woff[l]))) return rc;
@@ -1505,34 +1523,34 @@ int backward_layers(ttfld_ctx* c, GradWork* gw) {
   const int lblocks = GRID(VF), hblocks = GRID(V0);
   unsigned long long* count = reinterpret_cast<unsigned long long*>(n->loss_acc + 1);  // number of active cells
   TT_CHECK(cudaMemsetAsync(count, 0, sizeof(*count), s));
-  mask_count_kernel<<<lblocks, 256, 0, s>>>(n->mask, VF, count);
+  launch_after(mask_count_kernel, lblocks, 256, 0, s, n->mask, VF, count);
   count_launches(1);
-  loss_kernel<<<lblocks, 256, 0, s>>>(n->pred, n->target, n->mask, VF, count, n->gpred, gw->lpart);
-  sum_loss_kernel<<<1, 256, 0, s>>>(gw->lpart, lblocks, n->loss_acc);
-  pred_down_kernel<<<GRID(V0), 256, 0, s>>>(n->gpred, n->full, n->gpred_half, L(0));
-  head_bwd_kernel<<<hblocks, 256, 0, s>>>(n->gpred_half, n->a13, n->p + n->hoff, n->g_a13, gw->hpart, V0);
-  sum_parts_kernel<<<1, 32, 0, s>>>(gw->hpart, hblocks, 17, n->g + n->hoff);
+  launch_after(loss_kernel, lblocks, 256, 0, s, n->pred, n->target, n->mask, VF, count, n->gpred, gw->lpart);
+  launch_after(sum_loss_kernel, 1, 256, 0, s, gw->lpart, lblocks, n->loss_acc);
+  launch_after(pred_down_kernel, GRID(V0), 256, 0, s, n->gpred, n->full, n->gpred_half, L(0));
+  launch_after(head_bwd_kernel, hblocks, 256, 0, s, n->gpred_half, n->a13, n->p + n->hoff, n->g_a13, gw->hpart, V0);
+  launch_after(sum_parts_kernel, 1, 32, 0, s, gw->hpart, hblocks, 17, n->g + n->hoff);
   count_launches(5);
 #define BWD(l, gy, gcs, gco, y, ycs, yco, x, xcs, xco, gx, gxcs, gxco, acc, lev)                                  \
   if ((rc = conv_backward(c, gw, l, gy, gcs, gco, y, ycs, yco, x, xcs, xco, gx, gxcs, gxco, acc, lev))) return rc;
   BWD(13, n->g_a13, 16, 0, n->a13, 16, 0, n->a12, 16, 0, n->g_a12, 16, 0, 0, 0);
   BWD(12, n->g_a12, 16, 0, n->a12, 16, 0, n->cat0, 48, 0, n->g_cat0, 48, 0, 0, 0);
-  up_bwd_kernel<<<GRID(L(1).vox() * 32), 256, 0, s>>>(n->g_cat0, 48, 0, L(0), n->g_a11, 32, L(1), 32);
+  launch_after(up_bwd_kernel, GRID(L(1).vox() * 32), 256, 0, s, n->g_cat0, 48, 0, L(0), n->g_a11, 32, L(1), 32);
   BWD(11, n->g_a11, 32, 0, n->a11, 32, 0, n->a10, 32, 0, n->g_a10, 32, 0, 0, 1);
   BWD(10, n->g_a10, 32, 0, n->a10, 32, 0, n->cat1, 96, 0, n->g_cat1, 96, 0, 0, 1);
-  up_bwd_kernel<<<GRID(L(2).vox() * 64), 256, 0, s>>>(n->g_cat1, 96, 0, L(1), n->g_a9, 64, L(2), 64);
+  launch_after(up_bwd_kernel, GRID(L(2).vox() * 64), 256, 0, s, n->g_cat1, 96, 0, L(1), n->g_a9, 64, L(2), 64);
   BWD(9, n->g_a9, 64, 0, n->a9, 64, 0, n->a8, 64, 0, n->g_a8, 64, 0, 0, 2);
   BWD(8, n->g_a8, 64, 0, n->a8, 64, 0, n->cat2, 128, 0, n->g_cat2, 128, 0, 0, 2);
-  up_bwd_kernel<<<GRID(L(3).vox() * 64), 256, 0, s>>>(n->g_cat2, 128, 0, L(2), n->g_a7, 64, L(3), 64);
+  launch_after(up_bwd_kernel, GRID(L(3).vox() * 64), 256, 0, s, n->g_cat2, 128, 0, L(2), n->g_a7, 64, L(3), 64);
   BWD(7, n->g_a7, 64, 0, n->a7, 64, 0, n->a6, 64, 0, n->g_a6, 64, 0, 0, 3);
   BWD(6, n->g_a6, 64, 0, n->a6, 64, 0, n->p2, 64, 0, n->g_p2, 64, 0, 0, 3);
-  pool_bwd_kernel<<<GRID(L(2).vox() * 64), 256, 0, s>>>(n->g_p2, 64, 0, L(3), n->g_cat2, 128, 64, L(2), 64);
+  launch_after(pool_bwd_kernel, GRID(L(2).vox() * 64), 256, 0, s, n->g_p2, 64, 0, L(3), n->g_cat2, 128, 64, L(2), 64);
   BWD(5, n->g_cat2, 128, 64, n->cat2, 128, 64, n->a4, 64, 0, n->g_a4, 64, 0, 0, 2);
   BWD(4, n->g_a4, 64, 0, n->a4, 64, 0, n->p1, 32, 0, n->g_p1, 32, 0, 0, 2);
-  pool_bwd_kernel<<<GRID(L(1).vox() * 32), 256, 0, s>>>(n->g_p1, 32, 0, L(2), n->g_cat1, 96, 64, L(1), 32);
+  launch_after(pool_bwd_kernel, GRID(L(1).vox() * 32), 256, 0, s, n->g_p1, 32, 0, L(2), n->g_cat1, 96, 64, L(1), 32);
   BWD(3, n->g_cat1, 96, 64, n->cat1, 96, 64, n->a2, 32, 0, n->g_a2, 32, 0, 0, 1);
   BWD(2, n->g_a2, 32, 0, n->a2, 32, 0, n->p0, 16, 0, n->g_p0, 16, 0, 0, 1);
-  pool_bwd_kernel<<<GRID(L(0).vox() * 16), 256, 0, s>>>(n->g_p0, 16, 0, L(1), n->g_cat0, 48, 32, L(0), 16);
+  launch_after(pool_bwd_kernel, GRID(L(0).vox() * 16), 256, 0, s, n->g_p0, 16, 0, L(1), n->g_cat0, 48, 32, L(0), 16);
   BWD(1, n->g_cat0, 48, 32, n->cat0, 48, 32, n->a0, 16, 0, n->g_a0, 16, 0, 0, 0);
   BWD(0, n->g_a0, 16, 0, n->a0, 16, 0, n->feat, 16, 0, nullptr, 0, 0, 0, 0);
 #undef BWD
