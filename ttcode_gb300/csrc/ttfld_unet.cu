@@ -210,24 +210,37 @@ __global__ void __launch_bounds__(256) conv3_fwd_kernel(ConvArgs a) {
 // Shared-memory tiled form for the large levels (few output channels, many
 // voxels): a CTA computes 16 (x) x 8 (y) x 2 (z) output voxels and all
 // output channels.  The input tile with its one-voxel halo (18 x 10 x 4
-// voxels) and, when they fit, the weights are staged in shared memory with
-// every voxel/weight row padded by 8 channels, so that the 8 rows an
-// A/B-fragment read touches fall in distinct banks.  Warp w computes rows
-// (y0 + w, z0) and (y0 + w, z0 + 1), reusing each weight fragment for both.
-// Each input voxel is then read from global memory about 2.8 times (the
-// halo) instead of once per tap through the caches.
+// voxels) is staged in shared memory, and the weights a tap at a time, two
+// taps ahead (three stages), with every voxel/weight row padded by 8
+// channels, so that the 8 rows an A/B-fragment read touches fall in distinct
+// banks.  Warp w computes rows (y0 + w, z0) and (y0 + w, z0 + 1), reusing each
+// weight fragment for both.  Each input voxel is then read from global memory
+// about 2.8 times (the halo) instead of once per tap through the caches.  A
+// small level has a few tens of CTAs, whose time is what their reads wait for:
+// so the copies are asynchronous.  (Weights that did not fit beside the tile
+// were read from global memory 4 bytes a lane: 96 -> 32 channels on 8192
+// voxels 68 us, now 33; 32 -> 32 channels 28 and 17.)
 constexpr int kTX = 16, kTY = 8, kTZ = 2;
 constexpr int kHX = kTX + 2, kHY = kTY + 2, kHZ = kTZ + 2;
 constexpr int kHalo = kHX * kHY * kHZ;
 
-static size_t conv_smem_bytes(int cin, int cout, bool with_w) {
-  size_t b = (size_t)kHalo * (cin + 8) * 2;
-  if (with_w) b += (size_t)27 * cout * (cin + 8) * 2;
-  return b;
+constexpr int kTapStages = 3;
+
+__device__ __forceinline__ void ldmatrix4(uint32_t* r, const bf16* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"((uint32_t)__cvta_generic_to_shared(p))
+               : "memory");
 }
 
-template <int NB>
-__global__ void __launch_bounds__(256) conv3_smem_kernel(ConvArgs a, int w_in_smem) {
+static size_t conv_smem_bytes(int cin, int cout) {
+  return ((size_t)kHalo + (size_t)kTapStages * cout) * (cin + 8) * 2;
+}
+
+// KS = 2 adds the even taps and the odd taps apart and then the two, as
+// conv3_fwd_kernel<2> does.
+template <int NB, int KS>
+__global__ void __launch_bounds__(256) conv3_smem_kernel(ConvArgs a) {
   start_after();
   extern __shared__ __align__(16) unsigned char csm[];
   const int cst = a.cin + 8;  // padded row, in bf16
@@ -242,48 +255,73 @@ __global__ void __launch_bounds__(256) conv3_smem_kernel(ConvArgs a, int w_in_sm
     const int hx = hv % kHX, hy = (hv / kHX) % kHY, hz = hv / (kHX * kHY);
     const int x = x0 + hx - 1, z = z0 + hz - 1;
     const int y = ((y0 + hy - 1) % a.Y + a.Y) % a.Y;  // periodic phi
-    uint4 v = make_uint4(0u, 0u, 0u, 0u);
+    uint4* to = reinterpret_cast<uint4*>(tin + (size_t)hv * cst + c8 * 8);
     if (x >= 0 && x < a.X && z >= 0 && z < a.Z)
-      v = *reinterpret_cast<const uint4*>(a.in + (((size_t)z * a.Y + y) * a.X + x) * a.in_cs + a.in_co + c8 * 8);
-    *reinterpret_cast<uint4*>(tin + (size_t)hv * cst + c8 * 8) = v;
+      copy_async(to, reinterpret_cast<const uint4*>(a.in + (((size_t)z * a.Y + y) * a.X + x) * a.in_cs + a.in_co + c8 * 8));
+    else
+      *to = make_uint4(0u, 0u, 0u, 0u);
   }
-  if (w_in_smem) {
-    const int rows = 27 * a.cout;
-    for (int q = threadIdx.x; q < rows * c8n; q += blockDim.x) {
-      const int c8 = q % c8n, row = q / c8n;
-      *reinterpret_cast<uint4*>(tw + (size_t)row * cst + c8 * 8) =
-          *reinterpret_cast<const uint4*>(a.w + (size_t)row * a.cin + c8 * 8);
-    }
-  }
-  __syncthreads();
+  auto stage_tap = [&](int tap) {  // one group of copies per tap, empty behind the last
+    bf16* to = tw + (size_t)(tap % kTapStages) * a.cout * cst;
+    if (tap < 27)
+      for (int q = threadIdx.x; q < a.cout * c8n; q += blockDim.x) {
+        const int c8 = q % c8n, row = q / c8n;
+        copy_async(reinterpret_cast<uint4*>(to + (size_t)row * cst + c8 * 8),
+                   reinterpret_cast<const uint4*>(a.w + ((size_t)tap * a.cout + row) * a.cin + c8 * 8));
+      }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  stage_tap(0);  // with the tile
+  stage_tap(1);
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int r = lane >> 2, cq = (lane & 3) * 2;
-  const bf16* wbase = w_in_smem ? tw : a.w;
-  const int wst = w_in_smem ? cst : a.cin;
-  float acc[2][NB][4];
+  const int r = lane >> 2, cq = (lane & 3) * 2;  // of the accumulators
+  const int mr = lane & 7, mat = lane >> 3;  // the row of an 8 x 8 matrix whose address the lane gives, and which
+  const int aoff = (mr + (mat & 1) * 8) * cst + (mat >> 1) * 8;  // A: voxels r, r+8 at k; at k+8
+  const int boff = (mr + (mat >> 1) * 8) * cst + (mat & 1) * 8;  // B: channels n at k, k+8; n+8
+  float acc[KS][2][NB][4];
 #pragma unroll
-  for (int zz = 0; zz < 2; ++zz)
+  for (int ks = 0; ks < KS; ++ks)
 #pragma unroll
-    for (int nb = 0; nb < NB; ++nb) acc[zz][nb][0] = acc[zz][nb][1] = acc[zz][nb][2] = acc[zz][nb][3] = 0.f;
-  for (int tap = 0; tap < 27; ++tap) {
+    for (int zz = 0; zz < 2; ++zz)
+#pragma unroll
+      for (int nb = 0; nb < NB; ++nb)
+        acc[ks][zz][nb][0] = acc[ks][zz][nb][1] = acc[ks][zz][nb][2] = acc[ks][zz][nb][3] = 0.f;
+  auto add_tap = [&](int tap, float (&c)[2][NB][4]) {
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncthreads();  // the tap has landed for every thread, and the stage of the tap before is free
+    stage_tap(tap + 2);
     const int dz = tap / 9, dy = (tap / 3) % 3, dx = tap % 3;  // 0..2: halo offsets
-    const bf16* p0 = tin + ((size_t)((0 + dz) * kHY + (w + dy)) * kHX + r + dx) * cst + cq;
-    const bf16* p1 = tin + ((size_t)((1 + dz) * kHY + (w + dy)) * kHX + r + dx) * cst + cq;
-    const bf16* wt = wbase + (size_t)tap * a.cout * wst;
+    const bf16* p0 = tin + ((size_t)((0 + dz) * kHY + (w + dy)) * kHX + dx) * cst + aoff;
+    const bf16* p1 = p0 + (size_t)kHY * kHX * cst;
+    const bf16* wt = tw + (size_t)(tap % kTapStages) * a.cout * cst + boff;
+#pragma unroll 2
     for (int kc = 0; kc < a.cin; kc += 16) {
-      const uint32_t a00 = ld32(p0 + kc), a01 = ld32(p0 + 8 * cst + kc);
-      const uint32_t a02 = ld32(p0 + kc + 8), a03 = ld32(p0 + 8 * cst + kc + 8);
-      const uint32_t a10 = ld32(p1 + kc), a11 = ld32(p1 + 8 * cst + kc);
-      const uint32_t a12 = ld32(p1 + kc + 8), a13 = ld32(p1 + 8 * cst + kc + 8);
+      uint32_t f0[4], f1[4];
+      ldmatrix4(f0, p0 + kc);
+      ldmatrix4(f1, p1 + kc);
 #pragma unroll
-      for (int nb = 0; nb < NB; ++nb) {
-        const bf16* wp = wt + (size_t)(nb * 8 + r) * wst + kc + cq;
-        const uint32_t b0 = ld32(wp), b1 = ld32(wp + 8);
-        mma_bf16(acc[0][nb], a00, a01, a02, a03, b0, b1);
-        mma_bf16(acc[1][nb], a10, a11, a12, a13, b0, b1);
+      for (int nb = 0; nb < NB; nb += 2) {
+        uint32_t b[4];
+        ldmatrix4(b, wt + (size_t)(nb * 8) * cst + kc);
+        mma_bf16(c[0][nb], f0[0], f0[1], f0[2], f0[3], b[0], b[1]);
+        mma_bf16(c[1][nb], f1[0], f1[1], f1[2], f1[3], b[0], b[1]);
+        mma_bf16(c[0][nb + 1], f0[0], f0[1], f0[2], f0[3], b[2], b[3]);
+        mma_bf16(c[1][nb + 1], f1[0], f1[1], f1[2], f1[3], b[2], b[3]);
       }
     }
+  };
+#pragma unroll 1
+  for (int tap = 0; tap < 27; tap += KS) {
+    add_tap(tap, acc[0]);
+    if (KS == 2 && tap + 1 < 27) add_tap(tap + 1, acc[KS - 1]);
   }
+  if (KS == 2)
+#pragma unroll
+    for (int zz = 0; zz < 2; ++zz)
+#pragma unroll
+      for (int nb = 0; nb < NB; ++nb)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) acc[0][zz][nb][q] += acc[KS - 1][zz][nb][q];
   const int y = y0 + w;
   if (y >= a.Y) return;
 #pragma unroll
@@ -298,7 +336,7 @@ __global__ void __launch_bounds__(256) conv3_smem_kernel(ConvArgs a, int w_in_sm
       bf16* po = a.out + (rowo + x) * a.out_cs + a.out_co + cq;
 #pragma unroll
       for (int nb = 0; nb < NB; ++nb) {
-        float v0 = acc[zz][nb][half * 2], v1 = acc[zz][nb][half * 2 + 1];
+        float v0 = acc[0][zz][nb][half * 2], v1 = acc[0][zz][nb][half * 2 + 1];
         const int ch = nb * 8 + cq;
         if (a.bias) { v0 += a.bias[ch]; v1 += a.bias[ch + 1]; }
         if (a.act) { v0 = v0 > 0.f ? v0 : kLeak * v0; v1 = v1 > 0.f ? v1 : kLeak * v1; }
@@ -310,19 +348,18 @@ __global__ void __launch_bounds__(256) conv3_smem_kernel(ConvArgs a, int w_in_sm
   }
 }
 
-template <int NB>
+template <int NB, int KS>
 static int launch_conv_smem(cudaStream_t s, const ConvArgs& a) {
-  bool with_w = conv_smem_bytes(a.cin, a.cout, true) <= 100 * 1024;
-  const size_t smem = conv_smem_bytes(a.cin, a.cout, with_w);
+  const size_t smem = conv_smem_bytes(a.cin, a.cout);
   static size_t opted = 0;
   if (smem > 48 * 1024 && smem > opted) {
-    if (cudaFuncSetAttribute(conv3_smem_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) !=
+    if (cudaFuncSetAttribute(conv3_smem_kernel<NB, KS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) !=
         cudaSuccess)
       return TTFLD_E_CUDA;
     opted = 200 * 1024;
   }
   const long long blocks = (long long)((a.X + kTX - 1) / kTX) * ((a.Y + kTY - 1) / kTY) * ((a.Z + kTZ - 1) / kTZ);
-  launch_after(conv3_smem_kernel<NB>, (unsigned)blocks, 256, smem, s, a, with_w ? 1 : 0);
+  launch_after(conv3_smem_kernel<NB, KS>, (unsigned)blocks, 256, smem, s, a);
   count_launches(1);
   TT_CHECK_LAUNCH();
   return 0;
@@ -731,16 +768,21 @@ static int conv_fwd(cudaStream_t s, const ConvArgs& a) {
     if (a.cout == 16) return launch_conv_tc<16>(s, a);
     if (a.cout == 32) return launch_conv_tc<32>(s, a);
   }
-  // shared-memory tiles up to 96 input channels (a 150 KB input tile; the
-  // weights stay in global memory above 100 KB of tile + weights)
+  // shared-memory tiles up to 96 input channels (a 150 KB input tile)
   if (a.cin <= 96 && a.in_cs % 8 == 0 && a.in_co % 8 == 0) {
-    if (a.cout == 16) return launch_conv_smem<2>(s, a);
-    if (a.cout == 32) return launch_conv_smem<4>(s, a);
+    if (a.cout == 16) return launch_conv_smem<2, 1>(s, a);
+    if (a.cout == 32) return launch_conv_smem<4, 1>(s, a);
   }
   const long long tiles = (long long)((a.X + 15) >> 4) * a.Y * a.Z * (a.cout / 16);
   // split the taps over more warps until about two waves of warps are busy
   int ks = 1;
   while (ks < 8 && tiles * ks < 152LL * 128) ks *= 2;
+  // up to 48 output channels in shared-memory tiles too, where the taps are
+  // split in two at most: 16 -> 48 channels on 65,536 voxels 62 -> 28 us
+  if (a.cin == 16 && a.cout == 48 && a.in_cs % 8 == 0 && a.in_co % 8 == 0) {
+    if (ks == 1) return launch_conv_smem<6, 1>(s, a);
+    if (ks == 2) return launch_conv_smem<6, 2>(s, a);
+  }
   const long long tpc = 8 / ks;
   const int blocks = (int)((tiles + tpc - 1) / tpc);
   switch (ks) {
