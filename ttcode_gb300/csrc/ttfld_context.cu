@@ -3,6 +3,8 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <mutex>
+
 #include "ttfld_internal.cuh"
 
 namespace ttfld {
@@ -31,6 +33,49 @@ int grid_for(long long n, int threads) {
   if (blocks > cap) blocks = cap;
   if (blocks < 1) blocks = 1;
   return (int)blocks;
+}
+
+// L2 policies by sixteenths of the lines kept (0: every line leaves first).
+constexpr int kPolicies = 17;
+__device__ unsigned long long g_policies[kPolicies];
+__global__ void policies_kernel() {
+  unsigned long long p;
+  asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+  g_policies[0] = p;
+  for (int q = 1; q < kPolicies; ++q) {
+    asm volatile("createpolicy.fractional.L2::evict_last.L2::evict_first.b64 %0, %1;"
+                 : "=l"(p)
+                 : "f"((float)q / (kPolicies - 1)));
+    g_policies[q] = p;
+  }
+}
+
+uint64_t l2_policy(double keep) {
+  constexpr int kDevices = 64;
+  static std::mutex lock;
+  static unsigned long long table[kDevices][kPolicies];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev >= kDevices) return 0;
+  std::lock_guard<std::mutex> hold(lock);
+  if (!table[dev][0]) {
+    policies_kernel<<<1, 1>>>();
+    if (check_cuda(cudaGetLastError(), "L2 policies") ||
+        check_cuda(cudaMemcpyFromSymbol(table[dev], g_policies, sizeof(table[dev])), "L2 policies")) {
+      table[dev][0] = 0;
+      return 0;
+    }
+  }
+  const int q = (int)(keep * (kPolicies - 1) + 0.5);
+  return table[dev][q < 0 ? 0 : q < kPolicies ? q : kPolicies - 1];
+}
+
+L2Keep l2_keep(double iter_bytes, double coef_bytes) {
+  int dev = 0, l2 = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev);
+  const double room = 0.55 * l2, left = room - iter_bytes;
+  return L2Keep{l2_policy(left >= 0.0 ? 1.0 : room / iter_bytes),
+                l2_policy(left <= 0.0 ? 0.0 : coef_bytes <= left ? 1.0 : left / coef_bytes)};
 }
 
 // Copy between a box-shaped contiguous buffer and an internal array.
@@ -270,6 +315,10 @@ int ttfld_create(ttfld_ctx** out, const ttfld_dims* dims, const ttfld_metrics* m
       check_cuda(cudaEventCreate(&c->ev0), "event") || check_cuda(cudaEventCreate(&c->ev1), "event") ||
       check_cuda(cudaEventCreate(&c->evg), "event") ||
       check_cuda(cudaMallocHost((void**)&c->host_sol, sizeof(SolverDev)), "pinned")) {
+    ttfld_destroy(c);
+    return TTFLD_E_CUDA;
+  }
+  if (!l2_policy(0.0)) {  // made before the first solve
     ttfld_destroy(c);
     return TTFLD_E_CUDA;
   }

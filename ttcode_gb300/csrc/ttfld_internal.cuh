@@ -432,28 +432,17 @@ __device__ __forceinline__ bool grid_sum(SolverDev* sol, unsigned int nblocks, u
 // iterate goes first (it is read twice and written once per sweep), then the
 // coefficients.
 struct L2Keep {
-  float iter, coef;  // fractions of the lines
+  uint64_t iter, coef;  // policies of the accesses
 };
 // Of what the L2 holds, 0.55 (70 of 126 MB): over unique footprints of 79 to
 // 671 MB of the FP32 sweeps 60 to 80 MB is best, 90 MB up to 12 % slower.
-inline L2Keep l2_keep(double iter_bytes, double coef_bytes) {
-  int dev = 0, l2 = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev);
-  const double room = 0.55 * l2;
-  L2Keep k;
-  k.iter = (float)(iter_bytes <= room ? 1.0 : room / iter_bytes);
-  k.coef = (float)(iter_bytes >= room ? 0.0 : coef_bytes <= room - iter_bytes ? 1.0 : (room - iter_bytes) / coef_bytes);
-  return k;
-}
-__device__ __forceinline__ uint64_t l2_policy(float keep) {
-  uint64_t p;
-  if (keep > 0.f)
-    asm("createpolicy.fractional.L2::evict_last.L2::evict_first.b64 %0, %1;" : "=l"(p) : "f"(keep));
-  else
-    asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
-  return p;
-}
+L2Keep l2_keep(double iter_bytes, double coef_bytes);
+// The policy that keeps a fraction of the lines (in sixteenths).  A kernel
+// takes it as a parameter: made in the kernel it would live in a register of
+// each thread, and the accesses want it the same for a whole warp, whatever
+// the compiler does with that register where threads part.  0 after a CUDA
+// error.
+uint64_t l2_policy(double keep);
 
 // An asynchronous copy of one 8- or 16-byte word to shared memory.
 template <class W>

@@ -230,18 +230,15 @@ __device__ __forceinline__ float4 ldc4(const float* p) {
   return v;
 }
 
-// The same accesses with a part of the lines kept in L2 (L2Keep).
-struct KeepPolicy {
-  uint64_t coef, iter;
-};
-__device__ __forceinline__ float4 ldc4(const float* p, const KeepPolicy& k) {
+// The same accesses with a part of the lines kept in L2.
+__device__ __forceinline__ float4 ldc4(const float* p, const L2Keep& k) {
   float4 v;
   asm("ld.global.L1::no_allocate.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;"
       : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
       : "l"(p), "l"(k.coef));
   return v;
 }
-__device__ __forceinline__ float4 lde4(const float* p, const KeepPolicy& k) {
+__device__ __forceinline__ float4 lde4(const float* p, const L2Keep& k) {
   float4 v;
   asm volatile("ld.global.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;"
                : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
@@ -249,7 +246,7 @@ __device__ __forceinline__ float4 lde4(const float* p, const KeepPolicy& k) {
                : "memory");
   return v;
 }
-__device__ __forceinline__ void st4(float* p, float4 v, const KeepPolicy& k) {
+__device__ __forceinline__ void st4(float* p, float4 v, const L2Keep& k) {
   asm volatile("st.global.L2::cache_hint.v4.f32 [%4], {%0, %1, %2, %3}, %5;" ::"f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w),
                "l"(p), "l"(k.iter)
                : "memory");
@@ -519,7 +516,7 @@ __device__ __forceinline__ void fetch_vec(const Mix32& m, long long t, float4* t
 template <int COL, bool NORM, bool POLES, bool RESIDENT>
 __device__ __forceinline__ void sweep_local(const Cmp& g, const Mix32& m, float omega, long long t0, unsigned int n,
                                             int nv, size_t plane, const float4* slots, float& nacc,
-                                            const KeepPolicy& keep, bool back) {
+                                            const L2Keep& keep, bool back) {
   if constexpr (!RESIDENT) {
     const unsigned int rounds = (n + blockDim.x - 1) / blockDim.x;
     for (unsigned int q = 0; q < rounds; ++q) {
@@ -541,7 +538,7 @@ template <bool POLES, bool RESIDENT = false>
 __global__ void __launch_bounds__(kPersistThreads) sweeps32_local(Cmp g, Mix32 m, float omega, SolverDev* sol,
                                                                  Partial* gather, double stop_ratio, int nsweeps,
                                                                  int norm_every, int stall_check, unsigned int* flags,
-                                                                 unsigned int base, long long norms, L2Keep l2) {
+                                                                 unsigned int base, long long norms, L2Keep keep) {
   __shared__ double sh[32];
   __shared__ int stop_sh;
   extern __shared__ __align__(16) unsigned char slots_raw[];
@@ -570,7 +567,6 @@ __global__ void __launch_bounds__(kPersistThreads) sweeps32_local(Cmp g, Mix32 m
     asm volatile("cp.async.wait_all;" ::: "memory");
   }
   double last_ratio = -1.0;  // in-sweep ratio of the previous norm sweep (lane 0 of the last warp)
-  const KeepPolicy keep = {l2_policy(l2.coef), l2_policy(l2.iter)};
   const int it0 = sol->iter;
   unsigned int half = base;  // half-sweeps this block has finished
   int sw = 1;
@@ -1060,7 +1056,7 @@ struct SweepGrids {
 };
 template <bool POLES>
 static SweepGrids sweep_grids(long long nvec) {
-  static SweepGrids gr = {-1, -1, -1, -1, 0, 0, 0, {1.f, 1.f}};
+  static SweepGrids gr = {-1, -1, -1, -1, 0, 0, 0, {0, 0}};
   static long long sized_for = -1;
   if (sized_for != nvec) {
     gr.tma = persistent_grid(sweeps32_tma<POLES>, kTmaThreads, kTmaSmem, nvec);
@@ -1142,6 +1138,7 @@ static int launch_sweeps32_form(ttfld_ctx* c, int nsweeps, int norm_every, doubl
     Partial* gather = w->gather;
     long long norms = w->norm_base;  // no number is used twice, so nothing is cleared between launches
     L2Keep l2 = gr.l2;
+    if (!l2.iter || !l2.coef) return TTFLD_E_CUDA;
     void* largs[] = {&g, &m, &omega, &sol, &gather, &stop_ratio, &nsweeps, &norm_every, &stall, &flags, &base, &norms, &l2};
     if (gr.resident)
       TT_CHECK(cudaLaunchCooperativeKernel((const void*)sweeps32_local<POLES, true>, dim3(gr.local),

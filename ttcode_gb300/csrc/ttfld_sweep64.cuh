@@ -147,7 +147,7 @@ __device__ __forceinline__ double sweep_colour(const Sys& s, unsigned int r0, un
 template <class Sys, bool RESIDENT>
 __global__ void __launch_bounds__(Sys::kThreads, 1)
     sweeps64_persistent(Sys s, SolverDev* sol, Partial* gather, unsigned int* flags, typename Sys::Kept* keep,
-                        int nsweeps, int itmin, int itmax, double eps, float coef_keep,
+                        int nsweeps, int itmin, int itmax, double eps, uint64_t pol,
                         typename Sys::Word* copy) {
   __shared__ double sh[32];
   __shared__ int stop_sh, ok_sh;
@@ -168,7 +168,6 @@ __global__ void __launch_bounds__(Sys::kThreads, 1)
   const int it0 = sol->iter;
   extern __shared__ __align__(16) unsigned char slots_raw[];
   typename Sys::Word* slots = reinterpret_cast<typename Sys::Word*>(slots_raw);
-  const uint64_t pol = l2_policy(RESIDENT ? 0.f : coef_keep);  // resident: read once
   int stage = 0;
   if (RESIDENT) {  // each thread copies what it will read itself
     for (unsigned int u = threadIdx.x; u < n; u += blockDim.x) {
@@ -291,12 +290,13 @@ int launch_sweeps64_persistent(const Sys& s, cudaStream_t st, SolverDev* sol, do
   typename Sys::Kept* keep =
       (size_t)items * sizeof(typename Sys::Kept) <= kept_bytes ? (typename Sys::Kept*)kept : nullptr;
   const double word = 2.0 * (double)items * sizeof(typename Sys::Word);  // an array of both colours
-  float coef_keep = l2_keep(word, Sys::kWords * word).coef;
+  uint64_t pol = resident ? l2_policy(0.0) : l2_keep(word, Sys::kWords * word).coef;  // resident: read once
+  if (!pol) return TTFLD_E_CUDA;
   // the first sweep's stores cost about what half a sweep's reads do
   typename Sys::Word* copy = nullptr;
   if (Sys::kStrided && !resident && owner && nsweeps >= 4)
     copy = (typename Sys::Word*)sweep_copy(owner, (size_t)(Sys::kWords * word));
-  void* args[] = {&sys, &sol, &gather, &flags, &keep, &nsweeps, &itmin, &itmax, &eps, &coef_keep, &copy};
+  void* args[] = {&sys, &sol, &gather, &flags, &keep, &nsweeps, &itmin, &itmax, &eps, &pol, &copy};
   const cudaError_t e =
       cudaLaunchCooperativeKernel(kernel, dim3((unsigned int)nb), dim3(threads), args, smem, st);
   if (e == cudaErrorCooperativeLaunchTooLarge) {
