@@ -11,7 +11,9 @@
 // same stop decision -- one colour later: it begins the next sweep, keeping
 // the values that its first colour replaces, and reads the shares, by then
 // there, before the second; if the rule says stop it puts those values back.
-// (Where the values cannot be kept, the decision is waited for.)  The cells'
+// (Where the values cannot be kept, the decision is waited for.)  A block adds
+// up its own share behind its flag, which its neighbours wait for: 5.75 -> 5.48
+// ms for the exact SOR at 64x128x64 against adding it up before.  The cells'
 // updates and their operands are those of one launch per colour, so the
 // iterate is the same bit for bit; only the order in which the norm is
 // summed differs.
@@ -75,6 +77,13 @@ __device__ __forceinline__ int gather_norm(const Sys& s, const Partial* gather, 
     if (stop) sol->done = 1;
   }
   return stop;
+}
+
+// A block's share of the norm of sweep sw, from its warps' sums, by one warp.
+__device__ __forceinline__ void put_share(const double* sh, int nw, Partial* gather, int b, int sw) {
+  const int lane = threadIdx.x & 31;
+  const double part = warp_sum_all(lane < nw ? sh[lane] : 0.0);
+  if (lane == 0) put_partial(gather, b, sw, part);
 }
 
 // Put back the first colour's values from before the present sweep.
@@ -191,7 +200,10 @@ __global__ void __launch_bounds__(Sys::kThreads, 1)
   unsigned int half = 0;  // half-sweeps this block has finished
   int stop = 0;
   for (int sw = 1; sw <= nsweeps && !stop; ++sw) {
-    if (sw > 1 && !wait_flags(flags, lo, hi, half, sol)) break;
+    if (sw > 1) {
+      if (!wait_flags(flags, lo, hi, half, sol)) break;  // its block barrier also orders sh
+      if (mine && warp == 0) put_share(sh, nw, gather, b, sw - 1);
+    }
     s.template before<0>(r0, r1);
     double acc = sweep_colour<0, RESIDENT>(s, r0, n, sw == 1, slots, stage, sw > 1 ? mine : nullptr, pol,
                                             sw > 1 ? Copy{copy0, copy1, nullptr} : Copy{nullptr, nullptr, copy0});
@@ -214,14 +226,14 @@ __global__ void __launch_bounds__(Sys::kThreads, 1)
     acc += sweep_colour<1, RESIDENT>(s, r0, n, false, slots, stage, nullptr, pol,
                                       sw > 1 ? Copy{copy1, copy0, nullptr} : Copy{nullptr, copy0, copy1});
     s.template after<1>(r0, r1, false);
+    publish_flag(own, ++half);
+    // behind the flag, that the neighbours wait for; where the decision comes
+    // a colour later the block's share is put at the next sweep's start
     acc = warp_sum_all(acc);
     if (lane == 0) sh[warp] = acc;
-    publish_flag(own, ++half);  // its block barrier also orders sh
-    if (warp == 0) {
-      const double part = warp_sum_all(lane < nw ? sh[lane] : 0.0);
-      if (lane == 0) put_partial(gather, b, sw, part);
-    }
     if (!mine || sw == nsweeps) {
+      __syncthreads();
+      if (warp == 0) put_share(sh, nw, gather, b, sw);
       if (warp == nw - 1) {
         const int r = gather_norm(s, gather, nb, sw, it0, itmin, itmax, eps, rhsnorm, sol);
         if (lane == 0) stop_sh = r;
