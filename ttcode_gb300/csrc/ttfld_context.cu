@@ -337,6 +337,7 @@ int ttfld_destroy(ttfld_ctx* c) {
   mix_free(c);
   krylov_free(c);
   if (c->sweep_copy) cudaFree(c->sweep_copy);
+  if (c->rad_mem) cudaFree(c->rad_mem);
   if (c->opac) cudaFree(c->opac);
   if (c->freed) cudaFree(c->freed);
   if (c->wave) cudaFree(c->wave);

@@ -508,6 +508,7 @@ struct ttfld_ctx {
   ttfld::SolverDev* host_sol;  // pinned mirror
   void* sweep_copy;          // coefficients in the order of the FP64 sweeps (allocated on first use)
   size_t sweep_copy_bytes;
+  void* rad_mem;             // RADDIF's couplings (allocated on first use)
   // mixed-precision workspace (allocated on first use)
   void* mix_slab;
   size_t mix_bytes;

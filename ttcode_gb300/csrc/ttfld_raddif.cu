@@ -25,7 +25,6 @@ namespace {
 struct RadWork {
   double *ax, *cx, *ay, *cy, *az, *cz, *b, *rhs, *xs;
   double *volxb, *volyb, *volzb;  // (1:NX), (1:NY), (1:NZ)
-  void* mem;
 };
 
 __global__ void __launch_bounds__(kThreads) er_from_t_kernel(Dev d) {
@@ -383,8 +382,10 @@ extern "C" int ttfld_raddif(ttfld_ctx* c, const ttfld_raddif_params* p, ttfld_so
   RadWork w{};
   const size_t n = ncell(d);
   const size_t bytes = (9 * n + (size_t)d.nx + d.ny + d.nz) * sizeof(double);
-  TT_CHECK(cudaMallocAsync(&w.mem, bytes, c->stream));
-  double* q = (double*)w.mem;
+  // kept with the context: from the stream's pool it was mapped and unmapped
+  // again on every call
+  if (!c->rad_mem) TT_CHECK(cudaMalloc(&c->rad_mem, bytes));
+  double* q = (double*)c->rad_mem;
   double** arrs[] = {&w.ax, &w.cx, &w.ay, &w.cy, &w.az, &w.cz, &w.b, &w.rhs, &w.xs};
   for (double** a : arrs) { *a = q; q += n; }
   w.volxb = q; q += d.nx;
@@ -452,7 +453,6 @@ extern "C" int ttfld_raddif(ttfld_ctx* c, const ttfld_raddif_params* p, ttfld_so
     TT_CHECK_LAUNCH();
   }
   TT_CHECK(cudaEventRecord(c->ev1, c->stream));
-  TT_CHECK(cudaFreeAsync(w.mem, c->stream));
   TT_CHECK(cudaStreamSynchronize(c->stream));
   if (rc) return rc;
   float ms = 0.f;
