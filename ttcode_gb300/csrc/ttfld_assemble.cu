@@ -101,7 +101,9 @@ __device__ __forceinline__ int first_above(const double* node, int n, double v) 
 // table, 3: below it, 4: a non-positive opacity).  The powers of ten of the
 // node values alone are formed once per table (ttfld_set_opacity_table): three
 // per cell instead of nine, as exp10(), which is faster (26 against 6.7 G/s)
-// and nearer (1.04 against 1.32 ulp at most over 10^-20 .. 10^5) than pow().
+// and nearer (1.04 against 1.32 ulp at most over 10^-20 .. 10^5) than pow():
+// KAPPA from the table 562 us at 53x90x47 with nine pow(), 223 with three, now
+// 104.
 __device__ __forceinline__ int burrows_opc(const OpacTab& tb, double t, double rh, double& kp, double& kr,
                                            double& ka, double& dkp, double& dka) {
   if (!(t > 0.0)) return 1;
@@ -709,8 +711,8 @@ static int stellar_binned(ttfld_ctx* c) {
 // all its threads form the products of kTauChunk radii, a warp per column
 // (coalesced), and 32 of them then run the columns' sums through shared
 // memory.  (One thread per column walking global memory, a stride of a whole
-// radial row between the threads of a warp: 50 us at 100x256x128, 20 us at
-// 40x64x32.)
+// radial row between the threads of a warp: 50 us at 100x256x128, 21 us at
+// 40x64x32; so 38 and 12.)
 constexpr int kTauCols = 32, kTauChunk = 64;
 __global__ void __launch_bounds__(kThreads) stellar_tau_kernel(Dev d) {
   start_after();
@@ -794,7 +796,8 @@ static int stellarinput_heating(ttfld_ctx* c) {
 // ghosts by wrap for k = 1..NZ, then the k ghosts from k = 1 and NZ).  One
 // warp reads a column, 32 radii at once; its value goes to every place of the
 // plane that takes it.  (One thread per column, which reads its radii one
-// after another, and two more launches for the ghosts: 28 us at 100x256x128.)
+// after another, and two more launches for the ghosts: 30 us at 100x256x128 and
+// 18 at 40x64x32; so 13 and 4.)
 __global__ void __launch_bounds__(kThreads) upperbnd_kernel(Dev d) {
   start_after();
   const unsigned int col = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;

@@ -8,8 +8,8 @@
 // multiplications and some 30 other integer instructions, a quotient or a
 // square root 70 to 90, so on this chip the integer pipes do a product in
 // about the FP64 pipe's own time, beside it, and a quotient in a fifth of
-// it: measured alone, in G per second, mul_rn 479 (hardware 494; alternating
-// with sums, 464 against 249 pairs), div_rn 330 (67), sqrt_rn 306 (68).  The
+// it: measured alone, in G per second, mul_rn 570 (hardware 494), div_rn 335
+// (67), sqrt_rn 306 (68).  The
 // kernels of the FP64 path, which were bound by the FP64 pipe, use these for
 // their quotients and about half of their products and leave the sums to the
 // FP64 pipe: at 100x256x128 a face pass (FLIM, DIFF, flux of one direction)

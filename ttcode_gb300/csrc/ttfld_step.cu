@@ -50,19 +50,31 @@ __device__ __forceinline__ void left_column(const Dev& d, int j, int k) {
   HA(ER, -1, j, k) = TT_ARAD * p4(div_rn(qm, HA(RH, -1, j, k) * HA(CV, -1, j, k)));
 }
 
-// Both radial boundaries in one launch: the cells at i >= UPPERBND, and by the
-// thread of i = 1 the left one of its column.  They meet only in cell 1 of a
-// column with UPPERBND = 1, which that thread forms in the caller's order
-// (upper then left before the first outer iteration, ppenergy.f:80-167; left
-// then upper after each, :578-702).
+// Both radial boundaries in one launch: a thread per column first, for the left
+// one, then one per cell of i >= 2 for those at i >= UPPERBND.  They meet only
+// in cell 1 of a column with UPPERBND = 1, which the column's thread forms in
+// the caller's order (upper then left before the first outer iteration,
+// ppenergy.f:80-167; left then upper after each, :578-702).  (Two launches:
+// 43 us at 100x256x128 and 15 at 40x64x32; with the left boundary in the
+// threads of i = 1, one lane of every third warp, 66 and 11; so 32 and 8.)
 static int radial_bc(ttfld_ctx* c, bool upper_first) {
   Dev d = c->d;
   if (d.bcxmin != 9) return TTFLD_E_UNSUPPORTED;
-  launch_box(c->stream, box(1, d.nx + 2, -1, d.ny + 2, -1, d.nz + 2), [=] __device__(int i, int j, int k) {
+  const FastDiv by_cells = fast_div(d.nx + 1), by_j = fast_div(d.ny + 4);
+  const int cols = (d.ny + 4) * (d.nz + 4);
+  launch_box(c->stream, box(0, cols * (d.nx + 2) - 1, 0, 0, 0, 0), [=] __device__(int t, int, int) {
+    unsigned int col = (unsigned int)t, cell = 0, ju;
+    if (t >= cols) col = div_rem(by_cells, (unsigned int)(t - cols), cell);
+    const int k = (int)div_rem(by_j, col, ju) - 1, j = (int)ju - 1;
     const int ub = PA(UB, j, k);
-    if (i == 1 && !upper_first) left_column(d, j, k);
-    if (i >= ub && ub >= 1) upper_cell(d, i, j, k, ub);
-    if (i == 1 && upper_first) left_column(d, j, k);
+    if (t >= cols) {
+      const int i = (int)cell + 2;
+      if (i >= ub && ub >= 1) upper_cell(d, i, j, k, ub);
+      return;
+    }
+    if (!upper_first) left_column(d, j, k);
+    if (ub == 1) upper_cell(d, 1, j, k, ub);
+    if (upper_first) left_column(d, j, k);
   });
   TT_CHECK_LAUNCH();
   return 0;
