@@ -37,9 +37,10 @@
 // Gauss-Seidel sweep (half the iterations, three times the cost of one).
 //
 // Layout.  The FP32 inner arrays are line-major, q = (i-1)*NY*NZ +
-// (k-1)*NY + (j-1): in a line solve one thread walks one column and the
-// threads of a warp touch 32 consecutive columns of the same radius
-// (coalesced); in the operator pass the phi and theta neighbours are at q
+// (k-1)*NY + (j-1): in a line solve of block Jacobi one thread walks one
+// column and the threads of a warp touch 32 consecutive columns of the same
+// radius (coalesced), line Gauss-Seidel copies tiles of 32 such columns to
+// shared memory; in the operator pass the phi and theta neighbours are at q
 // +- 1 and q +- NY.  The inner iteration is one persistent cooperative
 // kernel with two grid barriers per iteration (after s = S p for alpha,
 // after the line solve for beta).
