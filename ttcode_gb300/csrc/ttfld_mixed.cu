@@ -540,7 +540,7 @@ __global__ void __launch_bounds__(kPersistThreads) sweeps32_local(Cmp g, Mix32 m
                                                                  int norm_every, int stall_check, unsigned int* flags,
                                                                  unsigned int base, long long norms, L2Keep keep) {
   __shared__ double sh[32];
-  __shared__ int stop_sh;
+  __shared__ int stop_sh, gave_up[2];
   extern __shared__ __align__(16) unsigned char slots_raw[];
   float4* slots = reinterpret_cast<float4*>(slots_raw);
   unsigned int* own = flags + (size_t)blockIdx.x * kFlagStride;
@@ -570,14 +570,31 @@ __global__ void __launch_bounds__(kPersistThreads) sweeps32_local(Cmp g, Mix32 m
   const int it0 = sol->iter;
   unsigned int half = base;  // half-sweeps this block has finished
   int sw = 1;
+  // RESIDENT, with few warps a block, each warp polls the flags itself and
+  // starts when it has seen them, a block barrier earlier; one that gives up
+  // says so in the slot of the wait's parity, which all read behind the next
+  // block barrier (implicit step 736 -> 714 us at 40x64x32, 1.50 -> 1.44 ms at
+  // 53x90x47 with poles)
+  if (RESIDENT) {
+    if (threadIdx.x < 2) gave_up[threadIdx.x] = 0;
+    __syncthreads();
+  }
+  auto wait = [&]() -> bool {
+    if (!RESIDENT) return wait_flags(flags, lo, hi, half, sol);
+    if (!poll_flags(flags, lo, hi, half, sol)) gave_up[half & 1] = 1;
+    __syncwarp();  // the other lanes' loads come after each lane's acquires
+    return true;
+  };
   for (; sw <= nsweeps; ++sw) {
     const bool norm = norm_every > 0 && (sw % norm_every == 0 || sw == nsweeps);
     float nacc = 0.f;
-    if (sw > 1 && !wait_flags(flags, lo, hi, half, sol)) break;
+    const unsigned int h0 = half;
+    if (sw > 1 && !wait()) break;
     if (norm) sweep_local<0, true, POLES, RESIDENT>(g, m, omega, t0, mine, nv, plane, slots, nacc, keep, (sw & 1) != 0);
     else sweep_local<0, false, POLES, RESIDENT>(g, m, omega, t0, mine, nv, plane, slots, nacc, keep, (sw & 1) != 0);
     publish_flag(own, ++half);
-    if (!wait_flags(flags, lo, hi, half, sol)) break;
+    if (RESIDENT && gave_up[h0 & 1]) break;
+    if (!wait()) break;
     if (norm) sweep_local<1, true, POLES, RESIDENT>(g, m, omega, t0, mine, nv, plane, slots, nacc, keep, (sw & 1) != 0);
     else sweep_local<1, false, POLES, RESIDENT>(g, m, omega, t0, mine, nv, plane, slots, nacc, keep, (sw & 1) != 0);
     if (norm) {
@@ -585,6 +602,7 @@ __global__ void __launch_bounds__(kPersistThreads) sweeps32_local(Cmp g, Mix32 m
       if (lane == 0) sh[warp] = v;
     }
     publish_flag(own, ++half);  // its block barrier also orders sh
+    if (RESIDENT && gave_up[~h0 & 1]) break;
     if (norm) {
       ++norms;
       if (warp == 0) {
