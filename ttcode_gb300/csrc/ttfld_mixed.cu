@@ -1513,7 +1513,7 @@ struct FastRows {
   typedef double2 Word;
   typedef double2 Kept;
   static constexpr int kWords = 8, kThreads = 768;  // 196 KB for two stages
-  static constexpr bool kStrided = false;
+  static constexpr bool kStrided = false, kBoundary = false;
   Fast64 m;
   double omega;
   long long rows;
@@ -1522,8 +1522,8 @@ struct FastRows {
   __device__ double norm(double sum) const { return sum; }
   template <int COL>
   __device__ void before(unsigned int, unsigned int) const {}
-  template <int COL>
-  __device__ void after(unsigned int, unsigned int, bool) const {}
+  __device__ bool boundary(bool) const { return false; }
+  __device__ void write_boundary(unsigned int, unsigned int, bool) const {}
   template <int COL>
   __device__ __forceinline__ void fetch(unsigned int row, unsigned int h, double2* to, unsigned int T, uint64_t pol) const {
     const size_t c = (size_t)row * nxp + 2 * h;

@@ -219,7 +219,14 @@ int radiativebound(ttfld_ctx* c, double d_t, double tinit_bottom) {
 // it is, is left out: T(1) never changes, so ER(1) = arad T(1)^4, which it
 // starts from, is simply not overwritten, ER at i <= 0 is set once, and the
 // top (but for IBDRAD = 9 with III > 1, whose top moves on with every
-// application) is set once and not overwritten.  The theta ghosts are
+// application) is set once and not overwritten.  An application writes cells
+// of both colours, which the neighbouring columns read in the colour before it
+// (ER at i >= UPPERBND of a column lies beside interior cells of another where
+// UPPERBND differs, and beside the top itself); so a block writes them once its
+// neighbours have finished that colour, and they begin the next once it has
+// written them (boundary_step): one exchange more per solve, or per colour
+// where the top moves (4.6 us a colour with a fixed top, 12.2 with a moving one,
+// whose decisions are waited for too, at 40x64x32).  The theta ghosts are
 // copies of the cell next to them, so after the first colour the cell itself
 // is read in their place, the phi neighbours by wrapping j.  The ghosts
 // themselves are filled after the last sweep (radbound_ghost_bottom, radbound_ghost_theta).
@@ -227,7 +234,7 @@ struct RadRows {
   typedef double Word;
   typedef double Kept;
   static constexpr int kWords = 8, kThreads = 1024;
-  static constexpr bool kStrided = true;
+  static constexpr bool kStrided = true, kBoundary = true;
   Dev d;
   RadWork w;
   double om, d_t, tinit_bottom;
@@ -263,10 +270,8 @@ struct RadRows {
     }
     __syncthreads();
   }
-  template <int COL>
-  __device__ void after(unsigned int r0, unsigned int r1, bool first) const {
-    if (!first && !moving_top) return;
-    __syncthreads();
+  __device__ bool boundary(bool first) const { return first || moving_top; }
+  __device__ void write_boundary(unsigned int r0, unsigned int r1, bool first) const {
     for (unsigned int r = r0 + threadIdx.x; r < r1; r += blockDim.x) {
       unsigned int j0;
       const int k = (int)div_rem(d.by_ny, r, j0) + 1, j = (int)j0 + 1;

@@ -46,8 +46,14 @@
 //                           has run yet; kept: where the old value (Kept) goes
 //   restore(row, h, kept)   puts a value of the first colour back
 //   kStrided                the items of a colour are not contiguous in memory
-//   before<COL>(r0, r1), after<COL>(r0, r1, first)  a block's own work around
-//                           a colour (all its threads; boundary values of its rows)
+//   before<COL>(r0, r1)     a block's own work ahead of a colour (all its threads),
+//                           on values that no update reads
+//   boundary(first)         whether boundary values of the rows are written
+//                           behind the colour (the same for all blocks)
+//   write_boundary(r0, r1, first)  the block's share of them (all its threads).
+//                           Its neighbours read these values in the colour, so
+//                           it is called once they have finished it
+//   kBoundary               there may be such values
 //   norm(sum)               the norm from the sum of the shares
 #pragma once
 #include "ttfld_internal.cuh"
@@ -153,6 +159,21 @@ __device__ __forceinline__ double sweep_colour(const Sys& s, unsigned int r0, un
   return acc;
 }
 
+// The boundary values behind a colour, if any, as a step of its own between
+// two flags: the first says that this block has read what its neighbours will
+// write, the caller's next one that its own values are there.  False if the
+// wait gave up.
+template <class Sys>
+__device__ __forceinline__ bool boundary_step(const Sys& s, unsigned int r0, unsigned int r1, bool first,
+                                              unsigned int* flags, int lo, int hi, unsigned int& half,
+                                              SolverDev* sol) {
+  if (!Sys::kBoundary || !s.boundary(first)) return true;
+  publish_flag(flags + (size_t)blockIdx.x * kFlagStride, ++half);
+  if (!wait_flags(flags, lo, hi, half, sol)) return false;
+  s.write_boundary(r0, r1, first);
+  return true;
+}
+
 template <class Sys, bool RESIDENT>
 __global__ void __launch_bounds__(Sys::kThreads, 1)
     sweeps64_persistent(Sys s, SolverDev* sol, Partial* gather, unsigned int* flags, typename Sys::Kept* keep,
@@ -197,7 +218,7 @@ __global__ void __launch_bounds__(Sys::kThreads, 1)
   typename Sys::Word* copy1 = copy ? copy0 + (size_t)Sys::kWords * n : nullptr;
   typename Sys::Kept* mine = keep ? keep + (size_t)r0 * s.by_items.d : nullptr;
   unsigned int* own = flags + (size_t)b * kFlagStride;
-  unsigned int half = 0;  // half-sweeps this block has finished
+  unsigned int half = 0;  // half-sweeps (and boundary steps) this block has finished
   int stop = 0;
   for (int sw = 1; sw <= nsweeps && !stop; ++sw) {
     if (sw > 1) {
@@ -207,7 +228,7 @@ __global__ void __launch_bounds__(Sys::kThreads, 1)
     s.template before<0>(r0, r1);
     double acc = sweep_colour<0, RESIDENT>(s, r0, n, sw == 1, slots, stage, sw > 1 ? mine : nullptr, pol,
                                             sw > 1 ? Copy{copy0, copy1, nullptr} : Copy{nullptr, nullptr, copy0});
-    s.template after<0>(r0, r1, sw == 1);
+    if (!boundary_step(s, r0, r1, sw == 1, flags, lo, hi, half, sol)) break;
     publish_flag(own, ++half);
     // the first warp waits for the neighbours, the last takes the last
     // sweep's rule, and with it whether this sweep begins at all
@@ -225,7 +246,7 @@ __global__ void __launch_bounds__(Sys::kThreads, 1)
     s.template before<1>(r0, r1);
     acc += sweep_colour<1, RESIDENT>(s, r0, n, false, slots, stage, nullptr, pol,
                                       sw > 1 ? Copy{copy1, copy0, nullptr} : Copy{nullptr, copy0, copy1});
-    s.template after<1>(r0, r1, false);
+    if (!boundary_step(s, r0, r1, false, flags, lo, hi, half, sol)) break;
     publish_flag(own, ++half);
     // behind the flag, that the neighbours wait for; where the decision comes
     // a colour later the block's share is put at the next sweep's start
@@ -332,7 +353,7 @@ struct SorRows {
   typedef double Word;
   typedef double Kept;
   static constexpr int kWords = 8, kThreads = 1024;
-  static constexpr bool kStrided = true;
+  static constexpr bool kStrided = true, kBoundary = false;
   const double *a, *xm, *xp, *jm, *jp, *km, *kp, *b;
   double* x;
   double omega;
@@ -341,8 +362,8 @@ struct SorRows {
   FastDiv by_items, by_ny;
   template <int COL>
   __device__ void before(unsigned int, unsigned int) const {}
-  template <int COL>
-  __device__ void after(unsigned int, unsigned int, bool) const {}
+  __device__ bool boundary(bool) const { return false; }
+  __device__ void write_boundary(unsigned int, unsigned int, bool) const {}
   __device__ double norm(double sum) const { return sum; }
   // radial index (from 0) of item h of a row: i + j + k, all from 1, has COL's parity
   template <int COL>
