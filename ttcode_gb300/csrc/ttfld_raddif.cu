@@ -275,7 +275,8 @@ struct RadRows {
     for (unsigned int r = r0 + threadIdx.x; r < r1; r += blockDim.x) {
       unsigned int j0;
       const int k = (int)div_rem(d.by_ny, r, j0) + 1, j = (int)j0 + 1;
-      if (first) radbound_bottom(d, j, k, d_t, tinit_bottom);
+      // (a top that begins at i <= 1 starts from the bottom's value each time)
+      if (first || PA(UB, j, k) <= 1) radbound_bottom(d, j, k, d_t, tinit_bottom);
       radbound_top(d, j, k);
     }
   }
@@ -331,8 +332,10 @@ struct RadRows {
 // ghosts' cells above i = 1 (RadRows::before).
 __global__ void __launch_bounds__(kThreads) radbound_ghost_bottom(Dev d, double d_t, double tinit_bottom) {
   const int n = (d.ny + 4) * (d.nz + 4);
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x)
-    radbound_bottom(d, t % (d.ny + 4) - 1, t / (d.ny + 4) - 1, d_t, tinit_bottom);
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+    const int j = t % (d.ny + 4) - 1, k = t / (d.ny + 4) - 1;
+    if (j < 1 || j > d.ny || k < 1 || k > d.nz) radbound_bottom(d, j, k, d_t, tinit_bottom);
+  }
 }
 __global__ void __launch_bounds__(kThreads) radbound_ghost_theta(Dev d) {
   const int nx = d.nx, ny = d.ny, nz = d.nz, n = (nx + 4) * (ny + 4);
