@@ -35,6 +35,19 @@ int grid_for(long long n, int threads) {
   return (int)blocks;
 }
 
+size_t smem_room(const void* kernel) {
+  int dev = 0, room = 0;
+  cudaFuncAttributes at;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&room, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
+      cudaFuncGetAttributes(&at, kernel) != cudaSuccess || (room -= (int)at.sharedSizeBytes) <= 0 ||
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, room) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return (size_t)room;
+}
+
 // L2 policies by sixteenths of the lines kept (0: every line leaves first).
 constexpr int kPolicies = 17;
 __device__ unsigned long long g_policies[kPolicies];

@@ -174,6 +174,13 @@ __global__ void __launch_bounds__(kThreads) box_kernel(Box b, Fn fn) {
 }
 
 int grid_for(long long n, int threads = kThreads);
+// The most dynamic shared memory that a block of `kernel` may have on the
+// current device, with the kernel allowed that much (0 after a CUDA error).
+// The limit belongs to the kernel on the device, for all contexts and host
+// threads, so it is set to the same value by every call: one set to what the
+// caller is about to launch with could be lowered by another thread before
+// that launch.
+size_t smem_room(const void* kernel);
 void count_launches(int n);
 
 template <class Fn>

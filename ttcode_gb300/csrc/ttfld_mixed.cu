@@ -65,8 +65,21 @@ struct Fast64 {
   double* x[2];     // iterate, with theta ghost planes
 };
 
+// Launch shapes of the persistent kernels: their blocks (0: not available) and
+// the product form's threads, shared memory and L2 marks.  Kept with the
+// context, whose grid, device and host thread are one: what a launch takes in
+// shared memory must be what its blocks were counted for.
+struct SweepGrids {
+  int sized;  // bit m: SweepForm m is
+  int pers, tma, wave, local;
+  int local_threads, resident;
+  size_t local_smem;
+  L2Keep l2;
+};
+
 struct MixWork {
   Cmp g;
+  SweepGrids grids;
   int have32, have64;
   void* mem32;
   void* mem64;
@@ -1029,11 +1042,7 @@ static int persistent_grid(K kernel, int threads, size_t smem, long long items) 
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (smem > 48 * 1024 &&
-      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-    cudaGetLastError();
-    return 0;
-  }
+  if (smem > 48 * 1024 && smem_room((const void*)kernel) < smem) return 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
   long long coresident = coop ? (long long)sms * per_sm : 0;
   if (coresident > kMaxPartials) coresident = kMaxPartials;
@@ -1064,22 +1073,20 @@ static int wave_planes(const Cmp& g) {
   return p;
 }
 
-// Blocks of the persistent kernels for nvec items (0: not available),
-// sized once per grid size and pole form.
-struct SweepGrids {
-  int pers, tma, wave, local;
-  int local_threads, resident;
-  size_t local_smem;
-  L2Keep l2;
-};
+// The launch shapes of a context with those of `form` sized, by its first solve
+// with it (all five of them would be 60 us of a context's first step, a fourteenth
+// of it at 40x64x32), and with the grid-barrier kernel's where that kernel takes
+// the form's place.
 template <bool POLES>
-static SweepGrids sweep_grids(long long nvec) {
-  static SweepGrids gr = {-1, -1, -1, -1, 0, 0, 0, {0, 0}};
-  static long long sized_for = -1;
-  if (sized_for != nvec) {
-    gr.tma = persistent_grid(sweeps32_tma<POLES>, kTmaThreads, kTmaSmem, nvec);
-    gr.pers = persistent_grid(sweeps32_persistent<POLES>, kPersistThreads, 0, nvec);
-    gr.wave = nvec < (1LL << 31) ? persistent_grid(sweeps32_wave<POLES>, kPersistThreads, 0, nvec) : 0;
+static const SweepGrids& sweep_grids(MixWork* w, SweepForm form) {
+  SweepGrids& gr = w->grids;
+  if (gr.sized & (1 << form)) return gr;
+  const long long nvec = w->g.rows * (w->g.nxp >> 2);
+  int own = 0;
+  if (form == kFormTma) own = gr.tma = persistent_grid(sweeps32_tma<POLES>, kTmaThreads, kTmaSmem, nvec);
+  if (form == kFormWave)
+    own = gr.wave = nvec < (1LL << 31) ? persistent_grid(sweeps32_wave<POLES>, kPersistThreads, 0, nvec) : 0;
+  if (form == kFormNeighbour) {
     // one block per SM, none of less than two warps' items, with the items
     // of both colours in shared memory where they fit
     const size_t item = 2 * kLocalWords * sizeof(float4);  // both colours
@@ -1104,13 +1111,14 @@ static SweepGrids sweep_grids(long long nvec) {
     }
     if (gr.local > kMaxLocalBlocks) gr.local = 0;
     gr.l2 = l2_keep(32.0 * (double)nvec, 7 * 32.0 * (double)nvec);  // e; the couplings and r-hat, of both colours
-    sized_for = nvec;
+    own = gr.local;
   }
+  if (form != kFormSplit && own <= 0) gr.pers = persistent_grid(sweeps32_persistent<POLES>, kPersistThreads, 0, nvec);
+  gr.sized |= 1 << form;
   return gr;
 }
-static SweepGrids sweep_grids_of(const Cmp& g) {
-  const long long nvec = g.rows * (g.nxp >> 2);
-  return g.poles ? sweep_grids<true>(nvec) : sweep_grids<false>(nvec);
+static const SweepGrids& sweep_grids_of(MixWork* w, SweepForm form) {
+  return w->g.poles ? sweep_grids<true>(w, form) : sweep_grids<false>(w, form);
 }
 // The form runs as one launch that stops itself.
 static bool one_launch_form(const SweepGrids& gr, SweepForm form) {
@@ -1139,7 +1147,7 @@ static int launch_sweeps32_form(ttfld_ctx* c, int nsweeps, int norm_every, doubl
   double* partials = c->partials;
   int stall = stall_check ? 1 : 0;
   void* args[] = {&g, &m, &omega, &sol, &partials, &stop_ratio, &nsweeps, &norm_every, &stall};
-  const SweepGrids gr = sweep_grids<POLES>(nvec);
+  const SweepGrids& gr = sweep_grids<POLES>(w, form);
   if (form != kFormSplit && form != kFormNeighbour)  // the grid barrier counts arrivals from zero
     TT_CHECK(cudaMemsetAsync(&sol->arrivals, 0, sizeof(unsigned long long), c->stream));
   if (form == kFormWave && gr.wave > 0) {
@@ -1256,7 +1264,7 @@ int solve_mixed(ttfld_ctx* c, double* x, const double* b, ttfld_solve_stats* st,
                          : c->opts.sweep_form == 4 ? kFormGrid
                                                    : kFormNeighbour;
   // one launch per anchor needs a persistent kernel (it stops itself)
-  const bool one_launch = one_launch_form(sweep_grids_of(g), form);
+  const bool one_launch = one_launch_form(sweep_grids_of(w, form), form);
   if (guess_test) {
     TT_CHECK(cudaMemsetAsync(&c->sol->done, 0, sizeof(int), c->stream));
     TT_CHECK(cudaMemsetAsync(w->m32.e[0], 0, 2 * g.gsz * sizeof(float), c->stream));
