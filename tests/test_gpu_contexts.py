@@ -26,7 +26,8 @@ def context(dims):
 
 
 def solve(f, solver):
-    f.set_solver(solver, tol=1e-10)
+    if solver != "hypre":
+        f.set_solver(solver, tol=1e-10)
     f.begin_step(new_run=True)
     st = f.solve_with_hypre(tol=1e-8, maxit=1000) if solver == "hypre" else f.solve_system()
     return st.sor_iter, st.status, f.download("DELTA_ER")
@@ -70,3 +71,7 @@ def in_turn_and_at_once(sizes, solvers, rounds):
 
 def test_product_solves():
     in_turn_and_at_once(SIZES, ["mixed"], 25)
+
+
+def test_other_solvers():
+    in_turn_and_at_once([(24, 16, 12), (40, 64, 32), (96, 112, 64)], ["sor64_exact", "sor64_fast", "pcg", "hypre"], 8)

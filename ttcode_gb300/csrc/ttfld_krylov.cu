@@ -914,7 +914,7 @@ PcgShape pcg_shape(const Kry& k, bool gs) {
   }
   const void* kern = pcg_kernel(gs, p.shared);
   int per_sm = 0;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem) != cudaSuccess ||
+  if (smem_room(kern) < p.smem ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, p.threads, p.smem) != cudaSuccess || per_sm < 1) {
     cudaGetLastError();
     return p;
@@ -970,11 +970,7 @@ StripShape strip_shape(const Kry& k, const void* kernel, int arrays) {
   s.blocks = s.strips < 1024 ? (int)s.strips : 1024;
   s.smem = (size_t)arrays * k.nx * kStripPitch * sizeof(float);
   s.staged = s.smem <= 200 * 1024;
-  if (s.staged && s.smem > 48 * 1024 &&
-      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.smem) != cudaSuccess) {
-    cudaGetLastError();
-    s.staged = 0;
-  }
+  if (s.staged && s.smem > 48 * 1024 && smem_room(kernel) < s.smem) s.staged = 0;
   if (!s.staged) s.smem = 0;
   return s;
 }

@@ -312,10 +312,7 @@ int launch_sweeps64_persistent(const Sys& s, cudaStream_t st, SolverDev* sol, do
   const bool resident = item * (size_t)most + 1024 <= (size_t)room;
   const size_t smem = item * (size_t)(resident ? most : threads);
   const void* kernel = resident ? (const void*)sweeps64_persistent<Sys, true> : (const void*)sweeps64_persistent<Sys, false>;
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-    cudaGetLastError();
-    return 1;
-  }
+  if (smem_room(kernel) < smem) return 1;
   TT_CHECK(cudaMemsetAsync(flags, 0, (size_t)nb * kFlagStride * sizeof(unsigned int), st));
   Partial* gather = (Partial*)partials;  // two a block
   TT_CHECK(cudaMemsetAsync(gather, 0, (size_t)nb * 2 * sizeof(Partial), st));
