@@ -512,9 +512,14 @@ int ttfld_guess_save(ttfld_ctx* ctx, void* blob, size_t bytes, size_t* needed);
  * call on a device (in each CUDA context: a caller's own context on the
  * device counts as a new one) looks up the array's device address in that
  * context.  Every call returns only after its solve has finished on the
- * GPU (it blocks the calling host thread): it waits on `stream` to read
- * the stopping flag between chunks of sweeps.  NY must be
- * even. */
+ * GPU (it blocks the calling host thread): it works on `stream` alone and
+ * waits for that stream, no other.  The sweeps are one cooperative launch, at
+ * most one block per SM with up to 1024 threads, all of an SM's registers and
+ * 227 KB of shared memory (288 threads and 35 KB at 40x64x33), which the GPU
+ * starts when all of its blocks fit beside what is running: behind kernels
+ * that leave the SMs less, it begins once they end, so no such kernel may wait
+ * for the result.  Where the stream has fewer SMs than the device, two
+ * launches per sweep take its place.  NY must be even. */
 int ttfld_sor_solve_noalloc(const double* sor_a, const double* sor_b, const double* sor_c,
                             const double* sor_d, const double* sor_e, const double* sor_f,
                             const double* sor_g, const double* rhs, double* x, int nx, int ny,

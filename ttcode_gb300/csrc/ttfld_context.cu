@@ -63,32 +63,40 @@ __global__ void policies_kernel() {
   }
 }
 
-uint64_t l2_policy(double keep) {
+// The first call on a device makes them, on the stream it is given, and waits
+// for that stream alone (without the lock: what that stream waits for may need
+// another thread's solve).
+uint64_t l2_policy(double keep, cudaStream_t st) {
   constexpr int kDevices = 64;
   static std::mutex lock;
   static unsigned long long table[kDevices][kPolicies];
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev >= kDevices) return 0;
-  std::lock_guard<std::mutex> hold(lock);
-  if (!table[dev][0]) {
-    policies_kernel<<<1, 1>>>();
-    if (check_cuda(cudaGetLastError(), "L2 policies") ||
-        check_cuda(cudaMemcpyFromSymbol(table[dev], g_policies, sizeof(table[dev])), "L2 policies")) {
-      table[dev][0] = 0;
-      return 0;
-    }
+  int q = (int)(keep * (kPolicies - 1) + 0.5);
+  q = q < 0 ? 0 : q < kPolicies ? q : kPolicies - 1;
+  {
+    std::lock_guard<std::mutex> hold(lock);
+    if (table[dev][0]) return table[dev][q];
   }
-  const int q = (int)(keep * (kPolicies - 1) + 0.5);
-  return table[dev][q < 0 ? 0 : q < kPolicies ? q : kPolicies - 1];
+  unsigned long long made[kPolicies];
+  policies_kernel<<<1, 1, 0, st>>>();
+  if (check_cuda(cudaGetLastError(), "L2 policies") ||
+      check_cuda(cudaMemcpyFromSymbolAsync(made, g_policies, sizeof(made), 0, cudaMemcpyDeviceToHost, st),
+                 "L2 policies") ||
+      check_cuda(cudaStreamSynchronize(st), "L2 policies"))
+    return 0;
+  std::lock_guard<std::mutex> hold(lock);
+  memcpy(table[dev], made, sizeof(made));
+  return made[q];
 }
 
-L2Keep l2_keep(double iter_bytes, double coef_bytes) {
+L2Keep l2_keep(double iter_bytes, double coef_bytes, cudaStream_t st) {
   int dev = 0, l2 = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev);
   const double room = 0.55 * l2, left = room - iter_bytes;
-  return L2Keep{l2_policy(left >= 0.0 ? 1.0 : room / iter_bytes),
-                l2_policy(left <= 0.0 ? 0.0 : coef_bytes <= left ? 1.0 : left / coef_bytes)};
+  return L2Keep{l2_policy(left >= 0.0 ? 1.0 : room / iter_bytes, st),
+                l2_policy(left <= 0.0 ? 0.0 : coef_bytes <= left ? 1.0 : left / coef_bytes, st)};
 }
 
 // Copy between a box-shaped contiguous buffer and an internal array.
@@ -331,7 +339,7 @@ int ttfld_create(ttfld_ctx** out, const ttfld_dims* dims, const ttfld_metrics* m
     ttfld_destroy(c);
     return TTFLD_E_CUDA;
   }
-  if (!l2_policy(0.0)) {  // made before the first solve
+  if (!l2_policy(0.0, c->stream)) {  // made before the first solve
     ttfld_destroy(c);
     return TTFLD_E_CUDA;
   }

@@ -443,13 +443,13 @@ struct L2Keep {
 };
 // Of what the L2 holds, 0.55 (70 of 126 MB): over unique footprints of 79 to
 // 671 MB of the FP32 sweeps 60 to 80 MB is best, 90 MB up to 12 % slower.
-L2Keep l2_keep(double iter_bytes, double coef_bytes);
+L2Keep l2_keep(double iter_bytes, double coef_bytes, cudaStream_t st);
 // The policy that keeps a fraction of the lines (in sixteenths).  A kernel
 // takes it as a parameter: made in the kernel it would live in a register of
 // each thread, and the accesses want it the same for a whole warp, whatever
-// the compiler does with that register where threads part.  0 after a CUDA
-// error.
-uint64_t l2_policy(double keep);
+// the compiler does with that register where threads part.  The first call on a
+// device waits for the stream.  0 after a CUDA error.
+uint64_t l2_policy(double keep, cudaStream_t st);
 
 // An asynchronous copy of one 8- or 16-byte word to shared memory.
 template <class W>

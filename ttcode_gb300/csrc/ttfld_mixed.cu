@@ -1078,7 +1078,8 @@ static int wave_planes(const Cmp& g) {
 // of it at 40x64x32), and with the grid-barrier kernel's where that kernel takes
 // the form's place.
 template <bool POLES>
-static const SweepGrids& sweep_grids(MixWork* w, SweepForm form) {
+static const SweepGrids& sweep_grids(ttfld_ctx* c, SweepForm form) {
+  MixWork* w = work(c);
   SweepGrids& gr = w->grids;
   if (gr.sized & (1 << form)) return gr;
   const long long nvec = w->g.rows * (w->g.nxp >> 2);
@@ -1110,15 +1111,16 @@ static const SweepGrids& sweep_grids(MixWork* w, SweepForm form) {
       gr.local = persistent_grid(sweeps32_local<POLES>, kPersistThreads, 0, nvec);
     }
     if (gr.local > kMaxLocalBlocks) gr.local = 0;
-    gr.l2 = l2_keep(32.0 * (double)nvec, 7 * 32.0 * (double)nvec);  // e; the couplings and r-hat, of both colours
+    // e; the couplings and r-hat, of both colours
+    gr.l2 = l2_keep(32.0 * (double)nvec, 7 * 32.0 * (double)nvec, c->stream);
     own = gr.local;
   }
   if (form != kFormSplit && own <= 0) gr.pers = persistent_grid(sweeps32_persistent<POLES>, kPersistThreads, 0, nvec);
   gr.sized |= 1 << form;
   return gr;
 }
-static const SweepGrids& sweep_grids_of(MixWork* w, SweepForm form) {
-  return w->g.poles ? sweep_grids<true>(w, form) : sweep_grids<false>(w, form);
+static const SweepGrids& sweep_grids_of(ttfld_ctx* c, SweepForm form) {
+  return work(c)->g.poles ? sweep_grids<true>(c, form) : sweep_grids<false>(c, form);
 }
 // The form runs as one launch that stops itself.
 static bool one_launch_form(const SweepGrids& gr, SweepForm form) {
@@ -1147,7 +1149,7 @@ static int launch_sweeps32_form(ttfld_ctx* c, int nsweeps, int norm_every, doubl
   double* partials = c->partials;
   int stall = stall_check ? 1 : 0;
   void* args[] = {&g, &m, &omega, &sol, &partials, &stop_ratio, &nsweeps, &norm_every, &stall};
-  const SweepGrids& gr = sweep_grids<POLES>(w, form);
+  const SweepGrids& gr = sweep_grids<POLES>(c, form);
   if (form != kFormSplit && form != kFormNeighbour)  // the grid barrier counts arrivals from zero
     TT_CHECK(cudaMemsetAsync(&sol->arrivals, 0, sizeof(unsigned long long), c->stream));
   if (form == kFormWave && gr.wave > 0) {
@@ -1264,7 +1266,7 @@ int solve_mixed(ttfld_ctx* c, double* x, const double* b, ttfld_solve_stats* st,
                          : c->opts.sweep_form == 4 ? kFormGrid
                                                    : kFormNeighbour;
   // one launch per anchor needs a persistent kernel (it stops itself)
-  const bool one_launch = one_launch_form(sweep_grids_of(w, form), form);
+  const bool one_launch = one_launch_form(sweep_grids_of(c, form), form);
   if (guess_test) {
     TT_CHECK(cudaMemsetAsync(&c->sol->done, 0, sizeof(int), c->stream));
     TT_CHECK(cudaMemsetAsync(w->m32.e[0], 0, 2 * g.gsz * sizeof(float), c->stream));

@@ -10,10 +10,10 @@
 // create a ttfld context (which allocates its arrays and workspaces).  This
 // entry point takes the SOR coefficients, the right-hand side and the
 // iterate as device pointers and allocates nothing: the only memory it needs
-// beyond them -- the per-row partial sums of the residual norm and the
-// loop's bookkeeping -- lives in one file-scope __device__ array of fixed
-// size, which every GPU that loads the library holds until the process
-// exits.
+// beyond them -- the shares of the residual norm, the blocks' flags, the
+// values kept for putting back and the loop's bookkeeping -- lives in one
+// file-scope __device__ array of fixed size, which every GPU that loads the
+// library holds until the process exits.
 //
 // Limits and sharing rules:
 //  * NY*NZ <= kNoAllocMaxRows (131072 rows, e.g. 512 x 256); larger grids are
@@ -29,7 +29,11 @@
 //    (cuCtxGetId): after cudaDeviceReset, or in a context the caller made
 //    itself with the driver API, the first call there looks it up again.
 //  * Each call returns once its solve has finished on the GPU (it
-//    synchronises its stream to read the stopping flag).
+//    synchronises its stream to read the stopping flag).  It works on that
+//    stream alone; the first call on a device waits for it once more, for the
+//    L2 policies (l2_policy).
+//  * The sweeps are one cooperative launch of a block per SM, which starts
+//    once all blocks fit beside what else is running.
 #include <mutex>
 
 #include "ttfld_sweep64.cuh"

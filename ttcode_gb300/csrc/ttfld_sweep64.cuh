@@ -320,7 +320,7 @@ int launch_sweeps64_persistent(const Sys& s, cudaStream_t st, SolverDev* sol, do
   typename Sys::Kept* keep =
       (size_t)items * sizeof(typename Sys::Kept) <= kept_bytes ? (typename Sys::Kept*)kept : nullptr;
   const double word = 2.0 * (double)items * sizeof(typename Sys::Word);  // an array of both colours
-  uint64_t pol = resident ? l2_policy(0.0) : l2_keep(word, Sys::kWords * word).coef;  // resident: read once
+  uint64_t pol = resident ? l2_policy(0.0, st) : l2_keep(word, Sys::kWords * word, st).coef;  // resident: read once
   if (!pol) return TTFLD_E_CUDA;
   // the first sweep's stores cost about what half a sweep's reads do
   typename Sys::Word* copy = nullptr;
