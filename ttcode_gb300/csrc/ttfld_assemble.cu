@@ -780,11 +780,11 @@ static int stellarinput_heating(ttfld_ctx* c) {
     if (i > d.nx) return;
     const double tinc = PA(TINC, j, k), mu = PA(MU, j, k);
     const double day = mul_rn(TT_SBCONST, div_rn(p4(tinc), mu));
-    // the night side (no incident flux) needs no exponential: any factor in
-    // (0, 1] gives the same signed zero, and an infinite tau has made dtaus
-    // non-finite too
+    // the night side (no incident flux) needs no exponential: with mu > 0 it is
+    // a factor in [0, 1], any of which gives the same signed zero, and an
+    // infinite tau has made dtaus non-finite too
     const double tau = HA(STAU, i, j, k);
-    const double ex = day == 0.0 && tau >= 0.0 ? 1.0 : exp(div_rn(-tau, mu));
+    const double ex = day == 0.0 && tau >= 0.0 && mu > 0.0 ? 1.0 : exp(div_rn(-tau, mu));
     HA(SI, i, j, k) = div_rn(mul_rn(mul_rn(day, ex), dtaus), G(dxb, i));
   });
   TT_CHECK_LAUNCH();
