@@ -61,6 +61,7 @@ struct OpacTab {
   int* err;
   const double *lt, *lrh, *ross, *plnk, *absk;
   const double *t10, *plnk10, *absk10;  // 10^ of the T nodes and of two of the means at the nodes
+  const double *lt_max, *lrh_max;       // the greatest node up to each (first_above)
 };
 
 static OpacTab opac_tab(const ttfld_ctx* c) {
@@ -76,17 +77,21 @@ static OpacTab opac_tab(const ttfld_ctx* c) {
   t.absk = p; p += (size_t)t.nt * t.nrh;
   t.t10 = p; p += t.nt;
   t.plnk10 = p; p += (size_t)t.nt * t.nrh;
-  t.absk10 = p;
+  t.absk10 = p; p += (size_t)t.nt * t.nrh;
+  t.lt_max = p; p += t.nt;
+  t.lrh_max = p;
   return t;
 }
 
 // The first node above v (1-based; n + 1: none), as the reference's loop from
-// the first node up finds it; the nodes increase.
-__device__ __forceinline__ int first_above(const double* node, int n, double v) {
+// the first node up finds it, in whatever order the nodes are: upto[m] is the
+// greatest of the first m + 1 (NaN left out), so the first one above v is that
+// of the first node above v.
+__device__ __forceinline__ int first_above(const double* upto, int n, double v) {
   int lo = 0, hi = n;
   while (lo < hi) {
     const int mid = (lo + hi) >> 1;
-    if (node[mid] > v) hi = mid;
+    if (upto[mid] > v) hi = mid;
     else lo = mid + 1;
   }
   return lo + 1;
@@ -112,7 +117,7 @@ __device__ __forceinline__ int burrows_opc(const OpacTab& tb, double t, double r
   if (tm1 > (double)3.69889f) tm1 = (double)3.69888f;
   if (rh1 < (double)-11.9996f) rh1 = (double)-11.9995f;
   if (rh1 > (double)-1.99993f) rh1 = (double)-1.99994f;
-  const int it = first_above(tb.lt, tb.nt, tm1);
+  const int it = first_above(tb.lt_max, tb.nt, tm1);
   if (it == tb.nt + 1) return 2;
   if (it == 1) return 3;
   const int it1 = it - 1;
@@ -120,7 +125,7 @@ __device__ __forceinline__ int burrows_opc(const OpacTab& tb, double t, double r
   double ws = tb.lt[it1 - 1] - tb.lt[it - 1];
   ws1 = div_rn(ws1, ws);
   ws = 1.0 - ws1;
-  const int iw = first_above(tb.lrh, tb.nrh, rh1);
+  const int iw = first_above(tb.lrh_max, tb.nrh, rh1);
   if (iw == tb.nrh + 1) return 2;
   if (iw == 1) return 3;
   const int iw1 = iw - 1;
@@ -155,7 +160,7 @@ __device__ __forceinline__ int burrows_wave(const OpacTab& tb, const double* wop
   if (tm1 > (double)3.69889f) tm1 = (double)3.69888f;
   if (rh1 < (double)-11.9996f) rh1 = (double)-11.9995f;
   if (rh1 > (double)-1.99993f) rh1 = (double)-1.99994f;
-  const int it = first_above(tb.lt, tb.nt, tm1);
+  const int it = first_above(tb.lt_max, tb.nt, tm1);
   if (it == tb.nt + 1) return 2;
   if (it == 1) return 3;
   const int it1 = it - 1;
@@ -163,7 +168,7 @@ __device__ __forceinline__ int burrows_wave(const OpacTab& tb, const double* wop
   double ws = tb.lt[it1 - 1] - tb.lt[it - 1];
   ws1 = div_rn(ws1, ws);
   ws = 1.0 - ws1;
-  const int iw = first_above(tb.lrh, tb.nrh, rh1);
+  const int iw = first_above(tb.lrh_max, tb.nrh, rh1);
   if (iw == tb.nrh + 1) return 2;
   if (iw == 1) return 3;
   const int iw1 = iw - 1;
@@ -949,7 +954,7 @@ int ttfld_set_opacity_table(ttfld_ctx* c, const ttfld_opacity_table* t) {
     return TTFLD_E_ARGS;
   const size_t nn = (size_t)t->nt * t->nrh;
   const size_t given = (size_t)t->nt + t->nrh + 3 * nn;
-  const size_t bytes = (1 + given + (size_t)t->nt + 2 * nn) * sizeof(double);
+  const size_t bytes = (1 + given + (size_t)t->nt + 2 * nn + (size_t)t->nt + t->nrh) * sizeof(double);
   TT_CHECK(cudaSetDevice(c->device));
   if (c->opac) {
     TT_CHECK(cudaStreamSynchronize(c->stream));
@@ -959,6 +964,7 @@ int ttfld_set_opacity_table(ttfld_ctx* c, const ttfld_opacity_table* t) {
   TT_CHECK(cudaMalloc(&c->opac, bytes));
   c->opac_nt = t->nt;
   c->opac_nrh = t->nrh;
+  const OpacTab tb = opac_tab(c);
   double* p = (double*)c->opac + 1;
   TT_CHECK(cudaMemcpy(p, t->log_t, t->nt * sizeof(double), cudaMemcpyHostToDevice));
   p += t->nt;
@@ -971,11 +977,17 @@ int ttfld_set_opacity_table(ttfld_ctx* c, const ttfld_opacity_table* t) {
   TT_CHECK(cudaMemcpy(p, t->log_abs, nn * sizeof(double), cudaMemcpyHostToDevice));
   // 10^ of the T nodes and of the Planck and absorption means, on the device,
   // whose exp10() the interpolation uses
-  const OpacTab tb = opac_tab(c);
   double* out = const_cast<double*>(tb.t10);
   const int nt = t->nt, n2 = (int)(nt + 2 * nn);
   launch_box(c->stream, box(0, n2 - 1, 0, 0, 0, 0), [=] __device__(int i, int, int) {
     out[i] = exp10(i < nt ? tb.lt[i] : tb.plnk[i - nt]);  // the two means lie one after the other
+  });
+  TT_CHECK_LAUNCH();
+  launch_box(c->stream, box(0, 1, 0, 0, 0, 0), [=] __device__(int q, int, int) {
+    const double* node = q ? tb.lrh : tb.lt;
+    double* upto = const_cast<double*>(q ? tb.lrh_max : tb.lt_max);
+    double top = -INFINITY;
+    for (int m = 0; m < (q ? tb.nrh : tb.nt); ++m) upto[m] = top = node[m] > top ? node[m] : top;
   });
   TT_CHECK_LAUNCH();
   TT_CHECK(cudaStreamSynchronize(c->stream));
