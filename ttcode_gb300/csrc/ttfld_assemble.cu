@@ -965,16 +965,11 @@ int ttfld_set_opacity_table(ttfld_ctx* c, const ttfld_opacity_table* t) {
   c->opac_nt = t->nt;
   c->opac_nrh = t->nrh;
   const OpacTab tb = opac_tab(c);
-  double* p = (double*)c->opac + 1;
-  TT_CHECK(cudaMemcpy(p, t->log_t, t->nt * sizeof(double), cudaMemcpyHostToDevice));
-  p += t->nt;
-  TT_CHECK(cudaMemcpy(p, t->log_rho, t->nrh * sizeof(double), cudaMemcpyHostToDevice));
-  p += t->nrh;
-  TT_CHECK(cudaMemcpy(p, t->log_ross, nn * sizeof(double), cudaMemcpyHostToDevice));
-  p += nn;
-  TT_CHECK(cudaMemcpy(p, t->log_plnk, nn * sizeof(double), cudaMemcpyHostToDevice));
-  p += nn;
-  TT_CHECK(cudaMemcpy(p, t->log_abs, nn * sizeof(double), cudaMemcpyHostToDevice));
+  struct { const double *to, *from; size_t n; } parts[] = {
+      {tb.lt, t->log_t, (size_t)t->nt}, {tb.lrh, t->log_rho, (size_t)t->nrh}, {tb.ross, t->log_ross, nn},
+      {tb.plnk, t->log_plnk, nn}, {tb.absk, t->log_abs, nn}};
+  for (const auto& p : parts)  // on the stream of the kernels below
+    TT_CHECK(cudaMemcpyAsync(const_cast<double*>(p.to), p.from, p.n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
   // 10^ of the T nodes and of the Planck and absorption means, on the device,
   // whose exp10() the interpolation uses
   double* out = const_cast<double*>(tb.t10);
