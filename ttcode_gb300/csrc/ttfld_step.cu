@@ -171,7 +171,10 @@ __global__ void __launch_bounds__(kThreads) delta_q_kernel(Dev d, double theta, 
     size_t h = hidx(d, i, j, k), q = cidx(d, i, j, k);
     const double q1 = -d.delt * (1.0 - theta);
     const double q2 = mul_rn(mul_rn(d.delt, d.RH[h]) * d.XKAPP[h], TT_FD);
-    double flow = 0.0;  // theta = 1 (ppenergy.f:60): the seven products are zeros
+    // theta = 1 (ppenergy.f:60): the seven products are zeros.  None hides a
+    // value that is not finite: x comes from a solve with a finite norm, and where
+    // a coefficient is not finite the cell's flux divergence, and so FQ, is not.
+    double flow = 0.0;
     if (q1 != 0.0)
       flow = q1 * d.E16[q] * x[h] - q1 * d.E1[q] * x[h + 1] - q1 * d.E2[q] * x[h - 1] - q1 * d.E3[q] * x[h + sj] -
              q1 * d.E4[q] * x[h - sj] - q1 * d.E5[q] * x[h + sk] - q1 * d.E6[q] * x[h - sk];
