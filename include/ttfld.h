@@ -241,7 +241,18 @@ typedef struct ttfld_ctx ttfld_ctx;
 #endif
 
 /* ---- lifetime (replaces the allocate* routines of ppmod.f for the
- *      arrays the step touches, and MPI_INIT's one-rank decomposition) ---- */
+ *      arrays the step touches, and MPI_INIT's one-rank decomposition) ----
+ * A context holds about 57 FP64 arrays (1.6 GB at 100x256x128) from
+ * ttfld_create on, and workspaces that the first call that wants one
+ * allocates and ttfld_destroy gives back, in bytes per cell: 40 for the
+ * FP32/FP64 solver, 72 for the scaled FP64 one, 56 for PCG and
+ * SOLVE_WITH_HYPRE, 72 for RADDIF, 8 for the previous solution, and for the
+ * exact SOR, DIFFUSION and RADDIF above 540,000 cells 64 for a copy of their
+ * coefficients (1.3 GB at 160x512x256; without it, where there is no room,
+ * they read the originals).  The network's are beside these.
+ * Solves are cooperative launches of at most one block per SM: the GPU starts
+ * one when all of its blocks fit beside what is running.  A context is used by
+ * one host thread at a time; contexts are independent of each other. */
 int ttfld_create(ttfld_ctx** out, const ttfld_dims* dims,
                  const ttfld_metrics* metrics, const ttfld_params* params,
                  int device);

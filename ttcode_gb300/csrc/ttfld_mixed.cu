@@ -486,9 +486,9 @@ __global__ void __launch_bounds__(kPersistThreads) sweeps32_persistent(Cmp g, Mi
 // barrier.  The relation is symmetric, so neighbours are never
 // more than one half-sweep apart and no block overwrites a colour that a
 // neighbour is still reading: every update reads the values it reads in the
-// grid-barrier form, whose iterate this is, bit for bit.  Norm sweeps still
-// end with a grid barrier: the stop decision needs every block's partial.
-// Flags count half-sweeps from a base that the host advances by 2 nsweeps
+// grid-barrier form, whose iterate this is, bit for bit.  Behind a norm sweep
+// every block waits for all blocks' shares of the norm (gather_sum), which the
+// stop decision needs, and for nothing else.  Flags count half-sweeps from a base that the host advances by 2 nsweeps
 // per launch, and every block leaves its flag at base + 2 nsweeps whenever
 // it returns, so all flags equal the base when the next launch starts.
 // Timed against the grid-barrier kernel in one process on a GB300: 4-6 %

@@ -12,7 +12,8 @@
 // and the top (ER at i >= upperbnd), copies the theta ghosts and shifts the
 // phi halo.  Every kernel keeps the reference's operation order (the library
 // is built with --fmad=false), so the iterates equal the reference loop's
-// except where pow() enters (the IBDRAD = 9 top and the final T).
+// except where pow() enters (the IBDRAD = 9 top and the final T), and beside a
+// column whose UPPERBND is 1, for whose faces the reference forms no limiter.
 #include <math.h>
 
 #include "ttfld_sweep64.cuh"

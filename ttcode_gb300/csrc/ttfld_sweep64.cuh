@@ -16,7 +16,8 @@
 // ms for the exact SOR at 64x128x64 against adding it up before.  The cells'
 // updates and their operands are those of one launch per colour, so the
 // iterate is the same bit for bit; only the order in which the norm is
-// summed differs.
+// summed differs.  Where boundary values are written behind a colour, that
+// takes a wait of its own (boundary_step).
 //
 // What does not change during a solve (the coefficients and b) each thread
 // copies for its next item into its own slots of shared memory (cp.async)
