@@ -76,10 +76,6 @@ struct KryWork {
   float* tiles;  // line tiles in global memory (lines too long for shared memory)
 };
 
-__host__ __device__ __forceinline__ size_t lq(const Kry& k, int i, int j, int kk) {
-  return (size_t)(i - 1) * k.ncol + (size_t)(kk - 1) * k.ny + (size_t)(j - 1);
-}
-
 // The rows of the system being solved: SOR_A..G, with the hypre changes.
 struct Row {
   double a, b, c, d, e, f, g;
@@ -137,49 +133,62 @@ __global__ void __launch_bounds__(kThreads) kry_weights_kernel(Dev d, Kry kr, in
 
 // The kernels between the cell order (radius fastest) and the line-major
 // order (phi fastest) work in strips of kStripCols neighbouring columns of
-// one theta row: NX * kStripCols consecutive cells, walked in cell order, with
-// the line-major side going through shared memory, so that both sides are
-// coalesced.  (A warp that writes its 32 radii straight to the line-major
-// arrays writes 32 sectors of 32 bytes for 4 bytes each: 140 us an anchor at
-// 100x256x128.)
+// one theta row, walked in cell order, with the line-major side going through
+// shared memory, so that both sides are coalesced.  (A warp that writes its 32
+// radii straight to the line-major arrays writes 32 sectors of 32 bytes for 4
+// bytes each: 140 us an anchor at 100x256x128.)  Strips are cut along the
+// radius into pieces of the same length (StripCut), so that few of them still
+// fill the SMs and a piece fits in shared memory.
 constexpr int kStripCols = 32;
+struct StripCut {
+  unsigned int pieces;  // strips times pieces of a strip
+  unsigned int per;     // pieces of a strip
+  FastDiv by_len;       // radii of a piece (the last may have fewer)
+};
 struct Strip {
   int j0, k, cols;        // columns j0 .. j0 + cols - 1 (from 1) of theta row k
+  int i0, ni;             // radii i0 + 1 .. i0 + ni
   unsigned int t0;        // first cell
 };
-__device__ __forceinline__ Strip strip_of(const Dev& d, unsigned int m) {
-  const unsigned int per = ((unsigned int)d.ny + kStripCols - 1) / kStripCols;
+__device__ __forceinline__ Strip strip_of(const Dev& d, const StripCut& cut, unsigned int m) {
+  const unsigned int across = ((unsigned int)d.ny + kStripCols - 1) / kStripCols, strip = m / cut.per;
   Strip p;
-  p.k = (int)(m / per) + 1;
-  p.j0 = (int)(m % per) * kStripCols + 1;
+  p.k = (int)(strip / across) + 1;
+  p.j0 = (int)(strip % across) * kStripCols + 1;
   p.cols = d.ny - p.j0 + 1 < kStripCols ? d.ny - p.j0 + 1 : kStripCols;
-  p.t0 = (unsigned int)cidx(d, 1, p.j0, p.k);
+  p.i0 = (int)((m % cut.per) * cut.by_len.d);
+  p.ni = d.nx - p.i0 < (int)cut.by_len.d ? d.nx - p.i0 : (int)cut.by_len.d;
+  p.t0 = (unsigned int)cidx(d, p.i0 + 1, p.j0, p.k);
   return p;
 }
 constexpr int kStripPitch = kStripCols + 1;
-// Write the staged values of a strip, stage[(i - 1) * kStripPitch + column], to
-// a line-major array.
+// Line-major index of a piece's radius i (from 0) in its column `lane`.
+__device__ __forceinline__ size_t strip_line(const Kry& kr, const Strip& p, int i, int lane) {
+  return (size_t)(p.i0 + i) * kr.ncol + (size_t)(p.k - 1) * kr.ny + (size_t)(p.j0 - 1 + lane);
+}
+// Write the staged values of a piece, stage[i * kStripPitch + column], to a
+// line-major array.
 __device__ __forceinline__ void strip_out(const Kry& kr, const Strip& p, const float* stage, float* to) {
   const int lane = threadIdx.x & 31;
   if (lane < p.cols)
-    for (int i = threadIdx.x >> 5; i < kr.nx; i += blockDim.x >> 5)
-      to[(size_t)i * kr.ncol + (size_t)(p.k - 1) * kr.ny + (size_t)(p.j0 - 1 + lane)] = stage[i * kStripPitch + lane];
+    for (int i = threadIdx.x >> 5; i < p.ni; i += blockDim.x >> 5)
+      to[strip_line(kr, p, i, lane)] = stage[i * kStripPitch + lane];
 }
 
 // Couplings of S (the symmetric part of Sigma W A Sigma) to the +i, +j, +k
-// neighbours, written line-major; stage holds three strips.
-__global__ void __launch_bounds__(kThreads) kry_couplings_kernel(Dev d, Kry kr, int hypre, unsigned int strips,
-                                                                 int staged) {
+// neighbours, written line-major; stage holds three pieces.
+__global__ void __launch_bounds__(kThreads) kry_couplings_kernel(Dev d, Kry kr, int hypre, StripCut cut) {
   extern __shared__ float stage[];
   const int nx = d.nx, ny = d.ny, nz = d.nz;
   const bool h = hypre != 0;
-  const int one = nx * kStripPitch;
-  for (unsigned int m = blockIdx.x; m < strips; m += gridDim.x) {
-    const Strip p = strip_of(d, m);
-    for (unsigned int u = threadIdx.x; u < (unsigned int)(nx * p.cols); u += blockDim.x) {
+  const int one = (int)cut.by_len.d * kStripPitch;
+  for (unsigned int m = blockIdx.x; m < cut.pieces; m += gridDim.x) {
+    const Strip p = strip_of(d, cut, m);
+    for (unsigned int u = threadIdx.x; u < cut.by_len.d * p.cols; u += blockDim.x) {
       unsigned int iu;
-      const int col = (int)div_rem(d.by_nx, u, iu), i = (int)iu + 1, j = p.j0 + col, k = p.k;
-      const size_t t = p.t0 + u;
+      const int col = (int)div_rem(cut.by_len, u, iu), i = p.i0 + (int)iu + 1, j = p.j0 + col, k = p.k;
+      if ((int)iu >= p.ni) continue;
+      const size_t t = p.t0 + (unsigned int)(nx * col) + iu;
       const Row r = row_of(d, t, i, j, k, h);
       const double wn = kr.wgt[t], sn = kr.sig[t];
       float cr = 0.f, cp = 0.f, ct = 0.f;
@@ -199,19 +208,11 @@ __global__ void __launch_bounds__(kThreads) kry_couplings_kernel(Dev d, Kry kr, 
         const Row rm = row_of(d, q, i, j, k + 1, h);
         ct = f32_rn(mul_rn(mul_rn(0.5 * (mul_rn(wn, r.g) + mul_rn(kr.wgt[q], rm.f)), sn), kr.sig[q]));
       }
-      if (staged) {
-        const int o = (int)iu * kStripPitch + col;
-        stage[o] = cr;
-        stage[one + o] = cp;
-        stage[2 * one + o] = ct;
-      } else {
-        const size_t q = lq(kr, i, j, k);
-        kr.cr[q] = cr;
-        kr.cp[q] = cp;
-        kr.ct[q] = ct;
-      }
+      const int o = (int)iu * kStripPitch + col;
+      stage[o] = cr;
+      stage[one + o] = cp;
+      stage[2 * one + o] = ct;
     }
-    if (!staged) continue;
     __syncthreads();
     strip_out(kr, p, stage, kr.cr);
     strip_out(kr, p, stage + one, kr.cp);
@@ -254,20 +255,20 @@ __global__ void __launch_bounds__(32) kry_factor_kernel(Kry kr, SolverDev* sol) 
 template <bool L2, bool WITH_B>
 __global__ void __launch_bounds__(kThreads) kry_anchor_kernel(Dev d, Kry kr, const double* __restrict__ x,
                                                               const double* __restrict__ b, int hypre,
-                                                              double* partials, int nbmax, unsigned int strips,
-                                                              int staged) {
+                                                              double* partials, int nbmax, StripCut cut) {
   extern __shared__ float stage[];
   __shared__ double sh[32];
   __shared__ bool last;
   const int nx = d.nx, ny = d.ny;
   const size_t sj = (size_t)(nx + 4), sk = (size_t)(nx + 4) * (ny + 4);
   double s[4] = {0.0, 0.0, 0.0, 0.0};
-  for (unsigned int m = blockIdx.x; m < strips; m += gridDim.x) {
-    const Strip p = strip_of(d, m);
-    for (unsigned int u = threadIdx.x; u < (unsigned int)(nx * p.cols); u += blockDim.x) {
+  for (unsigned int m = blockIdx.x; m < cut.pieces; m += gridDim.x) {
+    const Strip p = strip_of(d, cut, m);
+    for (unsigned int u = threadIdx.x; u < cut.by_len.d * p.cols; u += blockDim.x) {
       unsigned int iu;
-      const int col = (int)div_rem(d.by_nx, u, iu), i = (int)iu + 1, j = p.j0 + col, k = p.k;
-      const size_t t = p.t0 + u;
+      const int col = (int)div_rem(cut.by_len, u, iu), i = p.i0 + (int)iu + 1, j = p.j0 + col, k = p.k;
+      if ((int)iu >= p.ni) continue;
+      const size_t t = p.t0 + (unsigned int)(nx * col) + iu;
       const Row r = row_of(d, t, i, j, k, hypre != 0);
       const size_t q = hidx(d, i, j, k);
       const size_t qjm = (j == 1) ? hidx(d, i, ny, k) : q - sj;
@@ -291,20 +292,13 @@ __global__ void __launch_bounds__(kThreads) kry_anchor_kernel(Dev d, Kry kr, con
         s[2] += fabs(hypre ? bb : b[t]);  // RHSNORM over every row (ppsor.f:33)
         s[3] = fma(bs, bs, s[3]);
       }
-      if (staged) {
-        stage[(int)iu * kStripPitch + col] = f32_rn(rs);
-      } else {
-        const size_t l = lq(kr, i, j, k);
-        kr.r[l] = f32_rn(rs);
-        kr.e[l] = 0.f;
-      }
+      stage[(int)iu * kStripPitch + col] = f32_rn(rs);
     }
-    if (!staged) continue;
     __syncthreads();
     strip_out(kr, p, stage, kr.r);
     if ((threadIdx.x & 31) < p.cols)
-      for (int i = threadIdx.x >> 5; i < nx; i += blockDim.x >> 5)
-        kr.e[(size_t)i * kr.ncol + (size_t)(p.k - 1) * ny + (size_t)(p.j0 - 1 + (threadIdx.x & 31))] = 0.f;
+      for (int i = threadIdx.x >> 5; i < p.ni; i += blockDim.x >> 5)
+        kr.e[strip_line(kr, p, i, threadIdx.x & 31)] = 0.f;
     __syncthreads();
   }
   for (int m = 0; m < 4; ++m) {
@@ -333,24 +327,23 @@ __global__ void __launch_bounds__(kThreads) kry_anchor_kernel(Dev d, Kry kr, con
 }
 
 // x += Sigma e (x a halo array, e line-major).
-__global__ void __launch_bounds__(kThreads) kry_update_kernel(Dev d, Kry kr, double* x, unsigned int strips, int staged) {
+__global__ void __launch_bounds__(kThreads) kry_update_kernel(Dev d, Kry kr, double* x, StripCut cut) {
   extern __shared__ float stage[];
   const int nx = d.nx, lane = threadIdx.x & 31;
-  for (unsigned int m = blockIdx.x; m < strips; m += gridDim.x) {
-    const Strip p = strip_of(d, m);
-    if (staged) {
-      __syncthreads();
-      if (lane < p.cols)
-        for (int i = threadIdx.x >> 5; i < nx; i += blockDim.x >> 5)
-          stage[i * kStripPitch + lane] =
-              kr.e[(size_t)i * kr.ncol + (size_t)(p.k - 1) * kr.ny + (size_t)(p.j0 - 1 + lane)];
-      __syncthreads();
-    }
-    for (unsigned int u = threadIdx.x; u < (unsigned int)(nx * p.cols); u += blockDim.x) {
+  for (unsigned int m = blockIdx.x; m < cut.pieces; m += gridDim.x) {
+    const Strip p = strip_of(d, cut, m);
+    __syncthreads();
+    if (lane < p.cols)
+      for (int i = threadIdx.x >> 5; i < p.ni; i += blockDim.x >> 5)
+        stage[i * kStripPitch + lane] = kr.e[strip_line(kr, p, i, lane)];
+    __syncthreads();
+    for (unsigned int u = threadIdx.x; u < cut.by_len.d * p.cols; u += blockDim.x) {
       unsigned int iu;
-      const int col = (int)div_rem(d.by_nx, u, iu), i = (int)iu + 1, j = p.j0 + col;
-      const float e = staged ? stage[(int)iu * kStripPitch + col] : kr.e[lq(kr, i, j, p.k)];
-      x[hidx(d, i, j, p.k)] += mul_rn(kr.sig[p.t0 + u], f64_of_f32(e));
+      const int col = (int)div_rem(cut.by_len, u, iu);
+      if ((int)iu >= p.ni) continue;
+      const float e = stage[(int)iu * kStripPitch + col];
+      x[hidx(d, p.i0 + (int)iu + 1, p.j0 + col, p.k)] +=
+          mul_rn(kr.sig[p.t0 + (unsigned int)(nx * col) + iu], f64_of_f32(e));
     }
   }
 }
@@ -957,21 +950,35 @@ int launch_inner(ttfld_ctx* c, KryWork* w, int maxit, double stop_ratio, int gs,
   return 0;
 }
 
-// The strips of a grid, the blocks that walk them, and the shared memory of
-// `arrays` staged strips (0 and not staged where NX is too long for 200 KB).
+// The pieces of a grid's strips, the blocks that walk them, and the shared
+// memory of `arrays` staged pieces.  Strips are cut until there are two pieces
+// per SM, but to no less than 16 radii (two lines of an FP64 array), and in any
+// case to what 200 KB hold.  Uncut, 96 strips leave a third of the SMs without a
+// block and the others with one: at 180x64x48 the couplings took 101 us, an
+// anchor 57 and an update 39, cut 31, 34 and 14 (a PCG solve 1117 -> 976 us; 883
+// -> 839 at 100x64x70, 960 -> 883 at 98x70x52).  Seven pieces per SM instead of
+// two: 1014 us at 180x64x48, and 2-3 % slower than uncut at 64x96x100 and
+// 30x200x100, where the pieces were then 16 radii.
+constexpr int kStripPieces = 304, kStripBlocks = 1024;
 struct StripShape {
-  unsigned int strips;
-  int blocks, staged;
+  StripCut cut;
+  int blocks;
   size_t smem;
 };
 StripShape strip_shape(const Kry& k, const void* kernel, int arrays) {
   StripShape s;
-  s.strips = (unsigned int)k.nz * (((unsigned int)k.ny + kStripCols - 1) / kStripCols);
-  s.blocks = s.strips < 1024 ? (int)s.strips : 1024;
-  s.smem = (size_t)arrays * k.nx * kStripPitch * sizeof(float);
-  s.staged = s.smem <= 200 * 1024;
-  if (s.staged && s.smem > 48 * 1024 && smem_room(kernel) < s.smem) s.staged = 0;
-  if (!s.staged) s.smem = 0;
+  const unsigned int strips = (unsigned int)k.nz * (((unsigned int)k.ny + kStripCols - 1) / kStripCols);
+  const unsigned int nx = (unsigned int)k.nx, want = (kStripPieces + strips - 1) / strips;
+  const size_t radius = (size_t)arrays * kStripPitch * sizeof(float);
+  unsigned int len = (nx + want - 1) / want;
+  if (len < 16) len = nx < 16 ? nx : 16;
+  if (len * radius > 200 * 1024) len = (unsigned int)(200 * 1024 / radius);
+  if (len * radius > 48 * 1024 && smem_room(kernel) < len * radius) len = (unsigned int)(48 * 1024 / radius);
+  s.cut.per = (nx + len - 1) / len;
+  s.cut.pieces = strips * s.cut.per;
+  s.cut.by_len = fast_div((int)len);
+  s.blocks = s.cut.pieces < kStripBlocks ? (int)s.cut.pieces : kStripBlocks;
+  s.smem = len * radius;
   return s;
 }
 
@@ -979,7 +986,7 @@ template <bool L2, bool WITH_B>
 int launch_anchor(ttfld_ctx* c, KryWork* w, const double* x, const double* b, int h) {
   const StripShape s = strip_shape(w->k, (const void*)kry_anchor_kernel<L2, WITH_B>, 1);
   kry_anchor_kernel<L2, WITH_B><<<s.blocks, kThreads, s.smem, c->stream>>>(c->d, w->k, x, b, h, c->partials, 1024,
-                                                                           s.strips, s.staged);
+                                                                           s.cut);
   count_launches(1);
   TT_CHECK_LAUNCH();
   return 0;
@@ -998,7 +1005,7 @@ int prepare(ttfld_ctx* c, KryWork* w, bool hypre) {
   TT_CHECK(cudaMemsetAsync(&c->sol->bad_weights, 0, sizeof(int), c->stream));
   kry_weights_kernel<<<nb, kThreads, 0, c->stream>>>(c->d, w->k, hypre ? 1 : 0);
   const StripShape s = strip_shape(w->k, (const void*)kry_couplings_kernel, 3);
-  kry_couplings_kernel<<<s.blocks, kThreads, s.smem, c->stream>>>(c->d, w->k, hypre ? 1 : 0, s.strips, s.staged);
+  kry_couplings_kernel<<<s.blocks, kThreads, s.smem, c->stream>>>(c->d, w->k, hypre ? 1 : 0, s.cut);
   kry_factor_kernel<<<(unsigned int)((w->k.ncol + 31) / 32), 32, 0, c->stream>>>(w->k, c->sol);
   count_launches(3);
   TT_CHECK_LAUNCH();
@@ -1072,7 +1079,7 @@ int pcg_core(ttfld_ctx* c, double* x, const double* b, bool hypre, double tol, l
     ++anchors;
     if (c->host_sol->stalled) ++stalls;
     const StripShape up = strip_shape(w->k, (const void*)kry_update_kernel, 1);
-    kry_update_kernel<<<up.blocks, kThreads, up.smem, c->stream>>>(c->d, w->k, x, up.strips, up.staged);
+    kry_update_kernel<<<up.blocks, kThreads, up.smem, c->stream>>>(c->d, w->k, x, up.cut);
     count_launches(1);
     TT_CHECK_LAUNCH();
     if ((rc = anchor(c, w, x, b, hypre, l2, false))) return rc;
